@@ -144,10 +144,12 @@ struct gtk_tokenizer {
 
   // table in HBM
   DevBuf d_bpi;
-  DevBuf d_slots, d_overflow, d_bpr, d_mor, d_sor, d_adj, d_b2i, d_words, d_low_map, d_wide_slots;
+  DevBuf d_slots, d_overflow, d_bpr, d_mor, d_sor, d_adj, d_b2i, d_short_words, d_long_words, d_learned_words, d_low_map, d_wide_slots;
   DevBuf d_staging32, d_seg_scratch32;  // 32-bit kernel
   int id_space = GTK_IDS_REFERENCE;
   gtk::DeviceTable dtab{};
+  bool reset_learned = false;
+  gtk::DeviceTable call_tab{};  // what the kernels of the present call get: dtab, or with a long table of the call's own
 
   // arenas
   DevBuf d_bytes, d_text_off, d_text_chunk_base, d_chunk_off, d_tile_chunk0, d_staging, d_unit_first, d_unit_cnt,
@@ -213,10 +215,14 @@ void upload_table(gtk_tokenizer* h)
   upload(h->d_bpi, t.byte_pair_info.data(), t.byte_pair_info.size() * sizeof(uint16_t), h->stream);
   upload(h->d_mor, t.merged_of_rank.data(), t.merged_of_rank.size() * sizeof(uint32_t), h->stream);
   upload(h->d_sor, t.same_of_rank.data(), t.same_of_rank.size(), h->stream);
-  upload(h->d_adj, t.adj, sizeof(t.adj), h->stream);
+  uint32_t adj[2048];  // the device's layout: [v / 32][u]
+  for (int u = 0; u < 256; ++u)
+    for (int v = 0; v < 8; ++v) adj[v * 256 + u] = t.adj[u * 8 + v];
+  upload(h->d_adj, adj, sizeof(adj), h->stream);
   upload(h->d_b2i, t.byte_to_id, sizeof(t.byte_to_id), h->stream);
   upload(h->d_low_map, t.gpt2_low_id, sizeof(t.gpt2_low_id), h->stream);
-  upload(h->d_words, t.word_slots.data(), t.word_slots.size() * sizeof(gtk::WordSlot), h->stream);
+  upload(h->d_short_words, t.short_words.data(), t.short_words.size() * sizeof(gtk::ShortWord), h->stream);
+  upload(h->d_long_words, t.long_words.data(), t.long_words.size() * sizeof(gtk::LongWord), h->stream);
   if (h->wide) upload(h->d_wide_slots, t.slots.data(), t.slots.size() * sizeof(gtk::HashSlot), h->stream);
   GTK_CUDA(cudaStreamSynchronize(h->stream));
   h->dtab.pair_buckets = h->d_slots.as<uint4>();
@@ -228,14 +234,33 @@ void upload_table(gtk_tokenizer* h)
   h->dtab.same_of_rank = h->d_sor.as<uint8_t>();
   h->dtab.adj = h->d_adj.as<uint32_t>();
   h->dtab.byte_to_id = h->d_b2i.as<uint16_t>();
-  h->dtab.word_slots = h->d_words.as<uint4>();
-  h->dtab.word_log2_capacity = t.word_log2_capacity;
+  h->dtab.short_words = h->d_short_words.as<uint2>();
+  h->dtab.long_words = h->d_long_words.as<uint4>();
+  h->dtab.learn = 0;
   h->dtab.wide_slots = h->wide ? h->d_wide_slots.as<uint4>() : nullptr;
   h->dtab.wide_log2 = t.log2_capacity;
   h->dtab.wide_max_probe = t.max_probe;
   h->dtab.monotone = t.monotone ? 1 : 0;
   h->dtab.merged_is_256_plus_rank = t.merged_is_256_plus_rank ? 1 : 0;
   h->dtab.byte_ids_identity = t.byte_ids_identity ? 1 : 0;
+}
+
+// From this size on the tile kernel works on a copy of the long-string table and adds the segments it merges, so that a
+// word that is not in the vocabulary is merged once in a batch and looked up from then on.  Every call starts from the
+// vocabulary's own strings.  Where the line lies: the copy (8 MiB within L2, 3 us) and the first tiles, all of which miss
+// and add at once, have to be earned back.  English-like text of 4 / 8 / 16 / 64 MiB: 115 / 144 / 193 / 452 us with,
+// 101 / 141 / 204 / 588 us without; the sample novel 104 / 139 / 168 / 386 against 109 / 151 / 203 / 561 us.
+constexpr int64_t kLearnMinBytes = int64_t(12) << 20;
+
+void begin_call(gtk_tokenizer* h, int mode, int64_t n_bytes)
+{
+  h->call_tab     = h->dtab;
+  h->reset_learned = false;
+  if (h->wide || mode != GTK_MODE_OPT || n_bytes < kLearnMinBytes) return;
+  h->d_learned_words.reserve(h->table->long_words.size() * sizeof(gtk::LongWord));
+  h->call_tab.long_words = h->d_learned_words.as<uint4>();
+  h->call_tab.learn      = 1;
+  h->reset_learned       = true;  // by the first launch of the call (run_front)
 }
 
 // Upper bound on the number of chunks without touching the device: every text
@@ -350,9 +375,10 @@ void run_front(gtk_tokenizer* h, const gtk::EncodeBuffers& b, int mode, int* lau
   cudaStream_t s = h->stream;
   const bool stages = ev != nullptr || h->stage_timing;  // sliced batches always time their stages
   if (!ev) ev = h->ev;
-  if (!gtk::chunker_resets_counters(b)) {
-    GTK_CUDA(cudaMemsetAsync(b.counters, 0, 64, s));
-    GTK_CUDA(cudaMemsetAsync(b.chunk_cnt, 0, size_t(b.chunk_cap + 1) * 4, s));
+  const bool own_reset = gtk::chunker_resets_counters(b);
+  if (!own_reset || h->reset_learned) {
+    *launches += gtk::launch_begin_batch(b, !own_reset, h->dtab.long_words, h->reset_learned ? h->call_tab.long_words : nullptr, s);
+    h->reset_learned = false;
   }
   GTK_CUDA(cudaEventRecord(ev[0], s));
   *launches += gtk::launch_chunker(b, s);
@@ -360,7 +386,7 @@ void run_front(gtk_tokenizer* h, const gtk::EncodeBuffers& b, int mode, int* lau
   if (h->wide) *launches += gtk::launch_merge_wide(b, h->dtab, h->wide_grid, s);
   else if (mode == GTK_MODE_BASE) *launches += gtk::launch_merge_base(b, h->dtab, h->base_grid, h->base_block, s);
   else if (mode == GTK_MODE_LOCALMIN) *launches += gtk::launch_merge_localmin(b, h->dtab, h->localmin_grid, h->max_iters, s);
-  else *launches += gtk::launch_merge_opt(b, h->dtab, h->opt_grid, s);
+  else *launches += gtk::launch_merge_opt(b, h->call_tab, h->opt_grid, s);
   if (stages) GTK_CUDA(cudaEventRecord(ev[2], s));
   *launches += gtk::launch_output_scans(b, mode != GTK_MODE_OPT || h->wide, s);
   if (stages || !chained) GTK_CUDA(cudaEventRecord(ev[3], s));
@@ -626,6 +652,7 @@ int encode_host_sliced(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
   if (!h->out_stream) GTK_CUDA(cudaStreamCreateWithFlags(&h->out_stream, cudaStreamNonBlocking));
   if (!h->pack_stream) GTK_CUDA(cudaStreamCreateWithFlags(&h->pack_stream, cudaStreamNonBlocking));
   for (auto& a : h->slice) slice_arena_prepare(h, a, max_bytes, max_pieces);
+  begin_call(h, mode, n_bytes);
   GTK_CUDA(cudaStreamSynchronize(h->stream));
 
   for (int i = 0; i < ns; ++i) {
@@ -925,7 +952,7 @@ void release_handle(gtk_tokenizer* h)
   if (h->device >= 0) {
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
-    for (DevBuf* b : {&h->d_bpi, &h->d_slots, &h->d_overflow, &h->d_bpr, &h->d_mor, &h->d_sor, &h->d_adj, &h->d_b2i, &h->d_words, &h->d_low_map, &h->d_wide_slots, &h->d_staging32, &h->d_seg_scratch32, &h->d_bytes, &h->d_text_off,
+    for (DevBuf* b : {&h->d_bpi, &h->d_slots, &h->d_overflow, &h->d_bpr, &h->d_mor, &h->d_sor, &h->d_adj, &h->d_b2i, &h->d_short_words, &h->d_long_words, &h->d_learned_words, &h->d_low_map, &h->d_wide_slots, &h->d_staging32, &h->d_seg_scratch32, &h->d_bytes, &h->d_text_off,
                       &h->d_text_chunk_base, &h->d_chunk_off, &h->d_tile_chunk0, &h->d_staging, &h->d_unit_first,
                       &h->d_unit_cnt, &h->d_chunk_cnt, &h->d_unit_base, &h->d_chunk_id_off, &h->d_text_id_off,
                       &h->d_out_ids, &h->d_seg_scratch, &h->d_scan_sums, &h->d_totals, &h->d_out_pack, &h->d_fast_in})
@@ -1107,6 +1134,7 @@ GTK_API int gtk_encode_device(gtk_tokenizer* h, int mode, const uint8_t* d_bytes
     int64_t* chunk_dst = d_out_chunk_offsets;
     if (chunk_dst && chunk_capacity < need_chunks + 1) chunk_dst = nullptr;  // scan into the arena, copy what fits
     Plan p = plan_batch(h, d_bytes, n_bytes, d_text_offsets, n_texts, d_out_ids, out_capacity, chunk_dst, false);
+    begin_call(h, mode, n_bytes);
     int launches = 0;
     // When the chunk offsets are scanned straight into the caller's buffer (or not wanted), the pack follows
     // the front without a host round trip: the pack kernel itself never writes past out_capacity, and the
@@ -1197,6 +1225,7 @@ GTK_API int gtk_encode(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
                         reinterpret_cast<int32_t*>(dp + text_b + chunk_b), n_bytes,
                         reinterpret_cast<int64_t*>(dp + text_b), true);
     p.b.text_id_off = reinterpret_cast<int64_t*>(dp);
+    begin_call(h, mode, n_bytes);
     int launches = 0;
     // Up to 256 KiB of text a kernel behind the pack writes the results into mapped host memory and the host polls
     // its completion mark: no copy of the totals, no second copy sized by them, no stream synchronisation.

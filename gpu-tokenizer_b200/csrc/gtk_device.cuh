@@ -13,20 +13,16 @@ namespace gtk {
 // Tile geometry of the segment-parallel kernel: a CTA owns the segments that
 // start inside TILE consecutive bytes and sees HALO more bytes so that the
 // last owned segment can finish inside shared memory.
-#ifndef GTK_TILE
-#define GTK_TILE 4096
-#endif
 #ifndef GTK_OPT_THREADS
 #define GTK_OPT_THREADS 256
 #endif
-constexpr int kTile = GTK_TILE;
+constexpr int kOptThreads = GTK_OPT_THREADS;
+constexpr int kTile = kOptThreads * 16;  // sixteen positions per thread
 constexpr int kHalo = 256;
 constexpr int kWindow = kTile + kHalo;
-constexpr int kOptThreads = GTK_OPT_THREADS;
 constexpr int kBaseThreads = 512;
 constexpr int kBaseSmemTokens = 8192;  // chunks up to this length stay in shared memory in the local-minimum and allocation-free kernels
-constexpr int kBaseSmemMaxTokens = 49152;  // one-CTA-per-chunk kernel: longest chunk held in (dynamic) shared memory, 4 bytes per slot
-constexpr int kThreadSegMax = 32;      // longest segment a single thread merges on its own
+constexpr int kThreadSegMax = 16;      // longest segment a single thread merges on its own
 
 // Pointers into HBM, passed by value to every kernel.
 struct DeviceTable {
@@ -37,10 +33,11 @@ struct DeviceTable {
   const uint16_t* byte_pair_info;  // [65536]: 0xFFFF cut, 0xFFFE mergeable boundary without a byte-pair rank, else rank
   const uint32_t* merged_of_rank;  // [max_rank+1]
   const uint8_t* same_of_rank;     // [max_rank+1]
-  const uint32_t* adj;             // [2048]
+  const uint32_t* adj;             // [2048]: word [v / 32][u], bit v % 32: bytes u, v stand next to each other inside a merge result
   const uint16_t* byte_to_id;      // [256]
-  const uint4* word_slots;         // WordSlot[word capacity]: {k0, k1, k2, length << 16 | id}, two-choice cuckoo
-  uint32_t word_log2_capacity;
+  const uint2* short_words;        // ShortWord[1 << kShortBits]
+  uint4* long_words;               // LongWord[1 << kLongBits], two uint4 each
+  int learn;                       // 1: long_words is this call's own copy, merged segments may be added to it
   const uint4* wide_slots;         // tables beyond 16 bits: HashSlot[1 << wide_log2] {right, left, rank, merged id}
   uint32_t wide_log2;
   uint32_t wide_max_probe;         // longest displacement of a stored key
@@ -96,6 +93,8 @@ struct EncodeBuffers {
 };
 
 // Launchers (all asynchronous on `stream`; return the number of kernels launched).
+// resets the call's counters and per-chunk counts and, when learned is given, the learned long table to the vocabulary's
+int launch_begin_batch(const EncodeBuffers& b, bool counters, const uint4* long_words, uint4* learned, cudaStream_t stream);
 int launch_chunker(const EncodeBuffers& b, cudaStream_t stream);
 bool chunker_resets_counters(const EncodeBuffers& b);
 int launch_merge_opt(const EncodeBuffers& b, const DeviceTable& t, int grid, cudaStream_t stream);
@@ -142,6 +141,6 @@ bool handle_view(gtk_tokenizer* h, HandleView* out);
 int opt_kernel_max_blocks_per_sm();
 int base_kernel_max_blocks_per_sm(int chunk_bytes, int block_threads);
 int localmin_kernel_max_blocks_per_sm();
-void base_kernel_geometry(int chunk_bytes, int block_threads, int* warps, int* smem_tokens);
+int chunk_kernel_threads(int chunk_bytes, int block_threads);
 
 }  // namespace gtk

@@ -30,9 +30,11 @@
 // Kernels report trouble through a status word and never trap; every loop is
 // bounded.  -DGTK_CHECKED adds range checks on every data-dependent index.
 #include "gtk_device.cuh"
+#include "gtk_table.hpp"
 
 #include <algorithm>
 #include <cstddef>
+#include <type_traits>
 
 namespace gtk {
 namespace {
@@ -152,47 +154,15 @@ __device__ __forceinline__ uint32_t probe_rank_t(const DeviceTable& T, uint32_t 
   return probe_rank_wide(T, left, right);
 }
 
-// Whole-segment table: id of the vocabulary string (k0,k1,k2 = bytes zero padded, L = length)
-// if the greedy rule turns exactly that string into one token, else 0xFFFFFFFF.  Two-choice cuckoo
-// table: both candidate slots are loaded at once.
-__device__ __forceinline__ uint32_t word_lookup(const uint4* word_slots, uint32_t sh, uint32_t k0, uint32_t k1,
-                                                uint32_t k2, uint32_t L)
-{
-  uint32_t m = (k0 * 0x9E3779B1u) ^ (k1 * 0x85EBCA77u) ^ (k2 * 0xC2B2AE3Du);
-  m ^= m >> 15;
-  m *= 0x2C1B3C6Du;
-  const uint4 a = __ldg(word_slots + (m >> sh));
-  const uint4 c = __ldg(word_slots + (((m ^ (m >> 13)) * 0x165667B1u) >> sh));
-  const uint32_t meta = (L << 16);
-  if (a.x == k0 && a.y == k1 && a.z == k2 && (a.w & 0xFFFF0000u) == meta) return a.w & 0xFFFFu;
-  if (c.x == k0 && c.y == k1 && c.z == k2 && (c.w & 0xFFFF0000u) == meta) return c.w & 0xFFFFu;
-  return 0xFFFFFFFFu;
-}
-
-// segment bytes at shared-memory offset `at` (any alignment), zero padded to three words
-__device__ __forceinline__ void segment_key(const uint8_t* bytes, int at, int LL, uint32_t& k0, uint32_t& k1,
-                                            uint32_t& k2)
-{
-  const uint32_t* wp = reinterpret_cast<const uint32_t*>(bytes + (at & ~3));
-  const uint32_t sh  = uint32_t(at & 3) * 8u;
-  const uint32_t a0 = wp[0], a1 = wp[1], a2 = wp[2], a3 = wp[3];
-  k0 = __funnelshift_r(a0, a1, sh);
-  k1 = __funnelshift_r(a1, a2, sh);
-  k2 = __funnelshift_r(a2, a3, sh);
-  k0 &= (LL >= 4) ? 0xFFFFFFFFu : ((1u << (8 * LL)) - 1u);
-  k1 &= (LL >= 8) ? 0xFFFFFFFFu : ((LL <= 4) ? 0u : ((1u << (8 * (LL - 4))) - 1u));
-  k2 &= (LL >= 12) ? 0xFFFFFFFFu : ((LL <= 8) ? 0u : ((1u << (8 * (LL - 8))) - 1u));
-}
-
 __device__ __forceinline__ uint32_t merged_id(const DeviceTable& T, uint32_t rank)
 {
   return T.merged_is_256_plus_rank ? 256u + rank : __ldg(T.merged_of_rank + rank);
 }
 
+// may bytes u, v end up in one token (the matrix is laid out as [v / 32][u], bit v % 32)
 __device__ __forceinline__ bool adj_bit(const uint32_t* adj, uint32_t u, uint32_t v)
 {
-  const uint32_t bit = (u << 8) | v;
-  return (__ldg(adj + (bit >> 5)) >> (bit & 31u)) & 1u;
+  return (__ldg(adj + (((v >> 5) << 8) | u)) >> (v & 31u)) & 1u;
 }
 
 __device__ __forceinline__ uint32_t lanemask_lt()
@@ -200,82 +170,6 @@ __device__ __forceinline__ uint32_t lanemask_lt()
   uint32_t m;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
   return m;
-}
-
-// ------------------------------------------------------------------------------------------------
-// One short segment (<= 32 tokens) merged by a single thread.
-//
-// tok[0..L) / rk[0..L) live in shared memory; rk[i] is the rank of the pair
-// (token i, next live token), NONE for dead slots and for the last live one.
-// Dead slots become DEAD tombstones and stay where they are; the alive set is
-// a 32-bit register mask.  `best` = (rank << 16 | position) of the left-most
-// pair of lowest rank -- the pair Algorithm 1 restricted to the segment merges
-// next.  A step merges it, starts the two table probes for the pairs next to
-// the new token, scans the cached ranks of all other pairs while the probes are
-// in flight, and folds the two new ranks into the next `best`.
-// ------------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t segment_argmin(const uint16_t* rk_all, int s, int L)
-{
-  // two ranks per 32-bit load.  The words may reach one slot before the segment (when s is odd) and the
-  // segment's own last slot: both always hold NONE, so they never win.
-  uint32_t best         = 0xFFFFFFFFu;
-  const uint32_t* words = reinterpret_cast<const uint32_t*>(rk_all);
-  const int w_last      = (s + L - 2) >> 1;
-  uint32_t rel          = uint32_t(((s >> 1) << 1) - s);  // index of the low half relative to s: 0 or -1
-  for (int w = s >> 1; w <= w_last; ++w, rel += 2) {
-    const uint32_t x = words[w];
-    best = min(best, min((x << 16) | (rel & 0xFFFFu), (x & 0xFFFF0000u) | ((rel + 1u) & 0xFFFFu)));
-  }
-  return best;
-}
-
-// Returns false (and changes nothing) when no pair of the segment is mergeable any more.
-__device__ __forceinline__ bool thread_merge_step(uint16_t* tok_all, uint16_t* rk_all, int s, int L,
-                                                  uint32_t& alive, uint32_t& best, const PairTable& P)
-{
-  const uint32_t r = best >> 16;
-  if (r >= SEL) return false;
-  uint16_t* tok = tok_all + s;
-  uint16_t* rk  = rk_all + s;
-  const int j   = int(best & 0xFFFFu);
-  const int q   = j + __ffs(int(alive >> (j + 1)));  // next live slot after j (j <= 30)
-  if (!(GTK_IN(j, L - 1, 12) && GTK_IN(q - j - 1, L - j - 1, 13))) {
-    best = 0xFFFFFFFFu;
-    return false;
-  }
-  const uint32_t c = P.merged_of_rank ? __ldg(P.merged_of_rank + r) : 256u + r;
-  alive &= ~(1u << q);
-  const uint32_t right = (q >= 31) ? 0u : (alive >> (q + 1));
-  const uint32_t left  = alive & ((1u << j) - 1u);
-  const int p          = left ? 31 - __clz(int(left)) : j;  // j itself when there is no left neighbour
-  // both probes leave before anything waits for them; an absent neighbour reads as an empty slot
-  uint32_t keyR = 0xFFFFFFFFu, keyL = 0xFFFFFFFFu;
-  uint4 vR = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu), vL = vR;
-  if (right) {
-    keyR = (c << 16) | uint32_t(tok[q + __ffs(int(right))]);
-    vR   = __ldg(P.buckets + ((keyR * 0x9E3779B1u) >> 16));
-  }
-  if (left) {
-    keyL = (uint32_t(tok[p]) << 16) | c;
-    vL   = __ldg(P.buckets + ((keyL * 0x9E3779B1u) >> 16));
-  }
-  tok[j] = uint16_t(c);
-  tok[q] = uint16_t(DEAD);
-  rk[q]  = uint16_t(NONE);
-  rk[j]  = uint16_t(NONE);
-  rk[p]  = uint16_t(NONE);
-  best   = segment_argmin(rk_all, s, L);  // every pair but the two new ones
-  const uint32_t rr = resolve_rank_raw(vR, keyR, P.overflow, P.overflow_mask);
-  const uint32_t rl = resolve_rank_raw(vL, keyL, P.overflow, P.overflow_mask);
-  if (rr < SEL) {
-    rk[j] = uint16_t(rr);
-    best  = min(best, (rr << 16) | uint32_t(j));
-  }
-  if (rl < SEL) {
-    rk[p] = uint16_t(rl);
-    best  = min(best, (rl << 16) | uint32_t(p));
-  }
-  return true;
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -941,16 +835,12 @@ __global__ void k_tile_chunk0(const int64_t* __restrict__ chunk_off, const int64
 // merge kernel, segment-parallel ("opt")
 // ------------------------------------------------------------------------------------------------
 
-constexpr int kCutWords = kWindow / 32;  // 144
-constexpr int kSegCap   = kTile / 2 + 8;
-constexpr int kLongCap  = 128;
-
 // Optional per-phase cycle accounting of k_merge_opt (build with -DGTK_PHASE_TIMING): thread 0 of
 // every CTA accumulates clock64() deltas between phase boundaries; read with gtk_debug_phase_cycles.
 #ifdef GTK_PHASE_TIMING
 #define GTK_PHASE(k)                                              \
   do {                                                            \
-    if (tid == 0) {                                               \
+    if (threadIdx.x == 0) {                                       \
       const long long now__ = clock64();                          \
       atomicAdd(&g_phase_cycles[k], (unsigned long long)(now__ - phase_t0)); \
       phase_t0 = now__;                                           \
@@ -960,837 +850,121 @@ constexpr int kLongCap  = 128;
 #define GTK_PHASE(k) do { } while (0)
 #endif
 
+#include "gtk_tile.cuh"
 
-struct OptSmem {
-  // seg and bytes are adjacent on purpose: once the segments have been looked up, bytes and the unused tail of
-  // seg (entries from kOptThreads on) are the rank scratch of the merge loop (lane_scratch below)
-  alignas(16) uint16_t seg[kSegCap];  // starts of the segments that missed the lookup (length = distance to the next start)
-  alignas(16) uint8_t bytes[kWindow + 32];  // [15] = byte before the window, [16+i] = window position i
-  alignas(8) uint16_t tok[kWindow];
-  alignas(8) uint16_t rk[kWindow];  // reused as the compacted output buffer after merging
-  int hist[34];
-  uint32_t cut[kCutWords + 2];  // segment-start bits; reused as the alive bitmap
-  uint16_t woff[kCutWords + 2];
-  uint16_t longq[kLongCap];
-  GroupScratch gs;
-  int scanbuf[33];
-  int ticket;
-  int nseg, nlong, seg_next, nmiss;
-  int first_start, last_start, over_start;
-  int over_len;
-  long long over_end;
-  long long run_base;  // single-CTA kernel: ids written by the tiles so far
-  int over_chunk;
-  int end_owned;
-};
-
-// One instance per CTA; the kernels below and the out-of-line merge loop name it directly.
-__shared__ OptSmem g_tile;
-
-static_assert(kSegCap % 8 == 0 && offsetof(OptSmem, bytes) == offsetof(OptSmem, seg) + kSegCap * 2,
-              "seg and bytes must be adjacent");
-// Rank scratch of the one-segment-per-thread merge loop: 32-bit words from seg[kOptThreads] to the end of bytes.
-// Warp w owns kLaneWords words per lane at word offset w * 32 * kLaneWords, lane-interleaved (word k of lane l at
-// k * 32 + l), so the 32 lanes of a rank scan hit 32 different banks.  The last warp gets what is left.
-constexpr int kLaneWords        = 8;  // 16 ranks: segments of up to 16 tokens
-constexpr int kLaneScratchWords = ((kSegCap - kOptThreads) * 2 + kWindow + 32) / 4;
-__device__ __forceinline__ uint32_t* lane_scratch()
+// Window k of a batch walked in tiles of kTile bytes.
+__device__ __forceinline__ Span batch_span(const EncodeBuffers& b, int64_t k)
 {
-  return reinterpret_cast<uint32_t*>(g_tile.seg + kOptThreads);
+  const int64_t lo = k * kTile;
+  return Span{b.bytes, lo, 0, int(min(int64_t(kTile), b.n_bytes - lo)), int(min(int64_t(kWindow), b.n_bytes - lo)),
+              lo > 0, lo == 0};
 }
 
-// Every lane merges its own segment [s, s+L) to the end (s < 0: no segment).  Kept out of line so that
-// the loop gets registers of its own instead of sharing them with the tile code around the call.
-__device__ __noinline__ uint32_t thread_merge_segments(int s, int L, PairTable P)
+// start and end of the chunk that holds byte `at`; c0: a chunk at or before it
+__device__ __forceinline__ int64_t chunk_of(const EncodeBuffers& b, int64_t c0, int64_t C, int64_t at, int64_t* end)
 {
-  uint16_t* tok = g_tile.tok;  // named directly so that the accesses compile to shared-memory instructions
-  uint16_t* rk  = g_tile.rk;
-  uint32_t alive = 0, best = 0xFFFFFFFFu;
-  if (s >= 0 && !(GTK_IN(s + L, kWindow + 1, 10) && GTK_IN(L - 2, kThreadSegMax - 1, 11))) s = -1;
-  if (s >= 0) {
-    alive = (L >= 32) ? 0xFFFFFFFFu : ((1u << L) - 1u);
-    best  = segment_argmin(rk, s, L);
-  }
-#ifdef GTK_PHASE_TIMING
-  if (threadIdx.x == 0) {  // in-situ latency of one table load and of one rank scan
-    const long long a0 = clock64();
-    const uint4 v      = __ldg(P.buckets + (uint32_t(a0) * 2654435761u >> 16));
-    const long long a1 = clock64() + (v.x == 0x12345u);
-    atomicAdd(&g_phase_cycles[16], (unsigned long long)(a1 - a0));
-    atomicAdd(&g_phase_cycles[17], 1ull);
-    if (s >= 0) {
-      const long long b0 = clock64();
-      const uint32_t bb  = segment_argmin(rk, s, L);
-      const long long b1 = clock64() + (bb == 0x12345u);
-      atomicAdd(&g_phase_cycles[18], (unsigned long long)(b1 - b0));
-      atomicAdd(&g_phase_cycles[19], 1ull);
-      atomicAdd(&g_phase_cycles[20], (unsigned long long)L);
-    }
-  }
-  const long long t0 = clock64();
-  int steps          = 0;
-#endif
-  while (__any_sync(0xFFFFFFFFu, best < (SEL << 16))) {
-    if (best < (SEL << 16)) thread_merge_step(tok, rk, s, L, alive, best, P);
-#ifdef GTK_PHASE_TIMING
-    ++steps;
-#endif
-  }
-#ifdef GTK_PHASE_TIMING
-  if (threadIdx.x == 0) {  // warp 0: loop trips and their wall cycles
-    atomicAdd(&g_phase_cycles[14], (unsigned long long)(clock64() - t0));
-    atomicAdd(&g_phase_cycles[15], (unsigned long long)steps);
-  }
-#endif
-  return alive;
+  int64_t c = c0;
+  while (c + 1 < C && b.chunk_off[c + 1] <= at) ++c;
+  *end = b.chunk_off[c + 1];
+  return c;
 }
 
-// The same loop with the ranks of every segment copied into the lane-interleaved scratch first (WW words =
-// 2 * WW ranks per lane, uniform over the warp): the rank scan is unrolled, needs no alignment handling and is
-// free of bank conflicts; the tokens stay in place.
-template <int WW>
-__device__ __noinline__ uint32_t thread_merge_segments_lanes(int s, int L, PairTable P, int area, uint32_t alive)
-{
-  if (!GTK_IN(area + 32 * WW, kLaneScratchWords + 1, 14)) return alive;
-  if (s >= 0 && !(GTK_IN(s + L, kWindow + 1, 15) && GTK_IN(L - 2, 2 * WW - 1, 16))) {
-    s     = -1;
-    alive = 0;
-  }
-  uint32_t* scr = lane_scratch() + area + (threadIdx.x & 31);
-  uint16_t* tok = g_tile.tok + max(s, 0);
-#pragma unroll
-  for (int k = 0; k < WW; ++k) {
-    uint32_t lo = NONE, hi = NONE;
-    if (s >= 0 && 2 * k < L) lo = g_tile.rk[s + 2 * k];
-    if (s >= 0 && 2 * k + 1 < L) hi = g_tile.rk[s + 2 * k + 1];
-    scr[k * 32] = lo | (hi << 16);
-  }
-  auto scan = [&]() {
-    uint32_t b = 0xFFFFFFFFu;
-#pragma unroll
-    for (int k = 0; k < WW; ++k) {
-      const uint32_t x = scr[k * 32];
-      b = min(b, min((x << 16) | uint32_t(2 * k), (x & 0xFFFF0000u) | uint32_t(2 * k + 1)));
-    }
-    return b;
-  };
-  auto set_rank = [&](int i, uint32_t v) { reinterpret_cast<uint16_t*>(scr + (i >> 1) * 32)[i & 1] = uint16_t(v); };
-  uint32_t best = scan();
-#ifdef GTK_PHASE_TIMING
-  if (threadIdx.x == 0) {  // in-situ latency of one table load and of one rank scan
-    const long long a0 = clock64();
-    const uint4 v      = __ldg(P.buckets + (uint32_t(a0) * 2654435761u >> 16));
-    const long long a1 = clock64() + (v.x == 0x12345u);
-    atomicAdd(&g_phase_cycles[16], (unsigned long long)(a1 - a0));
-    atomicAdd(&g_phase_cycles[17], 1ull);
-    const long long b0 = clock64();
-    const uint32_t bb  = scan();
-    const long long b1 = clock64() + (bb == 0x12345u);
-    atomicAdd(&g_phase_cycles[18], (unsigned long long)(b1 - b0));
-    atomicAdd(&g_phase_cycles[19], 1ull);
-  }
-  const long long t0 = clock64();
-  int steps          = 0;
-#endif
-  while (__any_sync(0xFFFFFFFFu, best < (SEL << 16))) {
-#ifdef GTK_PHASE_TIMING
-    ++steps;
-    {  // merges done by this loop, all warps (each costs two bucket loads)
-      const uint32_t act = __ballot_sync(0xFFFFFFFFu, best < (SEL << 16));
-      if ((threadIdx.x & 31) == 0) atomicAdd(&g_phase_cycles[21], (unsigned long long)__popc(act));
-    }
-#endif
-    if (best < (SEL << 16)) {
-      const uint32_t r = best >> 16;
-      const int j      = int(best & 0xFFFFu);
-      const int q      = j + __ffs(int(alive >> (j + 1)));
-      if (!(GTK_IN(j, L - 1, 17) && GTK_IN(q - j - 1, L - j - 1, 18))) {
-        best = 0xFFFFFFFFu;
-        continue;
-      }
-      const uint32_t c = P.merged_of_rank ? __ldg(P.merged_of_rank + r) : 256u + r;
-      alive &= ~(1u << q);
-      const uint32_t right = (q >= 31) ? 0u : (alive >> (q + 1));
-      const uint32_t left  = alive & ((1u << j) - 1u);
-      const int p          = left ? 31 - __clz(int(left)) : j;
-      uint32_t keyR = 0xFFFFFFFFu, keyL = 0xFFFFFFFFu;
-      uint4 vR = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu), vL = vR;
-      if (right) {
-        keyR = (c << 16) | uint32_t(tok[q + __ffs(int(right))]);
-        vR   = __ldg(P.buckets + ((keyR * 0x9E3779B1u) >> 16));
-      }
-      if (left) {
-        keyL = (uint32_t(tok[p]) << 16) | c;
-        vL   = __ldg(P.buckets + ((keyL * 0x9E3779B1u) >> 16));
-      }
-      tok[j] = uint16_t(c);
-      tok[q] = uint16_t(DEAD);
-      set_rank(q, NONE);
-      set_rank(j, NONE);
-      set_rank(p, NONE);
-      best = scan();  // every pair but the two new ones
-      const uint32_t rr = resolve_rank_raw(vR, keyR, P.overflow, P.overflow_mask);
-      const uint32_t rl = resolve_rank_raw(vL, keyL, P.overflow, P.overflow_mask);
-      if (rr < SEL) {
-        set_rank(j, rr);
-        best = min(best, (rr << 16) | uint32_t(j));
-      }
-      if (rl < SEL) {
-        set_rank(p, rl);
-        best = min(best, (rl << 16) | uint32_t(p));
-      }
-    }
-  }
-#ifdef GTK_PHASE_TIMING
-  if (threadIdx.x == 0) {  // warp 0: loop trips and their wall cycles
-    atomicAdd(&g_phase_cycles[14], (unsigned long long)(clock64() - t0));
-    atomicAdd(&g_phase_cycles[15], (unsigned long long)steps);
-  }
-#endif
-  return alive;
-}
-
-// first segment start strictly after window position s (words past the window are all ones)
-__device__ __forceinline__ int next_cut(const uint32_t* cut, int s)
-{
-  int w      = (s + 1) >> 5;
-  if (!GTK_IN(w, kCutWords + 2, 1)) return kWindow;
-  uint32_t x = cut[w] & (0xFFFFFFFFu << ((s + 1) & 31));
-  while (!x) {
-    if (!GTK_IN(w + 1, kCutWords + 2, 2)) return kWindow;
-    x = cut[++w];
-  }
-  return w * 32 + __ffs(int(x)) - 1;
-}
-
-// One multi-byte segment that starts at window position ss: oversize and long ones are noted, a short one is
-// looked up as a whole; returns true when it has to be merged (it then joins the list of misses).
-__device__ __forceinline__ bool walk_one(int ss, const uint4* word_slots, uint32_t word_shift, int wlen, int* status)
-{
-  OptSmem& S   = g_tile;
-  const int e  = next_cut(S.cut, ss);
-  const int LL = e - ss;
-  if (e >= kWindow && wlen == kWindow) {
-    S.over_start = ss;  // runs past the window: finished in the HBM workspace
-    return false;
-  }
-  if (LL > kThreadSegMax) {
-    const int q = atomicAdd(&S.nlong, 1);
-    if (q < kLongCap && GTK_IN(ss, kWindow, 3)) S.longq[q] = uint16_t(ss);
-    else atomicMax(status, int(kStatusLongQueueOverflow));
-    return false;
-  }
-  if (LL <= 12 && GTK_IN(ss, kWindow, 4)) {
-    uint32_t k0, k1, k2;
-    segment_key(S.bytes, 16 + ss, LL, k0, k1, k2);
-    const uint32_t id = word_lookup(word_slots, word_shift, k0, k1, k2, uint32_t(LL));
-    if (id != 0xFFFFFFFFu) {
-      S.tok[ss] = uint16_t(id);
-      return false;
-    }
-  }
-  return true;
-}
-
-// Step D/E1 of a tile, out of line so that it gets registers of its own: every thread walks the multi-byte
-// segments that start in its 16 positions (window positions [16*tid, 16*tid+16), owned ones only).
-__device__ __noinline__ void walk_segments(const uint4* word_slots, uint32_t word_shift, int own, int wlen,
-                                           int* status)
-{
-  OptSmem& S     = g_tile;
-  const int tid  = threadIdx.x, lane = tid & 31;
-  const uint32_t lt = lanemask_lt();
-  const int base = tid * 16;
-  uint32_t m16   = 0;
-  if (base < own) {
-    const uint32_t w32     = __funnelshift_r(S.cut[tid >> 1], S.cut[(tid >> 1) + 1], (tid & 1) * 16);
-    const uint32_t ownmask = (base + 16 <= own) ? 0xFFFFu : ((1u << (own - base)) - 1u);
-    m16 = w32 & ~(w32 >> 1) & ownmask;  // starts whose next position is not a start
-  }
-#ifdef GTK_PHASE_TIMING
-  atomicAdd(&S.nseg, __popc(m16));
-#endif
-  while (__any_sync(0xFFFFFFFFu, m16 != 0)) {
-    bool miss = false;
-    int ss    = 0;
-    if (m16) {
-      ss = base + __ffs(int(m16)) - 1;
-      m16 &= m16 - 1;
-      miss = walk_one(ss, word_slots, word_shift, wlen, status);
-    }
-    const uint32_t bal = __ballot_sync(0xFFFFFFFFu, miss);
-    if (bal) {
-      int wbase = 0;
-      if (lane == 0) wbase = atomicAdd(&S.nmiss, __popc(bal));
-      wbase = __shfl_sync(0xFFFFFFFFu, wbase, 0);
-      if (miss && GTK_IN(wbase + __popc(bal & lt), kSegCap, 5)) S.seg[wbase + __popc(bal & lt)] = uint16_t(ss);
-    }
-  }
-}
-
-// The same step for a CTA that has its SM to itself (small batches, one tile at a time): the segments are listed
-// first (block-wide scan of the per-thread counts) and then dealt out one per thread and round.  A 512-byte text,
-// whose segments all start in the positions of the first 32 threads, is then looked up in one round of table loads
-// instead of one round per segment of the busiest thread.
-__device__ __noinline__ void walk_segments_cta(const uint4* word_slots, uint32_t word_shift, int own, int wlen,
-                                               int* status)
-{
-  OptSmem& S     = g_tile;
-  const int tid  = threadIdx.x, lane = tid & 31;
-  const uint32_t lt = lanemask_lt();
-  const int base = tid * 16;
-  uint32_t m16   = 0;
-  if (base < own) {
-    const uint32_t w32     = __funnelshift_r(S.cut[tid >> 1], S.cut[(tid >> 1) + 1], (tid & 1) * 16);
-    const uint32_t ownmask = (base + 16 <= own) ? 0xFFFFu : ((1u << (own - base)) - 1u);
-    m16 = w32 & ~(w32 >> 1) & ownmask;
-  }
-  constexpr int kListAt = kSegCap / 2, kListCap = kSegCap - kListAt;  // upper half of seg; misses fill the lower
-  int total;
-  int at = block_exclusive_scan(__popc(m16), S.scanbuf, &total);
-  if (total > kListCap) {  // CTA-uniform: too many for the list, walk per thread
-    walk_segments(word_slots, word_shift, own, wlen, status);
-    return;
-  }
-  for (uint32_t m = m16; m; m &= m - 1) S.seg[kListAt + at++] = uint16_t(base + __ffs(int(m)) - 1);
-  __syncthreads();
-  for (int g0 = 0; g0 < total; g0 += kOptThreads) {
-    const int g = g0 + tid;
-    bool miss   = false;
-    int ss      = 0;
-    if (g < total) {
-      ss   = S.seg[kListAt + g];
-      miss = walk_one(ss, word_slots, word_shift, wlen, status);
-    }
-    const uint32_t bal = __ballot_sync(0xFFFFFFFFu, miss);
-    if (bal) {
-      int wbase = 0;
-      if (lane == 0) wbase = atomicAdd(&S.nmiss, __popc(bal));
-      wbase = __shfl_sync(0xFFFFFFFFu, wbase, 0);
-      if (miss && GTK_IN(wbase + __popc(bal & lt), kListAt, 5)) S.seg[wbase + __popc(bal & lt)] = uint16_t(ss);
-    }
-  }
-}
-
-// The segment-start bitmap turns into the bitmap of live tokens as segments finish: the first token of a
-// segment is always live, so a finished segment adds the bits of its other live slots (`a`, relative to
-// its start s; bit 0 is ignored).  Only bits inside the segment change, so next_cut() of any other
-// segment still finds the same end.
-__device__ __forceinline__ void mark_alive(uint32_t* cut, int s, uint32_t a)
-{
-  a &= ~1u;
-  if (!a) return;
-  const int sh = s & 31;
-  if (!GTK_IN((s >> 5) + 1, kCutWords + 2, 6)) return;
-  atomicOr(&cut[s >> 5], a << sh);
-  if (sh && (a >> (32 - sh))) atomicOr(&cut[(s >> 5) + 1], a >> (32 - sh));
-}
-
-// one warp: positions [lo, hi) become live
-__device__ __forceinline__ void mark_alive_range(uint32_t* cut, int lo, int hi, int lane)
-{
-  if (hi <= lo || !GTK_IN(hi - 1, kWindow, 7) || !GTK_IN(lo, kWindow, 7)) return;
-  for (int w = (lo >> 5) + lane; w <= ((hi - 1) >> 5); w += 32) {
-    uint32_t x = 0xFFFFFFFFu;
-    if (w == (lo >> 5)) x &= 0xFFFFFFFFu << (lo & 31);
-    if (w == ((hi - 1) >> 5)) x &= 0xFFFFFFFFu >> (31 - ((hi - 1) & 31));
-    atomicOr(&cut[w], x);
-  }
-}
-
-// Per-CTA set-up shared by the kernels that process tiles: never-merge bitmap into shared memory and
-// the all-ones sentinel words behind the segment-start bitmap.
-__device__ __forceinline__ void opt_tile_setup(OptSmem& S, const DeviceTable& T)
-{
-  if (threadIdx.x < 2) S.cut[kCutWords + threadIdx.x] = 0xFFFFFFFFu;
-}
-
-// Reset of the per-tile words; call by one thread, then __syncthreads().
-__device__ __forceinline__ void opt_tile_reset(OptSmem& S)
-{
-  S.nlong       = 0;
-  S.nseg        = 0;
-  S.seg_next    = 0;
-  S.nmiss       = 0;
-  S.first_start = kWindow;
-  S.last_start  = -1;
-  S.over_start  = -1;
-  S.over_len    = 0;
-  S.end_owned   = 0;
-}
-
-// One tile of the byte stream: tokenises every segment that starts in bytes [k*kTile, (k+1)*kTile),
-// writes the tokens compacted to staging, the unit record and the per-chunk counts.
-// SEQ: the tiles of a batch are walked in order by one CTA (small batches); the tile then writes its ids and the
-// id offsets of its chunks straight to the output, at the running id count kept in S.run_base, instead of going
-// through staging, counts, scans and pack.
-template <bool SEQ>
-__device__ __forceinline__ void opt_tile(OptSmem& S, const EncodeBuffers& b, const DeviceTable& T, int64_t k,
+// One tile of a batch: tokenises every segment that starts in bytes [k*kTile, (k+1)*kTile), writes the tokens
+// compacted to staging, the unit record and the per-chunk counts.
+__device__ __forceinline__ void opt_tile(TileSmem<kOptThreads>& S, const EncodeBuffers& b, const DeviceTable& T, int64_t k,
                                          int64_t C)
 {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t lt = lanemask_lt();
-  const int64_t n   = b.n_bytes;
-  int* status       = b.counters + 1;
-  const bool aligned = (reinterpret_cast<uintptr_t>(b.bytes) & 15u) == 0;
-  const bool identity_ids = T.byte_ids_identity != 0;
+  int* status   = b.counters + 1;
+  const Span sp = batch_span(b, k);
 #ifdef GTK_PHASE_TIMING
   long long phase_t0 = clock64();
 #endif
-  {
-    const int64_t lo = k * kTile;
-    const int wlen   = int(min(int64_t(kWindow), n - lo));
-    const int own    = int(min(int64_t(kTile), n - lo));
-
-    // ---- A. stage the window ----
-    if (aligned) {
-      for (int v = tid; v < kWindow / 16; v += kOptThreads) {
-        const int64_t pos = lo + int64_t(v) * 16;
-        uint4 x = make_uint4(0, 0, 0, 0);
-        if (pos + 16 <= n) {
-          x = __ldg(reinterpret_cast<const uint4*>(b.bytes + pos));
-        } else if (pos < n) {
-          uint8_t tmp[16];
-          for (int j = 0; j < 16; ++j) tmp[j] = (pos + j < n) ? b.bytes[pos + j] : uint8_t(0);
-          x = *reinterpret_cast<uint4*>(tmp);
-        }
-        *reinterpret_cast<uint4*>(&S.bytes[16 + v * 16]) = x;
-      }
-    } else {
-      for (int i = tid; i < kWindow; i += kOptThreads) S.bytes[16 + i] = (lo + i < n) ? b.bytes[lo + i] : uint8_t(0);
+  const int64_t c0 = b.tile_chunk0[k];
+  tile_cut(S, sp, T, [&](auto mark) {
+    for (int64_t c = c0 + lane; c <= C; c += 32) {
+      const int64_t p = b.chunk_off[c] - sp.lo;
+      if (p >= sp.wlen) break;
+      if (p >= 0) mark(int(p));
     }
-    if (tid == 0) S.bytes[15] = (lo > 0) ? b.bytes[lo - 1] : uint8_t(0);
-    __syncthreads();
-
-    GTK_PHASE(0);
-    // Only the 32-position words that hold text are processed; the words behind them are all
-    // "segment start" (the window may be shorter than a tile at the end of the text or in small batches).
-    const int used_words  = (wlen + 31) >> 5;
-    const int used_groups = used_words * 8;
-    if (tid >= used_words && tid < kCutWords) S.cut[tid] = 0xFFFFFFFFu;
-    // ---- B. segment starts from the never-merge bitmap, initial ids and byte-pair ranks.
-    //         Four consecutive positions per thread; eight lanes assemble one 32-bit bitmap word ----
-    for (int g = tid; g < used_groups; g += kOptThreads) {
-      const int i0     = g * 4;
-      const uint32_t w = *reinterpret_cast<const uint32_t*>(&S.bytes[16 + i0]);
-      uint32_t by[6];
-      by[0] = S.bytes[15 + i0];
-      by[1] = w & 0xFFu;
-      by[2] = (w >> 8) & 0xFFu;
-      by[3] = (w >> 16) & 0xFFu;
-      by[4] = w >> 24;
-      by[5] = S.bytes[20 + i0];
-      // one 16-bit table entry per byte pair answers both questions: can this boundary ever merge
-      // (anything but 0xFFFF), and what is the rank of the byte pair (values below 0xFFFE)
-      uint32_t info[5];
-#pragma unroll
-      for (int k = 0; k < 5; ++k) info[k] = __ldg(T.byte_pair_info + ((by[k] << 8) | by[k + 1]));
-      uint32_t nib = 0, t[4], r[4];
-      if (i0 + 5 <= wlen && lo + i0 > 0) {  // the four positions and their right neighbours all hold text
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          nib |= uint32_t(info[k] == 0xFFFFu) << k;
-          t[k] = identity_ids ? by[k + 1] : uint32_t(__ldg(T.byte_to_id + by[k + 1]));
-          r[k] = (info[k + 1] < SEL) ? info[k + 1] : NONE;
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int i      = i0 + k;
-          const bool start = (i >= wlen) || (lo + i == 0) || (info[k] == 0xFFFFu);
-          nib |= uint32_t(start) << k;
-          t[k] = (i < wlen) ? (identity_ids ? by[k + 1] : uint32_t(__ldg(T.byte_to_id + by[k + 1]))) : DEAD;
-          r[k] = ((i + 1 < wlen) && info[k + 1] < SEL) ? info[k + 1] : NONE;
-        }
-      }
-      const uint32_t word = __reduce_or_sync(0xFFu << (lane & 24), nib << (4 * (lane & 7)));
-      if ((lane & 7) == 0) S.cut[g >> 3] = word;
-      *reinterpret_cast<uint2*>(&S.tok[i0]) = make_uint2(t[0] | (t[1] << 16), t[2] | (t[3] << 16));
-      *reinterpret_cast<uint2*>(&S.rk[i0])  = make_uint2(r[0] | (r[1] << 16), r[2] | (r[3] << 16));
-    }
-    __syncthreads();
-
-    GTK_PHASE(1);
-    // ---- C. chunk boundaries are segment starts too ----
-    {
-      const int64_t c0 = b.tile_chunk0[k];
-      for (int64_t c = c0 + tid; c <= C; c += kOptThreads) {
-        const int64_t p = b.chunk_off[c] - lo;
-        if (p >= wlen) break;
-        if (p >= 0 && GTK_IN(p, kWindow, 28)) {
-          atomicOr(&S.cut[p >> 5], 1u << (p & 31));
-          if (p > 0) S.rk[p - 1] = uint16_t(NONE);
-        }
-      }
-    }
-    __syncthreads();
-
-    GTK_PHASE(2);
-    // ---- D/E1. every thread walks the multi-byte segments that start in its 16 positions.
-    //      Whole-segment lookup: a segment whose bytes are a vocabulary string that the greedy rule
-    //      collapses to one id is finished with two independent table loads; the others go to the
-    //      list of misses (short), the warp queue (long) or the oversize slot (runs past the window) ----
-    {
-      if (tid < kTile / 32) {
-        const int w0        = tid * 32;
-        const uint32_t word = S.cut[tid];
-        const uint32_t ownmask = (w0 + 32 <= own) ? 0xFFFFFFFFu : (w0 >= own ? 0u : ((1u << (own - w0)) - 1u));
-        const uint32_t starts  = word & ownmask;
-        if (starts) {
-          const int last = w0 + 31 - __clz(int(starts));
-          atomicMin(&S.first_start, w0 + __ffs(int(starts)) - 1);
-          atomicMax(&S.last_start, last);
-          // end of the owned region = end of the last owned segment, taken while the bitmap still holds
-          // segment starts only (ends grow with starts, so the maximum is the last segment's end)
-          atomicMax(&S.end_owned, next_cut(S.cut, last));
-        }
-      }
-      if (SEQ) walk_segments_cta(T.word_slots, 32u - T.word_log2_capacity, own, wlen, status);
-      else walk_segments(T.word_slots, 32u - T.word_log2_capacity, own, wlen, status);
-    }
-    __syncthreads();
-    GTK_PHASE(3);
-    const int nmiss = S.nmiss;
-
-    // ---- E1c. the misses, sorted by length (longest first) so that the lanes of a warp work on segments of
-    //           similar length in step E2: thread j keeps entry j in registers while the list is rewritten ----
-    if (nmiss > 32 && nmiss <= kOptThreads) {
-      if (tid < 34) S.hist[tid] = 0;
-      __syncthreads();
-      int ss = 0, LL = 0, slot = 0;
-      if (tid < nmiss) {
-        ss   = S.seg[tid];
-        LL   = next_cut(S.cut, ss) - ss;
-        if (!GTK_IN(LL, 33, 8)) LL = 2;
-        slot = atomicAdd(&S.hist[LL], 1);
-      }
-      __syncthreads();
-      if (warp == 0) {  // exclusive prefix over lengths 32, 31, ... 2
-        const int len = 32 - lane;
-        const int v   = S.hist[len];
-        int inc       = v;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const int y = __shfl_up_sync(0xFFFFFFFFu, inc, d);
-          if (lane >= d) inc += y;
-        }
-        S.hist[len] = inc - v;
-      }
-      __syncthreads();
-      if (tid < nmiss && GTK_IN(S.hist[LL] + slot, kSegCap, 9)) S.seg[S.hist[LL] + slot] = uint16_t(ss);
-      __syncthreads();
-    }
-
-#ifdef GTK_PHASE_TIMING
-    if (tid == 0) {
-      atomicAdd(&g_phase_cycles[10], (unsigned long long)nmiss);
-      atomicAdd(&g_phase_cycles[11], (unsigned long long)S.nseg);
-    }
-#endif
-    // ---- E2. short segments that missed the lookup: one thread per segment (the usual case), or, when a
-    //          tile has more misses than threads, every lane pulls segments from a CTA-wide list and does one
-    //          merge step per loop trip ----
-    GTK_PHASE(12);
-    if (nmiss <= kOptThreads) {
-      // at most one segment per thread (the usual case): no queue, thread t takes entry t of the sorted list
-      int s = -1, L = 0;
-      if (tid < nmiss) {
-        s = S.seg[tid];
-        L = next_cut(S.cut, s) - s;
-      }
-      // The ranks go to the lane-interleaved scratch when the warp's longest segment fits its area (nobody
-      // needs the staged bytes any more).
-      // Two sizes only: every further copy of the loop costs instruction-cache hits on text with many long runs.
-      const int wmax  = __reduce_max_sync(0xFFFFFFFFu, L);
-      const int words = (wmax + 1) >> 1;
-      const int area  = warp * 32 * kLaneWords;
-      const int room  = min(kLaneWords, (kLaneScratchWords - area) / 32);
-      const uint32_t all = (s < 0) ? 0u : ((L >= 32) ? 0xFFFFFFFFu : ((1u << L) - 1u));
-      uint32_t alive;
-      if (words > room) alive = thread_merge_segments(s, L, pair_table(T));
-      else if (words <= 4) alive = thread_merge_segments_lanes<4>(s, L, pair_table(T), area, all);
-      else alive = thread_merge_segments_lanes<8>(s, L, pair_table(T), area, all);
-      if (s >= 0) mark_alive(S.cut, s, alive);
-    } else {
-      const int nseg   = nmiss;
-      int s            = -1, L = 0;
-      uint32_t alive   = 0, best = 0xFFFFFFFFu;
-      bool drained     = false;
-      const PairTable P = pair_table(T);
-      for (;;) {
-        const bool need   = (s < 0) && !drained;
-        const uint32_t nb = __ballot_sync(0xFFFFFFFFu, need);
-        if (nb) {
-          const int leader = __ffs(int(nb)) - 1;
-          int base         = 0;
-          if (lane == leader) base = atomicAdd(&S.seg_next, __popc(nb));
-          base = __shfl_sync(0xFFFFFFFFu, base, leader);
-          if (need) {
-            const int j = base + __popc(nb & lt);
-            if (j >= nseg) {
-              drained = true;
-            } else {
-              const int ss0 = S.seg[j];
-              const int LL0 = next_cut(S.cut, ss0) - ss0;
-              s     = ss0;
-              L     = LL0;
-              alive = (L >= 32) ? 0xFFFFFFFFu : ((1u << L) - 1u);
-              best  = segment_argmin(S.rk, s, L);
-            }
-          }
-        }
-        if (!__any_sync(0xFFFFFFFFu, s >= 0)) {
-          if (__all_sync(0xFFFFFFFFu, drained)) break;
-          continue;
-        }
-        if (s >= 0 && !thread_merge_step(S.tok, S.rk, s, L, alive, best, P)) {
-          mark_alive(S.cut, s, alive);
-          s = -1;
-        }
-      }
-    }
-    __syncthreads();
-
-    GTK_PHASE(13);
-    GTK_PHASE(4);
-    // ---- F. one warp per long segment ----
-    {
-      const int nl = min(S.nlong, kLongCap);
-      for (int q = warp; q < nl; q += kOptThreads / 32) {
-        const int s   = S.longq[q];
-        const int L   = next_cut(S.cut, s) - s;
-        if (!(GTK_IN(s, kWindow, 19) && GTK_IN(s + L, kWindow + 1, 20))) continue;
-        const int len = group_merge_dense<1>(S.tok + s, S.rk + s, L, T, nullptr, status);  // ids at the front
-        mark_alive_range(S.cut, s + 1, s + len, lane);
-        __syncwarp();
-      }
-    }
-    __syncthreads();
-
-    GTK_PHASE(5);
-    // ---- G/H. compact the owned region [first, end) into S.rk, then to staging ----
-    const int first     = S.first_start;
-    const int end_owned = min((S.over_start >= 0) ? S.over_start : S.end_owned, wlen);
-    int total;
-    {
+  });
+  GTK_PHASE(0);
+  tile_lookup(S, sp, T, status);
+  GTK_PHASE(1);
+  const int first = S.first;
+  const int end   = (S.over_start >= 0) ? S.over_start : S.end;
+  uint16_t* ws    = b.seg_scratch ? b.seg_scratch + int64_t(blockIdx.x) * 2 * b.seg_scratch_tokens : nullptr;
+  tile_merge(S, T, ws, b.seg_scratch_tokens, status);
+  GTK_PHASE(2);
+  const int64_t region_start = sp.lo + min(first, sp.wlen);
+  tile_emit<kOptThreads, false>(S, first, end, nullptr, [&](int off, const uint16_t* ids, int n) {
+    uint16_t* dst = b.staging + region_start + off;
+    for (int j = lane; j < n; j += 32)
+      if (GTK_IN(region_start + off + j, b.n_bytes, 22)) dst[j] = ids[j];
+  });
+  __syncthreads();
+  GTK_PHASE(3);
+  const int total = S.total;
+  if (S.no_space && tid == 0) atomicMax(status, int(kStatusScratchTooSmall));
+  GTK_PHASE(4);
+  // per-chunk token counts from the bitmap of live tokens
+  const int64_t region_end = sp.lo + end;
+  if (c0 < C && region_end <= b.chunk_off[c0 + 1]) {
+    // the owned region lies inside the chunk that holds the tile's first byte (CTA-uniform test): the tile's total
+    if (tid == 0 && total > 0 && GTK_IN(c0, b.chunk_cap, 24)) atomicAdd(b.chunk_cnt + c0, total);
+  } else {
+    for (int64_t c = c0 + warp; c < C; c += kOptThreads / 32) {
+      const int64_t cs_g = b.chunk_off[c];
+      if (cs_g >= region_end) break;
+      const int cs = int(max(cs_g, region_start) - sp.lo);
+      const int ce = int(min(b.chunk_off[c + 1], region_end) - sp.lo);
+      if (ce <= cs) continue;
       int cnt = 0;
-      if (tid < used_words) {  // the bitmap now marks live tokens; keep the owned range [first, end_owned)
-        const int w0 = tid * 32;
-        uint32_t x   = S.cut[tid];
-        x &= (first <= w0) ? 0xFFFFFFFFu : ((first >= w0 + 32) ? 0u : (0xFFFFFFFFu << (first - w0)));
-        x &= (end_owned >= w0 + 32) ? 0xFFFFFFFFu : ((end_owned <= w0) ? 0u : ((1u << (end_owned - w0)) - 1u));
-        S.cut[tid] = x;
-        cnt        = __popc(x);
-      }
-      const int off = block_exclusive_scan(cnt, S.scanbuf, &total);
-      if (tid < used_words) S.woff[tid] = uint16_t(off);
-    }
-    __syncthreads();
-    for (int g = tid; g < used_groups; g += kOptThreads) {
-      const int i0        = g * 4;
-      const int sh        = 4 * (lane & 7);
-      const uint32_t word = S.cut[g >> 3];
-      uint32_t nib        = (word >> sh) & 0xFu;
-      if (nib) {
-        int d          = S.woff[g >> 3] + __popc(word & ((1u << sh) - 1u));
-        const uint2 tk = *reinterpret_cast<const uint2*>(&S.tok[i0]);
-        const uint32_t t[4] = {tk.x & 0xFFFFu, tk.x >> 16, tk.y & 0xFFFFu, tk.y >> 16};
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (((nib >> k) & 1u) && GTK_IN(d, kWindow, 21)) S.rk[d++] = uint16_t(t[k]);
-      }
-    }
-    __syncthreads();
-    if (SEQ) {
-      // ---- single-CTA kernel: ids and chunk offsets go straight to the output ----
-      // J'. a segment that runs past the window is merged first (its tokens follow the tile's own ones)
-      int over_len         = 0;
-      const uint16_t* wtok = nullptr;
-      if (S.over_start >= 0) {  // CTA-uniform
-        const int64_t gs0 = lo + S.over_start;
-        if (tid == 0) {
-          int64_t c = b.tile_chunk0[k];
-          while (c + 1 < C && b.chunk_off[c + 1] <= gs0) ++c;
-          S.over_end = b.chunk_off[c + 1];
-        }
-        __syncthreads();
-        const int64_t cend = S.over_end;
-        int64_t ge         = cend;
-        for (int64_t pos = lo + kWindow; pos < cend; pos += kOptThreads) {
-          const int64_t p = pos + tid;
-          const bool cutp = (p < cend) && !adj_bit(T.adj, b.bytes[p - 1], b.bytes[p]);
-          if (__syncthreads_or(cutp)) {
-            if (cutp) atomicMin(reinterpret_cast<unsigned long long*>(&S.over_end), (unsigned long long)p);
-            __syncthreads();
-            ge = S.over_end;
-            break;
-          }
-        }
-        const int64_t L64 = ge - gs0;
-        if (L64 > b.seg_scratch_tokens || b.seg_scratch == nullptr) {
-          if (tid == 0) atomicMax(status, int(kStatusScratchTooSmall));
-        } else {
-          const int L   = int(L64);
-          uint16_t* wt  = b.seg_scratch + int64_t(blockIdx.x) * 2 * b.seg_scratch_tokens;
-          uint16_t* wrk = wt + b.seg_scratch_tokens;
-          for (int i = tid; i < L; i += kOptThreads) {
-            const uint32_t cur = b.bytes[gs0 + i];
-            wt[i]  = __ldg(T.byte_to_id + cur);
-            wrk[i] = (i + 1 < L) ? __ldg(T.byte_pair_rank + ((cur << 8) | b.bytes[gs0 + i + 1])) : uint16_t(NONE);
-          }
-          __syncthreads();
-          over_len = group_merge<kOptThreads / 32, true>(wt, wrk, L, T, &S.gs, status);
-          wtok     = wt;
-        }
-        __syncthreads();
-      }
-      const int64_t out_base = S.run_base;  // written by thread 0 behind the barrier at the end of the last tile
-      const uint16_t* map    = b.low_id_map;
-      for (int j = tid; j < total; j += kOptThreads) {
-        const uint32_t t = S.rk[j];
-        if (out_base + j < b.out_capacity)
-          b.out_ids[out_base + j] = int32_t((map && t < 256u) ? uint32_t(__ldg(map + t)) : t);
-      }
-      for (int j = tid; j < over_len; j += kOptThreads) {
-        const uint32_t t = wtok[j];
-        if (out_base + total + j < b.out_capacity)
-          b.out_ids[out_base + total + j] = int32_t((map && t < 256u) ? uint32_t(__ldg(map + t)) : t);
-      }
-      // id offset of every chunk that starts in this tile: the ids in front of the tile plus the live tokens of the
-      // tile in front of the chunk's first byte (a chunk start is a segment start, so it lies inside the owned
-      // region, or is the start of the oversize segment right behind it)
-      const int64_t c0 = b.tile_chunk0[k];
-      for (int64_t c = c0 + tid; c < C; c += kOptThreads) {
-        const int64_t p64 = b.chunk_off[c] - lo;
-        if (p64 >= own) break;
-        if (p64 >= 0) {
-          const int p = int(p64);
-          const int64_t at = out_base + S.woff[p >> 5] + __popc(S.cut[p >> 5] & ((1u << (p & 31)) - 1u));
-          b.chunk_id_off[c]    = at;
-          b.chunk_id_mirror[c] = at;
-        }
-      }
-      __syncthreads();
-      if (tid == 0) {
-        S.run_base = out_base + total + over_len;
-        if (k == b.n_tiles - 1) {  // the tile with the last byte closes the offsets
-          b.chunk_id_off[C]    = S.run_base;
-          b.chunk_id_mirror[C] = S.run_base;
-        }
-      }
-      return;
-    }
-    const int64_t region_start = lo + ((first < kWindow) ? first : 0);
-    for (int j = tid; j < total; j += kOptThreads)
-      if (GTK_IN(j, kWindow, 22) && GTK_IN(region_start + j, n, 23)) b.staging[region_start + j] = S.rk[j];
-
-    GTK_PHASE(6);
-    // ---- I. per-chunk token counts from the alive bitmap ----
-    {
-      const int64_t region_end = lo + end_owned;
-      const int64_t c0         = b.tile_chunk0[k];
-      if (c0 < C && region_end <= b.chunk_off[c0 + 1]) {
-        // the owned region lies inside the chunk that holds the tile's first byte (CTA-uniform test):
-        // the count is the tile's total
-        if (tid == 0 && total > 0 && GTK_IN(c0, b.chunk_cap, 24)) atomicAdd(b.chunk_cnt + c0, total);
-      } else
-      for (int64_t c = c0 + warp; c < C; c += kOptThreads / 32) {
-        const int64_t cs_g = b.chunk_off[c];
-        if (cs_g >= region_end) break;
-        const int64_t ce_g = b.chunk_off[c + 1];
-        const int cs = int(max(cs_g, region_start) - lo);
-        const int ce = int(min(ce_g, region_end) - lo);
-        if (ce <= cs) continue;
-        int cnt = 0;
-        for (int w = (cs >> 5) + lane; w <= ((ce - 1) >> 5); w += 32) {
-          uint32_t x = S.cut[w];
-          if (w == (cs >> 5)) x &= 0xFFFFFFFFu << (cs & 31);
-          if (w == ((ce - 1) >> 5)) x &= 0xFFFFFFFFu >> (31 - ((ce - 1) & 31));
-          cnt += __popc(x);
-        }
-        cnt = __reduce_add_sync(0xFFFFFFFFu, cnt);
-        if (lane == 0 && cnt && GTK_IN(c, b.chunk_cap, 25)) atomicAdd(b.chunk_cnt + c, cnt);
-      }
-    }
-
-    GTK_PHASE(7);
-    // ---- J. a segment that runs past the window (rare): whole CTA, HBM workspace ----
-    if (S.over_start >= 0) {  // CTA-uniform
-      const int64_t gs0 = lo + S.over_start;
-      if (tid == 0) {
-        int64_t c = b.tile_chunk0[k];
-        while (c + 1 < C && b.chunk_off[c + 1] <= gs0) ++c;
-        S.over_chunk = int(c);
-        S.over_end   = b.chunk_off[c + 1];
-      }
-      __syncthreads();
-      // first never-merge boundary after the window, at most the chunk end
-      const int64_t cend = S.over_end;
-      int64_t ge         = cend;
-      for (int64_t pos = lo + kWindow; pos < cend; pos += kOptThreads) {
-        const int64_t p = pos + tid;
-        const bool cutp = (p < cend) && !adj_bit(T.adj, b.bytes[p - 1], b.bytes[p]);
-        if (__syncthreads_or(cutp)) {
-          if (cutp) atomicMin(reinterpret_cast<unsigned long long*>(&S.over_end), (unsigned long long)p);
-          __syncthreads();
-          ge = S.over_end;
-          break;
-        }
-      }
-      const int64_t L64 = ge - gs0;
-      if (L64 > b.seg_scratch_tokens || b.seg_scratch == nullptr) {
-        if (tid == 0) atomicMax(status, int(kStatusScratchTooSmall));
-      } else {
-        const int L    = int(L64);
-        uint16_t* wtok = b.seg_scratch + int64_t(blockIdx.x) * 2 * b.seg_scratch_tokens;
-        uint16_t* wrk  = wtok + b.seg_scratch_tokens;
-        for (int i = tid; i < L; i += kOptThreads) {
-          const uint32_t cur = b.bytes[gs0 + i];
-          wtok[i] = __ldg(T.byte_to_id + cur);
-          wrk[i]  = (i + 1 < L) ? __ldg(T.byte_pair_rank + ((cur << 8) | b.bytes[gs0 + i + 1])) : uint16_t(NONE);
-        }
-        __syncthreads();
-        const int len = group_merge<kOptThreads / 32, true>(wtok, wrk, L, T, &S.gs, status);
-        for (int j = tid; j < len; j += kOptThreads)
-          if (GTK_IN(region_start + total + j, n, 26)) b.staging[region_start + total + j] = wtok[j];
-        if (tid == 0 && GTK_IN(S.over_chunk, b.chunk_cap, 27)) {
-          atomicAdd(b.chunk_cnt + S.over_chunk, len);
-          S.over_len = len;
-        }
-      }
-      __syncthreads();
-    }
-
-    GTK_PHASE(8);
-    // ---- K. unit record ----
-    if (tid == 0) {
-      b.unit_first[k] = region_start;
-      b.unit_cnt[k]   = total + S.over_len;
+      for (int w = (cs >> 5) + lane; w <= ((ce - 1) >> 5); w += 32) cnt += __popc(S.cut[w] & range_mask(w * 32, cs, ce));
+      cnt = __reduce_add_sync(0xFFFFFFFFu, cnt);
+      if (lane == 0 && cnt && GTK_IN(c, b.chunk_cap, 25)) atomicAdd(b.chunk_cnt + c, cnt);
     }
   }
+  int over = 0;
+  if (S.over_start >= 0) {  // CTA-uniform, rare
+    const int64_t start = sp.lo + S.over_start;
+    int64_t cend;
+    const int64_t c = chunk_of(b, c0, C, start, &cend);
+    over = merge_oversize<kOptThreads>(b.bytes, start, sp.lo + kWindow, cend, ws, b.seg_scratch_tokens, T, status);
+    for (int j = tid; j < over; j += kOptThreads)
+      if (GTK_IN(region_start + total + j, b.n_bytes, 26)) b.staging[region_start + total + j] = ws[j];
+    if (tid == 0 && over > 0 && GTK_IN(c, b.chunk_cap, 27)) atomicAdd(b.chunk_cnt + c, over);
+  }
+  if (tid == 0) {
+    b.unit_first[k] = region_start;
+    b.unit_cnt[k]   = total + over;
+  }
+  GTK_PHASE(5);
 }
 
-// Six CTAs per SM (40 registers per thread) measured faster than eight (32 registers, 120 bytes of spills): the
-// shared memory the two missing CTAs leave free becomes L1 for the table probes.
+// Bound by latency and issue together (see gtk_tile.cuh): 56 % of the issue slots, 54 % of the L1 data pipe, DRAM 3 %.
+// 128 MiB in 4 KiB chunks, this kernel alone: English-like text 1027 us before (five table loads and full token and rank
+// arrays per position, no reuse of merged segments within the batch), 580 us now; the sample novel 941 -> 490 us; 64 MiB
+// with multi-byte words and runs 750 -> 545 us.  Seven CTAs per SM with 36 registers: 443 us for the 64 MiB call on
+// English-like text, against 453 with six and 40, 467 with five and 48 registers; eight with 32 measure the same as seven.
 #ifndef GTK_OPT_CTAS
-#define GTK_OPT_CTAS 6
+#define GTK_OPT_CTAS 7
 #endif
-__global__ void __launch_bounds__(kOptThreads, GTK_OPT_CTAS) k_merge_opt(EncodeBuffers b, DeviceTable T)
+__global__ void __launch_bounds__(kOptThreads, GTK_OPT_CTAS) k_merge_opt(EncodeBuffers b, const __grid_constant__ DeviceTable T)
 {
-  OptSmem& S = g_tile;
-  const int tid   = threadIdx.x;
+  TileSmem<kOptThreads>& S = tile_smem<kOptThreads>();
   const int64_t C = b.totals[0];
-  opt_tile_setup(S, T);
-  for (;;) {
+  tile_setup(S);
+  int64_t k = blockIdx.x;  // the first tile of every CTA, the others by ticket
+  while (k < b.n_tiles) {
+    int next = 0;
+    if (threadIdx.x == 0) next = atomicAdd(b.counters + 0, 1);  // on its way while the tile is worked on
+    tile_reset(S);
     __syncthreads();
-    if (tid == 0) {
-      S.ticket = atomicAdd(b.counters + 0, 1);
-      opt_tile_reset(S);
-    }
+    opt_tile(S, b, T, k, C);
+    if (threadIdx.x == 0) S.ticket = next;
     __syncthreads();
-    const int64_t k = S.ticket;
-    if (k >= b.n_tiles) break;
-    opt_tile<false>(S, b, T, k, C);
+    k = int64_t(gridDim.x) + S.ticket;
   }
 }
 
@@ -1978,14 +1152,81 @@ __global__ void __launch_bounds__(kMediumThreads) k_scans_medium(EncodeBuffers b
     for (int64_t t = tid; t <= b.n_texts; t += kMediumThreads) b.text_id_off[t] = b.chunk_id_off[b.text_chunk_base[t]];
 }
 
-__global__ void __launch_bounds__(kOptThreads) k_encode_small(EncodeBuffers b, DeviceTable T)
+// One tile of a small batch: the tiles are walked in order by one CTA, so its ids and the id offsets of the chunks that
+// start in it go straight to the output, at the running id count S.run.
+__device__ __forceinline__ void small_tile(TileSmem<kOptThreads>& S, const EncodeBuffers& b, const DeviceTable& T, int64_t k,
+                                           int64_t C)
 {
-  OptSmem& S = g_tile;
+  __shared__ uint16_t woff[TileSmem<kOptThreads>::kWords];
+  const int tid = threadIdx.x, lane = tid & 31;
+  int* status   = b.counters + 1;
+  const Span sp = batch_span(b, k);
+  const int64_t c0 = b.tile_chunk0[k];
+  tile_cut(S, sp, T, [&](auto mark) {
+    for (int64_t c = c0 + lane; c <= C; c += 32) {
+      const int64_t p = b.chunk_off[c] - sp.lo;
+      if (p >= sp.wlen) break;
+      if (p >= 0) mark(int(p));
+    }
+  });
+  tile_lookup(S, sp, T, status);
+  const int first = S.first;
+  const int end   = (S.over_start >= 0) ? S.over_start : S.end;
+  tile_merge(S, T, b.seg_scratch, b.seg_scratch_tokens, status);
+  const int64_t out_base = S.run;  // written by thread 0 behind the barrier at the end of the last tile
+  const uint16_t* map    = b.low_id_map;
+  auto put = [&](int64_t at, uint32_t t) {
+    if (at < b.out_capacity) b.out_ids[at] = int32_t((map && t < 256u) ? uint32_t(__ldg(map + t)) : t);
+  };
+  tile_emit<kOptThreads, true>(S, first, end, woff, [&](int off, const uint16_t* ids, int n) {
+    for (int j = lane; j < n; j += 32) put(out_base + off + j, ids[j]);
+  });
+  __syncthreads();
+  const int total = S.total;
+  if (S.no_space && tid == 0) atomicMax(status, int(kStatusScratchTooSmall));
+  int over        = 0;
+  const uint16_t* over_ids = nullptr;
+  if (S.over_start >= 0) {  // CTA-uniform
+    const int64_t start = sp.lo + S.over_start;
+    int64_t cend;
+    chunk_of(b, c0, C, start, &cend);
+    over_ids = b.seg_scratch;
+    over = merge_oversize<kOptThreads>(b.bytes, start, sp.lo + kWindow, cend, b.seg_scratch, b.seg_scratch_tokens, T, status);
+  }
+  for (int j = tid; j < over; j += kOptThreads) put(out_base + total + j, over_ids[j]);
+  // id offset of every chunk that starts in this tile: the ids in front of the tile plus the live tokens of the
+  // tile in front of the chunk's first byte (a chunk start is a segment start, so it lies inside the owned
+  // region, or is the start of the oversize segment right behind it)
+  for (int64_t c = c0 + tid; c < C; c += kOptThreads) {
+    const int64_t p64 = b.chunk_off[c] - sp.lo;
+    if (p64 >= sp.own_hi) break;
+    if (p64 >= 0) {
+      const int p = int(p64);
+      const uint32_t in_front = S.cut[p >> 5] & range_mask(p & ~31, first, end) & ((1u << (p & 31)) - 1u);
+      const int64_t at = out_base + woff[p >> 5] + __popc(in_front);
+      b.chunk_id_off[c]    = at;
+      b.chunk_id_mirror[c] = at;
+    }
+  }
+  __syncthreads();
+  if (tid == 0) {
+    S.run = out_base + total + over;
+    if (k == b.n_tiles - 1) {  // the tile with the last byte closes the offsets
+      b.chunk_id_off[C]    = S.run;
+      b.chunk_id_mirror[C] = S.run;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kOptThreads) k_encode_small(EncodeBuffers b, const __grid_constant__ DeviceTable T)
+{
+  TileSmem<kOptThreads>& S = tile_smem<kOptThreads>();
+  __shared__ int scanbuf[33];
   __shared__ int64_t carry_s;
   const int tid = threadIdx.x;
   unsigned long long t_start = 0;
   if (tid == 0) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_start));
-  opt_tile_setup(S, T);
+  tile_setup(S);
   if (tid < 4) b.counters[tid] = 0;
   // One text of a few chunks (the one-string-per-call case): its chunk table is arithmetic and lives in shared
   // memory, so nothing is read over PCIe but the text itself and no search or scan runs.
@@ -2009,7 +1250,7 @@ __global__ void __launch_bounds__(kOptThreads) k_encode_small(EncodeBuffers b, D
   }
   // chunker: chunks per text -> offsets of every chunk -> first chunk of every tile
   C = cta_exclusive_scan(ChunksPerText{b.text_off, b.chunk_bytes}, b.n_texts, b.text_chunk_base,
-                         S.scanbuf, &carry_s);
+                         scanbuf, &carry_s);
   for (int64_t c = tid; c <= C; c += kOptThreads) {
     if (c == C) {
       b.chunk_off[c] = b.text_off[b.n_texts];
@@ -2034,18 +1275,18 @@ __global__ void __launch_bounds__(kOptThreads) k_encode_small(EncodeBuffers b, D
   }
   }
   // tiles, one after the other; each writes its ids and the id offsets of the chunks that start in it
-  if (tid == 0) S.run_base = 0;
+  if (tid == 0) S.run = 0;
   for (int64_t k = 0; k < b.n_tiles; ++k) {
     __syncthreads();
-    if (tid == 0) opt_tile_reset(S);
+    tile_reset(S);
     __syncthreads();
-    opt_tile<true>(S, b, T, k, C);
+    small_tile(S, b, T, k, C);
   }
   __syncthreads();
   // the offsets of the texts follow from those of their chunks; the caller-visible chunk offsets may live in
   // mapped host memory, so they are read back from the copy in device memory
   if (one_text) {
-    if (tid < 2) b.text_id_off[tid] = tid ? S.run_base : 0;
+    if (tid < 2) b.text_id_off[tid] = tid ? S.run : 0;
   } else {
     for (int64_t t = tid; t <= b.n_texts; t += kOptThreads) b.text_id_off[t] = b.chunk_id_mirror[b.text_chunk_base[t]];
   }
@@ -2056,7 +1297,7 @@ __global__ void __launch_bounds__(kOptThreads) k_encode_small(EncodeBuffers b, D
     unsigned long long t_end;
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t_end));
     b.totals[0] = C;
-    b.totals[1] = S.run_base;
+    b.totals[1] = S.run;
     b.totals[2] = int64_t(b.counters[1]);
     b.totals[4] = int64_t(t_end - t_start);
     __threadfence_system();
@@ -2065,56 +1306,84 @@ __global__ void __launch_bounds__(kOptThreads) k_encode_small(EncodeBuffers b, D
 }
 
 // ------------------------------------------------------------------------------------------------
-// merge kernel, one CTA per chunk ("base")
+// merge kernels, one CTA per chunk
 // ------------------------------------------------------------------------------------------------
-extern __shared__ __align__(16) unsigned char g_dyn_smem[];
 
-// The chunk lives in dynamic shared memory (tokens and cached ranks, 16 bits each, `smem_tokens` slots per
-// array); a chunk longer than that takes the HBM workspace.  NW warps per CTA: few for short chunks (the cost
-// of a pass is dominated by its fixed part, so many small CTAs per SM give the best throughput), many for
-// long ones.
-template <int NW>
-__global__ void __launch_bounds__(NW * 32) k_merge_base(EncodeBuffers b, DeviceTable T, int smem_tokens)
+// A CTA tokenises chunk [cs, ce) window by window; put(i, id) takes the chunk's i-th id, S.run counts them.  Returns false,
+// with the chunk half done, when a segment needs a workspace and there is none.
+template <int TH, class Put>
+__device__ __forceinline__ bool tokenise_chunk(TileSmem<TH>& S, const uint8_t* bytes, int64_t cs, int64_t ce,
+                                               const DeviceTable& T, uint16_t* scratch, int64_t scratch_tokens,
+                                               int* status, Put put)
 {
-  constexpr int G = NW * 32;
-  uint16_t* s_tok = reinterpret_cast<uint16_t*>(g_dyn_smem);
-  uint16_t* s_rk  = s_tok + smem_tokens;
-  __shared__ GroupScratch gs;
-  __shared__ int ticket;
+  // the first window starts at the 16-byte boundary in front of the chunk, so that every window loads whole vectors
+  const int skip = int(reinterpret_cast<uintptr_t>(bytes + cs) & 15u);
+  for (int64_t lo = cs - skip; lo < ce; lo += S.kOwn) {
+    const bool head = lo <= cs;
+    const Span sp{bytes, lo, head ? skip : 0, int(min(int64_t(S.kOwn), ce - lo)), int(min(int64_t(S.kWin), ce - lo)), !head,
+                  head};
+    __syncthreads();
+    tile_reset(S);
+    if (head && threadIdx.x == 0) S.run = 0;
+    __syncthreads();
+    tile_cut(S, sp, T, [](auto) {});
+    tile_lookup(S, sp, T, status);
+    const int first = S.first;
+    const int end   = (S.over_start >= 0) ? S.over_start : S.end;
+    tile_merge(S, T, scratch, scratch_tokens, status);
+    if (S.no_space || (S.over_start >= 0 && scratch == nullptr)) {  // CTA-uniform
+      __syncthreads();
+      return false;
+    }
+    const int64_t run = S.run;
+    tile_emit<TH, false>(S, first, end, nullptr, [&](int off, const uint16_t* ids, int n) {
+      for (int j = threadIdx.x & 31; j < n; j += 32) put(run + off + j, ids[j]);
+    });
+    __syncthreads();
+    const int total = S.total;
+    int over        = 0;
+    if (S.over_start >= 0) {  // CTA-uniform
+      over = merge_oversize<TH>(bytes, lo + S.over_start, lo + S.kWin, ce, scratch, scratch_tokens, T, status);
+      for (int j = threadIdx.x; j < over; j += TH) put(run + total + j, scratch[j]);
+    }
+    if (threadIdx.x == 0) S.run = run + total + over;
+  }
+  __syncthreads();
+  return true;
+}
+
+template <int TH>
+constexpr int chunk_kernel_ctas()  // 1536 resident threads per SM: 40 registers each, as in the tile kernel
+{
+  return 1536 / TH > 0 ? 1536 / TH : 1;
+}
+
+// GTK_MODE_BASE: one CTA per chunk from a ticket.  The threads per CTA are the caller's choice (the reference's
+// BLOCK_SIZE) or follow the chunk size: a CTA of TH threads works on windows of 16 * TH bytes.
+template <int TH>
+__global__ void __launch_bounds__(TH, chunk_kernel_ctas<TH>()) k_merge_base(EncodeBuffers b, const __grid_constant__ DeviceTable T)
+{
+  TileSmem<TH>& S = tile_smem<TH>();
   const int tid   = threadIdx.x;
   const int64_t C = b.totals[0];
   int* status     = b.counters + 1;
+  tile_setup(S);
+  uint16_t* ws = b.seg_scratch ? b.seg_scratch + int64_t(blockIdx.x) * 2 * b.seg_scratch_tokens : nullptr;
   for (;;) {
     __syncthreads();
-    if (tid == 0) ticket = atomicAdd(b.counters + 2, 1);
+    if (tid == 0) S.ticket = atomicAdd(b.counters + 2, 1);
     __syncthreads();
-    const int64_t c = ticket;
+    const int64_t c = S.ticket;
     if (c >= C) break;
-    const int64_t cs  = b.chunk_off[c];
-    const int64_t L64 = b.chunk_off[c + 1] - cs;
-    uint16_t *tok = s_tok, *rk = s_rk;
-    if (L64 > smem_tokens) {
-      if (L64 > b.seg_scratch_tokens || b.seg_scratch == nullptr) {
-        if (tid == 0) {
-          atomicMax(status, int(kStatusScratchTooSmall));
-          b.chunk_cnt[c] = 0;
-        }
-        continue;
-      }
-      tok = b.seg_scratch + int64_t(blockIdx.x) * 2 * b.seg_scratch_tokens;
-      rk  = tok + b.seg_scratch_tokens;
+    const int64_t cs = b.chunk_off[c];
+    const bool done = tokenise_chunk(S, b.bytes, cs, b.chunk_off[c + 1], T, ws, b.seg_scratch_tokens, status,
+                                     [&](int64_t at, uint32_t id) {
+      if (GTK_IN(cs + at, b.n_bytes, 31)) b.staging[cs + at] = uint16_t(id);
+    });
+    if (tid == 0) {
+      if (!done) atomicMax(status, int(kStatusScratchTooSmall));
+      b.chunk_cnt[c] = done ? int(S.run) : 0;
     }
-    const int L = int(L64);
-    for (int i = tid; i < L; i += G) {
-      const uint32_t cur = b.bytes[cs + i];
-      tok[i] = __ldg(T.byte_to_id + cur);
-      rk[i]  = (i + 1 < L) ? __ldg(T.byte_pair_rank + ((cur << 8) | b.bytes[cs + i + 1])) : uint16_t(NONE);
-    }
-    __syncthreads();
-    const int len = group_merge<NW, true>(tok, rk, L, T, &gs, status);
-    for (int j = tid; j < len; j += G)
-      if (GTK_IN(cs + j, b.n_bytes, 31)) b.staging[cs + j] = tok[j];
-    if (tid == 0) b.chunk_cnt[c] = len;
   }
 }
 
@@ -2386,6 +1655,34 @@ bool chunker_resets_counters(const EncodeBuffers& b)
   return medium_chunker_by_search(b) || medium_chunker_per_text(b);
 }
 
+// One launch instead of two memsets and a device-to-device copy, which take the stream 13 us: 8 MiB in L2 or HBM each way.
+__global__ void __launch_bounds__(512) k_begin_batch(int32_t* counters, int32_t* chunk_cnt, int64_t n_cnt,
+                                                     const uint4* __restrict__ from, uint4* __restrict__ to, int n_words)
+{
+  const int i0 = blockIdx.x * 512 + threadIdx.x, step = gridDim.x * 512;
+  if (counters && i0 < 16) counters[i0] = 0;
+  if (chunk_cnt)
+    for (int64_t i = i0; i < n_cnt; i += step) chunk_cnt[i] = 0;
+  if (to)
+    for (int i = i0; i < n_words; i += 4 * step) {
+      uint4 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (i + k * step < n_words) v[k] = __ldg(from + i + k * step);
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (i + k * step < n_words) to[i + k * step] = v[k];
+    }
+}
+
+int launch_begin_batch(const EncodeBuffers& b, bool counters, const uint4* long_words, uint4* learned, cudaStream_t stream)
+{
+  const int grid = learned ? 256 : grid_for(b.chunk_cap + 1, 512 * 4, 296);  // 256 CTAs: four words of the table per thread
+  k_begin_batch<<<grid, 512, 0, stream>>>(counters ? b.counters : nullptr, counters ? b.chunk_cnt : nullptr, b.chunk_cap + 1,
+                                          long_words, learned, learned ? 2 << kLongBits : 0);
+  return 1;
+}
+
 int launch_chunker(const EncodeBuffers& b, cudaStream_t stream)
 {
   if (medium_chunker_by_search(b) || medium_chunker_per_text(b)) {
@@ -2413,27 +1710,29 @@ int launch_merge_opt(const EncodeBuffers& b, const DeviceTable& t, int grid, cud
   return 1;
 }
 
-// Geometry of the one-CTA-per-chunk kernel for a chunk size: warps per CTA and slots of shared memory per array.
-// block_threads = 0 picks the warp count from the chunk size; 64 .. 1024 (a power of two) forces it, which is what
-// the reference's BLOCK_SIZE compile-time constant does (gputok_blockbpe.cu:313-315).
-void base_kernel_geometry(int chunk_bytes, int block_threads, int* warps, int* smem_tokens)
+// Threads per CTA of the one-CTA-per-chunk kernels.  block_threads = 0 picks them from the chunk size: a CTA covers 16
+// bytes per thread, so 64 threads take a chunk of up to 1 KiB in one window, 128 one of 2 KiB; beyond that 256 threads
+// work window by window (larger CTAs leave more of their threads waiting at barriers).  64 .. 1024 (a power of two)
+// forces it, which is what the reference's BLOCK_SIZE compile-time constant does (gputok_blockbpe.cu:313-315).
+int chunk_kernel_threads(int chunk_bytes, int block_threads)
 {
-  const int c  = std::max(chunk_bytes, 1);
-  const int w  = block_threads > 0 ? block_threads / 32 : (c + 1023) >> 10;  // one warp per KiB of chunk
-  *warps       = w <= 2 ? 2 : w <= 4 ? 4 : w <= 8 ? 8 : w <= 16 ? 16 : 32;
-  *smem_tokens = (std::min(c, kBaseSmemMaxTokens) + 63) & ~63;
+  if (block_threads > 0) return block_threads;
+  return chunk_bytes <= 1024 ? 64 : chunk_bytes <= 2048 ? 128 : 256;
 }
 
 namespace {
-template <int NW>
-int base_blocks_per_sm(int smem_tokens)
+template <int TH>
+constexpr int tile_dynamic_smem()
 {
-  const int bytes = smem_tokens * 4;
-  // opt in to the largest size any chunk length can ask for (a forced block size pairs any warp count with any
-  // chunk length), so that handles with different chunk sizes on one device never lower each other's limit
-  cudaFuncSetAttribute(k_merge_base<NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBaseSmemMaxTokens * 4);
+  return TH <= 256 ? 0 : int(sizeof(TileSmem<TH>));
+}
+template <int TH>
+int base_blocks_per_sm()
+{
+  if (tile_dynamic_smem<TH>())
+    cudaFuncSetAttribute(k_merge_base<TH>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile_dynamic_smem<TH>());
   int nb = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_merge_base<NW>, NW * 32, bytes);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_merge_base<TH>, TH, tile_dynamic_smem<TH>());
   return nb;
 }
 }  // namespace
@@ -2443,15 +1742,12 @@ int launch_merge_base(const EncodeBuffers& b, const DeviceTable& t, int grid, in
   if (b.n_bytes <= 0) return 0;
   if (grid > b.chunk_cap) grid = int(b.chunk_cap);
   if (grid < 1) grid = 1;
-  int nw = 0, st = 0;
-  base_kernel_geometry(b.chunk_bytes, block_threads, &nw, &st);
-  const size_t bytes = size_t(st) * 4;
-  switch (nw) {
-    case 2: k_merge_base<2><<<grid, 64, bytes, stream>>>(b, t, st); break;
-    case 4: k_merge_base<4><<<grid, 128, bytes, stream>>>(b, t, st); break;
-    case 8: k_merge_base<8><<<grid, 256, bytes, stream>>>(b, t, st); break;
-    case 16: k_merge_base<16><<<grid, 512, bytes, stream>>>(b, t, st); break;
-    default: k_merge_base<32><<<grid, 1024, bytes, stream>>>(b, t, st); break;
+  switch (chunk_kernel_threads(b.chunk_bytes, block_threads)) {
+    case 64: k_merge_base<64><<<grid, 64, 0, stream>>>(b, t); break;
+    case 128: k_merge_base<128><<<grid, 128, 0, stream>>>(b, t); break;
+    case 256: k_merge_base<256><<<grid, 256, 0, stream>>>(b, t); break;
+    case 512: k_merge_base<512><<<grid, 512, tile_dynamic_smem<512>(), stream>>>(b, t); break;
+    default: k_merge_base<1024><<<grid, 1024, tile_dynamic_smem<1024>(), stream>>>(b, t); break;
   }
   return 1;
 }
@@ -2697,14 +1993,12 @@ int opt_kernel_max_blocks_per_sm()
 // and returns the resident CTAs per SM.
 int base_kernel_max_blocks_per_sm(int chunk_bytes, int block_threads)
 {
-  int nw = 0, st = 0;
-  base_kernel_geometry(chunk_bytes, block_threads, &nw, &st);
-  switch (nw) {
-    case 2: return base_blocks_per_sm<2>(st);
-    case 4: return base_blocks_per_sm<4>(st);
-    case 8: return base_blocks_per_sm<8>(st);
-    case 16: return base_blocks_per_sm<16>(st);
-    default: return base_blocks_per_sm<32>(st);
+  switch (chunk_kernel_threads(chunk_bytes, block_threads)) {
+    case 64: return base_blocks_per_sm<64>();
+    case 128: return base_blocks_per_sm<128>();
+    case 256: return base_blocks_per_sm<256>();
+    case 512: return base_blocks_per_sm<512>();
+    default: return base_blocks_per_sm<1024>();
   }
 }
 

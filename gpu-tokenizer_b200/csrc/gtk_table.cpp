@@ -171,6 +171,13 @@ void HostTable::build_hash()
   }
 }
 
+// bytes of a string of up to 16 bytes as four zero-padded words
+static void word_key(const std::string& s, uint32_t k[4])
+{
+  k[0] = k[1] = k[2] = k[3] = 0;
+  for (size_t i = 0; i < s.size() && i < 16; ++i) k[i >> 2] |= uint32_t((unsigned char)s[i]) << (8 * (i & 3));
+}
+
 // A segment whose bytes equal a vocabulary string that the greedy rule collapses to that one id
 // needs no merging at all.  The entries are checked here, one by one, with the same greedy routine
 // that defines the result, so the shortcut cannot change any output.
@@ -185,32 +192,32 @@ void HostTable::build_words()
     greedy_chunk(reinterpret_cast<const uint8_t*>(bs.data()), int64_t(bs.size()), out);
     if (out.size() == 1 && out[0] == int32_t(id)) words.emplace_back(bs, int32_t(id));
   }
-  word_count = uint32_t(words.size());
-  word_log2_capacity = 10;
-  while ((size_t(1) << word_log2_capacity) < words.size() * 2 + 1) ++word_log2_capacity;
-  word_slots.assign(size_t(1) << word_log2_capacity, WordSlot{0, 0, 0, 0});
+  word_count   = uint32_t(words.size());
   word_dropped = 0;
-  auto home = [&](const WordSlot& w, int which) {
-    const uint32_t m = word_mix(w.k0, w.k1, w.k2);
-    return which ? word_hash_b(m, word_log2_capacity) : word_hash_a(m, word_log2_capacity);
-  };
-  for (auto& w : words) {
-    uint32_t k[3] = {0, 0, 0};
-    for (size_t i = 0; i < w.first.size(); ++i) k[i >> 2] |= uint32_t((unsigned char)w.first[i]) << (8 * (i & 3));
-    WordSlot cur{k[0], k[1], k[2], (uint32_t(w.first.size()) << 16) | uint32_t(w.second)};
-    // cuckoo insertion: take the first free choice, else evict from alternating choices
-    bool placed = false;
-    int which   = 0;
-    for (int kick = 0; kick < 500 && !placed; ++kick) {
-      const uint32_t ha = home(cur, 0), hb = home(cur, 1);
-      if (word_slots[ha].meta == 0) { word_slots[ha] = cur; placed = true; break; }
-      if (word_slots[hb].meta == 0) { word_slots[hb] = cur; placed = true; break; }
-      const uint32_t at = which ? hb : ha;
-      std::swap(cur, word_slots[at]);
-      // the evicted entry must move to its other choice next
-      which = (home(cur, 0) == at) ? 1 : 0;
+  short_words.assign(size_t(1) << kShortBits, ShortWord{0xFFFFFFFFu, 0xFFFFFFFFu});
+  long_words.assign(size_t(1) << kLongBits, LongWord{{0, 0, 0, 0}, 0, {0, 0, 0}});
+  for (auto& w : words) {  // in the order of ids: the more frequent of two strings comes first
+    const uint32_t len = uint32_t(w.first.size());
+    uint32_t k[4];
+    word_key(w.first, k);
+    if (len <= uint32_t(kShortMaxBytes)) {
+      const uint32_t k1 = k[1] | len << 24;
+      ShortWord& at     = short_words[short_slot(k[0], k1)];
+      if (at.k1 == 0xFFFFFFFFu) {
+        at = ShortWord{k1, (k[0] * kShortMulA) << kShortBits | uint32_t(w.second)};
+        continue;
+      }
     }
-    if (!placed) ++word_dropped;  // `cur` (some entry) is left out: it only loses the shortcut
+    const uint32_t h = long_slot(k, len);
+    uint32_t hop     = 0;
+    while (hop < kLongHops && long_words[h ^ hop].meta != 0) ++hop;
+    if (hop == kLongHops) {  // left out: it only loses the shortcut
+      ++word_dropped;
+      continue;
+    }
+    for (uint32_t j = 0; j < hop; ++j) long_words[h ^ j].meta |= kLongMore;
+    LongWord& at = long_words[h ^ hop];
+    at = LongWord{{k[0], k[1], k[2], k[3]}, len | 1u << 16, {0xFFFF0000u | (uint32_t(w.second) + 1u), 0xFFFFFFFFu, 0xFFFFFFFFu}};
   }
 }
 
@@ -260,17 +267,30 @@ void HostTable::verify_device_tables() const
     if (got != r.rank) throw std::runtime_error("internal error: device pair table does not return a merge's rank");
   }
   uint32_t found = 0;
-  for (const WordSlot& w : word_slots) {
-    if (w.meta == 0) continue;
-    const uint32_t m = word_mix(w.k0, w.k1, w.k2);
-    const WordSlot& a = word_slots[word_hash_a(m, word_log2_capacity)];
-    const WordSlot& c = word_slots[word_hash_b(m, word_log2_capacity)];
-    const bool at_a = a.k0 == w.k0 && a.k1 == w.k1 && a.k2 == w.k2 && a.meta == w.meta;
-    const bool at_c = c.k0 == w.k0 && c.k1 == w.k1 && c.k2 == w.k2 && c.meta == w.meta;
-    if (!at_a && !at_c) throw std::runtime_error("internal error: whole-segment table entry is not at either of its slots");
+  for (const ShortWord& w : short_words) {
+    if (w.k1 == 0xFFFFFFFFu) continue;
+    const std::string& bs = id_to_bytes[w.rest & 0xFFFFu];
+    uint32_t k[4];
+    word_key(bs, k);
+    const uint32_t k1 = k[1] | uint32_t(bs.size()) << 24;
+    const ShortWord& at = short_words[short_slot(k[0], k1)];
+    if (at.k1 != k1 || (at.rest ^ (k[0] * kShortMulA) << kShortBits) != (w.rest & 0xFFFFu))
+      throw std::runtime_error("internal error: short-string table does not return a string's id");
     ++found;
   }
-  if (found + word_dropped != word_count) throw std::runtime_error("internal error: whole-segment table lost entries");
+  for (const LongWord& w : long_words) {
+    if (w.meta == 0) continue;
+    const uint32_t h = long_slot(w.k, w.meta & 31u);
+    bool here        = false;
+    for (uint32_t hop = 0; hop < kLongHops && !here; ++hop) {
+      const LongWord& at = long_words[h ^ hop];
+      here = std::memcmp(at.k, w.k, sizeof(w.k)) == 0 && ((at.meta ^ w.meta) & 31u) == 0 && at.ids[0] == w.ids[0];
+      if (!here && !(at.meta & kLongMore)) break;
+    }
+    if (!here) throw std::runtime_error("internal error: long-string table entry is not where a lookup finds it");
+    ++found;
+  }
+  if (found + word_dropped != word_count) throw std::runtime_error("internal error: whole-segment tables lost entries");
 }
 
 bool HostTable::find(int32_t left, int32_t right, uint32_t* rank, int32_t* merged) const

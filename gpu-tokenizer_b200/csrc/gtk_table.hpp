@@ -6,7 +6,7 @@
 // an open-addressing table with 16-byte slots for host lookups, and for the
 // kernels a bucketed pair table answered by one 128-bit load, a dense 256x256
 // table for byte pairs, per-rank merged ids, a never-merge bigram bitmap and a
-// two-choice cuckoo table of vocabulary strings that are their own tokenisation.
+// tables of vocabulary strings that are their own tokenisation.
 #pragma once
 #include <cstdint>
 #include <string>
@@ -44,26 +44,44 @@ struct alignas(8) PairSlot {
   uint32_t rank;
 };
 
-// One slot of the whole-segment table: a byte string of 2..12 bytes (zero padded to three
-// words) whose greedy tokenisation is the single id in `meta` (length << 16 | id); meta 0 = empty.
-struct alignas(16) WordSlot {
-  uint32_t k0, k1, k2;
-  uint32_t meta;
+// Whole-segment tables: byte strings whose greedy tokenisation is known, so that a segment that equals one of them
+// needs no merging.
+//
+// Short strings (2..7 bytes), one 64-bit load per lookup, found or not.  k0 = first four bytes, k1 = bytes 4..6 with
+// the length in the top byte, zero padded.  p = k0 * kShortMulA is a bijection; the slot is the top bits of
+// p ^ k1 * kShortMulB, so (k1, slot) fix the top bits of p and the slot stores k1 and the other bits of p: an exact
+// key in 8 bytes beside the id.  One string per slot: of two that share a slot the more frequent (lower id) keeps it,
+// the other goes to the long table.
+struct alignas(8) ShortWord {
+  uint32_t k1;   // 0xFFFFFFFF = empty (no string is 255 bytes long)
+  uint32_t rest; // p << kShortBits | id
 };
-constexpr int kWordMaxBytes = 12;
+constexpr uint32_t kShortBits    = 18;  // 2 MiB; 17 bits put 12 % of the strings into the long table, 18 bits 6 %
+constexpr uint32_t kShortMulA    = 0x9E3779B1u;
+constexpr uint32_t kShortMulB    = 0x85EBCA77u;
+constexpr int kShortMaxBytes     = 7;
+inline uint32_t short_slot(uint32_t k0, uint32_t k1) { return ((k0 * kShortMulA) ^ (k1 * kShortMulB)) >> (32 - kShortBits); }
 
-// The whole-segment table is a two-choice cuckoo table: a string sits at word_hash_a or word_hash_b of its
-// key, so a lookup is two independent 128-bit loads and no loop, found or not.
-inline uint32_t word_mix(uint32_t k0, uint32_t k1, uint32_t k2)
+// Strings of up to 16 bytes and up to six ids: 32 bytes, one memory sector.  `meta` = length | bit 16 + i set when a
+// token starts at byte i; 0 = empty.  Ids are stored plus one, unused places hold 0xFFFF, so none of the last three
+// words of a filled slot is zero.  The vocabulary's own strings (one id) are placed when the table is built: at slot h,
+// or, when that is taken, at h ^ 1 .. h ^ 7, with kLongMore set in the slots that were passed over.  The kernels
+// of a large batch work on a copy and fill empty slots with segments they have merged (see merge_batch).
+struct alignas(32) LongWord {
+  uint32_t k[4];
+  uint32_t meta;
+  uint32_t ids[3];
+};
+constexpr uint32_t kLongBits = 18;  // 8 MiB
+constexpr uint32_t kLongHops = 8;
+constexpr uint32_t kLongMore = 0x80u;
+constexpr int kLongMaxIds    = 6;
+constexpr int kWordMaxBytes  = 16;
+inline uint32_t long_slot(const uint32_t k[4], uint32_t length)
 {
-  uint32_t h = (k0 * 0x9E3779B1u) ^ (k1 * 0x85EBCA77u) ^ (k2 * 0xC2B2AE3Du);
+  uint32_t h = k[0] * 0x9E3779B1u ^ k[1] * 0x85EBCA77u ^ k[2] * 0xC2B2AE3Du ^ (k[3] + length) * 0x27D4EB2Fu;
   h ^= h >> 15;
-  return h * 0x2C1B3C6Du;
-}
-inline uint32_t word_hash_a(uint32_t m, uint32_t log2_capacity) { return m >> (32 - log2_capacity); }
-inline uint32_t word_hash_b(uint32_t m, uint32_t log2_capacity)
-{
-  return ((m ^ (m >> 13)) * 0x165667B1u) >> (32 - log2_capacity);
+  return (h * 0x2C1B3C6Du) >> (32 - kLongBits);
 }
 
 struct MergeRow {
@@ -114,10 +132,10 @@ class HostTable {
   uint32_t adj[2048];                      // bit (u<<8|v): bigram occurs inside a merge result
   int adj_count = 0;
 
-  // whole-segment fast path: every vocabulary string of 2..12 bytes that the greedy rule turns
+  // whole-segment fast path: every vocabulary string of 2..16 bytes that the greedy rule turns
   // into exactly its own id (verified one by one with greedy_chunk at build time)
-  std::vector<WordSlot> word_slots;
-  uint32_t word_log2_capacity = 0;
+  std::vector<ShortWord> short_words;
+  std::vector<LongWord> long_words;
   uint32_t word_count = 0;    // strings that qualify
   uint32_t word_dropped = 0;  // of those, not placed (they take the merge path instead)
 

@@ -84,7 +84,7 @@ typedef struct gtk_table_info {
   int32_t  max_iters;
   int32_t  device;           /* CUDA device ordinal, -1 for a host-only handle */
   int32_t  sm_count;
-  int32_t  whole_segment_entries;   /* vocabulary strings (2..12 bytes) answered by one table probe */
+  int32_t  whole_segment_entries;   /* vocabulary strings (2..16 bytes) answered by one table probe */
   uint32_t whole_segment_dropped; /* qualifying strings that found no place (they are merged instead) */
 } gtk_table_info;
 

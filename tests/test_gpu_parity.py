@@ -232,6 +232,32 @@ def test_long_and_huge_segments_in_a_large_batch(lib, merges_path, oracle):
     assert t.decode(ids[:coff[20]]) == filler[:chunk_off[20]].tobytes()
 
 
+@pytest.mark.parametrize("mode", ["opt", "base"])
+@pytest.mark.parametrize("n_bytes", [65537, (12 << 20) - 1, (12 << 20) + 4097])
+def test_segment_lengths_at_the_edges(lib, merges_path, oracle, n_bytes, mode):
+    """Segments of every length around the limits of the tile code: 7 / 8 bytes (short and long string table), 16 / 17
+    (one thread or half a warp, one warp), runs with few and with more than 30 different tokens, segments beyond a warp's
+    272 places and beyond the window; batches below and above the size from which merged segments are added to the long
+    table while the batch runs.  Whole ids: no tolerance."""
+    rng = np.random.default_rng(n_bytes)
+    letters = np.frombuffer(b"etaoinshrdlu", np.uint8)
+    words = [bytes(rng.choice(letters, size=int(k))) for k in np.concatenate([np.arange(1, 40), rng.integers(6, 18, 400)])]
+    words += [b"a" * k for k in (15, 16, 17, 31, 32, 33, 255, 256, 271, 272, 273, 600)]
+    words += [b"x" * k + b"abcabc" + b"y" * k for k in (5, 100)] + [b"e\xcc\x81" * 60, bytes(rng.choice(letters, size=500))]
+    picks = rng.integers(0, len(words), size=n_bytes // 8)
+    blob = b" ".join(words[i] for i in picks)[:n_bytes]
+    if len(blob) < n_bytes:
+        blob += b"z" * (n_bytes - len(blob))
+    if mode == "base":
+        blob = blob[:3 << 20]
+    chunk = 5000
+    want, woff = oracle.encode_fixed(np.frombuffer(blob, np.uint8), chunk, mode=MODE_SEGMENTED, threads=NCPU)
+    t = make_tok(lib, merges_path, chunk)
+    for _ in range(2):  # the second call starts from the vocabulary's own strings again
+        ids, _, coff, _ = t.encode(blob, mode=lib.GTK_MODE_OPT if mode == "opt" else lib.GTK_MODE_BASE)
+        check_chunks(ids, coff, want, woff, f"segment lengths, {n_bytes} bytes, {mode}")
+
+
 def test_crowded_pair_bucket(lib, merges_path, tmp_path):
     """More than four pairs in one bucket of the device pair table: the fifth and later ones are found in
     the side table (second load), in every kernel that probes."""
