@@ -989,6 +989,7 @@ bool handle_view(gtk_tokenizer* h, HandleView* out)
 {
   if (!h || !out) return false;
   out->device = h->device;
+  out->sm_count = h->sm_count;
   out->stream = h->stream;
   out->table = h->dtab;
   out->wide = h->wide;

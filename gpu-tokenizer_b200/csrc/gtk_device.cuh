@@ -128,6 +128,7 @@ constexpr int kFinishMaxTiles = 32;  // batches through launch_finish_small_batc
 // What the allocation-free entry point needs from a handle (defined in gtk_api.cu).
 struct HandleView {
   int device;
+  int sm_count;
   cudaStream_t stream;
   DeviceTable table;
   const uint16_t* low_id_map;  // nullptr, or the 256-entry remap of ids < 256 (GPT-2 id space selected)

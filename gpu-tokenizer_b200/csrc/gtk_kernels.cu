@@ -2012,29 +2012,72 @@ int localmin_kernel_max_blocks_per_sm()
 }  // namespace gtk
 
 // ------------------------------------------------------------------------------------------------
-// Allocation-free entry point (declared in include/gputok_b200.h): the one-CTA-per-chunk merge
-// kernel with its ticket counter, status word and long-chunk workspace in a fixed device array
-// instead of buffers from cudaMalloc.
+// Allocation-free entry point (declared in include/gputok_b200.h): the one-CTA-per-chunk kernel with its ticket counter
+// and status words in a fixed device array instead of buffers from cudaMalloc.  The kernel needs no workspace but for
+// segments of several hundred bytes; chunks that have one are left to a second kernel, which merges the whole chunk pass
+// by pass with the workspace of the fixed array.
 // ------------------------------------------------------------------------------------------------
 #include "../../include/gputok_b200.h"
 
 namespace {
 
-constexpr int kNoAllocCtas        = 128;                          // persistent CTAs of the kernel
+constexpr int kNoAllocCtas        = 128;                          // CTAs of the second kernel
 constexpr int kNoAllocMaxTokens   = GTK_NOALLOC_MAX_CHUNK_BYTES;  // longest chunk (one token per byte at most)
-constexpr size_t kNoAllocHeader   = 256;                          // [0] chunk ticket, [1] status word
+constexpr size_t kNoAllocHeader   = 256;  // [0] chunk ticket, [1] status word, [2] chunks put off, [3] ticket of the second kernel
 constexpr size_t kNoAllocPerCta   = size_t(2) * kNoAllocMaxTokens * sizeof(uint16_t);  // tokens + ranks
 constexpr size_t kNoAllocBytes    = kNoAllocHeader + size_t(kNoAllocCtas) * kNoAllocPerCta;  // 8 MiB + 256 B
 constexpr int kMaxDevices         = 64;
+constexpr int32_t kPutOff         = -1;  // count of a chunk that waits for the second kernel
 
 // Lives in the library image on every GPU that loads it.  In host code this name is only a
 // stand-in for the symbol; the device address comes from cudaGetSymbolAddress below.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
+// 2 MiB of the sample novel in 4 KiB chunks, whole call: 5.9 ms when every chunk went through the kernel below (one pass
+// over the chunk per merge rank), 53 us now; see gtk_tile.cuh for what bounds it.
+template <int TH>
+__global__ void __launch_bounds__(TH, gtk::chunk_kernel_ctas<TH>())
+k_chunks_noalloc(const uint8_t* __restrict__ bytes, int64_t n_bytes, const int64_t* __restrict__ chunk_off,
+                 int64_t n_chunks, int max_chunk, int32_t* __restrict__ out_ids, int32_t* __restrict__ out_counts,
+                 const __grid_constant__ gtk::DeviceTable T, const uint16_t* __restrict__ low_id_map, int* header)
+{
+  using namespace gtk;
+  TileSmem<TH>& S = tile_smem<TH>();
+  const int tid   = threadIdx.x;
+  int* status     = header + 1;
+  tile_setup(S);
+  for (int64_t c = blockIdx.x; c < n_chunks;) {  // the first chunk of every CTA, the others by ticket
+    int next = 0;
+    if (tid == 0) next = atomicAdd(header, 1);
+    const int64_t cs  = chunk_off[c];
+    const int64_t L64 = chunk_off[c + 1] - cs;
+    // The offsets come from the caller's device memory and are used as indices below: a chunk that is not
+    // inside bytes[0, n_bytes) is skipped (count 0) and reported through the status word, never touched.
+    const bool outside = cs < 0 || L64 < 0 || cs > n_bytes || L64 > n_bytes - cs;
+    int count = 0;
+    if (outside || L64 > max_chunk) {
+      if (tid == 0) atomicMax(status, outside ? int(kStatusBadOffsets) : int(kStatusScratchTooSmall));
+    } else if (L64 > 0) {
+      const bool done = tokenise_chunk(S, bytes, cs, cs + L64, T, nullptr, 0, status, [&](int64_t at, uint32_t t) {
+        if (GTK_IN(at, L64, 32)) out_ids[cs + at] = int32_t((low_id_map && t < 256u) ? uint32_t(__ldg(low_id_map + t)) : t);
+      });
+      count = done ? int(S.run) : kPutOff;
+      if (!done && tid == 0) atomicAdd(header + 2, 1);
+    }
+    if (tid == 0) {
+      out_counts[c] = count;
+      S.ticket      = next;
+    }
+    __syncthreads();
+    c = int64_t(gridDim.x) + S.ticket;
+  }
+}
+
+// the chunks that the first kernel has put off
 __global__ void __launch_bounds__(gtk::kBaseThreads)
-k_merge_chunks_noalloc(const uint8_t* __restrict__ bytes, int64_t n_bytes, const int64_t* __restrict__ chunk_off,
-                       int64_t n_chunks, int max_chunk, int32_t* __restrict__ out_ids,
-                       int32_t* __restrict__ out_counts, gtk::DeviceTable T,
+k_merge_chunks_noalloc(const uint8_t* __restrict__ bytes, const int64_t* __restrict__ chunk_off,
+                       int64_t n_chunks, int32_t* __restrict__ out_ids,
+                       int32_t* __restrict__ out_counts, const __grid_constant__ gtk::DeviceTable T,
                        const uint16_t* __restrict__ low_id_map, unsigned char* scratch)
 {
   using namespace gtk;
@@ -2043,30 +2086,18 @@ k_merge_chunks_noalloc(const uint8_t* __restrict__ bytes, int64_t n_bytes, const
   __shared__ GroupScratch gs;
   __shared__ int ticket;
   const int tid   = threadIdx.x;
-  int* counter    = reinterpret_cast<int*>(scratch);
-  int* status     = counter + 1;
+  int* header     = reinterpret_cast<int*>(scratch);
   uint16_t* w_tok = reinterpret_cast<uint16_t*>(scratch + kNoAllocHeader + size_t(blockIdx.x) * kNoAllocPerCta);
   uint16_t* w_rk  = w_tok + kNoAllocMaxTokens;
   for (;;) {
     __syncthreads();
-    if (tid == 0) ticket = atomicAdd(counter, 1);
+    if (tid == 0) ticket = atomicAdd(header + 3, 1);
     __syncthreads();
     const int64_t c = ticket;
     if (c >= n_chunks) break;
-    const int64_t cs  = chunk_off[c];
-    const int64_t L64 = chunk_off[c + 1] - cs;
-    // The offsets come from the caller's device memory and are used as indices below: a chunk that is not
-    // inside bytes[0, n_bytes) is skipped (count 0) and reported through the status word, never touched.
-    const bool outside = cs < 0 || L64 < 0 || cs > n_bytes || L64 > n_bytes - cs;
-    if (outside || L64 == 0 || L64 > max_chunk) {
-      if (tid == 0) {
-        out_counts[c] = 0;
-        if (outside) atomicMax(status, int(kStatusBadOffsets));
-        else if (L64 != 0) atomicMax(status, int(kStatusScratchTooSmall));
-      }
-      continue;
-    }
-    const int L   = int(L64);
+    if (out_counts[c] != kPutOff) continue;
+    const int64_t cs = chunk_off[c];  // checked by the first kernel, as the length is
+    const int L      = int(chunk_off[c + 1] - cs);
     uint16_t* tok = (L <= kBaseSmemTokens) ? s_tok : w_tok;
     uint16_t* rk  = (L <= kBaseSmemTokens) ? s_rk : w_rk;
     for (int i = tid; i < L; i += kBaseThreads) {
@@ -2075,11 +2106,12 @@ k_merge_chunks_noalloc(const uint8_t* __restrict__ bytes, int64_t n_bytes, const
       rk[i]  = (i + 1 < L) ? __ldg(T.byte_pair_rank + ((cur << 8) | bytes[cs + i + 1])) : uint16_t(NONE);
     }
     __syncthreads();
-    const int len = group_merge<kBaseThreads / 32, true>(tok, rk, L, T, &gs, status);
+    const int len = group_merge<kBaseThreads / 32, true>(tok, rk, L, T, &gs, header + 1);
     for (int j = tid; j < len; j += kBaseThreads) {
       const uint32_t t = tok[j];
       out_ids[cs + j]  = int32_t((low_id_map && t < 256u) ? uint32_t(__ldg(low_id_map + t)) : t);
     }
+    __syncthreads();  // the count is read at the top of the loop
     if (tid == 0) out_counts[c] = len;
   }
 }
@@ -2129,16 +2161,37 @@ extern "C" GTK_API int gtk_encode_chunks_noalloc(gtk_tokenizer* h, const uint8_t
   unsigned char* scratch = nullptr;
   if (e == cudaSuccess) e = noalloc_scratch_for(v.device, &scratch);
   if (e != cudaSuccess) return fail(GTK_ERR_CUDA, std::string("fixed workspace lookup: ") + cudaGetErrorString(e));
-  // the previous call's ticket and status words must start at zero
+  // the previous call's tickets and status words must start at zero
   e = cudaMemsetAsync(scratch, 0, kNoAllocHeader, v.stream);
   if (e != cudaSuccess) return fail(GTK_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
-  const int grid = int(n_chunks < kNoAllocCtas ? n_chunks : kNoAllocCtas);
-  k_merge_chunks_noalloc<<<grid, gtk::kBaseThreads, 0, v.stream>>>(d_bytes, n_bytes, d_chunk_offsets, n_chunks,
-                                                                   max_chunk_bytes, d_out_ids, d_out_counts, v.table,
-                                                                   v.low_id_map, scratch);
-  e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaMemcpyAsync(v.pinned_words, scratch, 8, cudaMemcpyDeviceToHost, v.stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(v.stream);
+  const int threads = gtk::chunk_kernel_threads(max_chunk_bytes, 0);
+  const int grid    = int(std::min<int64_t>(n_chunks, int64_t(v.sm_count) * (1536 / threads)));
+  int* header       = reinterpret_cast<int*>(scratch);
+  switch (threads) {
+    case 64:
+      k_chunks_noalloc<64><<<grid, 64, 0, v.stream>>>(d_bytes, n_bytes, d_chunk_offsets, n_chunks, max_chunk_bytes, d_out_ids,
+                                                      d_out_counts, v.table, v.low_id_map, header);
+      break;
+    case 128:
+      k_chunks_noalloc<128><<<grid, 128, 0, v.stream>>>(d_bytes, n_bytes, d_chunk_offsets, n_chunks, max_chunk_bytes, d_out_ids,
+                                                        d_out_counts, v.table, v.low_id_map, header);
+      break;
+    default:
+      k_chunks_noalloc<256><<<grid, 256, 0, v.stream>>>(d_bytes, n_bytes, d_chunk_offsets, n_chunks, max_chunk_bytes, d_out_ids,
+                                                        d_out_counts, v.table, v.low_id_map, header);
+      break;
+  }
+  auto read_back = [&]() {
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(v.pinned_words, scratch, 16, cudaMemcpyDeviceToHost, v.stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(v.stream);
+  };
+  read_back();
+  if (e == cudaSuccess && v.pinned_words[2] > 0) {
+    k_merge_chunks_noalloc<<<int(std::min<int64_t>(n_chunks, kNoAllocCtas)), gtk::kBaseThreads, 0, v.stream>>>(
+      d_bytes, d_chunk_offsets, n_chunks, d_out_ids, d_out_counts, v.table, v.low_id_map, scratch);
+    read_back();
+  }
   if (e != cudaSuccess) return fail(GTK_ERR_CUDA, std::string("allocation-free merge kernel: ") + cudaGetErrorString(e));
   const int status = v.pinned_words[1];
   if (status == gtk::kStatusBadOffsets)

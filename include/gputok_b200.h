@@ -233,9 +233,10 @@ GTK_API int gtk_write_token_strings(const gtk_tokenizer* h, const char* path, co
  * with a frozen memory budget, under a framework whose caching allocator owns all of HBM, or
  * anywhere a cudaMalloc -- which synchronises the whole device -- would stall other streams.
  * Once the handle exists this call performs no cudaMalloc/cudaFree and calls no allocating
- * library routine: one kernel (the one-CTA-per-chunk greedy merge kernel) runs with its work
- * queue, status word and long-chunk workspace in a fixed array that is part of the library
- * image (8 MiB + 256 B of device memory on every GPU that loads the library, held until the
+ * library routine: the one-CTA-per-chunk greedy kernel runs with its work queue and status words
+ * in a fixed array that is part of the library image; chunks that hold a segment of several
+ * hundred bytes follow in a second kernel whose workspace is that array
+ * (8 MiB + 256 B of device memory on every GPU that loads the library, held until the
  * process exits).
  *
  *   d_bytes[n_bytes]              text on the handle's device
