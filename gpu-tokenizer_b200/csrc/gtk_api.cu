@@ -1375,19 +1375,9 @@ GTK_API int gtk_decode(const gtk_tokenizer* h, const int32_t* ids, int64_t n_ids
                        int64_t* n_out)
 {
   if (!h || (n_ids > 0 && !ids)) return GTK_ERR_INVALID_ARG;
-  const gtk::HostTable& t = *h->table;
-  int64_t k = 0;
-  for (int64_t i = 0; i < n_ids; ++i) {
-    const int32_t id = ids[i];
-    if (id < 0 || size_t(id) >= t.id_to_bytes.size() || !t.decodable[size_t(id)])
-      return h->fail(GTK_ERR_INVALID_ARG, "id " + std::to_string(id) + " has no byte string");
-    const std::string& s = t.id_to_bytes[size_t(id)];
-    if (out) {
-      if (k + int64_t(s.size()) > out_capacity) return h->fail(GTK_ERR_CAPACITY, "decode buffer too small");
-      std::memcpy(out + k, s.data(), s.size());
-    }
-    k += int64_t(s.size());
-  }
+  const int64_t k = h->table->decode(ids, n_ids, out, out_capacity);
+  if (k == -1 - n_ids) return h->fail(GTK_ERR_CAPACITY, "decode buffer too small");
+  if (k < 0) return h->fail(GTK_ERR_INVALID_ARG, "id " + std::to_string(ids[-1 - k]) + " has no byte string");
   if (n_out) *n_out = k;
   return GTK_OK;
 }

@@ -110,6 +110,9 @@ class HostTable {
   std::unordered_map<std::string, int32_t> symbols_to_id;
   std::vector<std::string> id_to_bytes;                 // token id -> raw bytes ("" + !decodable if impossible)
   std::vector<uint8_t> decodable;
+  // the same for the decoder: length of an id's byte string (0 = none, 255 = look in id_to_bytes) and its first 16 bytes
+  std::vector<uint8_t> decode_length;
+  std::vector<uint8_t> decode_bytes;  // [16 * id]
   uint16_t byte_to_id[256];
   uint16_t gpt2_low_id[256];  // id < 256 (reference id space) -> id of the same byte token in GPT-2's own vocabulary
 
@@ -144,6 +147,10 @@ class HostTable {
   bool merged_is_256_plus_rank = false;
   bool byte_ids_identity = false;
   bool fits_u16 = false;        // ids < 0xFFFF and ranks < 0xFFFE
+
+  // ids -> bytes.  Returns the byte count, or -1 - i when ids[i] has no byte string, or -1 - n_ids when `out` (null: count
+  // only) holds fewer than that.
+  int64_t decode(const int32_t* ids, int64_t n_ids, uint8_t* out, int64_t capacity) const;
 
   // host lookup through the same hash layout the device uses
   bool find(int32_t left, int32_t right, uint32_t* rank, int32_t* merged) const;

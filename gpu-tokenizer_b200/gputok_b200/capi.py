@@ -86,6 +86,12 @@ def load_library() -> C.CDLL:
     return lib
 
 
+_new_bytes = C.pythonapi.PyBytes_FromStringAndSize
+_new_bytes.argtypes, _new_bytes.restype = [C.c_char_p, C.c_ssize_t], C.py_object
+_bytes_address = C.pythonapi.PyBytes_AsString
+_bytes_address.argtypes, _bytes_address.restype = [C.py_object], C.c_void_p
+
+
 def _as_u8(data) -> np.ndarray:
     if isinstance(data, (bytes, bytearray, memoryview)):
         return np.frombuffer(data, dtype=np.uint8)
@@ -269,9 +275,10 @@ class Tokenizer:
         a = np.ascontiguousarray(ids, dtype=np.int32)
         n = C.c_int64()
         self._check(self._lib.gtk_decode(self._h, a.ctypes.data, len(a), None, 0, C.byref(n)))
-        out = np.empty(max(n.value, 1), dtype=np.uint8)
-        self._check(self._lib.gtk_decode(self._h, a.ctypes.data, len(a), out.ctypes.data, n.value, C.byref(n)))
-        return out[:n.value].tobytes()
+        out = _new_bytes(None, n.value)  # written in place: nobody else has seen it yet
+        if n.value:
+            self._check(self._lib.gtk_decode(self._h, a.ctypes.data, len(a), _bytes_address(out), n.value, C.byref(n)))
+        return out
 
     def token_symbols(self, tid: int) -> bytes:
         buf = C.create_string_buffer(1024)
