@@ -18,7 +18,10 @@
 #include <pybind11/pybind11.h>
 #include <pybind11/stl.h>
 
+#include <cstdlib>
 #include <cstring>
+#include <mutex>
+#include <new>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -42,26 +45,91 @@ class GpuTokenizer {
     int rc = gtk_create(merges_path.c_str(), chunk_tokens, max_iters, device, &h_);
     if (rc != GTK_OK) raise_status(rc, gtk_global_error());
   }
-  ~GpuTokenizer() { gtk_destroy(h_); }
+  ~GpuTokenizer()
+  {
+    for (PyObject* o : id_objects_) Py_XDECREF(o);
+    release_bytes();
+    gtk_destroy(h_);
+  }
   GpuTokenizer(const GpuTokenizer&) = delete;
   GpuTokenizer& operator=(const GpuTokenizer&) = delete;
 
-  // Flatten list[str] into one byte buffer + offsets (UTF-8, as pybind's
-  // str -> std::string caster does for the reference).
-  static void flatten(const std::vector<std::string>& texts, std::vector<uint8_t>& bytes,
-                      std::vector<int64_t>& off)
-  {
-    size_t total = 0;
-    for (auto& t : texts) total += t.size();
-    bytes.resize(total);
-    off.assign(1, 0);
-    off.reserve(texts.size() + 1);
-    size_t k = 0;
-    for (auto& t : texts) {
-      if (!t.empty()) std::memcpy(bytes.data() + k, t.data(), t.size());
-      k += t.size();
-      off.push_back(int64_t(k));
+  // One call at a time from flattening to reading the result.  Waiting happens without the GIL, which the holder needs.
+  class Turn {
+   public:
+    explicit Turn(GpuTokenizer& t) : lock_(t.mu_, std::try_to_lock)
+    {
+      if (lock_.owns_lock()) return;
+      py::gil_scoped_release nogil;
+      lock_.lock();
     }
+
+   private:
+    std::unique_lock<std::mutex> lock_;
+  };
+
+  // list[str] -> one byte buffer (page-locked, kept between calls: the upload is one DMA) + offsets, UTF-8 as pybind's
+  // str -> std::string caster does for the reference, without a std::string per text.
+  void flatten(const py::object& texts)
+  {
+    PyObject* seq = texts.ptr();
+    if (PyList_Check(seq) || PyTuple_Check(seq)) {
+      const Py_ssize_t n = PySequence_Fast_GET_SIZE(seq);
+      PyObject** items   = PySequence_Fast_ITEMS(seq);
+      parts_.resize(size_t(n));
+      off_.resize(size_t(n) + 1);
+      int64_t total = 0;
+      bool plain    = true;
+      for (Py_ssize_t i = 0; i < n && plain; ++i) {
+        Py_ssize_t len = 0;
+        const char* p  = PyUnicode_Check(items[i]) ? PyUnicode_AsUTF8AndSize(items[i], &len) : nullptr;
+        plain          = p != nullptr;
+        off_[size_t(i)]   = total;
+        parts_[size_t(i)] = p;
+        total += len;
+      }
+      if (plain) {
+        off_[size_t(n)] = total;
+        reserve(size_t(total));
+        for (Py_ssize_t i = 0; i < n; ++i) {
+          const size_t len = size_t(off_[size_t(i) + 1] - off_[size_t(i)]);
+          if (len) std::memcpy(bytes_ + off_[size_t(i)], parts_[size_t(i)], len);
+        }
+        return;
+      }
+      PyErr_Clear();  // something else than str, or a str without a UTF-8 form: the caster below decides
+    }
+    std::vector<std::string> strings;
+    try {
+      strings = texts.cast<std::vector<std::string>>();
+    } catch (const py::cast_error&) {
+      throw py::type_error("texts must be a sequence of str or bytes");
+    }
+    off_.assign(1, 0);
+    for (auto& t : strings) off_.push_back(off_.back() + int64_t(t.size()));
+    reserve(size_t(off_.back()));
+    for (size_t i = 0; i < strings.size(); ++i)
+      if (!strings[i].empty()) std::memcpy(bytes_ + off_[i], strings[i].data(), strings[i].size());
+  }
+  size_t n_texts() const { return off_.size() - 1; }
+
+  void reserve(size_t bytes)
+  {
+    if (bytes <= cap_) return;
+    release_bytes();
+    const size_t want = bytes + bytes / 4 + 4096;
+    bytes_  = static_cast<uint8_t*>(gtk_pinned_alloc(want));
+    pinned_ = bytes_ != nullptr;
+    if (!pinned_) bytes_ = static_cast<uint8_t*>(std::malloc(want));  // a host-only handle, no device to lock pages for
+    if (!bytes_) throw std::bad_alloc();
+    cap_ = want;
+  }
+  void release_bytes()
+  {
+    if (pinned_) gtk_pinned_free(bytes_);
+    else std::free(bytes_);
+    bytes_ = nullptr;
+    cap_   = 0;
   }
 
   void check(int rc) const
@@ -71,86 +139,105 @@ class GpuTokenizer {
 
   // (list[list[int]], kernel_ms); ([], 0.0) for an empty batch or a batch of
   // empty texts, as gputok_binding.cpp:707-709, 734-736.
-  py::tuple lists_from_result(size_t n_texts, float kernel_ms) const
+  py::tuple lists_from_result(size_t n_texts, float kernel_ms)
   {
     int64_t n_ids = 0, n_chunks = 0;
     gtk_result_sizes(h_, &n_ids, &n_chunks, nullptr);
     py::list batch;
     if (n_texts == 0 || n_chunks == 0) return py::make_tuple(batch, 0.0);
+    return py::make_tuple(id_lists(n_texts), double(kernel_ms));
+  }
+
+  // The last result as list[list[int]].  The int objects of the vocabulary are made once and shared (they are immutable, as
+  // Python's own small ints are): a reference count instead of an allocation per id.
+  py::list id_lists(size_t n_texts)
+  {
     const int32_t* ids;
     const int64_t* toff;
     gtk_result_view(h_, &ids, &toff, nullptr);
+    PyObject* batch = PyList_New(Py_ssize_t(n_texts));
+    if (!batch) throw py::error_already_set();
+    py::list owner = py::reinterpret_steal<py::list>(batch);
     for (size_t t = 0; t < n_texts; ++t) {
-      py::list one;
-      for (int64_t i = toff[t]; i < toff[t + 1]; ++i) one.append(py::int_(ids[i]));
-      batch.append(std::move(one));
+      const int64_t lo = toff[t], n = toff[t + 1] - lo;
+      PyObject* one    = PyList_New(Py_ssize_t(n));
+      if (!one) throw py::error_already_set();
+      PyList_SET_ITEM(batch, Py_ssize_t(t), one);
+      for (int64_t i = 0; i < n; ++i) {
+        const size_t id = size_t(uint32_t(ids[lo + i]));
+        if (id >= id_objects_.size()) id_objects_.resize(id + id / 2 + 1024, nullptr);
+        PyObject*& o = id_objects_[id];
+        if (!o && !(o = PyLong_FromLong(long(id)))) throw py::error_already_set();
+        Py_INCREF(o);
+        PyList_SET_ITEM(one, Py_ssize_t(i), o);
+      }
     }
-    return py::make_tuple(batch, double(kernel_ms));
+    return owner;
   }
 
-  py::tuple tokenize(const std::vector<std::string>& texts, int mode)
+  py::tuple tokenize(const py::object& texts, int mode)
   {
-    std::vector<uint8_t> bytes;
-    std::vector<int64_t> off;
-    flatten(texts, bytes, off);
+    Turn turn(*this);
+    flatten(texts);
     float ms = 0.f;
     int rc;
     {
       py::gil_scoped_release nogil;
-      rc = gtk_encode(h_, mode, bytes.data(), off.data(), int64_t(texts.size()), &ms);
+      rc = gtk_encode(h_, mode, bytes_, off_.data(), int64_t(n_texts()), &ms);
     }
     check(rc);
-    return lists_from_result(texts.size(), ms);
+    return lists_from_result(n_texts(), ms);
   }
 
-  py::list tokenize_cpu(const std::vector<std::string>& texts, const std::string& rule)
+  py::list tokenize_cpu(const py::object& texts, const std::string& rule)
   {
     int r;
     if (rule == "greedy") r = GTK_RULE_GREEDY;
     else if (rule == "localmin") r = GTK_RULE_LOCALMIN;
     else throw std::invalid_argument("merge_rule must be 'greedy' or 'localmin'");
-    std::vector<uint8_t> bytes;
-    std::vector<int64_t> off;
-    flatten(texts, bytes, off);
+    Turn turn(*this);
+    flatten(texts);
     int rc;
     {
       py::gil_scoped_release nogil;
-      rc = gtk_encode_cpu(h_, r, bytes.data(), off.data(), int64_t(texts.size()));
+      rc = gtk_encode_cpu(h_, r, bytes_, off_.data(), int64_t(n_texts()));
     }
     check(rc);
-    const int32_t* ids;
-    const int64_t* toff;
-    gtk_result_view(h_, &ids, &toff, nullptr);
-    py::list batch;
-    for (size_t t = 0; t < texts.size(); ++t) {
-      py::list one;
-      for (int64_t i = toff[t]; i < toff[t + 1]; ++i) one.append(py::int_(ids[i]));
-      batch.append(std::move(one));
-    }
-    return batch;
+    return id_lists(n_texts());
   }
 
-  py::tuple encode_packed(const std::vector<std::string>& texts, const std::string& mode)
+  py::tuple encode_packed(const py::object& texts, const std::string& mode)
   {
     int m;
     if (mode == "opt") m = GTK_MODE_OPT;
     else if (mode == "base") m = GTK_MODE_BASE;
     else throw std::invalid_argument("mode must be 'opt' or 'base'");
-    std::vector<uint8_t> bytes;
-    std::vector<int64_t> off;
-    flatten(texts, bytes, off);
+    Turn turn(*this);
+    flatten(texts);
     float ms = 0.f;
     int rc;
     {
       py::gil_scoped_release nogil;
-      rc = gtk_encode(h_, m, bytes.data(), off.data(), int64_t(texts.size()), &ms);
+      rc = gtk_encode(h_, m, bytes_, off_.data(), int64_t(n_texts()), &ms);
     }
     check(rc);
     int64_t n_ids = 0, n_chunks = 0;
     gtk_result_sizes(h_, &n_ids, &n_chunks, nullptr);
+    const int64_t n_text_off = int64_t(n_texts()) + 1, n_chunk_off = n_chunks + 1;
+    // large results are taken over, not copied: the arrays look at the page-locked memory that the ids were downloaded to
+    constexpr int64_t kTakeBytes = 128 << 10;
+    gtk_taken* taken = 4 * n_ids + 8 * (n_text_off + n_chunk_off) >= kTakeBytes ? gtk_result_take(h_) : nullptr;
+    if (taken) {
+      py::capsule owner(taken, [](void* p) { gtk_result_release(static_cast<gtk_taken*>(p)); });
+      const int32_t* ids;
+      const int64_t *toff, *coff;
+      gtk_result_view(h_, &ids, &toff, &coff);
+      return py::make_tuple(py::array_t<int32_t>(n_ids, ids, owner), py::array_t<int64_t>(n_text_off, toff, owner),
+                            py::array_t<int64_t>(n_chunk_off, coff, owner), double(ms));
+    }
     py::array_t<int32_t> ids(n_ids);
-    py::array_t<int64_t> toff(int64_t(texts.size()) + 1), coff(n_chunks + 1);
-    check(gtk_result_copy(h_, ids.mutable_data(), n_ids, toff.mutable_data(), coff.mutable_data(), n_chunks + 1));
+    py::array_t<int64_t> toff(n_text_off), coff(n_chunk_off);
+    check(gtk_result_copy(h_, ids.mutable_data(), n_ids, toff.mutable_data(), coff.mutable_data(), n_chunk_off));
     return py::make_tuple(ids, toff, coff, double(ms));
   }
 
@@ -206,6 +293,13 @@ class GpuTokenizer {
 
  private:
   gtk_tokenizer* h_ = nullptr;
+  std::mutex mu_;  // see Turn; guards what follows
+  uint8_t* bytes_ = nullptr;
+  size_t cap_     = 0;
+  bool pinned_    = false;
+  std::vector<int64_t> off_;
+  std::vector<const char*> parts_;
+  std::vector<PyObject*> id_objects_;
 };
 
 }  // namespace
@@ -218,7 +312,7 @@ PYBIND11_MODULE(gputok_gpu, m)
   py::class_<GpuTokenizer>(m, "GpuTokenizer")
     .def(py::init<const std::string&, int, int, int>(), py::arg("merges_path"), py::arg("chunk_tokens") = 2048,
          py::arg("max_iters") = 50, py::arg("device") = 0)
-    .def("tokenize_batch", [](GpuTokenizer& self, const std::vector<std::string>& texts, const std::string& rule) {
+    .def("tokenize_batch", [](GpuTokenizer& self, const py::object& texts, const std::string& rule) {
            if (rule == "greedy") return self.tokenize(texts, GTK_MODE_OPT);
            if (rule == "localmin") return self.tokenize(texts, GTK_MODE_LOCALMIN);
            throw std::invalid_argument("merge_rule must be 'greedy' or 'localmin'");
@@ -226,7 +320,7 @@ PYBIND11_MODULE(gputok_gpu, m)
          "Tokenize a batch of UTF-8 strings with the segment-parallel kernel (greedy rule).\n"
          "merge_rule='localmin' runs the reference method's own rule (local minimum, max_iters passes,\n"
          "per chunk) on the GPU instead.  Returns (list[list[int]], kernel_time_ms).")
-    .def("tokenize_batch_blockbpe_base", [](GpuTokenizer& self, const std::vector<std::string>& texts) {
+    .def("tokenize_batch_blockbpe_base", [](GpuTokenizer& self, const py::object& texts) {
            return self.tokenize(texts, GTK_MODE_BASE);
          }, py::arg("texts"),
          "Tokenize with the one-CTA-per-chunk Algorithm 1 kernel.\n"

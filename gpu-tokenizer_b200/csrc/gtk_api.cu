@@ -99,7 +99,62 @@ struct PinBuf {
   T* as() const { return static_cast<T*>(p); }
 };
 
+// Page-locked result buffers that callers have taken over (gtk_result_take) come back here when they are done with them.
+// Shared by the handle and by the results that are still out, so either may go first.  Bounded: at most kMaxTaken
+// results are out (further takes are refused and the caller copies), at most kMaxSpare buffers wait to be used again.
+struct ResultPool {
+  static constexpr int kMaxTaken = 4, kMaxSpare = 6;
+  static constexpr size_t kMaxTakenBytes = size_t(1) << 30, kMaxSpareBytes = size_t(512) << 20;
+  std::mutex mu;
+  std::vector<PinBuf> spare;
+  int taken = 0;
+  size_t taken_bytes = 0, spare_bytes = 0;
+  bool closed = false;  // the handle is gone
+
+  ~ResultPool()
+  {
+    for (PinBuf& b : spare) b.release();
+  }
+  // a buffer of at least `bytes`: the one in hand, else the smallest spare one that does, else a new one
+  void reserve(PinBuf& buf, size_t bytes)
+  {
+    if (buf.p && bytes <= buf.cap) return;
+    {
+      std::lock_guard<std::mutex> lock(mu);
+      size_t best = spare.size();
+      for (size_t i = 0; i < spare.size(); ++i)
+        if (spare[i].cap >= bytes && (best == spare.size() || spare[i].cap < spare[best].cap)) best = i;
+      if (best < spare.size()) {
+        std::swap(buf, spare[best]);
+        spare_bytes += spare[best].cap - buf.cap;
+        if (!spare[best].p) spare.erase(spare.begin() + long(best));
+        return;
+      }
+    }
+    buf.reserve(bytes);
+  }
+  void give_back(PinBuf& buf)
+  {
+    if (!buf.p) return;
+    std::lock_guard<std::mutex> lock(mu);
+    if (closed || int(spare.size()) >= kMaxSpare || spare_bytes + buf.cap > kMaxSpareBytes) {
+      buf.release();
+      return;
+    }
+    spare_bytes += buf.cap;
+    spare.push_back(buf);
+    buf = PinBuf();
+  }
+};
+
 }  // namespace
+
+// A result that its caller has taken over.
+struct gtk_taken {
+  std::shared_ptr<ResultPool> pool;
+  PinBuf bufs[3];
+  size_t bytes = 0;
+};
 
 // Buffers of one in-flight slice of a large host batch (kSliceArenas sets rotate).
 constexpr int kSliceArenas = 4;
@@ -169,11 +224,15 @@ struct gtk_tokenizer {
   DevBuf d_out_pack;
   PinBuf h_out_pack;
   bool result_is_packed = false;
+  std::shared_ptr<ResultPool> pool = std::make_shared<ResultPool>();
+  bool result_is_taken = false;
+  const int32_t* view_ids = nullptr;
+  const int64_t *view_text = nullptr, *view_chunk = nullptr;
+  PinBuf* result_bufs[3] = {nullptr, nullptr, nullptr};  // what the last result lives in, as far as it can be taken over
   size_t pack_text_bytes = 0, pack_chunk_bytes = 0;
   const uint8_t* pack_base = nullptr;  // h_out_pack, or the mapped block below behind its 64-byte header
   // batches of up to 256 KiB: a kernel writes the results into this mapped block and the host polls its header
-  uint8_t* mid_out_h = nullptr;
-  uint8_t* mid_out_d = nullptr;
+  PinBuf h_mid;
   int64_t mid_seq = 0;
   // one text of up to 64 KiB: chunk table, zeroed counters and the text travel in one copy (encode_host_one_text)
   PinBuf h_fast_in;
@@ -645,9 +704,9 @@ int encode_host_sliced(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
   h->h_piece_off.reserve(size_t(piece_at[nsz]) * 8);
   h->h_piece_id_off.reserve(size_t(piece_at[nsz]) * 8);
   h->h_chunk_id_all.reserve(size_t(chunk_at[nsz]) * 8);
-  h->h_text_id_off.reserve(size_t(n_texts + 1) * 8);
-  h->h_chunk_id_off.reserve(size_t(chunk_upper_bound(n_bytes, total_pieces, h->chunk_tokens) + 2) * 8);
-  h->h_ids.reserve(size_t(n_bytes) * 2);  // grown below if the batch yields more than one id per two bytes
+  h->pool->reserve(h->h_text_id_off, size_t(n_texts + 1) * 8);
+  h->pool->reserve(h->h_chunk_id_off, size_t(chunk_upper_bound(n_bytes, total_pieces, h->chunk_tokens) + 2) * 8);
+  h->pool->reserve(h->h_ids, size_t(n_bytes) * 2);  // grown below if the batch yields more than one id per two bytes
   if (!h->in_stream) GTK_CUDA(cudaStreamCreateWithFlags(&h->in_stream, cudaStreamNonBlocking));
   if (!h->out_stream) GTK_CUDA(cudaStreamCreateWithFlags(&h->out_stream, cudaStreamNonBlocking));
   if (!h->pack_stream) GTK_CUDA(cudaStreamCreateWithFlags(&h->pack_stream, cudaStreamNonBlocking));
@@ -760,6 +819,9 @@ int encode_host_sliced(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
   h->last_launches = launches;
   h->res_n_ids = R;
   h->res_n_chunks = Cbase;
+  h->result_bufs[0] = &h->h_ids;
+  h->result_bufs[1] = &h->h_text_id_off;
+  h->result_bufs[2] = &h->h_chunk_id_off;
   if (kernel_ms) *kernel_ms = h->stage_ms[4];
   return GTK_OK;
 }
@@ -794,12 +856,14 @@ void small_path_init(gtk_tokenizer* h)
   h->small_out_h = static_cast<uint8_t*>(oh);
   h->small_in_d = static_cast<uint8_t*>(id);
   h->small_out_d = static_cast<uint8_t*>(od);
-  void *mh = nullptr, *md = nullptr;
-  GTK_CUDA(cudaHostAlloc(&mh, kMappedResultBytes, cudaHostAllocMapped));
-  GTK_CUDA(cudaHostGetDevicePointer(&md, mh, 0));
-  std::memset(mh, 0, 64);
-  h->mid_out_h = static_cast<uint8_t*>(mh);
-  h->mid_out_d = static_cast<uint8_t*>(md);
+}
+
+// The mapped result block, its completion mark behind any call number that is still to come.
+uint8_t* mid_block(gtk_tokenizer* h)
+{
+  h->pool->reserve(h->h_mid, kMappedResultBytes);
+  std::memset(h->h_mid.p, 0, 64);
+  return h->h_mid.as<uint8_t>();
 }
 
 // Waits for a kernel's completion mark (the call number, its last store behind a system-wide fence) in a mapped
@@ -867,7 +931,7 @@ constexpr int64_t kTwoLaunchMaxChunks = 4096;
 // number of chunks of the batch, or -1 when it does not qualify for the two-launch path
 int64_t two_launch_chunks(const gtk_tokenizer* h, int mode, const int64_t* text_offsets, int64_t n_texts, int64_t n_bytes)
 {
-  if (h->wide || mode != GTK_MODE_OPT || !h->mid_out_h || h->stage_timing) return -1;
+  if (h->wide || mode != GTK_MODE_OPT || h->stage_timing) return -1;
   if (n_bytes > kTwoLaunchMaxBytes || n_texts > gtk::kSmallMaxTexts) return -1;
   const int64_t chunk = h->chunk_tokens;
   int64_t C = 0;
@@ -910,7 +974,7 @@ int encode_host_two_launches(gtk_tokenizer* h, const uint8_t* bytes, const int64
   GTK_CUDA(cudaMemcpyAsync(dp, hp, total, cudaMemcpyHostToDevice, s));
 
   const size_t text_b = up(size_t(n_texts + 1) * 8), chunk_b = up(size_t(C + 1) * 8);
-  uint8_t* md = h->mid_out_d;  // [64-byte header | text id offsets | chunk id offsets | ids]
+  uint8_t* md = mid_block(h);  // (page-locked memory has the same address on the device) [64-byte header | text id offsets | chunk id offsets | ids]
   Plan p = plan_batch(h, dp + o_bytes, n_bytes, nullptr, n_texts, reinterpret_cast<int32_t*>(md + 64 + text_b + chunk_b),
                       n_bytes, reinterpret_cast<int64_t*>(md + 64 + text_b), false);
   p.b.text_id_off     = reinterpret_cast<int64_t*>(md + 64);
@@ -928,7 +992,7 @@ int encode_host_two_launches(gtk_tokenizer* h, const uint8_t* bytes, const int64
   launches += gtk::launch_finish_small_batch(p.b, reinterpret_cast<int64_t*>(md), seq, s);
   GTK_CUDA(cudaEventRecord(h->ev[4], s));
   GTK_CUDA(cudaGetLastError());
-  volatile const int64_t* tot = reinterpret_cast<volatile const int64_t*>(h->mid_out_h);
+  volatile const int64_t* tot = h->h_mid.as<volatile const int64_t>();
   if (!wait_for_mark(tot + 3, seq, s, "finish kernel"))
     return h->fail(GTK_ERR_KERNEL, "finish kernel ended without publishing its results");
   if (tot[2] != gtk::kStatusOk) return h->fail(GTK_ERR_KERNEL, status_text(int(tot[2])));
@@ -936,7 +1000,8 @@ int encode_host_two_launches(gtk_tokenizer* h, const uint8_t* bytes, const int64
   GTK_CUDA(cudaEventSynchronize(h->ev[4]));  // completes a moment after the mark
   GTK_CUDA(cudaEventElapsedTime(&h->stage_ms[4], h->ev[0], h->ev[4]));
   h->result_is_packed = true;
-  h->pack_base        = h->mid_out_h + 64;
+  h->pack_base        = h->h_mid.as<uint8_t>() + 64;
+  h->result_bufs[0]   = &h->h_mid;
   h->pack_text_bytes  = text_b;
   h->pack_chunk_bytes = chunk_b;
   h->last_launches    = launches;
@@ -957,11 +1022,16 @@ void release_handle(gtk_tokenizer* h)
                       &h->d_unit_cnt, &h->d_chunk_cnt, &h->d_unit_base, &h->d_chunk_id_off, &h->d_text_id_off,
                       &h->d_out_ids, &h->d_seg_scratch, &h->d_scan_sums, &h->d_totals, &h->d_out_pack, &h->d_fast_in})
       b->release();
-    for (PinBuf* b : {&h->h_ids, &h->h_text_id_off, &h->h_chunk_id_off, &h->h_totals, &h->h_piece_off, &h->h_piece_id_off, &h->h_chunk_id_all, &h->h_out_pack, &h->h_fast_in}) b->release();
+    for (PinBuf* b : {&h->h_ids, &h->h_text_id_off, &h->h_chunk_id_off, &h->h_totals, &h->h_piece_off, &h->h_piece_id_off, &h->h_chunk_id_all, &h->h_out_pack, &h->h_mid, &h->h_fast_in}) b->release();
     for (DevBuf* b : {&h->d_piece_off, &h->d_piece_id_off, &h->d_chunk_id_all}) b->release();
     if (h->small_in_h) cudaFreeHost(h->small_in_h);
     if (h->small_out_h) cudaFreeHost(h->small_out_h);
-    if (h->mid_out_h) cudaFreeHost(h->mid_out_h);
+    {
+      std::lock_guard<std::mutex> lock(h->pool->mu);
+      h->pool->closed = true;
+      for (PinBuf& b : h->pool->spare) b.release();
+      h->pool->spare.clear();
+    }
     for (auto& sl : h->slice) sl.release();
     if (h->in_stream) cudaStreamDestroy(h->in_stream);
     if (h->out_stream) cudaStreamDestroy(h->out_stream);
@@ -1188,6 +1258,8 @@ GTK_API int gtk_encode(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
   h->result_is_cpu = false;
   h->result_is_small = false;
   h->result_is_packed = false;
+  h->result_is_taken = false;
+  h->result_bufs[0] = h->result_bufs[1] = h->result_bufs[2] = nullptr;
   h->res_n_ids = h->res_n_chunks = 0;
   h->res_n_texts = n_texts;
   h->last_launches = 0;
@@ -1196,10 +1268,10 @@ GTK_API int gtk_encode(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
   try {
     GTK_CUDA(cudaSetDevice(h->device));
     const int64_t n_bytes = n_texts ? text_offsets[n_texts] : 0;
-    h->h_text_id_off.reserve(size_t(n_texts + 1) * 8);
     if (n_bytes == 0) {  // empty batch or only empty texts: ([], 0.0) in the reference
+      h->pool->reserve(h->h_text_id_off, size_t(n_texts + 1) * 8);
       std::memset(h->h_text_id_off.p, 0, size_t(n_texts + 1) * 8);
-      h->h_chunk_id_off.reserve(8);
+      h->pool->reserve(h->h_chunk_id_off, 8);
       h->h_chunk_id_off.as<int64_t>()[0] = 0;
       return GTK_OK;
     }
@@ -1230,7 +1302,7 @@ GTK_API int gtk_encode(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
     int launches = 0;
     // Up to 256 KiB of text a kernel behind the pack writes the results into mapped host memory and the host polls
     // its completion mark: no copy of the totals, no second copy sized by them, no stream synchronisation.
-    const bool by_kernel = h->mid_out_h != nullptr && n_bytes <= kResultsByKernelMaxBytes &&
+    const bool by_kernel = n_bytes <= kResultsByKernelMaxBytes &&
                            64 + text_b + chunk_b + size_t(n_bytes) * 4 + 64 <= kMappedResultBytes;
     run_front(h, p.b, mode, &launches, nullptr, nullptr, nullptr, true);
     run_pack(h, p.b, mode, &launches, nullptr, nullptr, true, !by_kernel);
@@ -1238,14 +1310,15 @@ GTK_API int gtk_encode(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
     int status = gtk::kStatusOk;
     if (by_kernel) {
       const int64_t seq = ++h->mid_seq;
-      launches += gtk::launch_results_to_host(p.b, dp, h->mid_out_d + 64, int64_t(text_b + chunk_b),
-                                              reinterpret_cast<int64_t*>(h->mid_out_d), seq, s);
+      uint8_t* md = mid_block(h);
+      launches += gtk::launch_results_to_host(p.b, dp, md + 64, int64_t(text_b + chunk_b), reinterpret_cast<int64_t*>(md), seq, s);
       GTK_CUDA(cudaGetLastError());
-      volatile const int64_t* tot = reinterpret_cast<volatile const int64_t*>(h->mid_out_h);
+      volatile const int64_t* tot = h->h_mid.as<volatile const int64_t>();
       if (!wait_for_mark(tot + 3, seq, s, "result kernel"))
         return h->fail(GTK_ERR_KERNEL, "result kernel ended without publishing its results");
       C = tot[0], N = tot[1], status = int(tot[2]);
-      h->pack_base = h->mid_out_h + 64;
+      h->pack_base = h->h_mid.as<uint8_t>() + 64;
+      h->result_bufs[0] = &h->h_mid;
     } else {
       GTK_CUDA(cudaStreamSynchronize(s));
       const int64_t* ht = h->h_totals.as<int64_t>();
@@ -1255,10 +1328,11 @@ GTK_API int gtk_encode(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
     if (status != gtk::kStatusOk) return h->fail(GTK_ERR_KERNEL, status_text(status));
     if (N > n_bytes) return h->fail(GTK_ERR_KERNEL, "more ids than input bytes");
     if (!by_kernel) {
-      h->h_out_pack.reserve(text_b + chunk_b + size_t(N) * 4 + 64);
+      h->pool->reserve(h->h_out_pack, text_b + chunk_b + size_t(N) * 4 + 64);
       GTK_CUDA(cudaMemcpyAsync(h->h_out_pack.p, dp, text_b + chunk_b + size_t(N) * 4, cudaMemcpyDeviceToHost, s));
       GTK_CUDA(cudaStreamSynchronize(s));
       h->pack_base = h->h_out_pack.as<uint8_t>();
+      h->result_bufs[0] = &h->h_out_pack;
     }
     collect_stage_times(h, true);
     h->result_is_packed = true;
@@ -1304,6 +1378,8 @@ GTK_API int gtk_encode_cpu(gtk_tokenizer* h, int rule, const uint8_t* bytes, con
   h->result_is_cpu = true;
   h->result_is_small = false;
   h->result_is_packed = false;
+  h->result_is_taken = false;
+  h->result_bufs[0] = h->result_bufs[1] = h->result_bufs[2] = nullptr;
   h->res_n_ids = int64_t(h->cpu_ids.size());
   h->res_n_chunks = int64_t(h->cpu_chunk_off.size()) - 1;
   h->res_n_texts = n_texts;
@@ -1323,7 +1399,11 @@ GTK_API int gtk_result_view(const gtk_tokenizer* h, const int32_t** ids, const i
                             const int64_t** chunk_id_offsets)
 {
   if (!h) return GTK_ERR_INVALID_ARG;
-  if (h->result_is_cpu) {
+  if (h->result_is_taken) {
+    if (ids) *ids = h->view_ids;
+    if (text_id_offsets) *text_id_offsets = h->view_text;
+    if (chunk_id_offsets) *chunk_id_offsets = h->view_chunk;
+  } else if (h->result_is_cpu) {
     if (ids) *ids = h->cpu_ids.data();
     if (text_id_offsets) *text_id_offsets = h->cpu_text_off.data();
     if (chunk_id_offsets) *chunk_id_offsets = h->cpu_chunk_off.data();
@@ -1361,6 +1441,49 @@ GTK_API int gtk_result_copy(const gtk_tokenizer* h, int32_t* ids, int64_t ids_ca
     if (src_chunk) std::memcpy(chunk_id_offsets, src_chunk, size_t(h->res_n_chunks + 1) * 8);
   }
   return GTK_OK;
+}
+
+GTK_API gtk_taken* gtk_result_take(gtk_tokenizer* h)
+{
+  if (!h) return nullptr;
+  std::lock_guard<std::mutex> lock(h->mu);
+  if (!h->result_bufs[0]) return nullptr;
+  size_t bytes = 0;
+  for (PinBuf* b : h->result_bufs)
+    if (b) bytes += b->cap;
+  {
+    std::lock_guard<std::mutex> plock(h->pool->mu);
+    if (h->pool->taken >= ResultPool::kMaxTaken || h->pool->taken_bytes + bytes > ResultPool::kMaxTakenBytes) return nullptr;
+    ++h->pool->taken;
+    h->pool->taken_bytes += bytes;
+  }
+  gtk_taken* t = new (std::nothrow) gtk_taken();
+  if (!t) return nullptr;
+  t->pool  = h->pool;
+  t->bytes = bytes;
+  // the pointers of gtk_result_view stay what they are
+  const int32_t* ids;
+  const int64_t *text_off, *chunk_off;
+  gtk_result_view(h, &ids, &text_off, &chunk_off);
+  h->view_ids = ids, h->view_text = text_off, h->view_chunk = chunk_off;
+  for (int i = 0; i < 3; ++i) {
+    if (h->result_bufs[i]) std::swap(t->bufs[i], *h->result_bufs[i]);
+    h->result_bufs[i] = nullptr;
+  }
+  h->result_is_taken = true;
+  return t;
+}
+
+GTK_API void gtk_result_release(gtk_taken* t)
+{
+  if (!t) return;
+  {
+    std::lock_guard<std::mutex> lock(t->pool->mu);
+    --t->pool->taken;
+    t->pool->taken_bytes -= t->bytes;
+  }
+  for (PinBuf& b : t->bufs) t->pool->give_back(b);
+  delete t;
 }
 
 GTK_API int gtk_last_stage_ms(const gtk_tokenizer* h, float stage_ms[5], int32_t* kernel_launches)

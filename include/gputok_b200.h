@@ -169,6 +169,15 @@ GTK_API int gtk_encode_device(gtk_tokenizer* h, int mode, const uint8_t* d_bytes
                               int64_t out_capacity, int64_t* d_out_chunk_offsets, int64_t chunk_capacity,
                               int64_t* n_ids, int64_t* n_chunks, float* kernel_ms);
 
+/* Takes the buffers of the last result out of the handle instead of copying them (no counterpart in the reference): the
+ * pointers of gtk_result_view then stay valid until gtk_result_release, whatever the handle does meanwhile, also when it is
+ * destroyed first; the release hands the page-locked memory back for later results.  NULL when there is nothing to take
+ * -- small results and those of gtk_encode_cpu live in memory of the handle's own -- or when four results or 1 GiB are
+ * out already: the caller copies then.  May be called from any thread. */
+typedef struct gtk_taken gtk_taken;
+GTK_API gtk_taken* gtk_result_take(gtk_tokenizer* h);
+GTK_API void gtk_result_release(gtk_taken* result);
+
 /* Device time of the stages of the last GPU encode, in milliseconds:
  * [0] chunker, [1] merge kernel, [2] output scans, [3] pack, [4] whole pipeline.
  * Also the number of kernels launched by that call (for launch accounting).

@@ -258,6 +258,35 @@ def test_segment_lengths_at_the_edges(lib, merges_path, oracle, n_bytes, mode):
         check_chunks(ids, coff, want, woff, f"segment lengths, {n_bytes} bytes, {mode}")
 
 
+@pytest.mark.parametrize("n_bytes", [300_000, 1 << 20, 9 << 20])
+def test_results_outlive_later_calls_and_their_tokenizer(lib, merges_path, oracle, n_bytes):
+    """Arrays of large results look at memory taken over from the tokenizer: more of them than may be out at a time (the
+    others are copies), all still right after later calls, after some have been dropped and after the tokenizer is gone."""
+    import gputok_gpu
+
+    t, kept = make_tok(lib, merges_path, 2048), []
+    for seed in range(7):
+        data = lib.TextGen(40 + seed).text(n_bytes - seed)
+        kept.append((data, *t.encode(data)[:3]))
+        if seed == 4:
+            del kept[1]
+    t.close()
+    for data, ids, toff, coff in kept:
+        want, woff = oracle.encode_fixed(data, 2048, mode=MODE_SEGMENTED, threads=NCPU)
+        check_chunks(ids, coff, want, woff, "kept result")
+        assert toff.tolist() == [0, len(want)]
+    drop_in = gputok_gpu.GpuTokenizer(merges_path, 2048)
+    strings = [[lib.TextGen(seed).text(n_bytes // 3 + k).tobytes().decode() for k in range(3)] for seed in range(3)]
+    results = [drop_in.encode_packed(s) for s in strings]
+    lists = drop_in.tokenize_batch(strings[0])[0]
+    del drop_in
+    assert [len(x) for x in lists] == np.diff(results[0][1]).tolist() and lists[1] == results[0][0][results[0][1][1]:results[0][1][2]].tolist()
+    for texts, (ids, toff, coff, _) in zip(strings, results):
+        for k, text in enumerate(texts):
+            want, _ = oracle.encode_fixed(np.frombuffer(text.encode(), np.uint8), 2048, mode=MODE_SEGMENTED, threads=NCPU)
+            assert np.array_equal(ids[toff[k]:toff[k + 1]], want)
+
+
 def test_crowded_pair_bucket(lib, merges_path, tmp_path):
     """More than four pairs in one bucket of the device pair table: the fifth and later ones are found in
     the side table (second load), in every kernel that probes."""
