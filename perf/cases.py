@@ -28,7 +28,7 @@ import sys
 import numpy as np
 import torch
 
-ROOT = os.path.abspath(os.curdir)  # run from the root of the tree whose code is to be timed
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 GOLDEN = os.path.join(ROOT, "tests", "golden")
 MERGES = os.path.join(GOLDEN, "gpt2_merges.txt")
 for _p in (ROOT, os.path.join(ROOT, "gpu-tokenizer_b200")):
