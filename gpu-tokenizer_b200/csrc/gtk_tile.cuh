@@ -270,7 +270,9 @@ __device__ __forceinline__ void window_words(const TileSmem<TH>& S, int at, uint
 
 // A slot of the long table.  During a batch that learns, other threads fill empty slots word by word (see learn_segment):
 // every word goes from zero to its final value once, and a filled slot has no zero in its last four words, so a slot that
-// is seen half filled is recognised whatever order its words arrive in, and counts as empty.
+// is seen half filled is recognised whatever order its words arrive in, and counts as empty.  A key word that has not
+// arrived could only pass for the one that is looked for if that is zero too, four NUL bytes or what a string ends with:
+// such strings are not looked up while the table is being added to (blank_word).
 struct LongSlot {
   uint4 k, v;  // v = {meta, ids[3]}
 };
@@ -301,6 +303,12 @@ __device__ __forceinline__ bool long_matches(const LongSlot& s, const uint32_t k
   return diff == 0u && s.v.x != 0u && s.v.y != 0u && s.v.z != 0u && s.v.w != 0u;
 }
 
+// one of the words that hold the L bytes of a key is zero
+__device__ __forceinline__ bool blank_word(const uint32_t k[4], uint32_t L)
+{
+  return k[0] == 0u || (L > 4u && k[1] == 0u) || (L > 8u && k[2] == 0u) || (L > 12u && k[3] == 0u);
+}
+
 // Looks a listed segment up in the long table; a hit leaves its ids in tok and its live bits in the bitmap.
 template <int TH>
 __device__ __forceinline__ bool recall_segment(TileSmem<TH>& S, const DeviceTable& T, uint32_t ent)
@@ -311,6 +319,7 @@ __device__ __forceinline__ bool recall_segment(TileSmem<TH>& S, const DeviceTabl
   uint32_t k[4];
   window_words(S, s, k);
   k[0] &= km.x, k[1] &= km.y, k[2] &= km.z, k[3] &= km.w;
+  if (T.learn && blank_word(k, L)) return false;
   const uint32_t h = long_slot_of(k, L);
   LongSlot at      = load_long(T.long_words, h);
   bool found       = long_matches(at, k, L);

@@ -287,6 +287,26 @@ def test_results_outlive_later_calls_and_their_tokenizer(lib, merges_path, oracl
             assert np.array_equal(ids[toff[k]:toff[k + 1]], want)
 
 
+@pytest.mark.parametrize("n_bytes", [4096, (12 << 20) + 4097])
+def test_strings_of_nul_bytes(lib, merges_path, tmp_path, n_bytes):
+    """A table that merges NUL bytes, text full of strings whose key words are zero, below and above the size from which
+    merged segments are added to the long table while the batch runs.  Whole ids: no tolerance."""
+    from oracle.loader import Oracle
+
+    with open(merges_path, encoding="utf-8") as f:
+        lines = f.read().split("\n")[:3001]
+    nul = "\u0100"  # the symbol of byte 0
+    path = str(tmp_path / "nul_merges.txt")
+    with open(path, "w", encoding="utf-8") as f:
+        f.write("\n".join(lines + [f"{nul} {nul}", f"e {nul}", f"{nul}{nul} e", f"{nul} a"]) + "\n")
+    rng = np.random.default_rng(n_bytes)
+    parts = [b"\0" * k + t + b"\0" * j for k in range(9) for j in range(7) for t in (b"", b"e", b"a", b"the")]
+    blob = b" ".join(parts[i] for i in rng.integers(0, len(parts), n_bytes // 4))[:n_bytes]
+    want, woff = Oracle(path).encode_fixed(np.frombuffer(blob, np.uint8), 2048, mode=MODE_SEGMENTED, threads=NCPU)
+    ids, _, coff, _ = make_tok(lib, path, 2048).encode(blob)
+    check_chunks(ids, coff, want, woff, f"NUL strings, {n_bytes} bytes")
+
+
 def test_crowded_pair_bucket(lib, merges_path, tmp_path):
     """More than four pairs in one bucket of the device pair table: the fifth and later ones are found in
     the side table (second load), in every kernel that probes."""
