@@ -159,7 +159,9 @@ struct gtk_taken {
 // Buffers of one in-flight slice of a large host batch (kSliceArenas sets rotate).
 constexpr int kSliceArenas = 4;
 struct SliceArena {
-  DevBuf text_chunk_base, chunk_off, tile_chunk0, unit_first, unit_cnt, chunk_cnt, unit_base, scan_sums, counters,
+  DevBuf text_chunk_base, chunk_off, unit_first, unit_cnt, chunk_cnt, tile_info, chunk_rel, text_rel, group_base,
+      scan_sums,
+      counters,  // the 16 counter words, then the group counts
       totals;
   PinBuf h_totals;  // mapped: written by a kernel
   cudaEvent_t ev[6] = {};          // stage timing
@@ -169,8 +171,8 @@ struct SliceArena {
   cudaEvent_t ev_out = nullptr;    // results of the slice are on the host
   void release()
   {
-    for (DevBuf* b : {&text_chunk_base, &chunk_off, &tile_chunk0, &unit_first, &unit_cnt, &chunk_cnt, &unit_base,
-                      &scan_sums, &counters, &totals})
+    for (DevBuf* b : {&text_chunk_base, &chunk_off, &unit_first, &unit_cnt, &chunk_cnt, &tile_info, &chunk_rel,
+                      &text_rel, &group_base, &scan_sums, &counters, &totals})
       b->release();
     h_totals.release();
     for (auto& e : ev)
@@ -208,8 +210,8 @@ struct gtk_tokenizer {
 
   // arenas
   DevBuf d_bytes, d_text_off, d_text_chunk_base, d_chunk_off, d_tile_chunk0, d_staging, d_unit_first, d_unit_cnt,
-      d_chunk_cnt, d_unit_base, d_chunk_id_off, d_text_id_off, d_out_ids, d_seg_scratch, d_scan_sums,
-      d_totals;  // d_totals also holds the counters (plan_batch)
+      d_chunk_cnt, d_tile_info, d_chunk_rel, d_text_rel, d_group_base, d_chunk_id_off, d_text_id_off, d_out_ids, d_seg_scratch, d_scan_sums,
+      d_totals;  // d_totals also holds the counters and group counts (plan_batch)
   PinBuf h_ids, h_text_id_off, h_chunk_id_off, h_totals;
   // sliced host batches: offsets of all slices, moved once per batch
   DevBuf d_piece_off, d_piece_id_off, d_chunk_id_all;
@@ -233,8 +235,10 @@ struct gtk_tokenizer {
   const uint8_t* pack_base = nullptr;  // h_out_pack, or the mapped block below behind its 64-byte header
   // batches of up to 256 KiB: a kernel writes the results into this mapped block and the host polls its header
   PinBuf h_mid;
+  PinBuf h_out;                // results of encode_host_tiles
+  double ids_per_byte = 0.4;  // room for ids that encode_host_tiles starts with; grows with the texts it meets
   int64_t mid_seq = 0;
-  // one text of up to 64 KiB: chunk table, zeroed counters and the text travel in one copy (encode_host_one_text)
+  // zeroed counters, scanned chunk counts and, when it is short, the text travel in one copy (encode_host_tiles)
   PinBuf h_fast_in;
   DevBuf d_fast_in;
   int64_t small_seq = 0;  // calls of the small-batch kernel so far (the kernel echoes it as its completion mark)
@@ -346,12 +350,15 @@ Plan plan_batch(gtk_tokenizer* h, const uint8_t* d_bytes, int64_t n_bytes, const
   p.chunk_cap = chunk_cap;
   h->d_text_chunk_base.reserve(size_t(n_texts + 1) * 8);
   h->d_chunk_off.reserve(size_t(chunk_cap + 1) * 8);
-  h->d_tile_chunk0.reserve(size_t(n_tiles + 1) * 4);
+  h->d_tile_chunk0.reserve(size_t(gtk::kSmallMaxBytes / gtk::kTile + 1) * 4);
+  h->d_tile_info.reserve(size_t(n_tiles + 1) * sizeof(gtk::TileInfo));
+  h->d_chunk_rel.reserve(size_t(chunk_cap + 1) * 4);
+  h->d_text_rel.reserve(size_t(n_texts + 1) * 4);
+  h->d_group_base.reserve(size_t(n_tiles / gtk::kTileGroup + 2) * 8);
   h->d_staging.reserve(size_t(n_bytes + 16) * 2);
   h->d_unit_first.reserve(size_t(n_tiles + 1) * 8);
   h->d_unit_cnt.reserve(size_t(n_tiles + 1) * 4);
   h->d_chunk_cnt.reserve(size_t(chunk_cap + 1) * 4);
-  h->d_unit_base.reserve(size_t(n_tiles + 2) * 8);
   if (!d_chunk_id_off) {
     h->d_chunk_id_off.reserve(size_t(chunk_cap + 1) * 8);
     d_chunk_id_off = h->d_chunk_id_off.as<int64_t>();
@@ -359,7 +366,8 @@ Plan plan_batch(gtk_tokenizer* h, const uint8_t* d_bytes, int64_t n_bytes, const
   if (want_text_id_off) h->d_text_id_off.reserve(size_t(n_texts + 1) * 8);
   const int64_t scan_items = std::max<int64_t>(std::max(chunk_cap, n_tiles), n_texts);
   h->d_scan_sums.reserve(size_t(scan_items / 4096 + 2) * 8);
-  h->d_totals.reserve(128);  // [0] n_chunks, [1] n_ids as int64, then the 16 int32 counters: one copy brings both
+  // [0] n_chunks, [1] n_ids as int64, then the 16 int32 counters (one copy brings both) and the group counts
+  h->d_totals.reserve(80 + size_t(n_tiles / gtk::kTileGroup + 1) * 4);
   // workspace for segments / chunks that do not fit in shared memory
   const int64_t longest = std::min<int64_t>(h->chunk_tokens, n_bytes);
   int64_t scratch_tokens = 0;
@@ -385,7 +393,10 @@ Plan plan_batch(gtk_tokenizer* h, const uint8_t* d_bytes, int64_t n_bytes, const
   b.unit_first = h->d_unit_first.as<int64_t>();
   b.unit_cnt = h->d_unit_cnt.as<int32_t>();
   b.chunk_cnt = h->d_chunk_cnt.as<int32_t>();
-  b.unit_base = h->d_unit_base.as<int64_t>();
+  b.tile_info = h->d_tile_info.as<gtk::TileInfo>();
+  b.chunk_rel = h->d_chunk_rel.as<int32_t>();
+  b.text_rel = h->d_text_rel.as<int32_t>();
+  b.group_base = h->d_group_base.as<int64_t>();
   b.chunk_id_off = d_chunk_id_off;
   b.text_id_off = want_text_id_off ? h->d_text_id_off.as<int64_t>() : nullptr;
   b.out_ids = d_out_ids;
@@ -397,6 +408,7 @@ Plan plan_batch(gtk_tokenizer* h, const uint8_t* d_bytes, int64_t n_bytes, const
   b.scan_block_sums = h->d_scan_sums.as<int64_t>();
   b.totals = h->d_totals.as<int64_t>();
   b.counters = reinterpret_cast<int32_t*>(b.totals + 2);
+  b.group_cnt = b.counters + 16;
   b.low_id_map = (h->id_space == GTK_IDS_GPT2) ? h->d_low_map.as<uint16_t>() : nullptr;
   return p;
 }
@@ -412,6 +424,7 @@ const char* status_text(int s)
   }
 }
 
+// The kernels that work chunk by chunk (GTK_MODE_BASE, GTK_MODE_LOCALMIN, tables beyond 16 bits).
 // Chunker -> merge -> scans.  Leaves totals (n_chunks, n_ids) and the status
 // word in the pinned totals buffer; the caller synchronises and then packs.
 // n_chunks, n_ids and the status word to the host: totals and counters are adjacent in the handle's own arena
@@ -434,20 +447,18 @@ void run_front(gtk_tokenizer* h, const gtk::EncodeBuffers& b, int mode, int* lau
   cudaStream_t s = h->stream;
   const bool stages = ev != nullptr || h->stage_timing;  // sliced batches always time their stages
   if (!ev) ev = h->ev;
-  const bool own_reset = gtk::chunker_resets_counters(b);
-  if (!own_reset || h->reset_learned) {
-    *launches += gtk::launch_begin_batch(b, !own_reset, h->dtab.long_words, h->reset_learned ? h->call_tab.long_words : nullptr, s);
-    h->reset_learned = false;
+  if (!gtk::chunker_resets_counters(b)) {
+    GTK_CUDA(cudaMemsetAsync(b.counters, 0, 64, s));
+    GTK_CUDA(cudaMemsetAsync(b.chunk_cnt, 0, size_t(b.chunk_cap + 1) * 4, s));
   }
   GTK_CUDA(cudaEventRecord(ev[0], s));
   *launches += gtk::launch_chunker(b, s);
   if (stages) GTK_CUDA(cudaEventRecord(ev[1], s));
   if (h->wide) *launches += gtk::launch_merge_wide(b, h->dtab, h->wide_grid, s);
   else if (mode == GTK_MODE_BASE) *launches += gtk::launch_merge_base(b, h->dtab, h->base_grid, h->base_block, s);
-  else if (mode == GTK_MODE_LOCALMIN) *launches += gtk::launch_merge_localmin(b, h->dtab, h->localmin_grid, h->max_iters, s);
-  else *launches += gtk::launch_merge_opt(b, h->call_tab, h->opt_grid, s);
+  else *launches += gtk::launch_merge_localmin(b, h->dtab, h->localmin_grid, h->max_iters, s);
   if (stages) GTK_CUDA(cudaEventRecord(ev[2], s));
-  *launches += gtk::launch_output_scans(b, mode != GTK_MODE_OPT || h->wide, s);
+  *launches += gtk::launch_output_scans(b, s);
   if (stages || !chained) GTK_CUDA(cudaEventRecord(ev[3], s));
   GTK_CUDA(cudaGetLastError());
   if (mapped_totals) {  // one small kernel writes the four words into mapped host memory: no copy-engine round trips
@@ -458,7 +469,7 @@ void run_front(gtk_tokenizer* h, const gtk::EncodeBuffers& b, int mode, int* lau
   copy_totals(h, b, pinned_totals, s);
 }
 
-void run_pack(gtk_tokenizer* h, const gtk::EncodeBuffers& b, int mode, int* launches, cudaEvent_t* ev = nullptr,
+void run_pack(gtk_tokenizer* h, const gtk::EncodeBuffers& b, int* launches, cudaEvent_t* ev = nullptr,
               cudaStream_t on = nullptr, bool chained = false, bool totals_by_copy = true)
 {
   cudaStream_t s = on ? on : h->stream;
@@ -466,10 +477,37 @@ void run_pack(gtk_tokenizer* h, const gtk::EncodeBuffers& b, int mode, int* laun
   if (!ev) ev = h->ev;
   if (stages || !chained) GTK_CUDA(cudaEventRecord(ev[5], s));
   if (h->wide) *launches += gtk::launch_pack_wide(b, h->sm_count * 8, s);
-  else *launches += gtk::launch_pack(b, mode != GTK_MODE_OPT, h->sm_count * 8, s);
+  else *launches += gtk::launch_pack_chunks(b, h->sm_count * 8, s);
   GTK_CUDA(cudaEventRecord(ev[4], s));
   GTK_CUDA(cudaGetLastError());
   if (chained && totals_by_copy) copy_totals(h, b, nullptr, s);
+}
+
+// The tile kernel and what follows it (GTK_MODE_OPT): reset, chunks per text, tile records, tiles, pack.
+// `ready`: counters, group counts, scanned chunk counts and tile records are in place already.  The pack kernel publishes the totals (see
+// launch_pack_tiles).  The events between the stages are recorded when they are asked for.
+void run_tiles(gtk_tokenizer* h, const gtk::EncodeBuffers& b, bool ready, int64_t* publish, int64_t seq, int* launches,
+               cudaEvent_t* ev = nullptr)
+{
+  cudaStream_t s    = h->stream;
+  const bool stages = ev != nullptr || h->stage_timing;
+  if (!ev) ev = h->ev;
+  const bool learned = h->reset_learned;
+  if (!ready || learned) {
+    *launches += gtk::launch_begin_batch(b, h->dtab.long_words, learned ? h->call_tab.long_words : nullptr, s);
+  }
+  h->reset_learned = false;
+  if (stages) GTK_CUDA(cudaEventRecord(ev[0], s));
+  if (!ready) *launches += gtk::launch_scan_texts(b, learned, s) + gtk::launch_tile_info(b, s);
+  if (stages) GTK_CUDA(cudaEventRecord(ev[1], s));
+  *launches += gtk::launch_merge_opt(b, h->call_tab, h->opt_grid, s);
+  if (stages) GTK_CUDA(cudaEventRecord(ev[2], s));
+  const int scanned = ready ? 0 : gtk::launch_scan_groups(b, s);
+  if (stages)
+    for (int i : {3, 5}) GTK_CUDA(cudaEventRecord(ev[i], s));
+  *launches += scanned + gtk::launch_pack_tiles(b, h->sm_count, scanned != 0, publish, seq, s);
+  if (stages) GTK_CUDA(cudaEventRecord(ev[4], s));
+  GTK_CUDA(cudaGetLastError());
 }
 
 // Adds the stage times of one pipeline run (one batch, or one slice) to h->stage_ms.  The events must have
@@ -606,13 +644,15 @@ void slice_arena_prepare(gtk_tokenizer* h, SliceArena& a, int64_t max_bytes, int
   const int64_t n_tiles   = (max_bytes + gtk::kTile - 1) / gtk::kTile;
   a.text_chunk_base.reserve(size_t(max_pieces + 1) * 8);
   a.chunk_off.reserve(size_t(chunk_cap + 1) * 8);
-  a.tile_chunk0.reserve(size_t(n_tiles + 1) * 4);
+  a.tile_info.reserve(size_t(n_tiles + 1) * sizeof(gtk::TileInfo));
+  a.chunk_rel.reserve(size_t(chunk_cap + 1) * 4);
+  a.text_rel.reserve(size_t(max_pieces + 1) * 4);
+  a.group_base.reserve(size_t(n_tiles / gtk::kTileGroup + 2) * 8);
   a.unit_first.reserve(size_t(n_tiles + 1) * 8);
   a.unit_cnt.reserve(size_t(n_tiles + 1) * 4);
   a.chunk_cnt.reserve(size_t(chunk_cap + 1) * 4);
-  a.unit_base.reserve(size_t(n_tiles + 2) * 8);
   a.scan_sums.reserve(size_t(std::max<int64_t>(std::max(chunk_cap, n_tiles), max_pieces) / 4096 + 2) * 8);
-  a.counters.reserve(64);
+  a.counters.reserve(64 + size_t(n_tiles / gtk::kTileGroup + 1) * 4);
   a.totals.reserve(64);
   a.h_totals.reserve_mapped(64);
   for (auto& e : a.ev)
@@ -639,13 +679,15 @@ gtk::EncodeBuffers slice_buffers(gtk_tokenizer* h, SliceArena& a, const SlicePla
   b.text_chunk_base = a.text_chunk_base.as<int64_t>();
   b.chunk_off = a.chunk_off.as<int64_t>();
   b.chunk_cap = chunk_upper_bound(n_bytes, pieces, h->chunk_tokens);
-  b.tile_chunk0 = a.tile_chunk0.as<int32_t>();
   b.n_tiles = (n_bytes + gtk::kTile - 1) / gtk::kTile;
   b.staging = h->d_staging.as<uint16_t>() + dev_off;
   b.unit_first = a.unit_first.as<int64_t>();
   b.unit_cnt = a.unit_cnt.as<int32_t>();
   b.chunk_cnt = a.chunk_cnt.as<int32_t>();
-  b.unit_base = a.unit_base.as<int64_t>();
+  b.tile_info = a.tile_info.as<gtk::TileInfo>();
+  b.chunk_rel = a.chunk_rel.as<int32_t>();
+  b.text_rel = a.text_rel.as<int32_t>();
+  b.group_base = a.group_base.as<int64_t>();
   b.chunk_id_off = nullptr;
   b.text_id_off = nullptr;
   b.out_ids = h->d_out_ids.as<int32_t>() + dev_off;  // worst case one id per byte: slices never overlap
@@ -658,6 +700,7 @@ gtk::EncodeBuffers slice_buffers(gtk_tokenizer* h, SliceArena& a, const SlicePla
   b.seg_scratch_tokens = scratch_tokens;
   b.scan_block_sums = a.scan_sums.as<int64_t>();
   b.counters = a.counters.as<int32_t>();
+  b.group_cnt = b.counters + 16;
   b.totals = a.totals.as<int64_t>();
   b.low_id_map = (h->id_space == GTK_IDS_GPT2) ? h->d_low_map.as<uint16_t>() : nullptr;
   return b;
@@ -725,6 +768,7 @@ int encode_host_sliced(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
   std::vector<int64_t> sl_c(nsz), sl_r(nsz), sl_cbase(nsz);
   int launches = 0;
   int64_t R = 0, Cbase = 0;
+  const bool tiles = mode == GTK_MODE_OPT && !h->wide;  // its pack follows the tile kernel without a word from the host
 
   auto issue_front = [&](int i) {
     SliceArena& a = h->slice[i % kSliceArenas];
@@ -739,14 +783,15 @@ int encode_host_sliced(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
     b.text_off     = h->d_piece_off.as<int64_t>() + piece_at[size_t(i)];
     b.text_id_off  = h->d_piece_id_off.as<int64_t>() + piece_at[size_t(i)];
     b.chunk_id_off = h->d_chunk_id_all.as<int64_t>() + chunk_at[size_t(i)];
-    // the four result words of the front are written into mapped host memory by a one-thread kernel
-    run_front(h, b, mode, &launches, a.ev, nullptr, static_cast<int64_t*>(a.h_totals.dp));
+    // the result words reach the host through mapped memory
+    if (tiles) run_tiles(h, b, false, static_cast<int64_t*>(a.h_totals.dp), i + 1, &launches, a.ev);
+    else run_front(h, b, mode, &launches, a.ev, nullptr, static_cast<int64_t*>(a.h_totals.dp));
     GTK_CUDA(cudaEventRecord(a.ev_front, h->stream));
   };
   auto finish = [&](int i) {  // the ids of slice i are on the host
     SliceArena& a = h->slice[i % kSliceArenas];
     GTK_CUDA(cudaEventSynchronize(a.ev_out));
-    collect_pack_time(h, a.ev);
+    if (!tiles) collect_pack_time(h, a.ev);
   };
   auto sync_all = [&] {
     cudaStreamSynchronize(h->in_stream);
@@ -762,9 +807,10 @@ int encode_host_sliced(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
     if (i >= 2) finish(i - 2);
     GTK_CUDA(cudaEventSynchronize(a.ev_front));
     collect_front_times(h, a.ev);
+    if (tiles) collect_pack_time(h, a.ev);
     const int64_t* ht = a.h_totals.as<int64_t>();
     const int64_t C = ht[0], N = ht[1];
-    const int status = reinterpret_cast<const int32_t*>(ht + 2)[1];
+    const int status = tiles ? int(ht[2]) : reinterpret_cast<const int32_t*>(ht + 2)[1];
     if (status != gtk::kStatusOk) {
       sync_all();
       return h->fail(GTK_ERR_KERNEL, status_text(status));
@@ -777,11 +823,12 @@ int encode_host_sliced(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
       h->h_ids.release();
       h->h_ids = bigger;
     }
-    // the pack runs on a stream of its own: the compute stream already holds the fronts of later slices
-    GTK_CUDA(cudaStreamWaitEvent(h->pack_stream, a.ev_front, 0));
-    run_pack(h, bufs[size_t(i)], mode, &launches, a.ev, h->pack_stream);
-    GTK_CUDA(cudaEventRecord(a.ev_packed, h->pack_stream));
-    GTK_CUDA(cudaStreamWaitEvent(h->out_stream, a.ev_packed, 0));
+    if (!tiles) {  // the pack runs on a stream of its own: the compute stream already holds the fronts of later slices
+      GTK_CUDA(cudaStreamWaitEvent(h->pack_stream, a.ev_front, 0));
+      run_pack(h, bufs[size_t(i)], &launches, a.ev, h->pack_stream);
+      GTK_CUDA(cudaEventRecord(a.ev_packed, h->pack_stream));
+    }
+    GTK_CUDA(cudaStreamWaitEvent(h->out_stream, tiles ? a.ev_front : a.ev_packed, 0));
     GTK_CUDA(cudaMemcpyAsync(h->h_ids.as<int32_t>() + R, bufs[size_t(i)].out_ids, size_t(N) * 4, cudaMemcpyDeviceToHost,
                              h->out_stream));
     GTK_CUDA(cudaEventRecord(a.ev_out, h->out_stream));
@@ -921,92 +968,129 @@ int encode_host_small(gtk_tokenizer* h, const uint8_t* bytes, const int64_t* tex
   return GTK_OK;
 }
 
-// Batches of up to 64 KiB and 1024 texts (GTK_MODE_OPT, 16-bit table): two launches.  The host lays out the chunk
-// table (a few thousand entries at most) and sends it with zeroed counters and the text in ONE copy; the tile kernel
-// runs as for any batch; one more kernel (a CTA per tile) does the scans and the pack and writes the results into
-// mapped host memory, where the host polls the call number.  No chunker launch, no copy back, no synchronisation.
-constexpr int64_t kTwoLaunchMaxBytes  = int64_t(gtk::kFinishMaxTiles / 2) * gtk::kTile;  // 64 KiB
-constexpr int64_t kTwoLaunchMaxChunks = 4096;
+// Host batches below the slicing threshold (GTK_MODE_OPT, 16-bit table): two launches.  The host scans the chunk counts of
+// the texts and sends them with zeroed counters and, up to kTextInHeaderBytes, the text itself in one copy; tile kernel;
+// pack kernel, which writes ids and offsets into page-locked memory and then the call number, for which the host waits.
+// No chunker, no scan, no copy back, no synchronisation.
+constexpr int64_t kTextInHeaderBytes = 64 << 10;
 
-// number of chunks of the batch, or -1 when it does not qualify for the two-launch path
-int64_t two_launch_chunks(const gtk_tokenizer* h, int mode, const int64_t* text_offsets, int64_t n_texts, int64_t n_bytes)
+// The tile records of a batch, as k_tile_info makes them on the device.
+void lay_tiles(const int64_t* text_off, const int64_t* chunk_base, int64_t n_texts, int64_t n_bytes, int64_t chunk,
+               gtk::TileInfo* out)
 {
-  if (h->wide || mode != GTK_MODE_OPT || h->stage_timing) return -1;
-  if (n_bytes > kTwoLaunchMaxBytes || n_texts > gtk::kSmallMaxTexts) return -1;
-  const int64_t chunk = h->chunk_tokens;
-  int64_t C = 0;
-  for (int64_t t = 0; t < n_texts; ++t) C += (text_offsets[t + 1] - text_offsets[t] + chunk - 1) / chunk;
-  return C <= kTwoLaunchMaxChunks ? C : -1;
+  int64_t t = 0;  // first text that starts at or behind the tile's first byte
+  for (int64_t lo = 0; lo < n_bytes; lo += gtk::kTile) {
+    gtk::TileInfo& i = *out++;
+    if (n_texts == 1) {
+      const uint32_t past = uint32_t(lo) % uint32_t(chunk);
+      const int64_t p0    = past ? chunk - past : 0;
+      i = gtk::TileInfo{(lo + p0) / chunk, lo > 0, p0 < gtk::kWindow && lo + p0 < n_bytes ? int32_t(p0) : gtk::kTileNoCut,
+                        gtk::kTilePlain | (lo > 0 ? gtk::kTileRunsIn : 0)};
+      continue;
+    }
+    while (t < n_texts && text_off[t] < lo) ++t;
+    const bool runs_in = t > 0 && text_off[t] > lo;
+    i = gtk::TileInfo{chunk_base[t], t, gtk::kTileNoCut, runs_in ? gtk::kTileRunsIn : 0};
+    if (!runs_in) continue;
+    const int64_t n  = (uint32_t(lo - text_off[t - 1]) + uint32_t(chunk) - 1u) / uint32_t(chunk);
+    const int64_t at = text_off[t - 1] + n * chunk;
+    if (at < text_off[t]) {
+      i.c0 = chunk_base[t - 1] + n;
+      if (at - lo < gtk::kWindow) i.p0 = int32_t(at - lo);
+    }
+    if (text_off[t] >= std::min(lo + gtk::kWindow, n_bytes)) i.flags |= gtk::kTilePlain;
+  }
 }
 
-int encode_host_two_launches(gtk_tokenizer* h, const uint8_t* bytes, const int64_t* text_offsets, int64_t n_texts,
-                             int64_t n_bytes, int64_t C, float* kernel_ms)
+int encode_host_tiles(gtk_tokenizer* h, const uint8_t* bytes, const int64_t* text_offsets, int64_t n_texts, int64_t n_bytes,
+                      float* kernel_ms)
 {
   auto up = [](size_t x) { return (x + 63) & ~size_t(63); };
-  const int64_t chunk = h->chunk_tokens;
-  const int64_t K     = (n_bytes + gtk::kTile - 1) / gtk::kTile;
-  const size_t o_cnt = 128, o_coff = up(o_cnt + size_t(C + 1) * 4), o_tile = up(o_coff + size_t(C + 1) * 8);
-  const size_t o_tbase = up(o_tile + size_t(K) * 4), o_bytes = up(o_tbase + size_t(n_texts + 1) * 8);
-  const size_t total = o_bytes + size_t(n_bytes) + 32;
-  h->h_fast_in.reserve(total);
-  h->d_fast_in.reserve(total);
+  const int64_t chunk = h->chunk_tokens, K = (n_bytes + gtk::kTile - 1) / gtk::kTile;
+  const bool one = n_texts == 1, with_text = n_bytes <= kTextInHeaderBytes;
+  const size_t o_off = up(16 + 64 + size_t(K / gtk::kTileGroup + 1) * 4), o_base = up(o_off + (one ? 0 : size_t(n_texts + 1) * 8));
+  const size_t o_info = up(o_base + (one ? 0 : size_t(n_texts + 1) * 8)), o_text = up(o_info + size_t(K) * sizeof(gtk::TileInfo));
+  const size_t header = with_text ? o_text + size_t(n_bytes) : o_text;
+  h->h_fast_in.reserve(header + 32);
+  h->d_fast_in.reserve(header + 32);
   uint8_t* hp = static_cast<uint8_t*>(h->h_fast_in.p);
-  std::memset(hp, 0, o_coff);  // totals, counters, per-chunk counts
-  reinterpret_cast<int64_t*>(hp)[0] = C;
-  int64_t* coff  = reinterpret_cast<int64_t*>(hp + o_coff);
-  int64_t* tbase = reinterpret_cast<int64_t*>(hp + o_tbase);
-  int64_t c = 0;
-  for (int64_t t = 0; t < n_texts; ++t) {
-    tbase[t] = c;
-    for (int64_t pos = text_offsets[t]; pos < text_offsets[t + 1]; pos += chunk) coff[c++] = pos;
-  }
-  tbase[n_texts] = c;
-  coff[c]        = n_bytes;
-  int32_t* tile0 = reinterpret_cast<int32_t*>(hp + o_tile);
-  for (int64_t k = 0, cc = 0; k < K; ++k) {  // last chunk that starts at or before the tile's first byte
-    while (cc + 1 < C && coff[cc + 1] <= k * gtk::kTile) ++cc;
-    tile0[k] = int32_t(cc);
-  }
-  std::memcpy(hp + o_bytes, bytes, size_t(n_bytes));
-  std::memset(hp + o_bytes + n_bytes, 0, 32);
-  cudaStream_t s = h->stream;
   uint8_t* dp = h->d_fast_in.as<uint8_t>();
-  GTK_CUDA(cudaMemcpyAsync(dp, hp, total, cudaMemcpyHostToDevice, s));
+  cudaStream_t s = h->stream;
+  if (!with_text) {
+    h->d_bytes.reserve(size_t(n_bytes) + 32);
+    GTK_CUDA(cudaMemcpyAsync(h->d_bytes.p, bytes, size_t(n_bytes), cudaMemcpyHostToDevice, s));
+  }
+  std::memset(hp, 0, o_off);  // totals, counters, group counts
+  int64_t C = 0;
+  if (one) {
+    C = (n_bytes + chunk - 1) / chunk;
+  } else {
+    std::memcpy(hp + o_off, text_offsets, size_t(n_texts + 1) * 8);
+    int64_t* base = reinterpret_cast<int64_t*>(hp + o_base);
+    for (int64_t t = 0; t < n_texts; ++t) {  // lengths and chunk size are below 2^31 here: 32-bit divisions
+      base[t] = C;
+      const uint32_t len = uint32_t(text_offsets[t + 1] - text_offsets[t]);
+      C += len <= uint32_t(chunk) ? (len > 0) : (len + uint32_t(chunk) - 1u) / uint32_t(chunk);
+    }
+    base[n_texts] = C;
+  }
+  reinterpret_cast<int64_t*>(hp)[0] = C;
+  lay_tiles(text_offsets, reinterpret_cast<const int64_t*>(hp + o_base), n_texts, n_bytes, chunk,
+            reinterpret_cast<gtk::TileInfo*>(hp + o_info));
+  if (with_text) std::memcpy(hp + o_text, bytes, size_t(n_bytes));
+  GTK_CUDA(cudaMemcpyAsync(dp, hp, header, cudaMemcpyHostToDevice, s));
 
+  // [64-byte header | text id offsets | chunk id offsets | ids]
   const size_t text_b = up(size_t(n_texts + 1) * 8), chunk_b = up(size_t(C + 1) * 8);
-  uint8_t* md = mid_block(h);  // (page-locked memory has the same address on the device) [64-byte header | text id offsets | chunk id offsets | ids]
-  Plan p = plan_batch(h, dp + o_bytes, n_bytes, nullptr, n_texts, reinterpret_cast<int32_t*>(md + 64 + text_b + chunk_b),
-                      n_bytes, reinterpret_cast<int64_t*>(md + 64 + text_b), false);
-  p.b.text_id_off     = reinterpret_cast<int64_t*>(md + 64);
-  p.b.totals          = reinterpret_cast<int64_t*>(dp);
-  p.b.counters        = reinterpret_cast<int32_t*>(dp + 16);
-  p.b.chunk_cnt       = reinterpret_cast<int32_t*>(dp + o_cnt);
-  p.b.chunk_off       = reinterpret_cast<int64_t*>(dp + o_coff);
-  p.b.tile_chunk0     = reinterpret_cast<int32_t*>(dp + o_tile);
-  p.b.text_chunk_base = reinterpret_cast<int64_t*>(dp + o_tbase);
-  h->d_chunk_id_off.reserve(size_t(kTwoLaunchMaxChunks + 1) * 8);
-  p.b.chunk_id_mirror = h->d_chunk_id_off.as<int64_t>();  // the scan's own copy in HBM: the text offsets index it
-  const int64_t seq = ++h->mid_seq;
-  GTK_CUDA(cudaEventRecord(h->ev[0], s));
-  int launches = gtk::launch_merge_opt(p.b, h->dtab, h->opt_grid, s);
-  launches += gtk::launch_finish_small_batch(p.b, reinterpret_cast<int64_t*>(md), seq, s);
-  GTK_CUDA(cudaEventRecord(h->ev[4], s));
-  GTK_CUDA(cudaGetLastError());
-  volatile const int64_t* tot = h->h_mid.as<volatile const int64_t>();
-  if (!wait_for_mark(tot + 3, seq, s, "finish kernel"))
-    return h->fail(GTK_ERR_KERNEL, "finish kernel ended without publishing its results");
-  if (tot[2] != gtk::kStatusOk) return h->fail(GTK_ERR_KERNEL, status_text(int(tot[2])));
-  if (tot[0] != C || tot[1] > n_bytes) return h->fail(GTK_ERR_KERNEL, "inconsistent totals");
-  GTK_CUDA(cudaEventSynchronize(h->ev[4]));  // completes a moment after the mark
-  GTK_CUDA(cudaEventElapsedTime(&h->stage_ms[4], h->ev[0], h->ev[4]));
+  // room for the ids: by what this handle has met so far (English has one id in three or four bytes), at most one per byte
+  int64_t room = std::min<int64_t>(n_bytes, int64_t(double(n_bytes) * h->ids_per_byte) + 1024);
+  begin_call(h, GTK_MODE_OPT, n_bytes);
+  int launches = 0;
+  Plan p;
+  uint8_t* md = nullptr;
+  for (int attempt = 0;; ++attempt) {
+    h->pool->reserve(h->h_out, 64 + text_b + chunk_b + size_t(room) * 4);
+    md = h->h_out.as<uint8_t>();  // page-locked memory has the same address on the device
+    std::memset(md, 0, 64);
+    p = plan_batch(h, with_text ? dp + o_text : h->d_bytes.as<uint8_t>(), n_bytes, reinterpret_cast<int64_t*>(dp + o_off), n_texts,
+                   reinterpret_cast<int32_t*>(md + 64 + text_b + chunk_b), room, reinterpret_cast<int64_t*>(md + 64 + text_b), false);
+    p.b.text_id_off     = reinterpret_cast<int64_t*>(md + 64);
+    p.b.totals          = reinterpret_cast<int64_t*>(dp);
+    p.b.counters        = reinterpret_cast<int32_t*>(dp + 16);
+    p.b.group_cnt       = p.b.counters + 16;
+    p.b.text_chunk_base = reinterpret_cast<int64_t*>(dp + o_base);
+    p.b.tile_info       = reinterpret_cast<gtk::TileInfo*>(dp + o_info);
+    const int64_t seq   = ++h->mid_seq;
+    if (attempt == 0) {
+      run_tiles(h, p.b, true, reinterpret_cast<int64_t*>(md), seq, &launches);
+    } else {  // the tokens are still staged: pack them again
+      GTK_CUDA(cudaMemsetAsync(p.b.counters + 8, 0, 4, s));
+      launches += gtk::launch_pack_tiles(p.b, h->sm_count, false, reinterpret_cast<int64_t*>(md), seq, s);
+      GTK_CUDA(cudaGetLastError());
+    }
+    volatile const int64_t* tot = reinterpret_cast<volatile const int64_t*>(md);
+    if (!wait_for_mark(tot + 3, seq, s, "pack kernel"))
+      return h->fail(GTK_ERR_KERNEL, "pack kernel ended without publishing its results");
+    if (tot[2] != gtk::kStatusOk) return h->fail(GTK_ERR_KERNEL, status_text(int(tot[2])));
+    if (tot[0] != C || tot[1] > n_bytes) return h->fail(GTK_ERR_KERNEL, "inconsistent totals");
+    h->res_n_ids   = tot[1];
+    h->stage_ms[4] = float(double(tot[4]) * 1e-6);  // by the kernels' own clock
+    if (h->res_n_ids <= room) break;
+    h->ids_per_byte = std::min(1.0, 1.1 * double(h->res_n_ids) / double(n_bytes));
+    room = h->res_n_ids;
+  }
+  if (h->stage_timing) {
+    std::fill(h->stage_ms, h->stage_ms + 5, 0.f);
+    GTK_CUDA(cudaEventSynchronize(h->ev[4]));
+    collect_stage_times(h);
+  }
   h->result_is_packed = true;
-  h->pack_base        = h->h_mid.as<uint8_t>() + 64;
-  h->result_bufs[0]   = &h->h_mid;
+  h->pack_base        = md + 64;
+  h->result_bufs[0]   = &h->h_out;
   h->pack_text_bytes  = text_b;
   h->pack_chunk_bytes = chunk_b;
   h->last_launches    = launches;
   h->res_n_chunks     = C;
-  h->res_n_ids        = tot[1];
   if (kernel_ms) *kernel_ms = h->stage_ms[4];
   return GTK_OK;
 }
@@ -1019,10 +1103,10 @@ void release_handle(gtk_tokenizer* h)
     if (h->stream) cudaStreamSynchronize(h->stream);
     for (DevBuf* b : {&h->d_bpi, &h->d_slots, &h->d_overflow, &h->d_bpr, &h->d_mor, &h->d_sor, &h->d_adj, &h->d_b2i, &h->d_short_words, &h->d_long_words, &h->d_learned_words, &h->d_low_map, &h->d_wide_slots, &h->d_staging32, &h->d_seg_scratch32, &h->d_bytes, &h->d_text_off,
                       &h->d_text_chunk_base, &h->d_chunk_off, &h->d_tile_chunk0, &h->d_staging, &h->d_unit_first,
-                      &h->d_unit_cnt, &h->d_chunk_cnt, &h->d_unit_base, &h->d_chunk_id_off, &h->d_text_id_off,
+                      &h->d_unit_cnt, &h->d_chunk_cnt, &h->d_tile_info, &h->d_chunk_rel, &h->d_text_rel, &h->d_group_base, &h->d_chunk_id_off, &h->d_text_id_off,
                       &h->d_out_ids, &h->d_seg_scratch, &h->d_scan_sums, &h->d_totals, &h->d_out_pack, &h->d_fast_in})
       b->release();
-    for (PinBuf* b : {&h->h_ids, &h->h_text_id_off, &h->h_chunk_id_off, &h->h_totals, &h->h_piece_off, &h->h_piece_id_off, &h->h_chunk_id_all, &h->h_out_pack, &h->h_mid, &h->h_fast_in}) b->release();
+    for (PinBuf* b : {&h->h_ids, &h->h_text_id_off, &h->h_chunk_id_off, &h->h_totals, &h->h_piece_off, &h->h_piece_id_off, &h->h_chunk_id_all, &h->h_out_pack, &h->h_mid, &h->h_out, &h->h_fast_in}) b->release();
     for (DevBuf* b : {&h->d_piece_off, &h->d_piece_id_off, &h->d_chunk_id_all}) b->release();
     if (h->small_in_h) cudaFreeHost(h->small_in_h);
     if (h->small_out_h) cudaFreeHost(h->small_out_h);
@@ -1131,6 +1215,7 @@ GTK_API int gtk_create(const char* merges_path, int chunk_tokens, int max_iters,
       h->localmin_grid = h->sm_count * std::max(1, gtk::localmin_kernel_max_blocks_per_sm());
       h->wide_grid = h->sm_count * std::max(1, gtk::wide_kernel_max_blocks_per_sm());
       h->h_totals.reserve(64);
+      std::memset(h->h_totals.p, 0, 64);  // holds a completion mark: behind any call number that is still to come
       small_path_init(h);
     }
     *out = h;
@@ -1207,12 +1292,40 @@ GTK_API int gtk_encode_device(gtk_tokenizer* h, int mode, const uint8_t* d_bytes
     Plan p = plan_batch(h, d_bytes, n_bytes, d_text_offsets, n_texts, d_out_ids, out_capacity, chunk_dst, false);
     begin_call(h, mode, n_bytes);
     int launches = 0;
+    if (mode == GTK_MODE_OPT && !h->wide) {
+      volatile int64_t* tot = h->h_totals.as<int64_t>();
+      const int64_t seq     = ++h->mid_seq;
+      run_tiles(h, p.b, false, h->h_totals.as<int64_t>(), seq, &launches);
+      if (!wait_for_mark(tot + 3, seq, h->stream, "pack kernel"))
+        return h->fail(GTK_ERR_KERNEL, "pack kernel ended without publishing its results");
+      const int64_t C = tot[0], N = tot[1];
+      h->stage_ms[4]  = float(double(tot[4]) * 1e-6);  // by the kernels' own clock
+      if (tot[2] != gtk::kStatusOk) return h->fail(GTK_ERR_KERNEL, status_text(int(tot[2])));
+      if (N > out_capacity) return h->fail(GTK_ERR_CAPACITY, "d_out_ids too small: need " + std::to_string(N) + " ids");
+      if (d_out_chunk_offsets && !chunk_dst) {
+        if (chunk_capacity < C + 1)
+          return h->fail(GTK_ERR_CAPACITY, "d_out_chunk_offsets too small: need " + std::to_string(C + 1));
+        GTK_CUDA(cudaMemcpyAsync(d_out_chunk_offsets, p.b.chunk_id_off, size_t(C + 1) * 8, cudaMemcpyDeviceToDevice,
+                                 h->stream));
+        GTK_CUDA(cudaStreamSynchronize(h->stream));
+      }
+      if (h->stage_timing) {
+        std::fill(h->stage_ms, h->stage_ms + 5, 0.f);
+        GTK_CUDA(cudaEventSynchronize(h->ev[4]));
+        collect_stage_times(h);
+      }
+      h->last_launches = launches;
+      if (n_ids) *n_ids = N;
+      if (n_chunks) *n_chunks = C;
+      if (kernel_ms) *kernel_ms = h->stage_ms[4];
+      return GTK_OK;
+    }
     // When the chunk offsets are scanned straight into the caller's buffer (or not wanted), the pack follows
     // the front without a host round trip: the pack kernel itself never writes past out_capacity, and the
     // totals are checked once at the end.
     const bool one_sync = !d_out_chunk_offsets || chunk_dst;
     run_front(h, p.b, mode, &launches, nullptr, nullptr, nullptr, one_sync);
-    if (one_sync) run_pack(h, p.b, mode, &launches, nullptr, nullptr, true);
+    if (one_sync) run_pack(h, p.b, &launches, nullptr, nullptr, true);
     GTK_CUDA(cudaStreamSynchronize(h->stream));
     const int64_t* ht = h->h_totals.as<int64_t>();
     const int64_t C = ht[0], N = ht[1];
@@ -1233,7 +1346,7 @@ GTK_API int gtk_encode_device(gtk_tokenizer* h, int mode, const uint8_t* d_bytes
       GTK_CUDA(cudaMemcpyAsync(d_out_chunk_offsets, p.b.chunk_id_off, size_t(C + 1) * 8, cudaMemcpyDeviceToDevice,
                                h->stream));
     }
-    run_pack(h, p.b, mode, &launches);
+    run_pack(h, p.b, &launches);
     GTK_CUDA(cudaStreamSynchronize(h->stream));
     collect_stage_times(h);
     h->last_launches = launches;
@@ -1279,9 +1392,8 @@ GTK_API int gtk_encode(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
     if (h->wide && mode == GTK_MODE_LOCALMIN) return h->fail(GTK_ERR_TABLE, kWideNoLocalmin);
     if (!h->wide && mode == GTK_MODE_OPT && n_bytes <= gtk::kSmallMaxBytes && n_texts <= gtk::kSmallMaxTexts)
       return encode_host_small(h, bytes, text_offsets, n_texts, n_bytes, kernel_ms);
-    if (const int64_t C2 = two_launch_chunks(h, mode, text_offsets, n_texts, n_bytes); C2 >= 0)
-      return encode_host_two_launches(h, bytes, text_offsets, n_texts, n_bytes, C2, kernel_ms);
     if (n_bytes >= kSliceThresholdBytes) return encode_host_sliced(h, mode, bytes, text_offsets, n_texts, n_bytes, kernel_ms);
+    if (!h->wide && mode == GTK_MODE_OPT) return encode_host_tiles(h, bytes, text_offsets, n_texts, n_bytes, kernel_ms);
     cudaStream_t s = h->stream;
     h->d_bytes.reserve(size_t(n_bytes) + 32);
     h->d_text_off.reserve(size_t(n_texts + 1) * 8);
@@ -1298,14 +1410,13 @@ GTK_API int gtk_encode(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
                         reinterpret_cast<int32_t*>(dp + text_b + chunk_b), n_bytes,
                         reinterpret_cast<int64_t*>(dp + text_b), true);
     p.b.text_id_off = reinterpret_cast<int64_t*>(dp);
-    begin_call(h, mode, n_bytes);
     int launches = 0;
     // Up to 256 KiB of text a kernel behind the pack writes the results into mapped host memory and the host polls
     // its completion mark: no copy of the totals, no second copy sized by them, no stream synchronisation.
     const bool by_kernel = n_bytes <= kResultsByKernelMaxBytes &&
                            64 + text_b + chunk_b + size_t(n_bytes) * 4 + 64 <= kMappedResultBytes;
     run_front(h, p.b, mode, &launches, nullptr, nullptr, nullptr, true);
-    run_pack(h, p.b, mode, &launches, nullptr, nullptr, true, !by_kernel);
+    run_pack(h, p.b, &launches, nullptr, nullptr, true, !by_kernel);
     int64_t C = 0, N = 0;
     int status = gtk::kStatusOk;
     if (by_kernel) {

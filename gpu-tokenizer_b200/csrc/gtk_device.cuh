@@ -55,6 +55,16 @@ enum : int {
   kStatusBadOffsets = 4,  // caller-provided chunk offsets point outside the text or decrease
 };
 
+// Chunks and texts around a tile of the tile kernel.
+struct TileInfo {
+  int64_t c0, t0;  // chunks and texts that start in front of it
+  int32_t p0;      // position of the first chunk boundary of the text that runs into the tile, or kTileNoCut
+  int32_t flags;
+};
+constexpr int32_t kTileNoCut  = 0x40000000;
+constexpr int32_t kTilePlain  = 1;  // no text starts in the window (or there is only one): its cuts are p0 + i * chunk
+constexpr int32_t kTileRunsIn = 2;  // the last of the texts in front of the tile reaches into it
+
 struct EncodeBuffers {
   const uint8_t* bytes;      // input text, n_bytes
   int64_t n_bytes;
@@ -66,15 +76,19 @@ struct EncodeBuffers {
   int64_t* text_chunk_base;  // [n_texts+1] exclusive scan of chunks per text
   int64_t* chunk_off;        // [chunk_cap+1] start byte of each chunk, chunk_off[C] = n_bytes
   int64_t chunk_cap;         // upper bound on the number of chunks
-  int32_t* tile_chunk0;      // [n_tiles] chunk that contains the first byte of the tile
+  int32_t* tile_chunk0;      // [n_tiles] single-CTA kernel only: chunk that contains the first byte of the tile
   int64_t n_tiles;
   // merge outputs
   uint16_t* staging;         // [n_bytes] tokens of a unit, compacted at the unit's first byte
   int64_t* unit_first;       // [n_tiles] byte position where the unit's tokens start in staging (opt mode)
   int32_t* unit_cnt;         // [n_tiles] tokens produced by the unit (opt mode)
-  int32_t* chunk_cnt;        // [chunk_cap] tokens per chunk
+  int32_t* chunk_cnt;        // [chunk_cap] tokens per chunk (kernels that work chunk by chunk)
+  TileInfo* tile_info;       // [n_tiles] what starts where (tile kernel)
+  int32_t* chunk_rel;        // [chunk_cap] ids of its tile in front of a chunk
+  int32_t* text_rel;         // [n_texts] the same for the texts
+  int32_t* group_cnt;        // [n_tiles / kTileGroup + 1] ids per group of tiles (zero at the start)
+  int64_t* group_base;       // [n_tiles / kTileGroup + 2] the same, scanned
   // scan outputs
-  int64_t* unit_base;        // [n_tiles+1]
   int64_t* chunk_id_off;     // [chunk_cap+1] packed id offset of each chunk (caller visible)
   int64_t* text_id_off;      // [n_texts+1] or nullptr
   int64_t* chunk_id_mirror;  // single-CTA and finish kernels: device copy of chunk_id_off when that lives in host memory
@@ -88,13 +102,14 @@ struct EncodeBuffers {
   int32_t* staging32;        // [n_bytes] 32-bit kernel: tokens of a chunk, compacted at the chunk's first byte
   int64_t seg_scratch_tokens;  // tokens per CTA (two arrays of this length per CTA)
   int64_t* scan_block_sums;  // workspace of the multi-block scan
-  int32_t* counters;         // [0] tile ticket, [1] status word, [2] base-mode chunk ticket
+  int32_t* counters;         // [0] tile ticket, [1] status word, [2] chunk ticket, [8] CTAs done, [12..13] time the tile kernel began
   int64_t* totals;           // device: [0] n_chunks, [1] n_ids
 };
 
 // Launchers (all asynchronous on `stream`; return the number of kernels launched).
-// resets the call's counters and per-chunk counts and, when learned is given, the learned long table to the vocabulary's
-int launch_begin_batch(const EncodeBuffers& b, bool counters, const uint4* long_words, uint4* learned, cudaStream_t stream);
+// resets the call's counters and group counts and, when learned is given, the learned long table to the vocabulary's; for
+// medium batches without one also what launch_scan_texts does
+int launch_begin_batch(const EncodeBuffers& b, const uint4* long_words, uint4* learned, cudaStream_t stream);
 int launch_chunker(const EncodeBuffers& b, cudaStream_t stream);
 bool chunker_resets_counters(const EncodeBuffers& b);
 int launch_merge_opt(const EncodeBuffers& b, const DeviceTable& t, int grid, cudaStream_t stream);
@@ -103,18 +118,26 @@ int launch_merge_wide(const EncodeBuffers& b, const DeviceTable& t, int grid, cu
 int launch_pack_wide(const EncodeBuffers& b, int grid, cudaStream_t stream);
 int wide_kernel_max_blocks_per_sm();
 int launch_merge_localmin(const EncodeBuffers& b, const DeviceTable& t, int grid, int max_iters, cudaStream_t stream);
-int launch_output_scans(const EncodeBuffers& b, int mode_base, cudaStream_t stream);
-int launch_pack(const EncodeBuffers& b, int mode_base, int grid, cudaStream_t stream);
-// totals[0..1] and counters[0..3] to `mapped` (page-locked host memory as the device sees it), laid out as 4 x int64
-int launch_publish_totals(const EncodeBuffers& b, int64_t* mapped, cudaStream_t stream);
-// a batch of at most kFinishMaxTiles tiles with a host-made chunk table (chunk_off, tile_chunk0, text_chunk_base):
-// scans, pack and results into mapped host memory, then totals and the call number into mapped[0..3], in one launch
-// (one CTA per tile) behind the tile kernel; uses counters[8] (zero at the start of the call) and chunk_id_mirror
-int launch_finish_small_batch(const EncodeBuffers& b, int64_t* mapped, int64_t seq, cudaStream_t stream);
-// the device result arena of a single-piece batch into mapped host memory, then totals {n_chunks, n_ids, status} and,
+int launch_output_scans(const EncodeBuffers& b, cudaStream_t stream);
+// packs the ids of kernels that work chunk by chunk
+int launch_pack_chunks(const EncodeBuffers& b, int grid, cudaStream_t stream);
+// group_base from group_cnt for batches that are large enough for it (else nothing: returns 0)
+int launch_scan_groups(const EncodeBuffers& b, cudaStream_t stream);
+// tile_info from text_off and text_chunk_base
+int launch_tile_info(const EncodeBuffers& b, cudaStream_t stream);
+// text_chunk_base and totals[0] from text_off, for the tile kernel; nothing for one text, or when launch_begin_batch has
+// done it (learned: whether that was given a learned table): returns 0
+int launch_scan_texts(const EncodeBuffers& b, bool learned, cudaStream_t stream);
+// What follows the tile kernel: ids back to back, offsets of chunks and texts, totals[0] and [1].  publish: where the
+// host waits for the call, or nullptr: {n_chunks, n_ids, status, seq, nanoseconds since the tile kernel began}, seq last;
+// out_ids, chunk_id_off and text_id_off may then be page-locked host memory.  Uses counters[8] (zero at the start).
+int launch_pack_tiles(const EncodeBuffers& b, int sm_count, bool groups_scanned, int64_t* publish, int64_t seq, cudaStream_t stream);
+// the device result arena of a batch into mapped host memory, then totals {n_chunks, n_ids, status} and,
 // last, the call number into mapped[0..3]; uses counters[8] (zero at the start of the call)
 int launch_results_to_host(const EncodeBuffers& b, const void* src, void* dst, int64_t prefix_bytes, int64_t* mapped,
                            int64_t seq, cudaStream_t stream);
+// totals[0..1] and counters[0..3] to `mapped` (page-locked host memory as the device sees it), laid out as 4 x int64
+int launch_publish_totals(const EncodeBuffers& b, int64_t* mapped, cudaStream_t stream);
 // Whole pipeline in one single-CTA kernel for small batches; totals[0..2] receive n_chunks, n_ids, status,
 // totals[4] the kernel's own duration in nanoseconds and, as the very last store, totals[3] the call number.
 int launch_encode_small(const EncodeBuffers& b, const DeviceTable& t, cudaStream_t stream);
@@ -124,7 +147,7 @@ int launch_encode_small(const EncodeBuffers& b, const DeviceTable& t, cudaStream
 // two tiles one after the other in one CTA (57 us) still beat the two-launch path's 58..64 us; three (75 us) do not
 constexpr int64_t kSmallMaxBytes = GTK_SMALL_MAX_BYTES;
 constexpr int64_t kSmallMaxTexts = 1024;
-constexpr int kFinishMaxTiles = 32;  // batches through launch_finish_small_batch: at most this many tiles
+constexpr int kTileGroup = 64;  // tiles whose ids are counted together
 // What the allocation-free entry point needs from a handle (defined in gtk_api.cu).
 struct HandleView {
   int device;

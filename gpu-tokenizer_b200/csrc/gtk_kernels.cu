@@ -165,6 +165,13 @@ __device__ __forceinline__ bool adj_bit(const uint32_t* adj, uint32_t u, uint32_
   return (__ldg(adj + (((v >> 5) << 8) | u)) >> (v & 31u)) & 1u;
 }
 
+__device__ __forceinline__ unsigned long long global_timer()
+{
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
 __device__ __forceinline__ uint32_t lanemask_lt()
 {
   uint32_t m;
@@ -815,22 +822,6 @@ __global__ void k_chunk_fill(const int64_t* __restrict__ text_off, const int64_t
   }
 }
 
-// tile k -> chunk that contains byte k*kTile
-__global__ void k_tile_chunk0(const int64_t* __restrict__ chunk_off, const int64_t* __restrict__ n_chunks_ptr,
-                              int64_t n_tiles, int32_t* __restrict__ tile_chunk0)
-{
-  const int64_t C = *n_chunks_ptr;
-  for (int64_t k = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; k < n_tiles; k += int64_t(gridDim.x) * blockDim.x) {
-    const int64_t pos = k * kTile;
-    int64_t lo = 0, hi = C;  // last c with chunk_off[c] <= pos (chunk_off[0] == 0)
-    while (hi - lo > 1) {
-      const int64_t mid = (lo + hi) >> 1;
-      if (chunk_off[mid] <= pos) lo = mid; else hi = mid;
-    }
-    tile_chunk0[k] = int32_t(lo);
-  }
-}
-
 // ------------------------------------------------------------------------------------------------
 // merge kernel, segment-parallel ("opt")
 // ------------------------------------------------------------------------------------------------
@@ -860,34 +851,122 @@ __device__ __forceinline__ Span batch_span(const EncodeBuffers& b, int64_t k)
               lo > 0, lo == 0};
 }
 
-// start and end of the chunk that holds byte `at`; c0: a chunk at or before it
-__device__ __forceinline__ int64_t chunk_of(const EncodeBuffers& b, int64_t c0, int64_t C, int64_t at, int64_t* end)
+// first index in [0, n) whose value is not below x, n if there is none; one warp, 32 places per step
+__device__ __forceinline__ int64_t warp_lower_bound(const int64_t* v, int64_t n, int64_t x)
 {
-  int64_t c = c0;
-  while (c + 1 < C && b.chunk_off[c + 1] <= at) ++c;
-  *end = b.chunk_off[c + 1];
-  return c;
+  const int lane = threadIdx.x & 31;
+  int64_t lo = 0, hi = n;  // the answer is in [lo, hi]
+  while (hi > lo) {
+    const int64_t step = (hi - lo + 31) >> 5, i = lo + (lane + 1) * step - 1;
+    const int below    = __popc(__ballot_sync(0xFFFFFFFFu, i < hi && v[i] < x));
+    lo += below * step;
+    hi = min(hi, lo + step - 1);
+  }
+  return min(lo, n);
 }
 
-// One tile of a batch: tokenises every segment that starts in bytes [k*kTile, (k+1)*kTile), writes the tokens
-// compacted to staging, the unit record and the per-chunk counts.
-__device__ __forceinline__ void opt_tile(TileSmem<kOptThreads>& S, const EncodeBuffers& b, const DeviceTable& T, int64_t k,
-                                         int64_t C)
+// The tile records: one thread per tile.  The tile kernel would pay for the search and the divisions in every warp of every
+// tile (128 MiB: 710 us instead of 590).
+__global__ void __launch_bounds__(128) k_tile_info(EncodeBuffers b)
 {
+  const int64_t chunk = b.chunk_bytes;
+  for (int64_t k = int64_t(blockIdx.x) * 128 + threadIdx.x; k < b.n_tiles; k += int64_t(gridDim.x) * 128) {
+    const int64_t lo = k * kTile;
+    TileInfo i{0, 0, kTileNoCut, 0};
+    if (b.n_texts == 1) {
+      i.t0    = lo > 0;
+      i.c0    = (lo + chunk - 1) / chunk;
+      i.flags = kTilePlain | (lo > 0 ? kTileRunsIn : 0);
+      const int64_t p0 = i.c0 * chunk - lo;
+      if (p0 < kWindow && lo + p0 < b.n_bytes) i.p0 = int(p0);
+    } else {
+      int64_t a = 0, e = b.n_texts;  // first text that starts at or behind the tile's first byte
+      while (a < e) {
+        const int64_t mid = (a + e) >> 1;
+        if (b.text_off[mid] < lo) a = mid + 1; else e = mid;
+      }
+      const int64_t end = b.text_off[a];
+      i.t0 = a;
+      i.c0 = b.text_chunk_base[a];
+      if (a > 0 && end > lo) {
+        const int64_t s = b.text_off[a - 1], d = lo - s;
+        const int64_t n = d < (int64_t(1) << 31) ? int64_t((uint32_t(d) + uint32_t(chunk) - 1u) / uint32_t(chunk)) : (d + chunk - 1) / chunk;
+        const int64_t at = s + n * chunk;
+        i.flags = kTileRunsIn | (end >= min(lo + kWindow, b.n_bytes) ? kTilePlain : 0);
+        if (at < end) {
+          i.c0 = b.text_chunk_base[a - 1] + n;
+          if (at - lo < kWindow) i.p0 = int(at - lo);
+        }
+      }
+    }
+    b.tile_info[k] = i;
+  }
+}
+
+// Calls f(position, chunk number or -1, text number or -1) for everything that starts in window positions [0, limit): chunks
+// and texts (an empty text and the chunk behind it start at the same position, in calls of their own; the start of a batch's
+// only text is not reported).  The lanes of the calling warps share the texts between them, and the boundaries inside a text
+// that has more than a few in the window; `first`, `stride`: the calling warp's number and how many there are.
+template <class F>
+__device__ __forceinline__ void for_each_start(const EncodeBuffers& b, const TileInfo& ti, int64_t lo, int limit, int first,
+                                               int stride, F f)
+{
+  const int lane = threadIdx.x & 31;
+  const int step = min(b.chunk_bytes, 2 * kWindow);  // a longer one leaves the window just the same
+  if (ti.flags & kTilePlain) {
+    for (int i = first * 32 + lane; ti.p0 + i * step < limit; i += stride * 32) f(ti.p0 + i * step, ti.c0 + i, int64_t(-1));
+    return;
+  }
+  const int64_t t_lo = ti.t0 - ((ti.flags & kTileRunsIn) ? 1 : 0);
+  for (int64_t q0 = int64_t(first) * 32;; q0 += int64_t(stride) * 32) {
+    const int64_t t = t_lo + q0 + lane;
+    int at = kTileNoCut, end = 0;  // first boundary inside the text, where the text ends
+    int64_t c = 0;
+    bool more = false;
+    if (t < b.n_texts) {
+      const int64_t s = b.text_off[t];
+      more            = s < lo + limit;
+      if (more) {
+        const int64_t e = b.text_off[t + 1];
+        end = int(min(e - lo, int64_t(limit)));
+        if (s >= lo) {
+          c = b.text_chunk_base[t];
+          f(int(s - lo), e > s ? c : int64_t(-1), t);
+          at = int(s - lo) + step;
+          ++c;
+        } else {  // the text that runs in
+          at = ti.p0;
+          c  = ti.c0;
+        }
+      }
+    }
+    const bool many = at + 4 * step < end;
+    if (!many)
+      for (int p = at; p < end; p += step) f(p, c++, int64_t(-1));
+    for (uint32_t m = __ballot_sync(0xFFFFFFFFu, many); m; m &= m - 1) {
+      const int src    = __ffs(int(m)) - 1;
+      const int a0     = __shfl_sync(0xFFFFFFFFu, at, src), e0 = __shfl_sync(0xFFFFFFFFu, end, src);
+      const int64_t c0 = __shfl_sync(0xFFFFFFFFu, c, src);
+      for (int k = lane; a0 + k * step < e0; k += 32) f(a0 + k * step, c0 + k, int64_t(-1));
+    }
+    if (!__all_sync(0xFFFFFFFFu, more)) break;
+  }
+}
+
+// One tile of a batch: tokenises every segment that starts in bytes [k*kTile, (k+1)*kTile), writes the tokens compacted to
+// staging and what the pack kernel needs to know of the tile: number of ids, first chunk and text, and how many of its ids
+// stand in front of every chunk and text that starts in it.
+__device__ __forceinline__ void opt_tile(TileSmem<kOptThreads>& S, const EncodeBuffers& b, const DeviceTable& T, int64_t k)
+{
+  __shared__ uint16_t woff[TileSmem<kOptThreads>::kWords];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int* status   = b.counters + 1;
   const Span sp = batch_span(b, k);
 #ifdef GTK_PHASE_TIMING
   long long phase_t0 = clock64();
 #endif
-  const int64_t c0 = b.tile_chunk0[k];
-  tile_cut(S, sp, T, [&](auto mark) {
-    for (int64_t c = c0 + lane; c <= C; c += 32) {
-      const int64_t p = b.chunk_off[c] - sp.lo;
-      if (p >= sp.wlen) break;
-      if (p >= 0) mark(int(p));
-    }
-  });
+  const TileInfo ti = b.tile_info[k];
+  tile_cut(S, sp, T, [&](auto mark) { for_each_start(b, ti, sp.lo, sp.wlen, 0, 1, [&](int p, int64_t, int64_t) { mark(p); }); });
   GTK_PHASE(0);
   tile_lookup(S, sp, T, status);
   GTK_PHASE(1);
@@ -897,7 +976,7 @@ __device__ __forceinline__ void opt_tile(TileSmem<kOptThreads>& S, const EncodeB
   tile_merge(S, T, ws, b.seg_scratch_tokens, status);
   GTK_PHASE(2);
   const int64_t region_start = sp.lo + min(first, sp.wlen);
-  tile_emit<kOptThreads, false>(S, first, end, nullptr, [&](int off, const uint16_t* ids, int n) {
+  tile_emit<kOptThreads, true>(S, first, end, woff, [&](int off, const uint16_t* ids, int n) {
     uint16_t* dst = b.staging + region_start + off;
     for (int j = lane; j < n; j += 32)
       if (GTK_IN(region_start + off + j, b.n_bytes, 22)) dst[j] = ids[j];
@@ -906,38 +985,28 @@ __device__ __forceinline__ void opt_tile(TileSmem<kOptThreads>& S, const EncodeB
   GTK_PHASE(3);
   const int total = S.total;
   if (S.no_space && tid == 0) atomicMax(status, int(kStatusScratchTooSmall));
+  // ids of the tile in front of every chunk and text that starts in it (a chunk start is a segment start, so it lies inside
+  // the owned region, or is the start of the oversize segment right behind it)
+  for_each_start(b, ti, sp.lo, sp.own_hi, warp, kOptThreads / 32, [&](int p, int64_t c, int64_t t) {
+    const int rel = woff[p >> 5] + __popc(S.cut[p >> 5] & range_mask(p & ~31, first, end) & ((1u << (p & 31)) - 1u));
+    if (c >= 0 && GTK_IN(c, b.chunk_cap, 24)) b.chunk_rel[c] = rel;
+    if (t >= 0 && GTK_IN(t, b.n_texts, 25)) b.text_rel[t] = rel;
+  });
   GTK_PHASE(4);
-  // per-chunk token counts from the bitmap of live tokens
-  const int64_t region_end = sp.lo + end;
-  if (c0 < C && region_end <= b.chunk_off[c0 + 1]) {
-    // the owned region lies inside the chunk that holds the tile's first byte (CTA-uniform test): the tile's total
-    if (tid == 0 && total > 0 && GTK_IN(c0, b.chunk_cap, 24)) atomicAdd(b.chunk_cnt + c0, total);
-  } else {
-    for (int64_t c = c0 + warp; c < C; c += kOptThreads / 32) {
-      const int64_t cs_g = b.chunk_off[c];
-      if (cs_g >= region_end) break;
-      const int cs = int(max(cs_g, region_start) - sp.lo);
-      const int ce = int(min(b.chunk_off[c + 1], region_end) - sp.lo);
-      if (ce <= cs) continue;
-      int cnt = 0;
-      for (int w = (cs >> 5) + lane; w <= ((ce - 1) >> 5); w += 32) cnt += __popc(S.cut[w] & range_mask(w * 32, cs, ce));
-      cnt = __reduce_add_sync(0xFFFFFFFFu, cnt);
-      if (lane == 0 && cnt && GTK_IN(c, b.chunk_cap, 25)) atomicAdd(b.chunk_cnt + c, cnt);
-    }
-  }
   int over = 0;
   if (S.over_start >= 0) {  // CTA-uniform, rare
     const int64_t start = sp.lo + S.over_start;
-    int64_t cend;
-    const int64_t c = chunk_of(b, c0, C, start, &cend);
+    const int64_t t     = b.n_texts == 1 ? 0 : warp_lower_bound(b.text_off, b.n_texts, start + 1) - 1;  // text that holds it
+    const int64_t s     = b.n_texts == 1 ? 0 : b.text_off[t], e = b.n_texts == 1 ? b.n_bytes : b.text_off[t + 1];
+    const int64_t cend  = min(e, s + ((start - s) / b.chunk_bytes + 1) * b.chunk_bytes);
     over = merge_oversize<kOptThreads>(b.bytes, start, sp.lo + kWindow, cend, ws, b.seg_scratch_tokens, T, status);
     for (int j = tid; j < over; j += kOptThreads)
       if (GTK_IN(region_start + total + j, b.n_bytes, 26)) b.staging[region_start + total + j] = ws[j];
-    if (tid == 0 && over > 0 && GTK_IN(c, b.chunk_cap, 27)) atomicAdd(b.chunk_cnt + c, over);
   }
   if (tid == 0) {
     b.unit_first[k] = region_start;
     b.unit_cnt[k]   = total + over;
+    atomicAdd(b.group_cnt + k / kTileGroup, total + over);
   }
   GTK_PHASE(5);
 }
@@ -953,15 +1022,15 @@ __device__ __forceinline__ void opt_tile(TileSmem<kOptThreads>& S, const EncodeB
 __global__ void __launch_bounds__(kOptThreads, GTK_OPT_CTAS) k_merge_opt(EncodeBuffers b, const __grid_constant__ DeviceTable T)
 {
   TileSmem<kOptThreads>& S = tile_smem<kOptThreads>();
-  const int64_t C = b.totals[0];
   tile_setup(S);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long*>(b.counters + 12) = global_timer();
   int64_t k = blockIdx.x;  // the first tile of every CTA, the others by ticket
   while (k < b.n_tiles) {
     int next = 0;
     if (threadIdx.x == 0) next = atomicAdd(b.counters + 0, 1);  // on its way while the tile is worked on
     tile_reset(S);
     __syncthreads();
-    opt_tile(S, b, T, k, C);
+    opt_tile(S, b, T, k);
     if (threadIdx.x == 0) S.ticket = next;
     __syncthreads();
     k = int64_t(gridDim.x) + S.ticket;
@@ -1058,17 +1127,13 @@ __global__ void __launch_bounds__(kMediumThreads) k_chunker_medium(EncodeBuffers
 #endif
   if (tid == 0) b.totals[0] = C;
   if (per_text) {
-    // many short texts: every text writes the offsets of its own chunks and the first chunk of every tile that
-    // starts inside one of them (no search); a thread takes the texts of up to 32 chunks, a warp the longer ones.
+    // many short texts: every text writes the offsets of its own chunks (no search); a thread takes the texts of up to
+    // 32 chunks, a warp the longer ones.
     // A medium batch has at most 2048 tiles, so byte offsets and chunk numbers fit 32 bits.
     constexpr int kLongTexts = 128;
     __shared__ int n_long;
     __shared__ int long_text[kLongTexts];
     const uint32_t cb = uint32_t(b.chunk_bytes);
-    auto lay_chunk = [&](uint32_t c, uint32_t start, uint32_t end) {  // chunk c covers bytes [start, end)
-      b.chunk_off[c] = start;
-      for (uint32_t k = (start + kTile - 1) / kTile; k * kTile < end; ++k) b.tile_chunk0[k] = int32_t(c);
-    };
     if (tid == 0) {
       b.chunk_off[C] = b.text_off[b.n_texts];
       n_long         = 0;
@@ -1076,11 +1141,11 @@ __global__ void __launch_bounds__(kMediumThreads) k_chunker_medium(EncodeBuffers
     __syncthreads();
     for (int64_t t = tid; t < b.n_texts; t += kMediumThreads) {
       const uint32_t c0 = uint32_t(b.text_chunk_base[t]), nc = uint32_t(b.text_chunk_base[t + 1]) - c0;
-      const uint32_t at = uint32_t(b.text_off[t]), to = uint32_t(b.text_off[t + 1]);
+      const uint32_t at = uint32_t(b.text_off[t]);
       if (nc == 1) {
-        lay_chunk(c0, at, to);
+        b.chunk_off[c0] = at;
       } else if (nc <= 32) {
-        for (uint32_t c = 0; c < nc; ++c) lay_chunk(c0 + c, at + c * cb, min(at + (c + 1) * cb, to));
+        for (uint32_t c = 0; c < nc; ++c) b.chunk_off[c0 + c] = at + c * cb;
       } else {
         const int q = atomicAdd(&n_long, 1);
         if (q < kLongTexts) long_text[q] = int(t);
@@ -1095,8 +1160,8 @@ __global__ void __launch_bounds__(kMediumThreads) k_chunker_medium(EncodeBuffers
       for (int q = warp; q < n_long; q += kMediumThreads / 32) {
         const int64_t t   = long_text[q];
         const uint32_t cc = uint32_t(b.text_chunk_base[t]), nn = uint32_t(b.text_chunk_base[t + 1]) - cc;
-        const uint32_t at = uint32_t(b.text_off[t]), to = uint32_t(b.text_off[t + 1]);
-        for (uint32_t c = lane; c < nn; c += 32) lay_chunk(cc + c, at + c * cb, min(at + (c + 1) * cb, to));
+        const uint32_t at = uint32_t(b.text_off[t]);
+        for (uint32_t c = lane; c < nn; c += 32) b.chunk_off[cc + c] = at + c * cb;
       }
       return;
     }
@@ -1107,8 +1172,8 @@ __global__ void __launch_bounds__(kMediumThreads) k_chunker_medium(EncodeBuffers
       for (uint32_t m = __ballot_sync(0xFFFFFFFFu, nc > 32); m; m &= m - 1) {
         const int src     = __ffs(int(m)) - 1;
         const uint32_t cc = __shfl_sync(0xFFFFFFFFu, c0, src), nn = __shfl_sync(0xFFFFFFFFu, nc, src);
-        const uint32_t at = uint32_t(b.text_off[t0 + src]), to = uint32_t(b.text_off[t0 + src + 1]);
-        for (uint32_t c = lane; c < nn; c += 32) lay_chunk(cc + c, at + c * cb, min(at + (c + 1) * cb, to));
+        const uint32_t at = uint32_t(b.text_off[t0 + src]);
+        for (uint32_t c = lane; c < nn; c += 32) b.chunk_off[cc + c] = at + c * cb;
       }
     }
     return;
@@ -1126,19 +1191,34 @@ __global__ void __launch_bounds__(kMediumThreads) k_chunker_medium(EncodeBuffers
       b.chunk_off[c] = b.text_off[lo] + (c - b.text_chunk_base[lo]) * int64_t(b.chunk_bytes);
     }
   }
-  __syncthreads();
-  for (int64_t k = tid; k < b.n_tiles; k += kMediumThreads) {
-    const int64_t pos = k * kTile;
-    int64_t lo = 0, hi = C;  // last c with chunk_off[c] <= pos
-    while (hi - lo > 1) {
-      const int64_t mid = (lo + hi) >> 1;
-      if (b.chunk_off[mid] <= pos) lo = mid; else hi = mid;
-    }
-    b.tile_chunk0[k] = int32_t(lo);
-  }
 }
 
-__global__ void __launch_bounds__(kMediumThreads) k_scans_medium(EncodeBuffers b, int with_units)
+// ids per group of tiles, scanned (group_base), for large batches
+__global__ void __launch_bounds__(kMediumThreads) k_scan_groups(EncodeBuffers b)
+{
+  __shared__ int scanbuf[33];
+  __shared__ int64_t carry_s;
+  __shared__ __align__(16) int stage[4 * kMediumThreads];
+  cta_exclusive_scan_medium(CountsI32{b.group_cnt}, b.n_tiles / kTileGroup + 1, b.group_base, scanbuf, &carry_s, stage);
+}
+
+// chunks per text, scanned (totals[0], text_chunk_base), for the tile kernel; reset: the call's counters and group counts too
+__global__ void __launch_bounds__(kMediumThreads) k_scan_texts_medium(EncodeBuffers b, int reset)
+{
+  if (reset) {
+    if (threadIdx.x < 16) b.counters[threadIdx.x] = 0;
+    for (int64_t i = threadIdx.x; i <= b.n_tiles / kTileGroup; i += kMediumThreads) b.group_cnt[i] = 0;
+    if (b.n_texts == 1) return;
+  }
+  __shared__ int scanbuf[33];
+  __shared__ int64_t carry_s;
+  __shared__ __align__(16) int stage[4 * kMediumThreads];
+  const int64_t C = cta_exclusive_scan_medium(ChunksPerText{b.text_off, b.chunk_bytes}, b.n_texts, b.text_chunk_base,
+                                              scanbuf, &carry_s, stage);
+  if (threadIdx.x == 0) b.totals[0] = C;
+}
+
+__global__ void __launch_bounds__(kMediumThreads) k_scans_medium(EncodeBuffers b)
 {
   __shared__ int scanbuf[33];
   __shared__ int64_t carry_s;
@@ -1147,7 +1227,6 @@ __global__ void __launch_bounds__(kMediumThreads) k_scans_medium(EncodeBuffers b
   const int64_t C = b.totals[0];
   const int64_t N = cta_exclusive_scan_medium(CountsI32{b.chunk_cnt}, C, b.chunk_id_off, scanbuf, &carry_s, stage);
   if (tid == 0) b.totals[1] = N;
-  if (with_units) cta_exclusive_scan_medium(CountsI32{b.unit_cnt}, b.n_tiles, b.unit_base, scanbuf, &carry_s, stage);
   if (b.text_id_off)
     for (int64_t t = tid; t <= b.n_texts; t += kMediumThreads) b.text_id_off[t] = b.chunk_id_off[b.text_chunk_base[t]];
 }
@@ -1188,8 +1267,9 @@ __device__ __forceinline__ void small_tile(TileSmem<kOptThreads>& S, const Encod
   const uint16_t* over_ids = nullptr;
   if (S.over_start >= 0) {  // CTA-uniform
     const int64_t start = sp.lo + S.over_start;
-    int64_t cend;
-    chunk_of(b, c0, C, start, &cend);
+    int64_t c = c0;
+    while (c + 1 < C && b.chunk_off[c + 1] <= start) ++c;
+    const int64_t cend = b.chunk_off[c + 1];
     over_ids = b.seg_scratch;
     over = merge_oversize<kOptThreads>(b.bytes, start, sp.lo + kWindow, cend, b.seg_scratch, b.seg_scratch_tokens, T, status);
   }
@@ -1562,51 +1642,139 @@ __global__ void __launch_bounds__(kBaseThreads) k_merge_localmin(EncodeBuffers b
 // ------------------------------------------------------------------------------------------------
 // output: pack staged 16-bit tokens of every unit into the int32 id buffer
 // ------------------------------------------------------------------------------------------------
-// One warp per unit (a tile's or a chunk's compacted tokens): the ids of a unit are written in groups of
-// four as one 16-byte store once the destination is aligned; the 16-bit source tokens are read through L1.
-__global__ void __launch_bounds__(256) k_pack(const uint16_t* __restrict__ staging, const int64_t* __restrict__ first,
-                                              const int32_t* __restrict__ cnt, const int64_t* __restrict__ base,
-                                              int64_t n_units_imm, const int64_t* n_units_ptr,
-                                              int32_t* __restrict__ out, int64_t capacity,
-                                              const uint16_t* __restrict__ low_id_map)
+// A run of m tokens at sp -> ids at dp, by `stride` lanes of which this is number `lane`: groups of four as one 16-byte store
+// once the destination is aligned, sixteen 16-bit loads in flight per lane and trip.
+template <class Conv>
+__device__ __forceinline__ void pack_run(const uint16_t* sp, int32_t* dp, int m, int lane, int stride, Conv conv)
 {
-  const int64_t U    = n_units_ptr ? *n_units_ptr : n_units_imm;
+  const int head = min(m, int(((16u - uint32_t(reinterpret_cast<uintptr_t>(dp) & 15u)) >> 2) & 3u));
+  if (lane < head) dp[lane] = conv(sp[lane]);
+  const int quads = (m - head) >> 2;
+  for (int q0 = lane; q0 < quads; q0 += 4 * stride) {
+    uint32_t t[4][4];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const int q = q0 + stride * g;
+      if (q < quads) {
+        const uint16_t* s4 = sp + head + 4 * q;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) t[g][e] = s4[e];
+      }
+    }
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const int q = q0 + stride * g;
+      if (q < quads)
+        *reinterpret_cast<int4*>(dp + head + 4 * q) = make_int4(conv(t[g][0]), conv(t[g][1]), conv(t[g][2]), conv(t[g][3]));
+    }
+  }
+  const int done = head + 4 * quads;
+  if (done + lane < m) dp[done + lane] = conv(sp[done + lane]);
+}
+
+// One warp per chunk of the kernels that work chunk by chunk.
+__global__ void __launch_bounds__(256) k_pack_chunks(const uint16_t* __restrict__ staging, const int64_t* __restrict__ first,
+                                                     const int32_t* __restrict__ cnt, const int64_t* __restrict__ base,
+                                                     const int64_t* n_units_ptr, int32_t* __restrict__ out, int64_t capacity,
+                                                     const uint16_t* __restrict__ low_id_map)
+{
+  const int64_t U    = *n_units_ptr;
   const int lane     = threadIdx.x & 31;
   const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw   = (int64_t(gridDim.x) * blockDim.x) >> 5;
   for (int64_t u = warp; u < U; u += nw) {
-    const int64_t src = first[u], dst = base[u];
-    int64_t m = cnt[u];
-    if (dst + m > capacity) m = capacity > dst ? capacity - dst : 0;
-    const uint16_t* sp = staging + src;
-    int32_t* dp        = out + dst;
-    auto conv = [&](uint32_t t) { return int32_t((low_id_map && t < 256u) ? uint32_t(__ldg(low_id_map + t)) : t); };
-    // head: up to three ids until the destination is 16-byte aligned
-    const int64_t head = min(m, int64_t(((16u - uint32_t(reinterpret_cast<uintptr_t>(dp) & 15u)) >> 2) & 3u));
-    if (lane < head) dp[lane] = conv(sp[lane]);
-    const int64_t quads = (m - head) >> 2;
-    // four groups of four tokens per lane and trip: sixteen independent 16-bit loads in flight before the first
-    // store, because this kernel lives on memory latency (one warp per unit, nothing to overlap with)
-    for (int64_t q0 = lane; q0 < quads; q0 += 128) {
-      uint32_t t[4][4];
+    const int64_t dst = base[u];
+    pack_run(staging + first[u], out + dst, int(min(int64_t(cnt[u]), max(capacity - dst, int64_t(0)))), lane, 32,
+             [&](uint32_t t) { return int32_t((low_id_map && t < 256u) ? uint32_t(__ldg(low_id_map + t)) : t); });
+  }
+}
+
+// Everything behind the tile kernel.  A CTA packs a run of tiles, its warps one tile each, or (kWhole, for batches that leave
+// the chip idle otherwise) all of them one tile together.  Where its first tile's ids go is a sum over the counts of the
+// tile groups in front and of the tiles in front within the group, which every CTA forms for itself; for large batches
+// (a thousand groups at 256 MiB) k_scan_groups has formed the former.  The offsets of the chunks and texts that start in a tile are the tile's place plus
+// what the tile kernel has counted.  Bound by the latency of the staged tokens and by the stores.
+template <bool kWhole>
+__global__ void __launch_bounds__(256) k_pack_tiles(EncodeBuffers b, int64_t per_cta, int groups_scanned, int64_t* publish,
+                                                    int64_t seq)
+{
+  constexpr int kWarps = 8;
+  __shared__ int64_t warp_sum[kWarps];
+  __shared__ int last;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t K = b.n_tiles, a = min(int64_t(blockIdx.x) * per_cta, K), e = min(a + per_cta, K);
+  const uint16_t* map = b.low_id_map;
+  auto conv = [&](uint32_t t) { return int32_t((map && t < 256u) ? uint32_t(__ldg(map + t)) : t); };
+  const int64_t C = b.n_texts == 1 ? (b.n_bytes + b.chunk_bytes - 1) / b.chunk_bytes : b.totals[0];
+  if (a < e) {
+    const int64_t g = a / kTileGroup;
+    int64_t sum     = 0;
+    if (groups_scanned) {
+      if (tid == 0) sum = b.group_base[g];
+    } else {
+      for (int64_t i = tid; i < g; i += 256) sum += b.group_cnt[i];
+    }
+    for (int64_t i = g * kTileGroup + tid; i < a; i += 256) sum += b.unit_cnt[i];
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        const int64_t q = q0 + 32 * g;
-        if (q < quads) {
-          const uint16_t* s4 = sp + head + 4 * q;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) t[g][e] = s4[e];
+    for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, d);
+    if (lane == 0) warp_sum[warp] = sum;
+    __syncthreads();
+    int64_t base = 0;
+    for (int w = 0; w < kWarps; ++w) base += warp_sum[w];
+    constexpr int kStep = kWhole ? 1 : kWarps;
+    for (int64_t k0 = a; k0 < e; k0 += kStep) {
+      const int mine = kWhole ? 0 : warp;
+      const int cnt  = (lane < kStep && k0 + lane < e) ? b.unit_cnt[k0 + lane] : 0;
+      const int m    = __shfl_sync(0xFFFFFFFFu, cnt, mine);
+      const int64_t k = k0 + mine, dst = base + __reduce_add_sync(0xFFFFFFFFu, lane < mine ? cnt : 0);
+      base += __reduce_add_sync(0xFFFFFFFFu, cnt);
+      if (k >= e) continue;
+      const int l = kWhole ? tid : lane;
+      constexpr int kStride = kWhole ? 256 : 32;
+      pack_run(b.staging + b.unit_first[k], b.out_ids + dst, int(min(int64_t(m), max(b.out_capacity - dst, int64_t(0)))), l,
+               kStride, conv);
+      const bool end    = k == K - 1;
+      const int64_t c_e = end ? C : b.tile_info[k + 1].c0;
+      for (int64_t c = b.tile_info[k].c0 + l; c < c_e; c += kStride) b.chunk_id_off[c] = dst + b.chunk_rel[c];
+      if (b.text_id_off) {
+        const int64_t t_e = end ? b.n_texts : b.tile_info[k + 1].t0;
+        for (int64_t t = b.tile_info[k].t0 + l; t < t_e; t += kStride) {
+          if (b.n_texts == 1) {
+            b.text_id_off[0] = 0;
+          } else {
+            const bool behind = end && b.text_off[t] >= b.n_bytes;  // an empty text behind all bytes
+            b.text_id_off[t]  = behind ? dst + m : dst + b.text_rel[t];
+          }
         }
       }
-#pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        const int64_t q = q0 + 32 * g;
-        if (q < quads)
-          *reinterpret_cast<int4*>(dp + head + 4 * q) = make_int4(conv(t[g][0]), conv(t[g][1]), conv(t[g][2]), conv(t[g][3]));
+      if (end && l == 0) {
+        b.chunk_id_off[C] = dst + m;
+        if (b.text_id_off) b.text_id_off[b.n_texts] = dst + m;
+        b.totals[0] = C;
+        b.totals[1] = dst + m;
       }
     }
-    const int64_t done = head + 4 * quads;
-    if (done + lane < m) dp[done + lane] = conv(sp[done + lane]);
+  }
+  if (K == 0) {  // texts without a byte
+    if (b.text_id_off)
+      for (int64_t t = tid; t <= b.n_texts; t += 256) b.text_id_off[t] = 0;
+    if (tid == 0) b.chunk_id_off[0] = b.totals[0] = b.totals[1] = 0;
+  }
+  if (!publish) return;
+  // The CTA that finishes last (a counter, no waiting) tells the host, which may be polling the call number: the last store,
+  // behind a system-wide fence.
+  __threadfence_system();
+  __syncthreads();
+  if (tid == 0) last = atomicAdd(b.counters + 8, 1) == int(gridDim.x) - 1;
+  __syncthreads();
+  if (last && tid == 0) {
+    __threadfence();
+    publish[0] = C;
+    publish[1] = *reinterpret_cast<volatile int64_t*>(b.totals + 1);
+    publish[2] = int64_t(*reinterpret_cast<volatile int32_t*>(b.counters + 1));
+    publish[4] = int64_t(global_timer() - *reinterpret_cast<volatile unsigned long long*>(b.counters + 12));
+    __threadfence_system();
+    *reinterpret_cast<volatile int64_t*>(publish + 3) = seq;
   }
 }
 
@@ -1635,7 +1803,7 @@ inline unsigned grid_for(int64_t items, int threads, int64_t cap = 65535)
 // searches (one per chunk and one per tile) are latency-bound in a single CTA and only pay while there are few.
 static bool medium_scans(const EncodeBuffers& b)
 {
-  return b.n_texts <= kMediumMaxItems && b.chunk_cap <= kMediumMaxItems && b.n_tiles <= kMediumMaxItems;
+  return b.n_texts <= kMediumMaxItems && b.chunk_cap <= kMediumMaxItems;
 }
 // The single-CTA chunker finds the text of every chunk by binary search, which is cheap for a few texts and a few
 // thousand chunks; a batch of many short texts (no more chunk-sized pieces than texts) is laid out per text instead.
@@ -1655,14 +1823,13 @@ bool chunker_resets_counters(const EncodeBuffers& b)
   return medium_chunker_by_search(b) || medium_chunker_per_text(b);
 }
 
-// One launch instead of two memsets and a device-to-device copy, which take the stream 13 us: 8 MiB in L2 or HBM each way.
-__global__ void __launch_bounds__(512) k_begin_batch(int32_t* counters, int32_t* chunk_cnt, int64_t n_cnt,
+// One launch instead of memsets and a device-to-device copy, which take the stream 13 us: 8 MiB in L2 or HBM each way.
+__global__ void __launch_bounds__(512) k_begin_batch(int32_t* counters, int32_t* group_cnt, int64_t n_groups,
                                                      const uint4* __restrict__ from, uint4* __restrict__ to, int n_words)
 {
   const int i0 = blockIdx.x * 512 + threadIdx.x, step = gridDim.x * 512;
-  if (counters && i0 < 16) counters[i0] = 0;
-  if (chunk_cnt)
-    for (int64_t i = i0; i < n_cnt; i += step) chunk_cnt[i] = 0;
+  if (i0 < 16) counters[i0] = 0;
+  for (int64_t i = i0; i < n_groups; i += step) group_cnt[i] = 0;
   if (to)
     for (int i = i0; i < n_words; i += 4 * step) {
       uint4 v[4];
@@ -1675,11 +1842,55 @@ __global__ void __launch_bounds__(512) k_begin_batch(int32_t* counters, int32_t*
     }
 }
 
-int launch_begin_batch(const EncodeBuffers& b, bool counters, const uint4* long_words, uint4* learned, cudaStream_t stream)
+static bool medium_batch(const EncodeBuffers& b) { return medium_chunker_by_search(b) || medium_chunker_per_text(b); }
+
+int launch_begin_batch(const EncodeBuffers& b, const uint4* long_words, uint4* learned, cudaStream_t stream)
 {
-  const int grid = learned ? 256 : grid_for(b.chunk_cap + 1, 512 * 4, 296);  // 256 CTAs: four words of the table per thread
-  k_begin_batch<<<grid, 512, 0, stream>>>(counters ? b.counters : nullptr, counters ? b.chunk_cnt : nullptr, b.chunk_cap + 1,
-                                          long_words, learned, learned ? 2 << kLongBits : 0);
+  if (medium_batch(b) && !learned) {
+    k_scan_texts_medium<<<1, kMediumThreads, 0, stream>>>(b, 1);
+    return 1;
+  }
+  const int64_t n_groups = b.n_tiles / kTileGroup + 1;
+  const int grid = learned ? 256 : grid_for(n_groups, 512, 256);  // 256 CTAs: four words of the table per thread
+  k_begin_batch<<<grid, 512, 0, stream>>>(b.counters, b.group_cnt, n_groups, long_words, learned, learned ? 2 << kLongBits : 0);
+  return 1;
+}
+
+int launch_scan_texts(const EncodeBuffers& b, bool learned, cudaStream_t stream)
+{
+  if (b.n_texts == 1 || (medium_batch(b) && !learned)) return 0;
+  if (b.n_texts <= kMediumMaxItems && b.chunk_cap < (int64_t(1) << 30)) {  // its sums are 32 bits wide
+    k_scan_texts_medium<<<1, kMediumThreads, 0, stream>>>(b, 0);
+    return 1;
+  }
+  return run_scan(ChunksPerText{b.text_off, b.chunk_bytes}, b.n_texts, b.n_texts, nullptr, b.scan_block_sums,
+                  b.text_chunk_base, b.totals + 0, stream);
+}
+
+int launch_tile_info(const EncodeBuffers& b, cudaStream_t stream)
+{
+  if (b.n_tiles <= 0) return 0;
+  k_tile_info<<<grid_for(b.n_tiles, 128, 4096), 128, 0, stream>>>(b);
+  return 1;
+}
+
+// Medium batches: the pack kernel sums the group counts itself; beyond that one more launch does it once.
+int launch_scan_groups(const EncodeBuffers& b, cudaStream_t stream)
+{
+  if (medium_batch(b)) return 0;
+  k_scan_groups<<<1, kMediumThreads, 0, stream>>>(b);
+  return 1;
+}
+
+int launch_pack_tiles(const EncodeBuffers& b, int sm_count, bool groups_scanned, int64_t* publish, int64_t seq, cudaStream_t stream)
+{
+  // up to eight tiles per SM: a CTA for each, so that its 256 threads share the tile's 1400 ids
+  if (b.n_tiles <= int64_t(sm_count) * 8) {
+    k_pack_tiles<true><<<unsigned(std::max<int64_t>(b.n_tiles, 1)), 256, 0, stream>>>(b, 1, groups_scanned, publish, seq);
+    return 1;
+  }
+  const int64_t ctas = int64_t(sm_count) * 8, per = ((b.n_tiles + ctas - 1) / ctas + 7) & ~int64_t(7);
+  k_pack_tiles<false><<<unsigned((b.n_tiles + per - 1) / per), 256, 0, stream>>>(b, per, groups_scanned, publish, seq);
   return 1;
 }
 
@@ -1693,13 +1904,7 @@ int launch_chunker(const EncodeBuffers& b, cudaStream_t stream)
                           b.scan_block_sums, b.text_chunk_base, b.totals + 0, stream);
   k_chunk_fill<<<grid_for(b.chunk_cap + 1, 256, 2048), 256, 0, stream>>>(b.text_off, b.text_chunk_base, b.n_texts,
                                                                          b.chunk_bytes, b.chunk_off);
-  ++launches;
-  if (b.n_tiles > 0) {
-    k_tile_chunk0<<<grid_for(b.n_tiles, 256, 2048), 256, 0, stream>>>(b.chunk_off, b.totals + 0, b.n_tiles,
-                                                                      b.tile_chunk0);
-    ++launches;
-  }
-  return launches;
+  return launches + 1;
 }
 
 int launch_merge_opt(const EncodeBuffers& b, const DeviceTable& t, int grid, cudaStream_t stream)
@@ -1785,20 +1990,15 @@ int launch_merge_localmin(const EncodeBuffers& b, const DeviceTable& t, int grid
   return 1;
 }
 
-int launch_output_scans(const EncodeBuffers& b, int mode_base, cudaStream_t stream)
+int launch_output_scans(const EncodeBuffers& b, cudaStream_t stream)
 {
   if (medium_scans(b)) {
-    k_scans_medium<<<1, kMediumThreads, 0, stream>>>(b, (!mode_base && b.n_tiles > 0) ? 1 : 0);
+    k_scans_medium<<<1, kMediumThreads, 0, stream>>>(b);
     return 1;
   }
-  int launches = 0;
   // per-chunk counts -> packed id offset of every chunk (+ total id count)
-  launches += run_scan(CountsI32{b.chunk_cnt}, b.chunk_cap, 0, b.totals + 0, b.scan_block_sums, b.chunk_id_off,
-                       b.totals + 1, stream);
-  if (!mode_base && b.n_tiles > 0) {
-    launches += run_scan(CountsI32{b.unit_cnt}, b.n_tiles, b.n_tiles, nullptr, b.scan_block_sums, b.unit_base,
-                         nullptr, stream);
-  }
+  int launches = run_scan(CountsI32{b.chunk_cnt}, b.chunk_cap, 0, b.totals + 0, b.scan_block_sums, b.chunk_id_off,
+                          b.totals + 1, stream);
   if (b.text_id_off) {
     k_text_id_off<<<grid_for(b.n_texts + 1, 256, 2048), 256, 0, stream>>>(b.text_chunk_base, b.chunk_id_off,
                                                                           b.n_texts, b.text_id_off);
@@ -1807,16 +2007,11 @@ int launch_output_scans(const EncodeBuffers& b, int mode_base, cudaStream_t stre
   return launches;
 }
 
-int launch_pack(const EncodeBuffers& b, int mode_base, int grid, cudaStream_t stream)
+int launch_pack_chunks(const EncodeBuffers& b, int grid, cudaStream_t stream)
 {
   if (b.n_bytes <= 0) return 0;
-  if (mode_base) {
-    k_pack<<<grid, 256, 0, stream>>>(b.staging, b.chunk_off, b.chunk_cnt, b.chunk_id_off, 0, b.totals + 0, b.out_ids,
-                                     b.out_capacity, b.low_id_map);
-  } else {
-    k_pack<<<grid, 256, 0, stream>>>(b.staging, b.unit_first, b.unit_cnt, b.unit_base, b.n_tiles, nullptr, b.out_ids,
-                                     b.out_capacity, b.low_id_map);
-  }
+  k_pack_chunks<<<grid, 256, 0, stream>>>(b.staging, b.chunk_off, b.chunk_cnt, b.chunk_id_off, b.totals + 0, b.out_ids,
+                                          b.out_capacity, b.low_id_map);
   return 1;
 }
 
@@ -1904,68 +2099,6 @@ __global__ void __launch_bounds__(256) k_results_to_host(const uint4* __restrict
     __threadfence_system();
     *reinterpret_cast<volatile int64_t*>(mapped + 3) = seq;
   }
-}
-
-// A batch of a few tiles whose chunk table the host has laid out (chunk_off, tile_chunk0, text_chunk_base):
-// everything behind the tile kernel in one launch, one CTA per tile -- the CTA packs its tile's token run into int32
-// ids (the runs' offsets are a sum over at most kFinishMaxTiles counts, which every CTA forms for itself), CTA 0
-// also scans the per-chunk counts into id offsets (into chunk_id_mirror in HBM, then out) and writes the texts' id
-// offsets -- straight into mapped host memory (b.chunk_id_off, b.text_id_off, b.out_ids point there).  The CTA
-// that finishes last (a counter, no waiting) adds {n_chunks, n_ids, status} and, as the very last store behind a
-// system-wide fence, the call number the host polls for.
-__global__ void __launch_bounds__(kMediumThreads) k_finish_small_batch(EncodeBuffers b, int64_t* mapped, int64_t seq)
-{
-  __shared__ int scanbuf[33];
-  __shared__ int64_t carry_s;
-  __shared__ __align__(16) int stage[4 * kMediumThreads];
-  __shared__ int64_t s_base, s_total;
-  __shared__ int last;
-  const int tid   = threadIdx.x;
-  const int64_t u = blockIdx.x;
-  const int64_t C = b.totals[0];
-  if (tid == 0) {
-    int64_t run = 0, base = 0;
-    for (int64_t v = 0; v < b.n_tiles; ++v) {
-      if (v == u) base = run;
-      run += b.unit_cnt[v];
-    }
-    s_base  = base;
-    s_total = run;
-  }
-  __syncthreads();
-  const int64_t N = s_total;
-  {
-    const uint16_t* sp = b.staging + b.unit_first[u];
-    int32_t* dp        = b.out_ids + s_base;
-    int64_t m          = b.unit_cnt[u];
-    if (s_base + m > b.out_capacity) m = b.out_capacity > s_base ? b.out_capacity - s_base : 0;
-    for (int64_t i = tid; i < m; i += kMediumThreads) {
-      const uint32_t t = sp[i];
-      dp[i] = int32_t((b.low_id_map && t < 256u) ? uint32_t(__ldg(b.low_id_map + t)) : t);
-    }
-  }
-  if (u == 0) {
-    cta_exclusive_scan_medium(CountsI32{b.chunk_cnt}, C, b.chunk_id_mirror, scanbuf, &carry_s, stage);
-    for (int64_t c = tid; c <= C; c += kMediumThreads) b.chunk_id_off[c] = b.chunk_id_mirror[c];
-    for (int64_t t = tid; t <= b.n_texts; t += kMediumThreads) b.text_id_off[t] = b.chunk_id_mirror[b.text_chunk_base[t]];
-  }
-  __threadfence_system();
-  __syncthreads();
-  if (tid == 0) last = (atomicAdd(b.counters + 8, 1) == int(gridDim.x) - 1);
-  __syncthreads();
-  if (last && tid == 0) {
-    mapped[0] = C;
-    mapped[1] = N;
-    mapped[2] = int64_t(b.counters[1]);  // status word
-    __threadfence_system();
-    *reinterpret_cast<volatile int64_t*>(mapped + 3) = seq;
-  }
-}
-
-int launch_finish_small_batch(const EncodeBuffers& b, int64_t* mapped, int64_t seq, cudaStream_t stream)
-{
-  k_finish_small_batch<<<unsigned(b.n_tiles), kMediumThreads, 0, stream>>>(b, mapped, seq);
-  return 1;
 }
 
 int launch_results_to_host(const EncodeBuffers& b, const void* src, void* dst, int64_t prefix_bytes, int64_t* mapped,
