@@ -159,9 +159,7 @@ struct gtk_taken {
 // Buffers of one in-flight slice of a large host batch (kSliceArenas sets rotate).
 constexpr int kSliceArenas = 4;
 struct SliceArena {
-  DevBuf text_chunk_base, chunk_off, unit_first, unit_cnt, chunk_cnt, tile_info, chunk_rel, text_rel, group_base,
-      scan_sums,
-      counters,  // the 16 counter words, then the group counts
+  DevBuf text_chunk_base, chunk_off, unit_first, unit_cnt, chunk_cnt, scan_sums, counters,
       totals;
   PinBuf h_totals;  // mapped: written by a kernel
   cudaEvent_t ev[6] = {};          // stage timing
@@ -171,8 +169,8 @@ struct SliceArena {
   cudaEvent_t ev_out = nullptr;    // results of the slice are on the host
   void release()
   {
-    for (DevBuf* b : {&text_chunk_base, &chunk_off, &unit_first, &unit_cnt, &chunk_cnt, &tile_info, &chunk_rel,
-                      &text_rel, &group_base, &scan_sums, &counters, &totals})
+    for (DevBuf* b : {&text_chunk_base, &chunk_off, &unit_first, &unit_cnt, &chunk_cnt, &scan_sums,
+                       &counters, &totals})
       b->release();
     h_totals.release();
     for (auto& e : ev)
@@ -226,6 +224,7 @@ struct gtk_tokenizer {
   DevBuf d_out_pack;
   PinBuf h_out_pack;
   bool result_is_packed = false;
+  bool ids_apart = false;  // of a packed result: the ids are in h_ids
   std::shared_ptr<ResultPool> pool = std::make_shared<ResultPool>();
   bool result_is_taken = false;
   const int32_t* view_ids = nullptr;
@@ -235,8 +234,11 @@ struct gtk_tokenizer {
   const uint8_t* pack_base = nullptr;  // h_out_pack, or the mapped block below behind its 64-byte header
   // batches of up to 256 KiB: a kernel writes the results into this mapped block and the host polls its header
   PinBuf h_mid;
-  PinBuf h_out;                // results of encode_host_tiles
-  double ids_per_byte = 0.4;  // room for ids that encode_host_tiles starts with; grows with the texts it meets
+  PinBuf h_out;                // results of encode_host_tiles, offsets of encode_host_pieces
+  DevBuf d_piece_ids;          // ids in front of every piece
+  PinBuf h_marks;              // completion mark and id count of every piece
+  std::vector<cudaEvent_t> piece_ev;
+  double ids_per_byte = 0.4;  // room for ids that they start with; grows with the texts it meets
   int64_t mid_seq = 0;
   // zeroed counters, scanned chunk counts and, when it is short, the text travel in one copy (encode_host_tiles)
   PinBuf h_fast_in;
@@ -409,6 +411,8 @@ Plan plan_batch(gtk_tokenizer* h, const uint8_t* d_bytes, int64_t n_bytes, const
   b.totals = h->d_totals.as<int64_t>();
   b.counters = reinterpret_cast<int32_t*>(b.totals + 2);
   b.group_cnt = b.counters + 16;
+  b.ticket = b.counters;
+  b.tile_hi = n_tiles;
   b.low_id_map = (h->id_space == GTK_IDS_GPT2) ? h->d_low_map.as<uint16_t>() : nullptr;
   return p;
 }
@@ -644,15 +648,11 @@ void slice_arena_prepare(gtk_tokenizer* h, SliceArena& a, int64_t max_bytes, int
   const int64_t n_tiles   = (max_bytes + gtk::kTile - 1) / gtk::kTile;
   a.text_chunk_base.reserve(size_t(max_pieces + 1) * 8);
   a.chunk_off.reserve(size_t(chunk_cap + 1) * 8);
-  a.tile_info.reserve(size_t(n_tiles + 1) * sizeof(gtk::TileInfo));
-  a.chunk_rel.reserve(size_t(chunk_cap + 1) * 4);
-  a.text_rel.reserve(size_t(max_pieces + 1) * 4);
-  a.group_base.reserve(size_t(n_tiles / gtk::kTileGroup + 2) * 8);
   a.unit_first.reserve(size_t(n_tiles + 1) * 8);
   a.unit_cnt.reserve(size_t(n_tiles + 1) * 4);
   a.chunk_cnt.reserve(size_t(chunk_cap + 1) * 4);
   a.scan_sums.reserve(size_t(std::max<int64_t>(std::max(chunk_cap, n_tiles), max_pieces) / 4096 + 2) * 8);
-  a.counters.reserve(64 + size_t(n_tiles / gtk::kTileGroup + 1) * 4);
+  a.counters.reserve(64);
   a.totals.reserve(64);
   a.h_totals.reserve_mapped(64);
   for (auto& e : a.ev)
@@ -684,10 +684,6 @@ gtk::EncodeBuffers slice_buffers(gtk_tokenizer* h, SliceArena& a, const SlicePla
   b.unit_first = a.unit_first.as<int64_t>();
   b.unit_cnt = a.unit_cnt.as<int32_t>();
   b.chunk_cnt = a.chunk_cnt.as<int32_t>();
-  b.tile_info = a.tile_info.as<gtk::TileInfo>();
-  b.chunk_rel = a.chunk_rel.as<int32_t>();
-  b.text_rel = a.text_rel.as<int32_t>();
-  b.group_base = a.group_base.as<int64_t>();
   b.chunk_id_off = nullptr;
   b.text_id_off = nullptr;
   b.out_ids = h->d_out_ids.as<int32_t>() + dev_off;  // worst case one id per byte: slices never overlap
@@ -700,7 +696,6 @@ gtk::EncodeBuffers slice_buffers(gtk_tokenizer* h, SliceArena& a, const SlicePla
   b.seg_scratch_tokens = scratch_tokens;
   b.scan_block_sums = a.scan_sums.as<int64_t>();
   b.counters = a.counters.as<int32_t>();
-  b.group_cnt = b.counters + 16;
   b.totals = a.totals.as<int64_t>();
   b.low_id_map = (h->id_space == GTK_IDS_GPT2) ? h->d_low_map.as<uint16_t>() : nullptr;
   return b;
@@ -754,7 +749,6 @@ int encode_host_sliced(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
   if (!h->out_stream) GTK_CUDA(cudaStreamCreateWithFlags(&h->out_stream, cudaStreamNonBlocking));
   if (!h->pack_stream) GTK_CUDA(cudaStreamCreateWithFlags(&h->pack_stream, cudaStreamNonBlocking));
   for (auto& a : h->slice) slice_arena_prepare(h, a, max_bytes, max_pieces);
-  begin_call(h, mode, n_bytes);
   GTK_CUDA(cudaStreamSynchronize(h->stream));
 
   for (int i = 0; i < ns; ++i) {
@@ -768,7 +762,6 @@ int encode_host_sliced(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
   std::vector<int64_t> sl_c(nsz), sl_r(nsz), sl_cbase(nsz);
   int launches = 0;
   int64_t R = 0, Cbase = 0;
-  const bool tiles = mode == GTK_MODE_OPT && !h->wide;  // its pack follows the tile kernel without a word from the host
 
   auto issue_front = [&](int i) {
     SliceArena& a = h->slice[i % kSliceArenas];
@@ -784,14 +777,13 @@ int encode_host_sliced(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
     b.text_id_off  = h->d_piece_id_off.as<int64_t>() + piece_at[size_t(i)];
     b.chunk_id_off = h->d_chunk_id_all.as<int64_t>() + chunk_at[size_t(i)];
     // the result words reach the host through mapped memory
-    if (tiles) run_tiles(h, b, false, static_cast<int64_t*>(a.h_totals.dp), i + 1, &launches, a.ev);
-    else run_front(h, b, mode, &launches, a.ev, nullptr, static_cast<int64_t*>(a.h_totals.dp));
+    run_front(h, b, mode, &launches, a.ev, nullptr, static_cast<int64_t*>(a.h_totals.dp));
     GTK_CUDA(cudaEventRecord(a.ev_front, h->stream));
   };
   auto finish = [&](int i) {  // the ids of slice i are on the host
     SliceArena& a = h->slice[i % kSliceArenas];
     GTK_CUDA(cudaEventSynchronize(a.ev_out));
-    if (!tiles) collect_pack_time(h, a.ev);
+    collect_pack_time(h, a.ev);
   };
   auto sync_all = [&] {
     cudaStreamSynchronize(h->in_stream);
@@ -807,10 +799,9 @@ int encode_host_sliced(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
     if (i >= 2) finish(i - 2);
     GTK_CUDA(cudaEventSynchronize(a.ev_front));
     collect_front_times(h, a.ev);
-    if (tiles) collect_pack_time(h, a.ev);
     const int64_t* ht = a.h_totals.as<int64_t>();
     const int64_t C = ht[0], N = ht[1];
-    const int status = tiles ? int(ht[2]) : reinterpret_cast<const int32_t*>(ht + 2)[1];
+    const int status = reinterpret_cast<const int32_t*>(ht + 2)[1];
     if (status != gtk::kStatusOk) {
       sync_all();
       return h->fail(GTK_ERR_KERNEL, status_text(status));
@@ -823,12 +814,11 @@ int encode_host_sliced(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
       h->h_ids.release();
       h->h_ids = bigger;
     }
-    if (!tiles) {  // the pack runs on a stream of its own: the compute stream already holds the fronts of later slices
-      GTK_CUDA(cudaStreamWaitEvent(h->pack_stream, a.ev_front, 0));
-      run_pack(h, bufs[size_t(i)], &launches, a.ev, h->pack_stream);
-      GTK_CUDA(cudaEventRecord(a.ev_packed, h->pack_stream));
-    }
-    GTK_CUDA(cudaStreamWaitEvent(h->out_stream, tiles ? a.ev_front : a.ev_packed, 0));
+    // the pack runs on a stream of its own: the compute stream already holds the fronts of later slices
+    GTK_CUDA(cudaStreamWaitEvent(h->pack_stream, a.ev_front, 0));
+    run_pack(h, bufs[size_t(i)], &launches, a.ev, h->pack_stream);
+    GTK_CUDA(cudaEventRecord(a.ev_packed, h->pack_stream));
+    GTK_CUDA(cudaStreamWaitEvent(h->out_stream, a.ev_packed, 0));
     GTK_CUDA(cudaMemcpyAsync(h->h_ids.as<int32_t>() + R, bufs[size_t(i)].out_ids, size_t(N) * 4, cudaMemcpyDeviceToHost,
                              h->out_stream));
     GTK_CUDA(cudaEventRecord(a.ev_out, h->out_stream));
@@ -1058,6 +1048,7 @@ int encode_host_tiles(gtk_tokenizer* h, const uint8_t* bytes, const int64_t* tex
     p.b.totals          = reinterpret_cast<int64_t*>(dp);
     p.b.counters        = reinterpret_cast<int32_t*>(dp + 16);
     p.b.group_cnt       = p.b.counters + 16;
+    p.b.ticket          = p.b.counters;
     p.b.text_chunk_base = reinterpret_cast<int64_t*>(dp + o_base);
     p.b.tile_info       = reinterpret_cast<gtk::TileInfo*>(dp + o_info);
     const int64_t seq   = ++h->mid_seq;
@@ -1095,6 +1086,170 @@ int encode_host_tiles(gtk_tokenizer* h, const uint8_t* bytes, const int64_t* tex
   return GTK_OK;
 }
 
+// Larger host batches (GTK_MODE_OPT, 16-bit table): the text goes up in pieces, and while a piece travels the one before it
+// is in the tile and pack kernels and the ids of earlier ones are on their way back.  The pack kernel of a piece knows where
+// its ids go; a mark with the id count is left in page-locked memory, where the host polls for it and then sends the ids with
+// the copy engine.  (Ids written by the pack kernel itself: 3.8 instead of 3.1 ms for
+// 96 MiB, since beside the next piece's tile kernel no pack CTA finds room on an SM.)  Bound by the host link, which carries
+// one byte up and 1.0 .. 2.4 bytes of ids down per byte of text.
+// While the link is busy every step from one stream to another takes 25 .. 55 us (commands and marks travel behind the
+// text), so pieces are few: 96 MiB of the novel 2.70 ms with pieces of 2 .. 12 MiB, 2.76 with 0.5 .. 16 MiB; below 6 MiB the
+// single upload of encode_host_tiles is quicker (4 MiB page-locked 256 against 281 us, 7 MiB 431 against 433, from
+// ordinary memory 680 against 610).
+constexpr int64_t kPiecesMinBytes = int64_t(6) << 20;
+constexpr int64_t kPieceMin = int64_t(2) << 20, kPieceMax = int64_t(12) << 20;
+
+// Ends of the pieces: small ones first and last, because the first upload and the last piece's kernels and download are what
+// nothing overlaps; whole tile groups.
+std::vector<int64_t> piece_ends(int64_t n_bytes)
+{
+  constexpr int64_t kGroup = int64_t(gtk::kTileGroup) * gtk::kTile;
+  std::vector<int64_t> ends;
+  for (int64_t at = 0; at < n_bytes;) {
+    const int64_t left = n_bytes - at;
+    int64_t take = std::max(std::min({std::max(at, kPieceMin), left / 2, kPieceMax}), kPieceMin) / kGroup * kGroup;
+    if (left - take < kPieceMin / 2) take = left;
+    at += take;
+    ends.push_back(at);
+  }
+  return ends;
+}
+
+int encode_host_pieces(gtk_tokenizer* h, const uint8_t* bytes, const int64_t* text_offsets, int64_t n_texts, int64_t n_bytes,
+                       float* kernel_ms)
+{
+  auto up = [](size_t x) { return (x + 63) & ~size_t(63); };
+  const int64_t chunk = h->chunk_tokens, K = (n_bytes + gtk::kTile - 1) / gtk::kTile, groups = K / gtk::kTileGroup + 1;
+  int64_t C = 0;
+  if (n_texts == 1) {
+    C = (n_bytes + chunk - 1) / chunk;
+  } else {
+    for (int64_t t = 0; t < n_texts; ++t) {
+      const int64_t len = text_offsets[t + 1] - text_offsets[t];
+      C += len <= chunk ? (len > 0) : (len + chunk - 1) / chunk;
+    }
+  }
+  const std::vector<int64_t> ends = piece_ends(n_bytes);
+  const size_t np = ends.size();
+  const size_t text_b = up(size_t(n_texts + 1) * 8), chunk_b = up(size_t(C + 1) * 8);
+  // everything is sized before the first copy is issued: nothing may be reallocated in flight
+  h->pool->reserve(h->h_out, text_b + chunk_b);
+  h->pool->reserve(h->h_ids, std::min(size_t(n_bytes), size_t(double(n_bytes) * h->ids_per_byte) + 1024) * 4);  // grown below
+  h->h_marks.reserve(np * 64);
+  std::memset(h->h_marks.p, 0, np * 64);
+  h->d_bytes.reserve(size_t(n_bytes) + 32);
+  h->d_out_ids.reserve(size_t(n_bytes) * 4);
+  if (n_texts > 1) h->d_text_off.reserve(size_t(n_texts + 1) * 8);
+  h->d_totals.reserve(80 + size_t(groups) * 8);
+  h->d_piece_ids.reserve((np + 1) * 8);
+  for (cudaStream_t* c : {&h->in_stream, &h->pack_stream, &h->out_stream})
+    if (!*c) GTK_CUDA(cudaStreamCreateWithFlags(c, cudaStreamNonBlocking));
+  while (h->piece_ev.size() < np * 4) {  // per piece: uploaded; in front of, between and behind its kernels
+    cudaEvent_t e;
+    GTK_CUDA(cudaEventCreateWithFlags(&e, h->piece_ev.size() % 4 == 0 ? cudaEventDisableTiming : cudaEventDefault));
+    h->piece_ev.push_back(e);
+  }
+  gtk::EncodeBuffers b = plan_batch(h, h->d_bytes.as<uint8_t>(), n_bytes, h->d_text_off.as<int64_t>(), n_texts,
+                                    h->d_out_ids.as<int32_t>(), n_bytes, nullptr, true).b;
+  int32_t* tickets = b.group_cnt + groups;
+  cudaStream_t s   = h->stream;
+  int launches     = 0;
+  begin_call(h, GTK_MODE_OPT, n_bytes);
+  const bool learned = h->reset_learned;
+  h->reset_learned   = false;
+  if (n_texts > 1) GTK_CUDA(cudaMemcpyAsync(h->d_text_off.p, text_offsets, size_t(n_texts + 1) * 8, cudaMemcpyHostToDevice, s));
+  GTK_CUDA(cudaMemsetAsync(tickets, 0, np * 4, s));
+  launches += gtk::launch_begin_batch(b, h->dtab.long_words, learned ? h->call_tab.long_words : nullptr, s);
+  launches += gtk::launch_scan_texts(b, learned, s) + gtk::launch_tile_info(b, s);
+  GTK_CUDA(cudaGetLastError());
+
+  int64_t have = 0;  // ids whose copy has been issued
+  // the ids of piece i, once its mark is there; wait: for the mark.  false: not there yet
+  auto collect = [&](size_t i, bool wait) {
+    volatile const int64_t* m = h->h_marks.as<int64_t>() + 8 * i;
+    if (!wait && m[3] != int64_t(i) + 1) return false;
+    if (!wait_for_mark(m + 3, int64_t(i) + 1, h->pack_stream, "pack kernel"))
+      throw CudaFail{"pack kernel ended without publishing its results"};
+    const int64_t n = m[1];
+    if (n < have || n > n_bytes) throw CudaFail{"inconsistent id count"};
+    if (size_t(n) * 4 > h->h_ids.cap) {  // grow the pinned id buffer, keeping what has arrived
+      h->ids_per_byte = std::min(1.0, std::max(h->ids_per_byte, 1.1 * double(n) / double(ends[i])));
+      GTK_CUDA(cudaStreamSynchronize(h->out_stream));
+      PinBuf bigger;
+      h->pool->reserve(bigger, std::max(size_t(n), std::min(size_t(n_bytes), size_t(double(n_bytes) * h->ids_per_byte) + 1024)) * 4);
+      std::memcpy(bigger.p, h->h_ids.p, size_t(have) * 4);
+      h->pool->give_back(h->h_ids);
+      h->h_ids = bigger;
+    }
+    if (n > have)
+      GTK_CUDA(cudaMemcpyAsync(h->h_ids.as<int32_t>() + have, h->d_out_ids.as<int32_t>() + have, size_t(n - have) * 4,
+                               cudaMemcpyDeviceToHost, h->out_stream));
+    have = n;
+    return true;
+  };
+  try {
+    size_t done = 0;  // pieces collected
+    for (size_t i = 0; i < np; ++i) {
+      cudaEvent_t* ev  = &h->piece_ev[4 * i];
+      const int64_t lo = i ? ends[i - 1] : 0;
+      GTK_CUDA(cudaMemcpyAsync(h->d_bytes.as<uint8_t>() + lo, bytes + lo, size_t(ends[i] - lo), cudaMemcpyHostToDevice, h->in_stream));
+      GTK_CUDA(cudaEventRecord(ev[0], h->in_stream));
+      GTK_CUDA(cudaStreamWaitEvent(s, ev[0], 0));
+      // a tile may need the text to the end of its last chunk: such tiles wait for the next piece
+      const bool last   = i + 1 == np;
+      const int64_t own = ends[i] - gtk::kWindow - std::min(chunk, n_bytes);
+      b.tile_hi         = last ? K : std::max(b.tile_lo, own / gtk::kTile / gtk::kTileGroup * gtk::kTileGroup);
+      b.ticket          = tickets + i;
+      b.piece_ids       = h->d_piece_ids.as<int64_t>() + i;
+      GTK_CUDA(cudaEventRecord(ev[1], s));
+      launches += gtk::launch_merge_opt(b, h->call_tab, h->opt_grid, s);
+      GTK_CUDA(cudaEventRecord(ev[2], s));
+      // a piece without a tile hands the count of the pieces in front of it on
+      launches += gtk::launch_pack_tiles(b, h->sm_count, false, nullptr, 0, s);
+      GTK_CUDA(cudaEventRecord(ev[3], s));
+      GTK_CUDA(cudaStreamWaitEvent(h->pack_stream, ev[3], 0));
+      launches += gtk::launch_publish_piece(b, h->h_marks.as<int64_t>() + 8 * i, int64_t(i) + 1, h->pack_stream);  // page-locked: same address on the device
+      GTK_CUDA(cudaGetLastError());
+      b.tile_lo = b.tile_hi;
+      while (done < i && collect(done, false)) ++done;
+    }
+    while (done < np) collect(done++, true);
+    GTK_CUDA(cudaMemcpyAsync(h->h_out.p, b.text_id_off, size_t(n_texts + 1) * 8, cudaMemcpyDeviceToHost, h->out_stream));
+    GTK_CUDA(cudaMemcpyAsync(h->h_out.as<uint8_t>() + text_b, b.chunk_id_off, size_t(C + 1) * 8, cudaMemcpyDeviceToHost, h->out_stream));
+    GTK_CUDA(cudaStreamSynchronize(h->out_stream));
+  } catch (...) {  // nothing of the call may be in flight when it returns
+    cudaStreamSynchronize(h->in_stream);
+    cudaStreamSynchronize(s);
+    cudaStreamSynchronize(h->pack_stream);
+    cudaStreamSynchronize(h->out_stream);
+    throw;
+  }
+  const int64_t* end = h->h_marks.as<int64_t>() + 8 * (np - 1);
+  if (end[2] != gtk::kStatusOk) return h->fail(GTK_ERR_KERNEL, status_text(int(end[2])));
+  if (end[0] != C) return h->fail(GTK_ERR_KERNEL, "inconsistent totals");
+  GTK_CUDA(cudaEventSynchronize(h->piece_ev[4 * np - 1]));
+  for (size_t i = 0; i < np; ++i) {
+    float merge = 0, pack = 0;
+    GTK_CUDA(cudaEventElapsedTime(&merge, h->piece_ev[4 * i + 1], h->piece_ev[4 * i + 2]));
+    GTK_CUDA(cudaEventElapsedTime(&pack, h->piece_ev[4 * i + 2], h->piece_ev[4 * i + 3]));
+    h->stage_ms[1] += merge;
+    h->stage_ms[3] += pack;
+  }
+  h->stage_ms[4]      = h->stage_ms[1] + h->stage_ms[3];
+  h->result_is_packed = true;
+  h->ids_apart        = true;
+  h->pack_base        = h->h_out.as<uint8_t>();
+  h->result_bufs[0]   = &h->h_out;
+  h->result_bufs[1]   = &h->h_ids;
+  h->pack_text_bytes  = text_b;
+  h->pack_chunk_bytes = chunk_b;
+  h->last_launches    = launches;
+  h->res_n_ids        = have;
+  h->res_n_chunks     = C;
+  if (kernel_ms) *kernel_ms = h->stage_ms[4];
+  return GTK_OK;
+}
+
 // frees every device / pinned buffer, stream and event of a handle (also used when gtk_create fails half way)
 void release_handle(gtk_tokenizer* h)
 {
@@ -1106,8 +1261,8 @@ void release_handle(gtk_tokenizer* h)
                       &h->d_unit_cnt, &h->d_chunk_cnt, &h->d_tile_info, &h->d_chunk_rel, &h->d_text_rel, &h->d_group_base, &h->d_chunk_id_off, &h->d_text_id_off,
                       &h->d_out_ids, &h->d_seg_scratch, &h->d_scan_sums, &h->d_totals, &h->d_out_pack, &h->d_fast_in})
       b->release();
-    for (PinBuf* b : {&h->h_ids, &h->h_text_id_off, &h->h_chunk_id_off, &h->h_totals, &h->h_piece_off, &h->h_piece_id_off, &h->h_chunk_id_all, &h->h_out_pack, &h->h_mid, &h->h_out, &h->h_fast_in}) b->release();
-    for (DevBuf* b : {&h->d_piece_off, &h->d_piece_id_off, &h->d_chunk_id_all}) b->release();
+    for (PinBuf* b : {&h->h_ids, &h->h_text_id_off, &h->h_chunk_id_off, &h->h_totals, &h->h_piece_off, &h->h_piece_id_off, &h->h_chunk_id_all, &h->h_out_pack, &h->h_mid, &h->h_out, &h->h_marks, &h->h_fast_in}) b->release();
+    for (DevBuf* b : {&h->d_piece_off, &h->d_piece_id_off, &h->d_chunk_id_all, &h->d_piece_ids}) b->release();
     if (h->small_in_h) cudaFreeHost(h->small_in_h);
     if (h->small_out_h) cudaFreeHost(h->small_out_h);
     {
@@ -1120,6 +1275,7 @@ void release_handle(gtk_tokenizer* h)
     if (h->in_stream) cudaStreamDestroy(h->in_stream);
     if (h->out_stream) cudaStreamDestroy(h->out_stream);
     if (h->pack_stream) cudaStreamDestroy(h->pack_stream);
+    for (cudaEvent_t ev : h->piece_ev) cudaEventDestroy(ev);
     for (auto& ev : h->ev)
       if (ev) cudaEventDestroy(ev);
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
@@ -1371,6 +1527,7 @@ GTK_API int gtk_encode(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
   h->result_is_cpu = false;
   h->result_is_small = false;
   h->result_is_packed = false;
+  h->ids_apart = false;
   h->result_is_taken = false;
   h->result_bufs[0] = h->result_bufs[1] = h->result_bufs[2] = nullptr;
   h->res_n_ids = h->res_n_chunks = 0;
@@ -1392,8 +1549,10 @@ GTK_API int gtk_encode(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
     if (h->wide && mode == GTK_MODE_LOCALMIN) return h->fail(GTK_ERR_TABLE, kWideNoLocalmin);
     if (!h->wide && mode == GTK_MODE_OPT && n_bytes <= gtk::kSmallMaxBytes && n_texts <= gtk::kSmallMaxTexts)
       return encode_host_small(h, bytes, text_offsets, n_texts, n_bytes, kernel_ms);
+    if (!h->wide && mode == GTK_MODE_OPT)
+      return n_bytes >= kPiecesMinBytes ? encode_host_pieces(h, bytes, text_offsets, n_texts, n_bytes, kernel_ms)
+                                        : encode_host_tiles(h, bytes, text_offsets, n_texts, n_bytes, kernel_ms);
     if (n_bytes >= kSliceThresholdBytes) return encode_host_sliced(h, mode, bytes, text_offsets, n_texts, n_bytes, kernel_ms);
-    if (!h->wide && mode == GTK_MODE_OPT) return encode_host_tiles(h, bytes, text_offsets, n_texts, n_bytes, kernel_ms);
     cudaStream_t s = h->stream;
     h->d_bytes.reserve(size_t(n_bytes) + 32);
     h->d_text_off.reserve(size_t(n_texts + 1) * 8);
@@ -1489,6 +1648,7 @@ GTK_API int gtk_encode_cpu(gtk_tokenizer* h, int rule, const uint8_t* bytes, con
   h->result_is_cpu = true;
   h->result_is_small = false;
   h->result_is_packed = false;
+  h->ids_apart = false;
   h->result_is_taken = false;
   h->result_bufs[0] = h->result_bufs[1] = h->result_bufs[2] = nullptr;
   h->res_n_ids = int64_t(h->cpu_ids.size());
@@ -1524,7 +1684,7 @@ GTK_API int gtk_result_view(const gtk_tokenizer* h, const int32_t** ids, const i
     if (chunk_id_offsets) *chunk_id_offsets = reinterpret_cast<const int64_t*>(h->small_out_h + kSmallOutChunk);
   } else if (h->result_is_packed) {
     const uint8_t* base = h->pack_base;
-    if (ids) *ids = reinterpret_cast<const int32_t*>(base + h->pack_text_bytes + h->pack_chunk_bytes);
+    if (ids) *ids = h->ids_apart ? h->h_ids.as<int32_t>() : reinterpret_cast<const int32_t*>(base + h->pack_text_bytes + h->pack_chunk_bytes);
     if (text_id_offsets) *text_id_offsets = reinterpret_cast<const int64_t*>(base);
     if (chunk_id_offsets) *chunk_id_offsets = reinterpret_cast<const int64_t*>(base + h->pack_text_bytes);
   } else {

@@ -78,6 +78,9 @@ struct EncodeBuffers {
   int64_t chunk_cap;         // upper bound on the number of chunks
   int32_t* tile_chunk0;      // [n_tiles] single-CTA kernel only: chunk that contains the first byte of the tile
   int64_t n_tiles;
+  int64_t tile_lo, tile_hi;  // the launch works on these (all, or those of a piece that starts with a group)
+  int32_t* ticket;           // tile ticket of the launch (zero at the start)
+  int64_t* piece_ids;        // nullptr, or [0] ids in front of the piece, [1] the same for the next one (pack kernel)
   // merge outputs
   uint16_t* staging;         // [n_bytes] tokens of a unit, compacted at the unit's first byte
   int64_t* unit_first;       // [n_tiles] byte position where the unit's tokens start in staging (opt mode)
@@ -102,7 +105,7 @@ struct EncodeBuffers {
   int32_t* staging32;        // [n_bytes] 32-bit kernel: tokens of a chunk, compacted at the chunk's first byte
   int64_t seg_scratch_tokens;  // tokens per CTA (two arrays of this length per CTA)
   int64_t* scan_block_sums;  // workspace of the multi-block scan
-  int32_t* counters;         // [0] tile ticket, [1] status word, [2] chunk ticket, [8] CTAs done, [12..13] time the tile kernel began
+  int32_t* counters;         // [0] tile ticket of whole batches, [1] status word, [2] chunk ticket, [8] CTAs done, [12..13] time the tile kernel began
   int64_t* totals;           // device: [0] n_chunks, [1] n_ids
 };
 
@@ -132,6 +135,8 @@ int launch_scan_texts(const EncodeBuffers& b, bool learned, cudaStream_t stream)
 // host waits for the call, or nullptr: {n_chunks, n_ids, status, seq, nanoseconds since the tile kernel began}, seq last;
 // out_ids, chunk_id_off and text_id_off may then be page-locked host memory.  Uses counters[8] (zero at the start).
 int launch_pack_tiles(const EncodeBuffers& b, int sm_count, bool groups_scanned, int64_t* publish, int64_t seq, cudaStream_t stream);
+// {n_chunks, ids up to the end of the piece, status, seq} to `publish` in page-locked host memory, seq last
+int launch_publish_piece(const EncodeBuffers& b, int64_t* publish, int64_t seq, cudaStream_t stream);
 // the device result arena of a batch into mapped host memory, then totals {n_chunks, n_ids, status} and,
 // last, the call number into mapped[0..3]; uses counters[8] (zero at the start of the call)
 int launch_results_to_host(const EncodeBuffers& b, const void* src, void* dst, int64_t prefix_bytes, int64_t* mapped,

@@ -1023,17 +1023,18 @@ __global__ void __launch_bounds__(kOptThreads, GTK_OPT_CTAS) k_merge_opt(EncodeB
 {
   TileSmem<kOptThreads>& S = tile_smem<kOptThreads>();
   tile_setup(S);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long*>(b.counters + 12) = global_timer();
-  int64_t k = blockIdx.x;  // the first tile of every CTA, the others by ticket
-  while (k < b.n_tiles) {
+  if (b.tile_lo == 0 && blockIdx.x == 0 && threadIdx.x == 0)
+    *reinterpret_cast<unsigned long long*>(b.counters + 12) = global_timer();
+  int64_t k = b.tile_lo + blockIdx.x;  // the first tile of every CTA, the others by ticket
+  while (k < b.tile_hi) {
     int next = 0;
-    if (threadIdx.x == 0) next = atomicAdd(b.counters + 0, 1);  // on its way while the tile is worked on
+    if (threadIdx.x == 0) next = atomicAdd(b.ticket, 1);  // on its way while the tile is worked on
     tile_reset(S);
     __syncthreads();
     opt_tile(S, b, T, k);
     if (threadIdx.x == 0) S.ticket = next;
     __syncthreads();
-    k = int64_t(gridDim.x) + S.ticket;
+    k = b.tile_lo + int64_t(gridDim.x) + S.ticket;
   }
 }
 
@@ -1700,9 +1701,8 @@ __global__ void __launch_bounds__(256) k_pack_tiles(EncodeBuffers b, int64_t per
 {
   constexpr int kWarps = 8;
   __shared__ int64_t warp_sum[kWarps];
-  __shared__ int last;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t K = b.n_tiles, a = min(int64_t(blockIdx.x) * per_cta, K), e = min(a + per_cta, K);
+  const int64_t K = b.n_tiles, a = min(b.tile_lo + int64_t(blockIdx.x) * per_cta, b.tile_hi), e = min(a + per_cta, b.tile_hi);
   const uint16_t* map = b.low_id_map;
   auto conv = [&](uint32_t t) { return int32_t((map && t < 256u) ? uint32_t(__ldg(map + t)) : t); };
   const int64_t C = b.n_texts == 1 ? (b.n_bytes + b.chunk_bytes - 1) / b.chunk_bytes : b.totals[0];
@@ -1712,7 +1712,8 @@ __global__ void __launch_bounds__(256) k_pack_tiles(EncodeBuffers b, int64_t per
     if (groups_scanned) {
       if (tid == 0) sum = b.group_base[g];
     } else {
-      for (int64_t i = tid; i < g; i += 256) sum += b.group_cnt[i];
+      for (int64_t i = b.tile_lo / kTileGroup + tid; i < g; i += 256) sum += b.group_cnt[i];
+      if (tid == 0 && b.tile_lo > 0) sum += b.piece_ids[0];
     }
     for (int64_t i = g * kTileGroup + tid; i < a; i += 256) sum += b.unit_cnt[i];
 #pragma unroll
@@ -1747,6 +1748,7 @@ __global__ void __launch_bounds__(256) k_pack_tiles(EncodeBuffers b, int64_t per
           }
         }
       }
+      if (k == b.tile_hi - 1 && l == 0 && b.piece_ids) b.piece_ids[1] = dst + m;
       if (end && l == 0) {
         b.chunk_id_off[C] = dst + m;
         if (b.text_id_off) b.text_id_off[b.n_texts] = dst + m;
@@ -1755,6 +1757,7 @@ __global__ void __launch_bounds__(256) k_pack_tiles(EncodeBuffers b, int64_t per
       }
     }
   }
+  if (a >= e && b.tile_lo == b.tile_hi && b.piece_ids && tid == 0) b.piece_ids[1] = b.tile_lo > 0 ? b.piece_ids[0] : 0;
   if (K == 0) {  // texts without a byte
     if (b.text_id_off)
       for (int64_t t = tid; t <= b.n_texts; t += 256) b.text_id_off[t] = 0;
@@ -1762,13 +1765,12 @@ __global__ void __launch_bounds__(256) k_pack_tiles(EncodeBuffers b, int64_t per
   }
   if (!publish) return;
   // The CTA that finishes last (a counter, no waiting) tells the host, which may be polling the call number: the last store,
-  // behind a system-wide fence.
-  __threadfence_system();
+  // behind a system-wide fence, which covers what the other CTAs have published to this one.
   __syncthreads();
-  if (tid == 0) last = atomicAdd(b.counters + 8, 1) == int(gridDim.x) - 1;
-  __syncthreads();
-  if (last && tid == 0) {
+  if (tid == 0) {
     __threadfence();
+    if (atomicAdd(b.counters + 8, 1) != int(gridDim.x) - 1) return;
+    __threadfence_system();
     publish[0] = C;
     publish[1] = *reinterpret_cast<volatile int64_t*>(b.totals + 1);
     publish[2] = int64_t(*reinterpret_cast<volatile int32_t*>(b.counters + 1));
@@ -1856,6 +1858,23 @@ int launch_begin_batch(const EncodeBuffers& b, const uint4* long_words, uint4* l
   return 1;
 }
 
+// {n_chunks, ids up to the end of the piece, status, seq} to the host, seq last.  A kernel of its own on a stream of its own: the
+// fence behind stores to the host takes tens of microseconds while the link is busy, and the next piece need not wait for it.
+__global__ void k_publish_piece(EncodeBuffers b, int64_t* publish, int64_t seq)
+{
+  publish[0] = b.totals[0];
+  publish[1] = b.piece_ids[1];
+  publish[2] = int64_t(b.counters[1]);
+  __threadfence_system();
+  *reinterpret_cast<volatile int64_t*>(publish + 3) = seq;
+}
+
+int launch_publish_piece(const EncodeBuffers& b, int64_t* publish, int64_t seq, cudaStream_t stream)
+{
+  k_publish_piece<<<1, 1, 0, stream>>>(b, publish, seq);
+  return 1;
+}
+
 int launch_scan_texts(const EncodeBuffers& b, bool learned, cudaStream_t stream)
 {
   if (b.n_texts == 1 || (medium_batch(b) && !learned)) return 0;
@@ -1885,12 +1904,14 @@ int launch_scan_groups(const EncodeBuffers& b, cudaStream_t stream)
 int launch_pack_tiles(const EncodeBuffers& b, int sm_count, bool groups_scanned, int64_t* publish, int64_t seq, cudaStream_t stream)
 {
   // up to eight tiles per SM: a CTA for each, so that its 256 threads share the tile's 1400 ids
-  if (b.n_tiles <= int64_t(sm_count) * 8) {
-    k_pack_tiles<true><<<unsigned(std::max<int64_t>(b.n_tiles, 1)), 256, 0, stream>>>(b, 1, groups_scanned, publish, seq);
+  const int64_t n = b.tile_hi - b.tile_lo;
+  if (n <= int64_t(sm_count) * 8) {
+    k_pack_tiles<true><<<unsigned(std::max<int64_t>(n, 1)), 256, 0, stream>>>(b, 1, groups_scanned, publish, seq);
     return 1;
   }
-  const int64_t ctas = int64_t(sm_count) * 8, per = ((b.n_tiles + ctas - 1) / ctas + 7) & ~int64_t(7);
-  k_pack_tiles<false><<<unsigned((b.n_tiles + per - 1) / per), 256, 0, stream>>>(b, per, groups_scanned, publish, seq);
+  // beyond that one tile per warp: 128 MiB of English-like text 72 us, with four times as many tiles per CTA 82 us
+  const int64_t per = 8;
+  k_pack_tiles<false><<<unsigned((n + per - 1) / per), 256, 0, stream>>>(b, per, groups_scanned, publish, seq);
   return 1;
 }
 
@@ -1909,8 +1930,8 @@ int launch_chunker(const EncodeBuffers& b, cudaStream_t stream)
 
 int launch_merge_opt(const EncodeBuffers& b, const DeviceTable& t, int grid, cudaStream_t stream)
 {
-  if (b.n_tiles <= 0) return 0;
-  if (grid > b.n_tiles) grid = int(b.n_tiles);
+  if (b.tile_hi <= b.tile_lo) return 0;
+  if (grid > b.tile_hi - b.tile_lo) grid = int(b.tile_hi - b.tile_lo);
   k_merge_opt<<<grid, kOptThreads, 0, stream>>>(b, t);
   return 1;
 }
@@ -2084,15 +2105,14 @@ __global__ void __launch_bounds__(256) k_results_to_host(const uint4* __restrict
                                                          const int64_t* totals, int32_t* counters, int64_t* mapped,
                                                          int64_t seq)
 {
-  __shared__ int last;
   const int64_t n16 = (prefix_bytes + totals[1] * 4 + 15) / 16;
   for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n16; i += int64_t(gridDim.x) * blockDim.x)
     dst[i] = src[i];
-  __threadfence_system();
   __syncthreads();
-  if (threadIdx.x == 0) last = (atomicAdd(counters + 8, 1) == int(gridDim.x) - 1);
-  __syncthreads();
-  if (last && threadIdx.x == 0) {
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(counters + 8, 1) != int(gridDim.x) - 1) return;
+    __threadfence_system();
     mapped[0] = totals[0];
     mapped[1] = totals[1];
     mapped[2] = int64_t(counters[1]);  // status word
