@@ -241,20 +241,6 @@ __device__ __forceinline__ void tile_cut(TileSmem<TH>& S, const Span& sp, const 
   __syncthreads();
 }
 
-// A segment of more than kThreadSegMax bytes: to the long list, or noted as the one that runs past the window.
-template <int TH>
-__device__ __noinline__ void note_long_segment(int s, int wlen, int* status)
-{
-  TileSmem<TH>& S = tile_smem<TH>();
-  if (next_cut(S, s) >= S.kWin && wlen == S.kWin) {
-    S.over_start = s;
-    return;
-  }
-  const int q = atomicAdd(&S.nlong, 1);
-  if (q < S.kLong && GTK_IN(s, S.kOwn, 3)) S.longq[q] = uint16_t(s);
-  else atomicMax(status, int(kStatusLongQueueOverflow));
-}
-
 // the 16 bytes from window position `at` on
 template <int TH>
 __device__ __forceinline__ void window_words(const TileSmem<TH>& S, int at, uint32_t k[4])
@@ -303,6 +289,26 @@ __device__ __forceinline__ bool long_matches(const LongSlot& s, const uint32_t k
   return diff == 0u && s.v.x != 0u && s.v.y != 0u && s.v.z != 0u && s.v.w != 0u;
 }
 
+__device__ __forceinline__ bool find_long(const DeviceTable& T, const uint32_t k[4], uint32_t length, LongSlot& at)
+{
+  const uint32_t h = long_slot_of(k, length);
+  at         = load_long(T.long_words, h);
+  bool found = long_matches(at, k, length);
+  for (uint32_t hop = 1; !found && (at.v.x & kLongMore) && hop < kLongHops; ++hop) {
+    at    = load_long(T.long_words, h ^ hop);
+    found = long_matches(at, k, length);
+  }
+  if (T.learn && !found) {  // nothing that this SM's L1 knows of
+    at    = load_long_l2(T.long_words, h);
+    found = long_matches(at, k, length);
+    for (uint32_t hop = 1; !found && (at.v.x & kLongMore) && hop < kLongHops; ++hop) {
+      at    = load_long_l2(T.long_words, h ^ hop);
+      found = long_matches(at, k, length);
+    }
+  }
+  return found;
+}
+
 // one of the words that hold the L bytes of a key is zero
 __device__ __forceinline__ bool blank_word(const uint32_t k[4], uint32_t L)
 {
@@ -320,22 +326,8 @@ __device__ __forceinline__ bool recall_segment(TileSmem<TH>& S, const DeviceTabl
   window_words(S, s, k);
   k[0] &= km.x, k[1] &= km.y, k[2] &= km.z, k[3] &= km.w;
   if (T.learn && blank_word(k, L)) return false;
-  const uint32_t h = long_slot_of(k, L);
-  LongSlot at      = load_long(T.long_words, h);
-  bool found       = long_matches(at, k, L);
-  for (uint32_t hop = 1; !found && (at.v.x & kLongMore) && hop < kLongHops; ++hop) {
-    at    = load_long(T.long_words, h ^ hop);
-    found = long_matches(at, k, L);
-  }
-  if (T.learn && !found) {  // nothing that this SM's L1 knows of
-    at    = load_long_l2(T.long_words, h);
-    found = long_matches(at, k, L);
-    for (uint32_t hop = 1; !found && (at.v.x & kLongMore) && hop < kLongHops; ++hop) {
-      at    = load_long_l2(T.long_words, h ^ hop);
-      found = long_matches(at, k, L);
-    }
-  }
-  if (!found) return false;
+  LongSlot at;
+  if (!find_long(T, k, L, at)) return false;
   const uint32_t starts = at.v.x >> 16;
   S.tok[s]              = uint16_t((at.v.y & 0xFFFFu) - 1u);
   uint32_t m            = starts & (starts - 1u);
@@ -591,82 +583,106 @@ __device__ __noinline__ void merge_two(uint32_t ent, PairTable P, const uint16_t
 // ---- A long segment is hardly ever anything but a run of one byte with a few others around it.  One warp merges it as a
 //      list of (token, count) items, one per lane: a step merges either the pair inside an item, all its occurrences at
 //      once (left to right, which is what Algorithm 1 does over consecutive steps when no merge exposes a lower rank), or
-//      one pair across two items; it costs two table loads and some shuffles whatever the length of the run, where the
-//      pass routine sweeps the whole segment once per merge rank.  tok[0..L) holds the segment's byte tokens and receives
-//      the ids; list: room for 32 entries.  Returns the number of ids, or -1 when the segment has too many items (tok is then
+//      one pair across two items; it costs one round of table loads and some shuffles whatever the length of the run, where
+//      the pass routine sweeps the whole segment once per merge rank.  The segment's L tokens, still its bytes, stand at s
+//      and make way for the ids; list: room for 32 entries.  Returns the number of ids, or -1 when the segment has too many items (tok is then
 //      unchanged).  Monotone tables only. ----
 constexpr int kRunItems = 30;
-__device__ __noinline__ int merge_runs(uint16_t* tok, uint16_t* list, int L, const PairTable P)
+constexpr int kRunKept  = 3;           // items of a result that learn_run can keep
+constexpr int kRunMany  = 0x10000;     // flag on the result of merge_runs: more than that
+template <int TH>
+__device__ __noinline__ int merge_runs(int s, uint16_t* list, int L, const PairTable P)
 {
+  TileSmem<TH>& S   = tile_smem<TH>();
+  uint16_t* tok     = S.tok + s;
   const int lane    = threadIdx.x & 31;
-  const uint32_t lt = lanemask_lt();
   int m             = 0;  // items
-  for (int base = 0; base < L; base += 32) {
-    const int i       = base + lane;
-    const bool first  = i < L && (i == 0 || tok[i] != tok[i - 1]);
-    const uint32_t bb = __ballot_sync(0xFFFFFFFFu, first);
-    if (m + __popc(bb) > kRunItems) return -1;
-    if (first) list[m + __popc(bb & lt)] = uint16_t(i);
-    m += __popc(bb);
+  uint32_t carry    = 0;  // last byte of the 256 before
+  for (int base = 0; base < L; base += 256) {  // eight bytes per lane
+    const int i0 = base + 8 * lane;
+    uint32_t x0 = 0, x1 = 0;
+    if (i0 < L) {
+      const int at       = 16 + s + i0;
+      const uint32_t* wp = reinterpret_cast<const uint32_t*>(S.bytes + (at & ~3));
+      const uint32_t sh  = uint32_t(at & 3) * 8u;
+      x0 = __funnelshift_r(wp[0], wp[1], sh);
+      x1 = __funnelshift_r(wp[1], wp[2], sh);
+    }
+    uint32_t before = __shfl_up_sync(0xFFFFFFFFu, x1, 1);
+    if (lane == 0) before = carry;
+    carry = __shfl_sync(0xFFFFFFFFu, x1, 31);
+    const uint32_t d0 = __vcmpne4(x0, __funnelshift_l(before, x0, 8)), d1 = __vcmpne4(x1, __funnelshift_l(x0, x1, 8));
+    uint32_t starts   = (((d0 & 0x01010101u) * 0x01020408u) >> 24 & 15u) | ((((d1 & 0x01010101u) * 0x01020408u) >> 20) & 0xF0u);
+    if (i0 == 0) starts |= 1u;
+    starts &= low_bits(max(min(L - i0, 8), 0));
+    const int cnt = __popc(starts);
+    int inc       = cnt;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int y = __shfl_up_sync(0xFFFFFFFFu, inc, d);
+      if (lane >= d) inc += y;
+    }
+    const int total = __shfl_sync(0xFFFFFFFFu, inc, 31);
+    if (m + total > kRunItems) return -1;
+    for (int at = m + inc - cnt; starts; starts &= starts - 1) list[at++] = uint16_t(i0 + __ffs(int(starts)) - 1);
+    m += total;
   }
   __syncwarp();
-  auto rank_of = [&](uint32_t a, uint32_t b) {
-    const uint32_t key = (a << 16) | b;
-    return resolve_rank(__ldg(P.buckets + ((key * 0x9E3779B1u) >> 16)), key, P.overflow, P.overflow_mask);
-  };
+  // tc = token << 16 | count; rank = rank of (t, t) << 16 | rank of (t, next item's token)
   const int start = lane < m ? int(list[lane]) : L;
-  int cnt         = __shfl_down_sync(0xFFFFFFFFu, start, 1) - start;
-  uint32_t t      = lane < m ? uint32_t(tok[start]) : 0xFFFFu;
-  uint32_t next   = __shfl_down_sync(0xFFFFFFFFu, t, 1);
-  if (lane >= m) cnt = 0;
-  uint32_t inner = NONE, cross = NONE;  // rank of (t, t) and of (t, next item's token)
-  if (lane < m) inner = rank_of(t, t);
-  if (lane + 1 < m) cross = rank_of(t, next);
+  uint32_t tc     = uint32_t(__shfl_down_sync(0xFFFFFFFFu, start, 1) - start);
+  tc              = lane < m ? uint32_t(tok[start]) << 16 | tc : 0xFFFF0000u;
+  uint32_t rank   = 0xFFFFFFFFu;
+  auto probe = [&](uint32_t next, bool inner, bool cross) {  // both loads leave before anything waits for them
+    const uint32_t t = tc >> 16, key_i = t << 16 | t, key_c = t << 16 | next;
+    uint4 vi = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu), vc = vi;
+    if (inner) vi = __ldg(P.buckets + ((key_i * 0x9E3779B1u) >> 16));
+    if (cross) vc = __ldg(P.buckets + ((key_c * 0x9E3779B1u) >> 16));
+    if (inner) rank = (rank & 0xFFFFu) | resolve_rank(vi, key_i, P.overflow, P.overflow_mask) << 16;
+    if (cross) rank = (rank & 0xFFFF0000u) | resolve_rank(vc, key_c, P.overflow, P.overflow_mask);
+  };
+  probe(__shfl_down_sync(0xFFFFFFFFu, tc, 1) >> 16, lane < m && (tc & 0xFFFFu) >= 2u, lane + 1 < m);
   for (int step = 0; step < 2 * L; ++step) {
-    const uint32_t in   = cnt >= 2 ? inner : NONE;
+    const uint32_t in = (tc & 0xFFFFu) >= 2u ? rank >> 16 : NONE, cross = rank & 0xFFFFu;
     const uint32_t best = __reduce_min_sync(0xFFFFFFFFu, (min(in, cross) << 6) | uint32_t(lane << 1) | (in <= cross ? 0u : 1u));
     const uint32_t r    = best >> 6;
     if (r >= SEL || m > kRunItems) break;
-    const int a      = int(best >> 1) & 31;
-    const uint32_t c = P.merged_of_rank ? __ldg(P.merged_of_rank + r) : 256u + r;
-    const uint32_t ta = __shfl_sync(0xFFFFFFFFu, t, a), tb = __shfl_sync(0xFFFFFFFFu, t, a + 1);
-    const int na = __shfl_sync(0xFFFFFFFFu, cnt, a), nb = __shfl_sync(0xFFFFFFFFu, cnt, a + 1);
+    const int a       = int(best >> 1) & 31;
+    const uint32_t c  = P.merged_of_rank ? __ldg(P.merged_of_rank + r) : 256u + r;
+    const uint32_t xa = __shfl_sync(0xFFFFFFFFu, tc, a), xb = __shfl_sync(0xFFFFFFFFu, tc, a + 1);
+    const uint32_t na = xa & 0xFFFFu, nb = xb & 0xFFFFu;
     // the items that take the place of item a (and a + 1)
-    uint32_t xt[3];
-    int xn[3], k = 0, w;
+    uint32_t y0, y1, y2 = 0;
+    int k, w;
     if ((best & 1u) == 0u) {
-      w = 1;
-      xt[0] = c, xn[0] = na >> 1, k = 1;
-      xt[1] = ta, xn[1] = 1;
-      xt[2] = 0, xn[2] = 0;
-      k += na & 1;
+      w  = 1;
+      y0 = c << 16 | na >> 1;
+      y1 = (xa & 0xFFFF0000u) | 1u;
+      k  = 1 + int(na & 1u);
     } else {
       w = 2;
-      const bool keep_a = na > 1, keep_b = nb > 1;
-      xt[0] = keep_a ? ta : c, xn[0] = keep_a ? na - 1 : 1;
-      xt[1] = keep_a ? c : tb, xn[1] = keep_a ? 1 : nb - 1;
-      xt[2] = tb, xn[2] = nb - 1;
-      k = 1 + int(keep_a) + int(keep_b);
+      const bool keep_a = na > 1u, keep_b = nb > 1u;
+      const uint32_t one = c << 16 | 1u;
+      y0 = keep_a ? xa - 1u : one;
+      y1 = keep_a ? one : xb - 1u;
+      y2 = xb - 1u;
+      k  = 1 + int(keep_a) + int(keep_b);
     }
-    const int from      = (lane - (k - w)) & 31;
-    const uint32_t st   = __shfl_sync(0xFFFFFFFFu, t, from), si = __shfl_sync(0xFFFFFFFFu, inner, from), sc = __shfl_sync(0xFFFFFFFFu, cross, from);
-    const int sn        = __shfl_sync(0xFFFFFFFFu, cnt, from);
+    const int from    = (lane - (k - w)) & 31;
+    const uint32_t st = __shfl_sync(0xFFFFFFFFu, tc, from), sr = __shfl_sync(0xFFFFFFFFu, rank, from);
     m += k - w;
-    if (lane >= a + k) t = st, cnt = sn, inner = si, cross = sc;
+    if (lane >= a + k) tc = st, rank = sr;
     const int e = lane - a;
     if (e >= 0 && e < k) {
-      t     = e == 0 ? xt[0] : e == 1 ? xt[1] : xt[2];
-      cnt   = e == 0 ? xn[0] : e == 1 ? xn[1] : xn[2];
-      inner = NONE;
+      tc   = e == 0 ? y0 : e == 1 ? y1 : y2;
+      rank = 0xFFFFFFFFu;
     }
-    if (lane >= m) t = 0xFFFFu, cnt = 0, inner = NONE, cross = NONE;
-    next = __shfl_down_sync(0xFFFFFFFFu, t, 1);
-    if (e >= -1 && e < k && lane < m) {
-      cross = (lane + 1 < m) ? rank_of(t, next) : NONE;
-      if (cnt >= 2) inner = rank_of(t, t);
-    }
+    if (lane >= m) tc = 0xFFFF0000u, rank = 0xFFFFFFFFu;
+    const uint32_t next = __shfl_down_sync(0xFFFFFFFFu, tc, 1) >> 16;
+    if (e == -1) rank |= 0xFFFFu;
+    probe(next, e >= 0 && e < k && lane < m && (tc & 0xFFFFu) >= 2u, e >= -1 && e < k && lane + 1 < m);
   }
-  int inc = cnt;
+  int inc = int(tc & 0xFFFFu);
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
     const int y = __shfl_up_sync(0xFFFFFFFFu, inc, d);
@@ -674,38 +690,119 @@ __device__ __noinline__ int merge_runs(uint16_t* tok, uint16_t* list, int L, con
   }
   __syncwarp();
   for (int i = 0; i < m; ++i) {
-    const uint32_t ti = __shfl_sync(0xFFFFFFFFu, t, i);
-    const int hi = __shfl_sync(0xFFFFFFFFu, inc, i), lo = hi - __shfl_sync(0xFFFFFFFFu, cnt, i);
+    const uint32_t x = __shfl_sync(0xFFFFFFFFu, tc, i);
+    const int hi = __shfl_sync(0xFFFFFFFFu, inc, i), lo = hi - int(x & 0xFFFFu);
     for (int j = lo + lane; j < hi; j += 32)
-      if (GTK_IN(j, L, 13)) tok[j] = uint16_t(ti);
+      if (GTK_IN(j, L, 13)) tok[j] = uint16_t(x >> 16);
   }
   const int len = __shfl_sync(0xFFFFFFFFu, inc, 31);
+  if (lane < kRunKept) reinterpret_cast<uint32_t*>(list)[lane] = lane < m ? tc : 0xFFFF0000u;  // for learn_run
   __syncwarp();
-  return m > kRunItems ? -2 - len : len;
+  return m > kRunItems ? -2 - len : m > kRunKept ? len | kRunMany : len;
+}
+
+// Runs are remembered too, in a batch that learns: a long segment of up to three runs of a byte (a rule of dashes, padding in
+// front of a number) that ends as up to three runs of a token.  Key: bytes, where the runs start, length, and a word that no
+// text has in that place together with length code 31.  Value: token + 1 | count << 16 of each run.  A third of the time of
+// merge_runs, whose code is hardly ever in the instruction cache.
+constexpr uint32_t kRunCode = 31u;
+template <int TH>
+__device__ __forceinline__ bool run_key(const TileSmem<TH>& S, int s, int L, uint32_t k[4])
+{
+  if (L > 256) return false;
+  const int lane = threadIdx.x & 31, i0 = 8 * lane;
+  uint32_t starts = 0;
+  if (i0 < L) {  // starts of runs among eight bytes, but for the first of the segment
+    const int at       = 16 + s + i0;
+    const uint32_t* wp = reinterpret_cast<const uint32_t*>(S.bytes + (at & ~3));
+    const uint32_t sh  = uint32_t(at & 3) * 8u;
+    const uint32_t x0 = __funnelshift_r(wp[0], wp[1], sh), x1 = __funnelshift_r(wp[1], wp[2], sh);
+    const uint32_t d0 = __vcmpne4(x0, x0 << 8 | S.bytes[at - 1]), d1 = __vcmpne4(x1, __funnelshift_l(x0, x1, 8));
+    starts = (((d0 & 0x01010101u) * 0x01020408u) >> 24 & 15u) | ((((d1 & 0x01010101u) * 0x01020408u) >> 20) & 0xF0u);
+    starts &= low_bits(L - i0) & (lane == 0 ? 0xFEu : 0xFFu);
+  }
+  if (__reduce_add_sync(0xFFFFFFFFu, __popc(starts)) > 2) return false;
+  const int p1 = int(__reduce_min_sync(0xFFFFFFFFu, starts ? uint32_t(i0 + __ffs(int(starts)) - 1) : uint32_t(L)));
+  const int p2 = int(__reduce_max_sync(0xFFFFFFFFu, starts ? uint32_t(i0 + 31 - __clz(int(starts))) : 0u));
+  const uint8_t* bp = S.bytes + 16 + s;
+  k[0] = uint32_t(bp[0]) | uint32_t(bp[p1 < L ? p1 : 0]) << 8 | uint32_t(bp[p2]) << 16 | 1u << 24;
+  k[1] = uint32_t(p1) | uint32_t(p2) << 16;  // p1 > 0
+  k[2] = uint32_t(L);
+  k[3] = 0x736E7572u;
+  return true;
+}
+template <int TH>
+__device__ __noinline__ int recall_run(int s, int L, const DeviceTable& T)
+{
+  TileSmem<TH>& S = tile_smem<TH>();
+  uint32_t k[4];
+  LongSlot at;
+  if (!run_key(S, s, L, k) || !find_long(T, k, kRunCode, at)) return -1;
+  const int n0 = int(at.v.y >> 16), n1 = n0 + int(at.v.z >> 16), n2 = n1 + int(at.v.w >> 16);
+  for (int j = threadIdx.x & 31; j < n2; j += 32)
+    if (GTK_IN(j, L, 16)) S.tok[s + j] = uint16_t(((j < n0 ? at.v.y : j < n1 ? at.v.z : at.v.w) & 0xFFFFu) - 1u);
+  __syncwarp();
+  return n2;
+}
+template <int TH>
+__device__ __noinline__ void learn_run(int s, int L, const uint32_t* items, uint4* words)
+{
+  const int lane = threadIdx.x & 31;
+  uint32_t k[4];
+  if (!run_key(tile_smem<TH>(), s, L, k)) return;
+  const uint32_t h = long_slot_of(k, kRunCode), want = kRunCode | (k[0] * 0x9E3779B1u ^ k[1] * 0x85EBCA77u ^ k[2]) << 16;
+  uint32_t meta = 1;
+  if (lane < int(kLongHops))
+    asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(meta) : "l"(reinterpret_cast<uint32_t*>(words + 2 * (h ^ uint32_t(lane))) + 4));
+  const int hop = __ffs(int(__ballot_sync(0xFFFFFFFFu, meta == 0u))) - 1;  // first empty slot of the row
+  if (hop < 0 || __any_sync(0xFFFFFFFFu, (meta & ~kLongMore) == want)) return;
+  uint32_t* slot = reinterpret_cast<uint32_t*>(words + 2 * (h ^ uint32_t(hop)));
+  if (lane < hop && !(meta & kLongMore)) atomicOr(reinterpret_cast<uint32_t*>(words + 2 * (h ^ uint32_t(lane))) + 4, kLongMore);
+  uint32_t was = 1;
+  if (lane == 0) was = atomicCAS(slot + 4, 0u, want);
+  if (__shfl_sync(0xFFFFFFFFu, was, 0) != 0u) return;  // taken meanwhile
+  if (lane == 0) *reinterpret_cast<uint4*>(slot) = make_uint4(k[0], k[1], k[2], k[3]);
+  if (lane < kRunKept) slot[5 + lane] = ((items[lane] >> 16) + 1u & 0xFFFFu) | items[lane] << 16 | (items[lane] == 0xFFFF0000u ? 0xFFFFu : 0u);
 }
 
 // ---- multi-byte segments, every warp those that start in its own 512 positions: listed, looked up in the table of short
 //      strings, what is left in the table of long ones.  One or two misses are merged on the spot (a batch that learns has
-//      hardly more), others join the CTA's list.  Ends with a barrier. ----
+//      hardly more), others join the CTA's list, as the long segments do theirs.  Ends with a barrier. ----
 template <int TH>
 __device__ __forceinline__ void tile_lookup(TileSmem<TH>& S, const Span& sp, const DeviceTable& T, int* status)
 {
   using Entry = typename TileSmem<TH>::Entry;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t lt = lanemask_lt();
-  if (warp == TileSmem<TH>::kWarps - 1 && lane == 0) {  // while the bitmap still holds segment starts only
+  // Everything that is read from the bitmap of starts is read in front of the barrier, because segments that are done mark
+  // their tokens in it, also those that reach into the next warp's positions.
+  const int base    = tid * 16;
+  const uint32_t w0 = S.cut[tid >> 1], w1 = S.cut[(tid >> 1) + 1], w2 = S.cut[(tid >> 1) + 2];
+  const uint32_t a  = __funnelshift_r(w0, w1, (tid & 1) * 16), a2 = __funnelshift_r(w1, w2, (tid & 1) * 16);  // 64 positions from base on
+  uint32_t m = a & ~(a >> 1) & range_mask(base, sp.own_lo, sp.own_hi) & 0xFFFFu;  // starts whose next position is no start
+  if (m) {  // only the last of the segments that start in sixteen positions can be a long one
+    const int b = 31 - __clz(int(m));
+    if (unsigned(__ffs(int(__funnelshift_r(a, a2, b + 1))) - 1) >= unsigned(kThreadSegMax)) {
+      const int long_at = base + b;
+      m ^= 1u << b;
+      if (next_cut(S, long_at) >= S.kWin && sp.wlen == S.kWin) {
+        S.over_start = long_at;
+      } else {
+        const int q = atomicAdd(&S.nlong, 1);
+        if (q < S.kLong && GTK_IN(long_at, S.kOwn, 3)) S.longq[q] = uint16_t(long_at);
+        else atomicMax(status, int(kStatusLongQueueOverflow));
+      }
+    }
+  }
+  if (warp == TileSmem<TH>::kWarps - 1 && lane == 0) {
     S.first = next_cut(S, sp.own_lo - 1);
     S.end   = min(next_cut(S, sp.own_hi - 1), sp.wlen);
   }
+  __syncthreads();
   if (warp * 512 < sp.own_hi) {
     Entry* list = S.work + warp * TileSmem<TH>::kRegion;
     int tot;
     {
-      const int base    = tid * 16;
-      const uint32_t w0 = S.cut[tid >> 1], w1 = S.cut[(tid >> 1) + 1], w2 = S.cut[(tid >> 1) + 2];
-      const int sh      = (tid & 1) * 16;
-      const uint32_t a  = __funnelshift_r(w0, w1, sh), a2 = __funnelshift_r(w1, w2, sh);  // 64 positions from base on
-      uint32_t m = a & ~(a >> 1) & range_mask(base, sp.own_lo, sp.own_hi) & 0xFFFFu;  // starts whose next position is no start
       const int cnt = __popc(m);
       int inc       = cnt;
 #pragma unroll
@@ -718,11 +815,9 @@ __device__ __forceinline__ void tile_lookup(TileSmem<TH>& S, const Span& sp, con
       while (m) {
         const int b = __ffs(int(m)) - 1;
         m &= m - 1;
-        const int len = __ffs(int(__funnelshift_r(a, a2, b + 1)));  // 0: more than 32
-        const bool is_short = unsigned(len - 1) < unsigned(kThreadSegMax);
-        if (GTK_IN(at, 256, 4)) list[at] = is_short ? Entry(((base + b) << 4) | (len - 1)) : Entry(0);
+        const int len = __ffs(int(__funnelshift_r(a, a2, b + 1)));
+        if (GTK_IN(at, 256, 4)) list[at] = Entry(((base + b) << 4) | (len - 1));
         ++at;
-        if (!is_short) note_long_segment<TH>(base + b, sp.wlen, status);
       }
     }
     __syncwarp();
@@ -791,7 +886,14 @@ __device__ __noinline__ void merge_long_segments(const DeviceTable& T, int* stat
     const int L = next_cut(S, s) - s;
     if (!(GTK_IN(s, S.kWin, 19) && GTK_IN(s + L, S.kWin + 1, 20))) continue;
     int len = -1;
-    if (T.monotone) len = merge_runs(S.tok + s, area, L, pair_table(T));
+    if (T.monotone) {
+      if (T.learn) len = recall_run<TH>(s, L, T);
+      if (len < 0) {
+        len = merge_runs<TH>(s, area, L, pair_table(T));
+        if (T.learn && len >= 0 && !(len & kRunMany)) learn_run<TH>(s, L, reinterpret_cast<const uint32_t*>(area), T.long_words);
+        if (len >= 0) len &= kRunMany - 1;
+      }
+    }
     if (len < 0) {
       // too many different tokens (len -1: from the start; else -2 - len tokens are left to go on with)
       const int left = len == -1 ? L : -2 - len;
