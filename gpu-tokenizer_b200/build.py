@@ -45,7 +45,7 @@ def _run(cmd: list[str]) -> None:
 
 def build_cuda(force: bool = False, ptxas_verbose: bool = False) -> str:
     srcs = [os.path.join(CSRC, f) for f in ("gtk_kernels.cu", "gtk_api.cu", "gtk_table.cpp")]
-    deps = srcs + [os.path.join(CSRC, f) for f in ("gtk_device.cuh", "gtk_tile.cuh", "gtk_table.hpp")] + \
+    deps = srcs + [os.path.join(CSRC, f) for f in ("gtk_device.cuh", "gtk_tile.cuh", "gtk_table.hpp", "gtk_crew.hpp")] + \
         [os.path.join(INCLUDE, "gputok_b200.h")]
     if force or _stale(LIB, deps):
         nvcc = os.environ.get("NVCC", "nvcc")
@@ -57,7 +57,7 @@ def build_cuda(force: bool = False, ptxas_verbose: bool = False) -> str:
 def build_cuda_checked(force: bool = False) -> str:
     """The bounds-checked build (stands in for a memory sanitizer, which this pool does not offer)."""
     srcs = [os.path.join(CSRC, f) for f in ("gtk_kernels.cu", "gtk_api.cu", "gtk_table.cpp")]
-    deps = srcs + [os.path.join(CSRC, f) for f in ("gtk_device.cuh", "gtk_tile.cuh", "gtk_table.hpp")] + \
+    deps = srcs + [os.path.join(CSRC, f) for f in ("gtk_device.cuh", "gtk_tile.cuh", "gtk_table.hpp", "gtk_crew.hpp")] + \
         [os.path.join(INCLUDE, "gputok_b200.h")]
     if force or _stale(LIB_CHECKED, deps):
         nvcc = os.environ.get("NVCC", "nvcc")

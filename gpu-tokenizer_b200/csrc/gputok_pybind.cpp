@@ -18,10 +18,8 @@
 #include <pybind11/pybind11.h>
 #include <pybind11/stl.h>
 
-#include <cstdlib>
 #include <cstring>
 #include <mutex>
-#include <new>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -48,13 +46,12 @@ class GpuTokenizer {
   ~GpuTokenizer()
   {
     for (PyObject* o : id_objects_) Py_XDECREF(o);
-    release_bytes();
     gtk_destroy(h_);
   }
   GpuTokenizer(const GpuTokenizer&) = delete;
   GpuTokenizer& operator=(const GpuTokenizer&) = delete;
 
-  // One call at a time from flattening to reading the result.  Waiting happens without the GIL, which the holder needs.
+  // One call at a time from collecting the strings to reading the result.  Waiting happens without the GIL, which the holder needs.
   class Turn {
    public:
     explicit Turn(GpuTokenizer& t) : lock_(t.mu_, std::try_to_lock)
@@ -68,69 +65,59 @@ class GpuTokenizer {
     std::unique_lock<std::mutex> lock_;
   };
 
-  // list[str] -> one byte buffer (page-locked, kept between calls: the upload is one DMA) + offsets, UTF-8 as pybind's
-  // str -> std::string caster does for the reference, without a std::string per text.
-  void flatten(const py::object& texts)
+  // Where the strings lie and their offsets, UTF-8 as pybind's str -> std::string caster gives it to the reference; they are
+  // gathered inside the call (gtk_encode_strings).  `keep` holds them meanwhile: the caller's list may change while
+  // the GIL is released.
+  struct Keep {
+    py::object items;
+    std::vector<std::string> strings;
+  };
+  void collect(const py::object& texts, Keep& keep)
   {
     PyObject* seq = texts.ptr();
     if (PyList_Check(seq) || PyTuple_Check(seq)) {
-      const Py_ssize_t n = PySequence_Fast_GET_SIZE(seq);
-      PyObject** items   = PySequence_Fast_ITEMS(seq);
+      keep.items = PyTuple_Check(seq) ? texts : py::reinterpret_steal<py::object>(PyList_AsTuple(seq));
+      if (!keep.items) throw py::error_already_set();
+      const Py_ssize_t n = PyTuple_GET_SIZE(keep.items.ptr());
       parts_.resize(size_t(n));
       off_.resize(size_t(n) + 1);
       int64_t total = 0;
       bool plain    = true;
       for (Py_ssize_t i = 0; i < n && plain; ++i) {
+        PyObject* o = PyTuple_GET_ITEM(keep.items.ptr(), i);
+        if (i + 16 < n) __builtin_prefetch(PyTuple_GET_ITEM(keep.items.ptr(), i + 16));  // strings lie all over the heap
         Py_ssize_t len = 0;
-        const char* p  = PyUnicode_Check(items[i]) ? PyUnicode_AsUTF8AndSize(items[i], &len) : nullptr;
-        plain          = p != nullptr;
+        const char* p  = nullptr;
+        if (PyUnicode_Check(o)) {
+          if (PyUnicode_IS_COMPACT_ASCII(o)) {
+            p   = reinterpret_cast<const char*>(PyUnicode_1BYTE_DATA(o));
+            len = PyUnicode_GET_LENGTH(o);
+          } else {
+            p = PyUnicode_AsUTF8AndSize(o, &len);
+          }
+        }
+        plain             = p != nullptr;
         off_[size_t(i)]   = total;
-        parts_[size_t(i)] = p;
+        parts_[size_t(i)] = reinterpret_cast<const uint8_t*>(p);
         total += len;
       }
-      if (plain) {
-        off_[size_t(n)] = total;
-        reserve(size_t(total));
-        for (Py_ssize_t i = 0; i < n; ++i) {
-          const size_t len = size_t(off_[size_t(i) + 1] - off_[size_t(i)]);
-          if (len) std::memcpy(bytes_ + off_[size_t(i)], parts_[size_t(i)], len);
-        }
-        return;
-      }
+      off_[size_t(n)] = total;
+      if (plain) return;
       PyErr_Clear();  // something else than str, or a str without a UTF-8 form: the caster below decides
     }
-    std::vector<std::string> strings;
     try {
-      strings = texts.cast<std::vector<std::string>>();
+      keep.strings = texts.cast<std::vector<std::string>>();
     } catch (const py::cast_error&) {
       throw py::type_error("texts must be a sequence of str or bytes");
     }
+    parts_.clear();
     off_.assign(1, 0);
-    for (auto& t : strings) off_.push_back(off_.back() + int64_t(t.size()));
-    reserve(size_t(off_.back()));
-    for (size_t i = 0; i < strings.size(); ++i)
-      if (!strings[i].empty()) std::memcpy(bytes_ + off_[i], strings[i].data(), strings[i].size());
+    for (auto& t : keep.strings) {
+      parts_.push_back(reinterpret_cast<const uint8_t*>(t.data()));
+      off_.push_back(off_.back() + int64_t(t.size()));
+    }
   }
   size_t n_texts() const { return off_.size() - 1; }
-
-  void reserve(size_t bytes)
-  {
-    if (bytes <= cap_) return;
-    release_bytes();
-    const size_t want = bytes + bytes / 4 + 4096;
-    bytes_  = static_cast<uint8_t*>(gtk_pinned_alloc(want));
-    pinned_ = bytes_ != nullptr;
-    if (!pinned_) bytes_ = static_cast<uint8_t*>(std::malloc(want));  // a host-only handle, no device to lock pages for
-    if (!bytes_) throw std::bad_alloc();
-    cap_ = want;
-  }
-  void release_bytes()
-  {
-    if (pinned_) gtk_pinned_free(bytes_);
-    else std::free(bytes_);
-    bytes_ = nullptr;
-    cap_   = 0;
-  }
 
   void check(int rc) const
   {
@@ -178,12 +165,13 @@ class GpuTokenizer {
   py::tuple tokenize(const py::object& texts, int mode)
   {
     Turn turn(*this);
-    flatten(texts);
+    Keep keep;
+    collect(texts, keep);
     float ms = 0.f;
     int rc;
     {
       py::gil_scoped_release nogil;
-      rc = gtk_encode(h_, mode, bytes_, off_.data(), int64_t(n_texts()), &ms);
+      rc = gtk_encode_strings(h_, mode, parts_.data(), off_.data(), int64_t(n_texts()), &ms);
     }
     check(rc);
     return lists_from_result(n_texts(), ms);
@@ -196,11 +184,15 @@ class GpuTokenizer {
     else if (rule == "localmin") r = GTK_RULE_LOCALMIN;
     else throw std::invalid_argument("merge_rule must be 'greedy' or 'localmin'");
     Turn turn(*this);
-    flatten(texts);
+    Keep keep;
+    collect(texts, keep);
+    std::vector<uint8_t> bytes(size_t(off_.back()));
+    for (size_t t = 0; t < n_texts(); ++t)
+      if (off_[t + 1] > off_[t]) std::memcpy(bytes.data() + off_[t], parts_[t], size_t(off_[t + 1] - off_[t]));
     int rc;
     {
       py::gil_scoped_release nogil;
-      rc = gtk_encode_cpu(h_, r, bytes_, off_.data(), int64_t(n_texts()));
+      rc = gtk_encode_cpu(h_, r, bytes.data(), off_.data(), int64_t(n_texts()));
     }
     check(rc);
     return id_lists(n_texts());
@@ -213,12 +205,13 @@ class GpuTokenizer {
     else if (mode == "base") m = GTK_MODE_BASE;
     else throw std::invalid_argument("mode must be 'opt' or 'base'");
     Turn turn(*this);
-    flatten(texts);
+    Keep keep;
+    collect(texts, keep);
     float ms = 0.f;
     int rc;
     {
       py::gil_scoped_release nogil;
-      rc = gtk_encode(h_, m, bytes_, off_.data(), int64_t(n_texts()), &ms);
+      rc = gtk_encode_strings(h_, m, parts_.data(), off_.data(), int64_t(n_texts()), &ms);
     }
     check(rc);
     int64_t n_ids = 0, n_chunks = 0;
@@ -294,11 +287,8 @@ class GpuTokenizer {
  private:
   gtk_tokenizer* h_ = nullptr;
   std::mutex mu_;  // see Turn; guards what follows
-  uint8_t* bytes_ = nullptr;
-  size_t cap_     = 0;
-  bool pinned_    = false;
   std::vector<int64_t> off_;
-  std::vector<const char*> parts_;
+  std::vector<const uint8_t*> parts_;
   std::vector<PyObject*> id_objects_;
 };
 

@@ -20,6 +20,7 @@
 #include <string>
 #include <vector>
 
+#include "gtk_crew.hpp"
 #include "gtk_device.cuh"
 #include "gtk_table.hpp"
 
@@ -236,6 +237,8 @@ struct gtk_tokenizer {
   PinBuf h_mid;
   PinBuf h_out;                // results of encode_host_tiles, offsets of encode_host_pieces
   DevBuf d_piece_ids;          // ids in front of every piece
+  PinBuf h_gather;             // strings of gtk_encode_strings, back to back
+  mutable gtk::Crew crew;
   PinBuf h_marks;              // completion mark and id count of every piece
   std::vector<cudaEvent_t> piece_ev;
   double ids_per_byte = 0.4;  // room for ids that they start with; grows with the texts it meets
@@ -923,11 +926,64 @@ bool wait_for_mark(volatile const int64_t* mark, int64_t seq, cudaStream_t s, co
   return true;
 }
 
-int encode_host_small(gtk_tokenizer* h, const uint8_t* bytes, const int64_t* text_offsets, int64_t n_texts,
+// The text of a call: in one buffer, or every string where it lies (gtk_encode_strings).
+struct Source {
+  const uint8_t* bytes;         // nullptr: strings
+  const uint8_t* const* parts;  // text t is parts[t][0 .. text_offsets[t + 1] - text_offsets[t])
+  const int64_t* text_offsets;
+  int64_t n_texts;
+
+  void copy_texts(uint8_t* all, int64_t t, int64_t end) const  // to where they belong in the whole
+  {
+    for (; t < end; ++t)
+      if (const size_t n = size_t(text_offsets[t + 1] - text_offsets[t])) std::memcpy(all + text_offsets[t], parts[t], n);
+  }
+  void copy_all(uint8_t* to) const
+  {
+    if (bytes) std::memcpy(to, bytes, size_t(text_offsets[n_texts]));
+    else copy_texts(to, 0, n_texts);
+  }
+};
+
+// Gathers the strings of a source block by block, with the crew's help, into page-locked memory; ready(hi) returns the whole
+// buffer once its first hi bytes are there.  A plain buffer is ready as it is.
+class Gather {
+ public:
+  Gather(gtk_tokenizer* h, const Source& src) : src_(src)
+  {
+    if (src.bytes) return;
+    const int64_t n = src.text_offsets[src.n_texts];
+    h->h_gather.reserve(size_t(n));
+    to_ = h->h_gather.as<uint8_t>();
+    first_.push_back(0);
+    for (int64_t t = 1; t < src.n_texts; ++t)
+      if (src.text_offsets[t] - src.text_offsets[first_.back()] >= kBlock) first_.push_back(t);
+    first_.push_back(src.n_texts);
+    job_.reset(new gtk::Crew::Job(h->crew, int64_t(first_.size()) - 1, [this](int64_t i) {
+      src_.copy_texts(to_, first_[size_t(i)], first_[size_t(i) + 1]);
+    }));
+  }
+  const uint8_t* ready(int64_t hi)
+  {
+    if (!job_) return src_.bytes;
+    while (at_ + 1 < first_.size() && src_.text_offsets[first_[at_]] < hi) job_->wait(int64_t(at_++));
+    return to_;
+  }
+
+ private:
+  static constexpr int64_t kBlock = 64 << 10;
+  const Source src_;
+  uint8_t* to_ = nullptr;
+  std::vector<int64_t> first_;  // first text of every block
+  size_t at_ = 0;
+  std::unique_ptr<gtk::Crew::Job> job_;
+};
+
+int encode_host_small(gtk_tokenizer* h, const Source& src, const int64_t* text_offsets, int64_t n_texts,
                       int64_t n_bytes, float* kernel_ms)
 {
   std::memcpy(h->small_in_h + kSmallInOff, text_offsets, size_t(n_texts + 1) * 8);
-  std::memcpy(h->small_in_h + kSmallInBytes, bytes, size_t(n_bytes));
+  src.copy_all(h->small_in_h + kSmallInBytes);
   Plan p = plan_batch(h, h->small_in_d + kSmallInBytes, n_bytes,
                       reinterpret_cast<const int64_t*>(h->small_in_d + kSmallInOff), n_texts,
                       reinterpret_cast<int32_t*>(h->small_out_d + kSmallOutIds), gtk::kSmallMaxBytes,
@@ -963,6 +1019,7 @@ int encode_host_small(gtk_tokenizer* h, const uint8_t* bytes, const int64_t* tex
 // pack kernel, which writes ids and offsets into page-locked memory and then the call number, for which the host waits.
 // No chunker, no scan, no copy back, no synchronisation.
 constexpr int64_t kTextInHeaderBytes = 64 << 10;
+constexpr int64_t kGatherStep        = 512 << 10;  // strings go up in steps of this while the next ones are gathered
 
 // The tile records of a batch, as k_tile_info makes them on the device.
 void lay_tiles(const int64_t* text_off, const int64_t* chunk_base, int64_t n_texts, int64_t n_bytes, int64_t chunk,
@@ -992,7 +1049,7 @@ void lay_tiles(const int64_t* text_off, const int64_t* chunk_base, int64_t n_tex
   }
 }
 
-int encode_host_tiles(gtk_tokenizer* h, const uint8_t* bytes, const int64_t* text_offsets, int64_t n_texts, int64_t n_bytes,
+int encode_host_tiles(gtk_tokenizer* h, const Source& src, const int64_t* text_offsets, int64_t n_texts, int64_t n_bytes,
                       float* kernel_ms)
 {
   auto up = [](size_t x) { return (x + 63) & ~size_t(63); };
@@ -1008,7 +1065,12 @@ int encode_host_tiles(gtk_tokenizer* h, const uint8_t* bytes, const int64_t* tex
   cudaStream_t s = h->stream;
   if (!with_text) {
     h->d_bytes.reserve(size_t(n_bytes) + 32);
-    GTK_CUDA(cudaMemcpyAsync(h->d_bytes.p, bytes, size_t(n_bytes), cudaMemcpyHostToDevice, s));
+    Gather gather(h, src);
+    const int64_t step = src.bytes ? n_bytes : kGatherStep;
+    for (int64_t lo = 0; lo < n_bytes; lo += step) {
+      const int64_t hi = std::min(lo + step, n_bytes);
+      GTK_CUDA(cudaMemcpyAsync(h->d_bytes.as<uint8_t>() + lo, gather.ready(hi) + lo, size_t(hi - lo), cudaMemcpyHostToDevice, s));
+    }
   }
   std::memset(hp, 0, o_off);  // totals, counters, group counts
   int64_t C = 0;
@@ -1027,7 +1089,7 @@ int encode_host_tiles(gtk_tokenizer* h, const uint8_t* bytes, const int64_t* tex
   reinterpret_cast<int64_t*>(hp)[0] = C;
   lay_tiles(text_offsets, reinterpret_cast<const int64_t*>(hp + o_base), n_texts, n_bytes, chunk,
             reinterpret_cast<gtk::TileInfo*>(hp + o_info));
-  if (with_text) std::memcpy(hp + o_text, bytes, size_t(n_bytes));
+  if (with_text) src.copy_all(hp + o_text);
   GTK_CUDA(cudaMemcpyAsync(dp, hp, header, cudaMemcpyHostToDevice, s));
 
   // [64-byte header | text id offsets | chunk id offsets | ids]
@@ -1115,7 +1177,7 @@ std::vector<int64_t> piece_ends(int64_t n_bytes)
   return ends;
 }
 
-int encode_host_pieces(gtk_tokenizer* h, const uint8_t* bytes, const int64_t* text_offsets, int64_t n_texts, int64_t n_bytes,
+int encode_host_pieces(gtk_tokenizer* h, const Source& src, const int64_t* text_offsets, int64_t n_texts, int64_t n_bytes,
                        float* kernel_ms)
 {
   auto up = [](size_t x) { return (x + 63) & ~size_t(63); };
@@ -1163,6 +1225,7 @@ int encode_host_pieces(gtk_tokenizer* h, const uint8_t* bytes, const int64_t* te
   launches += gtk::launch_scan_texts(b, learned, s) + gtk::launch_tile_info(b, s);
   GTK_CUDA(cudaGetLastError());
 
+  Gather gather(h, src);
   int64_t have = 0;  // ids whose copy has been issued
   // the ids of piece i, once its mark is there; wait: for the mark.  false: not there yet
   auto collect = [&](size_t i, bool wait) {
@@ -1192,7 +1255,7 @@ int encode_host_pieces(gtk_tokenizer* h, const uint8_t* bytes, const int64_t* te
     for (size_t i = 0; i < np; ++i) {
       cudaEvent_t* ev  = &h->piece_ev[4 * i];
       const int64_t lo = i ? ends[i - 1] : 0;
-      GTK_CUDA(cudaMemcpyAsync(h->d_bytes.as<uint8_t>() + lo, bytes + lo, size_t(ends[i] - lo), cudaMemcpyHostToDevice, h->in_stream));
+      GTK_CUDA(cudaMemcpyAsync(h->d_bytes.as<uint8_t>() + lo, gather.ready(ends[i]) + lo, size_t(ends[i] - lo), cudaMemcpyHostToDevice, h->in_stream));
       GTK_CUDA(cudaEventRecord(ev[0], h->in_stream));
       GTK_CUDA(cudaStreamWaitEvent(s, ev[0], 0));
       // a tile may need the text to the end of its last chunk: such tiles wait for the next piece
@@ -1261,7 +1324,7 @@ void release_handle(gtk_tokenizer* h)
                       &h->d_unit_cnt, &h->d_chunk_cnt, &h->d_tile_info, &h->d_chunk_rel, &h->d_text_rel, &h->d_group_base, &h->d_chunk_id_off, &h->d_text_id_off,
                       &h->d_out_ids, &h->d_seg_scratch, &h->d_scan_sums, &h->d_totals, &h->d_out_pack, &h->d_fast_in})
       b->release();
-    for (PinBuf* b : {&h->h_ids, &h->h_text_id_off, &h->h_chunk_id_off, &h->h_totals, &h->h_piece_off, &h->h_piece_id_off, &h->h_chunk_id_all, &h->h_out_pack, &h->h_mid, &h->h_out, &h->h_marks, &h->h_fast_in}) b->release();
+    for (PinBuf* b : {&h->h_ids, &h->h_text_id_off, &h->h_chunk_id_off, &h->h_totals, &h->h_piece_off, &h->h_piece_id_off, &h->h_chunk_id_all, &h->h_out_pack, &h->h_mid, &h->h_out, &h->h_gather, &h->h_marks, &h->h_fast_in}) b->release();
     for (DevBuf* b : {&h->d_piece_off, &h->d_piece_id_off, &h->d_chunk_id_all, &h->d_piece_ids}) b->release();
     if (h->small_in_h) cudaFreeHost(h->small_in_h);
     if (h->small_out_h) cudaFreeHost(h->small_out_h);
@@ -1515,8 +1578,8 @@ GTK_API int gtk_encode_device(gtk_tokenizer* h, int mode, const uint8_t* d_bytes
   }
 }
 
-GTK_API int gtk_encode(gtk_tokenizer* h, int mode, const uint8_t* bytes, const int64_t* text_offsets,
-                       int64_t n_texts, float* kernel_ms)
+static int encode_host(gtk_tokenizer* h, int mode, const uint8_t* bytes, const uint8_t* const* parts,
+                       const int64_t* text_offsets, int64_t n_texts, float* kernel_ms)
 {
   if (!h) return GTK_ERR_INVALID_ARG;
   std::lock_guard<std::mutex> lock(h->mu);
@@ -1545,13 +1608,16 @@ GTK_API int gtk_encode(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
       h->h_chunk_id_off.as<int64_t>()[0] = 0;
       return GTK_OK;
     }
-    if (!bytes) return h->fail(GTK_ERR_INVALID_ARG, "bytes is null");
+    if (!bytes && !parts) return h->fail(GTK_ERR_INVALID_ARG, "bytes is null");
+    const Source src{bytes, parts, text_offsets, n_texts};
     if (h->wide && mode == GTK_MODE_LOCALMIN) return h->fail(GTK_ERR_TABLE, kWideNoLocalmin);
     if (!h->wide && mode == GTK_MODE_OPT && n_bytes <= gtk::kSmallMaxBytes && n_texts <= gtk::kSmallMaxTexts)
-      return encode_host_small(h, bytes, text_offsets, n_texts, n_bytes, kernel_ms);
+      return encode_host_small(h, src, text_offsets, n_texts, n_bytes, kernel_ms);
     if (!h->wide && mode == GTK_MODE_OPT)
-      return n_bytes >= kPiecesMinBytes ? encode_host_pieces(h, bytes, text_offsets, n_texts, n_bytes, kernel_ms)
-                                        : encode_host_tiles(h, bytes, text_offsets, n_texts, n_bytes, kernel_ms);
+      return n_bytes >= kPiecesMinBytes ? encode_host_pieces(h, src, text_offsets, n_texts, n_bytes, kernel_ms)
+                                        : encode_host_tiles(h, src, text_offsets, n_texts, n_bytes, kernel_ms);
+    Gather gather(h, src);
+    bytes = gather.ready(n_bytes);  // the kernels that work chunk by chunk take one buffer
     if (n_bytes >= kSliceThresholdBytes) return encode_host_sliced(h, mode, bytes, text_offsets, n_texts, n_bytes, kernel_ms);
     cudaStream_t s = h->stream;
     h->d_bytes.reserve(size_t(n_bytes) + 32);
@@ -1616,6 +1682,18 @@ GTK_API int gtk_encode(gtk_tokenizer* h, int mode, const uint8_t* bytes, const i
   } catch (const CudaFail& f) {
     return h->fail(GTK_ERR_CUDA, f.what);
   }
+}
+
+GTK_API int gtk_encode(gtk_tokenizer* h, int mode, const uint8_t* bytes, const int64_t* text_offsets, int64_t n_texts,
+                       float* kernel_ms)
+{
+  return encode_host(h, mode, bytes, nullptr, text_offsets, n_texts, kernel_ms);
+}
+
+GTK_API int gtk_encode_strings(gtk_tokenizer* h, int mode, const uint8_t* const* texts, const int64_t* text_offsets,
+                               int64_t n_texts, float* kernel_ms)
+{
+  return encode_host(h, mode, nullptr, texts, text_offsets, n_texts, kernel_ms);
 }
 
 GTK_API int gtk_encode_cpu(gtk_tokenizer* h, int rule, const uint8_t* bytes, const int64_t* text_offsets,
@@ -1769,7 +1847,29 @@ GTK_API int gtk_decode(const gtk_tokenizer* h, const int32_t* ids, int64_t n_ids
                        int64_t* n_out)
 {
   if (!h || (n_ids > 0 && !ids)) return GTK_ERR_INVALID_ARG;
-  const int64_t k = h->table->decode(ids, n_ids, out, out_capacity);
+  // Long ones block by block with the crew's help: the lengths first, then every block to its place.  Whatever is not plain
+  // (an unknown id, too little room) is left to the one pass that finds out what.
+  constexpr int64_t kBlock = 16384;
+  int64_t k = -1;
+  if (n_ids >= 4 * kBlock) {
+    const int64_t nb = (n_ids + kBlock - 1) / kBlock;
+    std::vector<int64_t> at(size_t(nb) + 1, 0);
+    gtk::Crew::Job(h->crew, nb, [&](int64_t i) {
+      at[size_t(i) + 1] = h->table->decode(ids + i * kBlock, std::min(kBlock, n_ids - i * kBlock), nullptr, 0);
+    }).finish();
+    bool plain = true;
+    for (int64_t i = 0; i < nb; ++i) {
+      plain = plain && at[size_t(i) + 1] >= 0;
+      at[size_t(i) + 1] += at[size_t(i)];
+    }
+    plain = plain && (!out || at[size_t(nb)] <= out_capacity);
+    if (plain && out)
+      gtk::Crew::Job(h->crew, nb, [&](int64_t i) {
+        h->table->decode(ids + i * kBlock, std::min(kBlock, n_ids - i * kBlock), out + at[size_t(i)], at[size_t(i) + 1] - at[size_t(i)]);
+      }).finish();
+    if (plain) k = at[size_t(nb)];
+  }
+  if (k < 0) k = h->table->decode(ids, n_ids, out, out_capacity);
   if (k == -1 - n_ids) return h->fail(GTK_ERR_CAPACITY, "decode buffer too small");
   if (k < 0) return h->fail(GTK_ERR_INVALID_ARG, "id " + std::to_string(ids[-1 - k]) + " has no byte string");
   if (n_out) *n_out = k;

@@ -388,8 +388,9 @@ void HostTable::build_derived()
 }
 
 // Bound by the loads of the lengths and strings from the host's L2 and by the unaligned stores.  1 MiB of the sample novel
-// (a quarter of a million ids): 2.1 ms per pass through one std::string per id and a memcpy of its length; 0.1 ms to count
-// (four lengths at a time, one test for all) and 0.35 ms to write (16 bytes into place whatever the length) now.
+// (a quarter of a million ids) through the Python call: 2.5 ms with one std::string per id and a memcpy of its length; four
+// lengths at a time with one test for all to count, 16 bytes into place whatever the length to write: 384 us on one core;
+// 204 us with three helpers (gtk_decode).
 int64_t HostTable::decode(const int32_t* ids, int64_t n_ids, uint8_t* out, int64_t capacity) const
 {
   const uint8_t* length = decode_length.data();

@@ -134,6 +134,12 @@ GTK_API int gtk_table_info_get(const gtk_tokenizer* h, gtk_table_info* out);
 GTK_API int gtk_encode(gtk_tokenizer* h, int mode, const uint8_t* bytes, const int64_t* text_offsets,
                        int64_t n_texts, float* kernel_ms);
 
+/* The same for strings that lie anywhere: text t is texts[t][0 .. text_offsets[t+1] - text_offsets[t]).  They are gathered
+ * into page-locked memory inside the call, by up to three helper threads of the handle's when there is much to gather,
+ * while what has been gathered is on its way to the device. */
+GTK_API int gtk_encode_strings(gtk_tokenizer* h, int mode, const uint8_t* const* texts, const int64_t* text_offsets,
+                               int64_t n_texts, float* kernel_ms);
+
 /* Replaces tokenize_batch_cpu (gputok_binding.cu:992-1003): host-only
  * reference tokenizer.  GTK_RULE_GREEDY (default of the Python surface) runs
  * the greedy rule per chunk; GTK_RULE_LOCALMIN reproduces the reference

@@ -307,6 +307,41 @@ def test_strings_of_nul_bytes(lib, merges_path, tmp_path, n_bytes):
     check_chunks(ids, coff, want, woff, f"NUL strings, {n_bytes} bytes")
 
 
+@pytest.mark.parametrize("n_texts", [1, 63, 3000, 12000])
+def test_strings_gathered_by_the_helpers(lib, merges_path, oracle, n_texts):
+    """Strings of every kind (ASCII, other scripts, empty, longer than a block of the gather) through the drop-in class, from
+    several threads at once, in sizes on both sides of the two-launch and pieces paths; decoding with helpers."""
+    import threading
+
+    import gputok_gpu
+
+    rng = np.random.default_rng(n_texts)
+    text = lib.TextGen(3).text(10 << 20, mix=lib.MIX_STRESS).tobytes().decode("utf-8", "ignore")
+    cuts = np.sort(rng.integers(0, min(len(text), 800 * n_texts), n_texts * 2))
+    texts = [text[a:b] for a, b in zip(cuts[::2], cuts[1::2])] + ["", text[:150_000], "caf\u00e9 \U0001f600 " * 40]
+    blobs = [t.encode() for t in texts]
+    off = np.concatenate([[0], np.cumsum([len(b) for b in blobs])]).astype(np.int64)
+    chunk = 2048
+    coff = np.unique(np.concatenate([[0], off] + [np.arange(s, e, chunk) for s, e in zip(off[:-1], off[1:])])).astype(np.int64)
+    want, woff = oracle.encode_chunks(np.frombuffer(b"".join(blobs), np.uint8), coff, mode=MODE_SEGMENTED, threads=NCPU)
+    tok = gputok_gpu.GpuTokenizer(merges_path, chunk)
+    bad = []
+
+    def work():
+        ids, toff, got_off, _ = tok.encode_packed(texts)
+        if not (np.array_equal(ids, want) and np.array_equal(got_off, woff) and np.array_equal(toff, woff[np.searchsorted(coff, off)])):
+            bad.append("encode_packed")
+        if tok.decode(ids.tolist()) != b"".join(blobs):
+            bad.append("decode")
+
+    threads = [threading.Thread(target=work) for _ in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
+
+
 def test_crowded_pair_bucket(lib, merges_path, tmp_path):
     """More than four pairs in one bucket of the device pair table: the fifth and later ones are found in
     the side table (second load), in every kernel that probes."""
