@@ -1011,13 +1011,13 @@ __device__ __forceinline__ void opt_tile(TileSmem<kOptThreads>& S, const EncodeB
   GTK_PHASE(5);
 }
 
-// Bound by latency and issue together (see gtk_tile.cuh): 56 % of the issue slots, 54 % of the L1 data pipe, DRAM 3 %.
-// 128 MiB in 4 KiB chunks, this kernel alone: English-like text 1027 us before (five table loads and full token and rank
-// arrays per position, no reuse of merged segments within the batch), 580 us now; the sample novel 941 -> 490 us; 64 MiB
-// with multi-byte words and runs 750 -> 545 us.  Seven CTAs per SM with 36 registers: 443 us for the 64 MiB call on
-// English-like text, against 453 with six and 40, 467 with five and 48 registers; eight with 32 measure the same as seven.
+// Bound by latency and issue together (see gtk_tile.cuh): about 60 % of the issue slots, DRAM 3 %.  This kernel alone, 128 MiB
+// in 4 KiB chunks: English-like text 1027 us with five table loads and full token and rank arrays per position and no
+// reuse of merged segments within the batch, 565 us now; the sample novel 941 -> 490 us; 64 MiB with multi-byte words and runs
+// 750 -> 500 us.  Six CTAs per SM with 40 registers: 16 MiB of English-like text 147 us per call, 128 MiB 657; seven with 36
+// registers 163 and 657, five with 48 registers 153 and 708 (128 MiB with runs 1050 / 1073 / 1088).  CTAs of 128 threads: the same.
 #ifndef GTK_OPT_CTAS
-#define GTK_OPT_CTAS 7
+#define GTK_OPT_CTAS 6
 #endif
 __global__ void __launch_bounds__(kOptThreads, GTK_OPT_CTAS) k_merge_opt(EncodeBuffers b, const __grid_constant__ DeviceTable T)
 {
