@@ -342,6 +342,23 @@ def test_strings_gathered_by_the_helpers(lib, merges_path, oracle, n_texts):
     assert not bad
 
 
+@pytest.mark.parametrize("n_bytes", [(512 << 10) - 1, 512 << 10, (1 << 20) + 1, (6 << 20) - 1, 6 << 20, (64 << 20) + 1])
+def test_ordinary_and_page_locked_memory(lib, merges_path, oracle, n_bytes):
+    """Both sides of the sizes at which ordinary memory is staged by the helpers and at which the text goes up in pieces; chunk
+    sizes that let tiles of a piece wait for the next one; results of the second call on the same buffers."""
+    from gputok_b200.capi import PinnedArray
+
+    data = lib.TextGen(n_bytes % 97).text(n_bytes, mix=lib.MIX_STRESS if n_bytes < (8 << 20) else lib.MIX_PLAIN)
+    pin = PinnedArray(n_bytes)
+    pin.array[:] = data
+    for chunk in (2048, 70_001):
+        want, woff = oracle.encode_fixed(data, chunk, mode=MODE_SEGMENTED, threads=NCPU)
+        t = make_tok(lib, merges_path, chunk)
+        for src, what in ((data, "ordinary"), (pin.array, "page-locked"), (data, "ordinary again")):
+            ids, toff, coff, _ = t.encode(src)
+            check_chunks(ids, coff, want, woff, f"{what}, {n_bytes} bytes, chunk {chunk}")
+
+
 def test_crowded_pair_bucket(lib, merges_path, tmp_path):
     """More than four pairs in one bucket of the device pair table: the fifth and later ones are found in
     the side table (second load), in every kernel that probes."""
