@@ -1432,6 +1432,22 @@ int validate_offsets(gtk_tokenizer* h, const int64_t* text_offsets, int64_t n_te
 }  // namespace
 
 namespace gtk {
+cudaError_t wait_for_word(volatile const int32_t* word, int32_t seq, cudaStream_t stream)
+{
+  for (unsigned spin = 1; *word != seq; ++spin) {
+    if ((spin & 0xFFFFu) == 0u) {
+      const cudaError_t q = cudaStreamQuery(stream);
+      if (q == cudaSuccess && *word != seq) return cudaErrorUnknown;
+      if (q != cudaSuccess && q != cudaErrorNotReady) return q;
+    }
+#if defined(__x86_64__) || defined(__i386__)
+    __builtin_ia32_pause();
+#endif
+  }
+  std::atomic_thread_fence(std::memory_order_acquire);
+  return cudaSuccess;
+}
+
 bool handle_view(gtk_tokenizer* h, HandleView* out)
 {
   if (!h || !out) return false;

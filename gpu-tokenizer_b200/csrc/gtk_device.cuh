@@ -149,7 +149,7 @@ int launch_encode_small(const EncodeBuffers& b, const DeviceTable& t, cudaStream
 #ifndef GTK_SMALL_MAX_BYTES
 #define GTK_SMALL_MAX_BYTES 8192
 #endif
-// two tiles one after the other in one CTA (57 us) still beat the two-launch path's 58..64 us; three (75 us) do not
+// 8 KiB as two tiles one after the other in one CTA 48 us, as two launches 47; 4 KiB 31 us
 constexpr int64_t kSmallMaxBytes = GTK_SMALL_MAX_BYTES;
 constexpr int64_t kSmallMaxTexts = 1024;
 constexpr int kTileGroup = 64;  // tiles whose ids are counted together
@@ -166,6 +166,8 @@ struct HandleView {
   std::string* last_error;
 };
 bool handle_view(gtk_tokenizer* h, HandleView* out);
+// waits for a kernel's last store, the call number, in page-locked memory; an error when the stream fails or goes idle without it
+cudaError_t wait_for_word(volatile const int32_t* word, int32_t seq, cudaStream_t stream);
 
 int opt_kernel_max_blocks_per_sm();
 int base_kernel_max_blocks_per_sm(int chunk_bytes, int block_threads);

@@ -188,7 +188,7 @@ GTK_API void gtk_result_release(gtk_taken* result);
  * [0] chunker, [1] merge kernel, [2] output scans, [3] pack, [4] whole pipeline.
  * Also the number of kernels launched by that call (for launch accounting).
  * [4] is always measured (it is the kernel_ms the encode entry points return, the reference's one event pair,
- * gputok_binding.cu:790-805).  [0]..[3] are measured for batches that the host path cuts into slices, and for
+ * gputok_binding.cu:790-805).  [0]..[3] are measured for batches that the host path cuts into pieces, and for
  * batches that run in one piece only after gtk_set_stage_timing(h, 1); otherwise they are 0.  The events between
  * the stages cost a call of a few hundred KiB to a few MiB about a tenth of its time, which is why they are off
  * by default. */
