@@ -956,7 +956,12 @@ __device__ __forceinline__ void tile_merge(TileSmem<TH>& S, const DeviceTable& T
   constexpr int cap = TileSmem<TH>::kScratchBytes / 128;  // columns of 32 words in the scratch
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n   = min(S.nmiss, S.kMisses);
-  if (n > 0) {  // CTA-uniform
+  if (n > 0 && n <= 2 * NW) {  // few: two for each warp, quicker than one warp's loop over all (128-byte call 20.8 -> 19.7 us)
+    const int k = 2 * warp + (lane >> 4);
+    if (2 * warp < n)
+      merge_two<TH>(k < n ? uint32_t(S.miss[k]) : 0u, pair_table(T), T.byte_pair_info, T.learn ? T.long_words : nullptr);
+    __syncthreads();
+  } else if (n > 0) {  // CTA-uniform
     Entry* ml = S.miss;
     if (n > 32) {
       // counting sort, longest first, so that the lanes of a warp work on segments of similar length
