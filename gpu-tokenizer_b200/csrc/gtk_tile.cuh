@@ -837,7 +837,7 @@ __device__ __forceinline__ void tile_lookup(TileSmem<TH>& S, const Span& sp, con
         const uint32_t k0 = __funnelshift_r(a0, a1, sh) & low_bits(8 * L);
         k1[e] = (__funnelshift_r(a1, a2, sh) & low_bits(max(8 * L - 32, 0))) | uint32_t(L) << 24;
         p[e]  = k0 * kShortMulA;
-        v[e]  = make_uint2(0xFFFFFFFFu, 0u);
+        v[e]  = make_uint2(0xFFFFFFFFu, 0xFFFFFFFFu);  // an empty place: whatever k1 is, bits 16 and 17 of the id stay set
         if (L <= kShortMaxBytes) v[e] = __ldg(T.short_words + ((p[e] ^ (k1[e] * kShortMulB)) >> (32 - kShortBits)));
       }
 #pragma unroll

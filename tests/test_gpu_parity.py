@@ -307,6 +307,42 @@ def test_strings_of_nul_bytes(lib, merges_path, tmp_path, n_bytes):
     check_chunks(ids, coff, want, woff, f"NUL strings, {n_bytes} bytes")
 
 
+@pytest.mark.parametrize("n_bytes", [4096, 100_000, (12 << 20) + 4097])
+def test_long_segments_whose_key_words_look_empty(lib, merges_path, tmp_path, n_bytes):
+    """Segments of 8..16 bytes are not in the table of short strings, but their first words are formed all the same: with FF in
+    bytes 4..7 they equal the mark of an empty place, with zeros in front the id that is left over is 0.  Every kernel that
+    looks segments up.  Whole ids: no tolerance."""
+    import torch
+
+    from oracle.loader import Oracle
+
+    with open(merges_path, encoding="utf-8") as f:
+        lines = f.read().split("\n")[:3001]
+    nul, last = "\u0100", "\u00ff"  # the symbols of bytes 0 and 255
+    path = str(tmp_path / "edge_merges.txt")
+    with open(path, "w", encoding="utf-8") as f:
+        f.write("\n".join(lines + [f"{nul} {nul}", f"{nul} {last}", f"{last} {last}", f"{nul} @", f"@ {last}"]) + "\n")
+    rng = np.random.default_rng(n_bytes)
+    parts = [b"\0" * i + t + b"\xff" * j for i in range(9) for j in range(12) for t in (b"", b"@", b"@\0\0")] + [b"the", b" of"]
+    blob = b" ".join(parts[i] for i in rng.integers(0, len(parts), n_bytes // 3))[:n_bytes]
+    data, chunk = np.frombuffer(blob, np.uint8), 2048
+    want, woff = Oracle(path).encode_fixed(data, chunk, mode=MODE_SEGMENTED, threads=NCPU)
+    t = make_tok(lib, path, chunk)
+    for mode in (lib.GTK_MODE_OPT, lib.GTK_MODE_BASE):
+        ids, _, coff, _ = t.encode(blob, mode=mode)
+        check_chunks(ids, coff, want, woff, f"mode {mode}, {n_bytes} bytes")
+    off = np.minimum(np.arange(0, n_bytes + chunk, chunk), n_bytes).astype(np.int64)
+    d_bytes, d_off = torch.from_numpy(data.copy()).cuda(), torch.from_numpy(off).cuda()
+    d_ids = torch.zeros(n_bytes, dtype=torch.int32, device="cuda")
+    d_cnt = torch.zeros(len(off) - 1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    t.encode_chunks_noalloc(d_bytes.data_ptr(), n_bytes, d_off.data_ptr(), len(off) - 1, chunk, d_ids.data_ptr(), d_cnt.data_ptr())
+    cnt = d_cnt.cpu().numpy()
+    assert np.array_equal(cnt, np.diff(woff))
+    place = np.repeat(off[:-1] - woff[:-1], cnt) + np.arange(len(want))
+    assert np.array_equal(d_ids.cpu().numpy()[place], want), "allocation-free"
+
+
 @pytest.mark.parametrize("n_texts", [1, 63, 3000, 12000])
 def test_strings_gathered_by_the_helpers(lib, merges_path, oracle, n_texts):
     """Strings of every kind (ASCII, other scripts, empty, longer than a block of the gather) through the drop-in class, from
