@@ -1524,7 +1524,7 @@ GTK_API int gtk_create(const char* merges_path, int chunk_tokens, int max_iters,
       h->localmin_grid = h->sm_count * std::max(1, gtk::localmin_kernel_max_blocks_per_sm());
       h->wide_grid = h->sm_count * std::max(1, gtk::wide_kernel_max_blocks_per_sm());
       h->h_totals.reserve(64);
-      std::memset(h->h_totals.p, 0, 64);  // holds a completion mark: behind any call number that is still to come
+      std::memset(h->h_totals.p, 0, 64);
       small_path_init(h);
     }
     *out = h;
@@ -1604,6 +1604,7 @@ GTK_API int gtk_encode_device(gtk_tokenizer* h, int mode, const uint8_t* d_bytes
     if (mode == GTK_MODE_OPT && !h->wide) {
       volatile int64_t* tot = h->h_totals.as<int64_t>();
       const int64_t seq     = ++h->mid_seq;
+      tot[3] = 0;  // copy_totals of an earlier call in another mode has left its chunk ticket there, which may equal the call number
       run_tiles(h, p.b, false, h->h_totals.as<int64_t>(), seq, &launches);
       if (!wait_for_mark(tot + 3, seq, h->stream, "pack kernel"))
         return h->fail(GTK_ERR_KERNEL, "pack kernel ended without publishing its results");

@@ -707,6 +707,46 @@ def test_device_resident_entry_point(lib, merges_path, oracle):
     assert e.value.code == 4
 
 
+@pytest.mark.parametrize("between", ["base", "localmin", "host base"])
+def test_device_calls_of_different_modes_on_one_handle(lib, merges_path, oracle, between):
+    """The segment-parallel mode waits for its call number in page-locked words that the other modes fill with totals and
+    counters; every number of calls in front, so that the number meets whatever the call in between has left there (a batch
+    of one short text: chunk ticket 3).  Texts of different sizes, every call's counts and ids; whole ids, no tolerance."""
+    import torch
+
+    chunk = 4096
+    texts = [lib.TextGen(70 + i).text(n) for i, n in enumerate((3 << 20, 1000, (2 << 20) + 777))]
+    want = [oracle.encode_fixed(x, chunk, mode=MODE_SEGMENTED, threads=NCPU) for x in texts]
+    on_gpu = [(torch.from_numpy(x.copy()).cuda(), torch.tensor([0, len(x)], dtype=torch.int64, device="cuda")) for x in texts]
+    host_text = lib.TextGen(80).text((1 << 20) + 5)  # above the size up to which a kernel brings the results of that mode
+    torch.cuda.synchronize()
+
+    def device_call(t, i, mode):
+        d_bytes, d_off = on_gpu[i]
+        n = len(texts[i])
+        d_ids = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+        d_coff = torch.full((n // chunk + 8,), -1, dtype=torch.int64, device="cuda")
+        torch.cuda.synchronize()
+        n_ids, n_chunks, _ = t.encode_device(d_bytes.data_ptr(), n, d_off.data_ptr(), 1, d_ids.data_ptr(), n,
+                                             d_coff.data_ptr(), d_coff.numel(), mode=mode)
+        if mode == lib.GTK_MODE_LOCALMIN:
+            return
+        ids, woff = want[i]
+        assert (n_ids, n_chunks) == (len(ids), len(woff) - 1), (i, mode)
+        assert np.array_equal(d_ids[:n_ids].cpu().numpy(), ids) and np.array_equal(d_coff[:n_chunks + 1].cpu().numpy(), woff)
+
+    for calls in range(1, 7):
+        t = make_tok(lib, merges_path, chunk)
+        for _ in range(calls):
+            device_call(t, 0, lib.GTK_MODE_OPT)
+        if between == "host base":
+            t.encode(host_text, mode=lib.GTK_MODE_BASE)
+        else:
+            device_call(t, 1, lib.GTK_MODE_BASE if between == "base" else lib.GTK_MODE_LOCALMIN)
+        device_call(t, 2, lib.GTK_MODE_OPT)
+        t.close()
+
+
 def test_batch_beyond_2_gib_uses_64_bit_offsets(lib, merges_path, oracle):
     """2.25 GiB in one call (byte positions and id offsets beyond 2^31): every chunk must decode to exactly its own
     bytes (token byte lengths summed per chunk), a seeded sample of chunks must equal the oracle, and the
