@@ -1602,6 +1602,7 @@ GTK_API int gtk_encode_device(gtk_tokenizer* h, int mode, const uint8_t* d_bytes
     begin_call(h, mode, n_bytes);
     int launches = 0;
     if (mode == GTK_MODE_OPT && !h->wide) {
+      p.b.text_end = d_text_offsets + n_texts;
       volatile int64_t* tot = h->h_totals.as<int64_t>();
       const int64_t seq     = ++h->mid_seq;
       tot[3] = 0;  // copy_totals of an earlier call in another mode has left its chunk ticket there, which may equal the call number

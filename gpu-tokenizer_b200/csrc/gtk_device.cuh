@@ -71,6 +71,7 @@ struct EncodeBuffers {
   const int64_t* text_off;   // [n_texts+1]
   int64_t* text_off_copy;    // small-batch kernel only: device copy of text_off when that lives in host memory
   int64_t n_texts;
+  const int64_t* text_end;   // tile kernel, device-resident batches: where the last text ends, bytes behind it belong to none; nullptr = n_bytes
   int chunk_bytes;
   // chunker outputs
   int64_t* text_chunk_base;  // [n_texts+1] exclusive scan of chunks per text

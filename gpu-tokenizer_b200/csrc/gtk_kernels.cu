@@ -834,12 +834,17 @@ __global__ void k_chunk_fill(const int64_t* __restrict__ text_off, const int64_t
 
 #include "gtk_tile.cuh"
 
-// Window k of a batch walked in tiles of kTile bytes.
-__device__ __forceinline__ Span batch_span(const EncodeBuffers& b, int64_t k)
+// Window k of a batch walked in tiles of kTile bytes: n_tiles that hold text, `tail` bytes of it in the last of them.
+__device__ __forceinline__ Span batch_span(const EncodeBuffers& b, int k, int n_tiles, int tail)
 {
-  const int64_t lo = k * kTile;
-  return Span{b.bytes, lo, 0, int(min(int64_t(kTile), b.n_bytes - lo)), int(min(int64_t(kWindow), b.n_bytes - lo)),
-              lo > 0, lo == 0};
+  const int rest = min(n_tiles - 1 - k, 2) * kTile + tail;  // as far as it matters
+  return Span{b.bytes, int64_t(k) * kTile, 0, min(kTile, rest), min(kWindow, rest), k > 0, k == 0};
+}
+
+// Where the texts of a batch end.  A caller's device buffer may be longer than they are.
+__device__ __forceinline__ int64_t text_end(const EncodeBuffers& b)
+{
+  return b.text_end ? max(min(__ldg(reinterpret_cast<const long long*>(b.text_end)), (long long)b.n_bytes), 0ll) : b.n_bytes;
 }
 
 // first index in [0, n) whose value is not below x, n if there is none; one warp, 32 places per step
@@ -860,16 +865,20 @@ __device__ __forceinline__ int64_t warp_lower_bound(const int64_t* v, int64_t n,
 // tile (128 MiB: 710 us instead of 590).
 __global__ void __launch_bounds__(128) k_tile_info(EncodeBuffers b)
 {
-  const int64_t chunk = b.chunk_bytes;
+  const int64_t chunk = b.chunk_bytes, n_end = text_end(b);
   for (int64_t k = int64_t(blockIdx.x) * 128 + threadIdx.x; k < b.n_tiles; k += int64_t(gridDim.x) * 128) {
     const int64_t lo = k * kTile;
     TileInfo i{0, 0, kTileNoCut, 0};
+    if (lo >= n_end) {  // the tile kernel leaves it out
+      b.unit_first[k] = lo;
+      b.unit_cnt[k]   = 0;
+    }
     if (b.n_texts == 1) {
       i.t0    = lo > 0;
-      i.c0    = (lo + chunk - 1) / chunk;
+      i.c0    = (min(lo, n_end) + chunk - 1) / chunk;
       i.flags = kTilePlain | (lo > 0 ? kTileRunsIn : 0);
       const int64_t p0 = i.c0 * chunk - lo;
-      if (p0 < kWindow && lo + p0 < b.n_bytes) i.p0 = int(p0);
+      if (p0 < kWindow && lo + p0 < n_end) i.p0 = int(p0);
     } else {
       int64_t a = 0, e = b.n_texts;  // first text that starts at or behind the tile's first byte
       while (a < e) {
@@ -883,7 +892,7 @@ __global__ void __launch_bounds__(128) k_tile_info(EncodeBuffers b)
         const int64_t s = b.text_off[a - 1], d = lo - s;
         const int64_t n = d < (int64_t(1) << 31) ? int64_t((uint32_t(d) + uint32_t(chunk) - 1u) / uint32_t(chunk)) : (d + chunk - 1) / chunk;
         const int64_t at = s + n * chunk;
-        i.flags = kTileRunsIn | (end >= min(lo + kWindow, b.n_bytes) ? kTilePlain : 0);
+        i.flags = kTileRunsIn | (end >= min(lo + kWindow, n_end) ? kTilePlain : 0);
         if (at < end) {
           i.c0 = b.text_chunk_base[a - 1] + n;
           if (at - lo < kWindow) i.p0 = int(at - lo);
@@ -947,12 +956,12 @@ __device__ __forceinline__ void for_each_start(const EncodeBuffers& b, const Til
 // One tile of a batch: tokenises every segment that starts in bytes [k*kTile, (k+1)*kTile), writes the tokens compacted to
 // staging and what the pack kernel needs to know of the tile: number of ids, first chunk and text, and how many of its ids
 // stand in front of every chunk and text that starts in it.
-__device__ __forceinline__ void opt_tile(TileSmem<kOptThreads>& S, const EncodeBuffers& b, const DeviceTable& T, int64_t k)
+__device__ __forceinline__ void opt_tile(TileSmem<kOptThreads>& S, const EncodeBuffers& b, const DeviceTable& T, int k)
 {
   __shared__ uint16_t woff[TileSmem<kOptThreads>::kWords];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int* status   = b.counters + 1;
-  const Span sp = batch_span(b, k);
+  const Span sp = batch_span(b, k, S.n_tiles, S.tail);
 #ifdef GTK_PHASE_TIMING
   long long phase_t0 = clock64();
 #endif
@@ -988,7 +997,7 @@ __device__ __forceinline__ void opt_tile(TileSmem<kOptThreads>& S, const EncodeB
   if (S.over_start >= 0) {  // CTA-uniform, rare
     const int64_t start = sp.lo + S.over_start;
     const int64_t t     = b.n_texts == 1 ? 0 : warp_lower_bound(b.text_off, b.n_texts, start + 1) - 1;  // text that holds it
-    const int64_t s     = b.n_texts == 1 ? 0 : b.text_off[t], e = b.n_texts == 1 ? b.n_bytes : b.text_off[t + 1];
+    const int64_t s     = b.n_texts == 1 ? 0 : b.text_off[t], e = b.n_texts == 1 ? int64_t(S.n_tiles - 1) * kTile + S.tail : b.text_off[t + 1];
     const int64_t cend  = min(e, s + ((start - s) / b.chunk_bytes + 1) * b.chunk_bytes);
     over = merge_oversize<kOptThreads>(b.bytes, start, sp.lo + kWindow, cend, ws, b.seg_scratch_tokens, T, status);
     for (int j = tid; j < over; j += kOptThreads)
@@ -1014,10 +1023,17 @@ __global__ void __launch_bounds__(kOptThreads, GTK_OPT_CTAS) k_merge_opt(EncodeB
 {
   TileSmem<kOptThreads>& S = tile_smem<kOptThreads>();
   tile_setup(S);
+  if (threadIdx.x == 0) {
+    const int64_t n = text_end(b);
+    S.n_tiles = int((n + kTile - 1) / kTile);
+    S.tail    = int(n - int64_t(S.n_tiles - 1) * kTile);
+  }
   if (b.tile_lo == 0 && blockIdx.x == 0 && threadIdx.x == 0)
     *reinterpret_cast<unsigned long long*>(b.counters + 12) = global_timer();
-  int64_t k = b.tile_lo + blockIdx.x;  // the first tile of every CTA, the others by ticket
-  while (k < b.tile_hi) {
+  __syncthreads();
+  const int lo = int(b.tile_lo);  // tiles are counted in 32 bits: 8 TB of text
+  int k        = lo + int(blockIdx.x);  // the first tile of every CTA, the others by ticket
+  while (k < min(int(b.tile_hi), S.n_tiles)) {
     int next = 0;
     if (threadIdx.x == 0) next = atomicAdd(b.ticket, 1);  // on its way while the tile is worked on
     tile_reset(S);
@@ -1025,7 +1041,7 @@ __global__ void __launch_bounds__(kOptThreads, GTK_OPT_CTAS) k_merge_opt(EncodeB
     opt_tile(S, b, T, k);
     if (threadIdx.x == 0) S.ticket = next;
     __syncthreads();
-    k = b.tile_lo + int64_t(gridDim.x) + S.ticket;
+    k = lo + int(gridDim.x) + S.ticket;
   }
 }
 
@@ -1231,7 +1247,7 @@ __device__ __forceinline__ void small_tile(TileSmem<kOptThreads>& S, const Encod
   __shared__ uint16_t woff[TileSmem<kOptThreads>::kWords];
   const int tid = threadIdx.x, lane = tid & 31;
   int* status   = b.counters + 1;
-  const Span sp = batch_span(b, k);
+  const Span sp = batch_span(b, int(k), int(b.n_tiles), int(b.n_bytes - (b.n_tiles - 1) * kTile));
   const int64_t c0 = b.tile_chunk0[k];
   tile_cut(S, sp, T, [&](auto mark) {
     for (int64_t c = c0 + lane; c <= C; c += 32) {
@@ -1696,7 +1712,7 @@ __global__ void __launch_bounds__(256) k_pack_tiles(EncodeBuffers b, int64_t per
   const int64_t K = b.n_tiles, a = min(b.tile_lo + int64_t(blockIdx.x) * per_cta, b.tile_hi), e = min(a + per_cta, b.tile_hi);
   const uint16_t* map = b.low_id_map;
   auto conv = [&](uint32_t t) { return int32_t((map && t < 256u) ? uint32_t(__ldg(map + t)) : t); };
-  const int64_t C = b.n_texts == 1 ? (b.n_bytes + b.chunk_bytes - 1) / b.chunk_bytes : b.totals[0];
+  const int64_t C = b.n_texts == 1 ? (text_end(b) + b.chunk_bytes - 1) / b.chunk_bytes : b.totals[0];
   if (a < e) {
     const int64_t g = a / kTileGroup;
     int64_t sum     = 0;

@@ -50,6 +50,7 @@ struct TileSmem {
   int ticket;
   int merged;          // ids of the sequence that the whole CTA has merged
   long long over_end;
+  int n_tiles, tail;   // tiles that hold text, bytes of it in the last of them (tile kernel)
   long long run;       // ids written so far (kernels that walk tiles in order)
 
   static constexpr int kScratchBytes = int(sizeof(work));

@@ -167,6 +167,7 @@ GTK_API int gtk_result_copy(const gtk_tokenizer* h, int32_t* ids, int64_t ids_ca
  * d_bytes (16-byte aligned for full speed), d_text_offsets[n_texts+1] (int64),
  * d_out_ids[out_capacity] and d_out_chunk_offsets[chunk_capacity] (>= number
  * of chunks + 1, may be NULL) are device pointers on the handle's device.
+ * d_text_offsets[0] is 0; bytes from d_text_offsets[n_texts] to n_bytes belong to no text and yield no ids.
  * *n_ids / *n_chunks are host outputs.  Synchronous on return.  GTK_ERR_CAPACITY
  * if a buffer is too small: nothing is written past a capacity, what was
  * written before the error is unspecified. */

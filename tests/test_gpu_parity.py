@@ -747,6 +747,34 @@ def test_device_calls_of_different_modes_on_one_handle(lib, merges_path, oracle,
         t.close()
 
 
+@pytest.mark.parametrize("mode", ["opt", "base"])
+@pytest.mark.parametrize("n, ends", [
+    (100_000, [61_234]), (100_000, [65_536]), (100_000, [99_990]), (100_000, [100_000]), (100_000, [0]), (100_000, [3000, 61_234]),
+    (5000, [17]), (1 << 20, 2000), (14_000_000, [9_000_123]), (14_000_000, 12_000),
+])
+def test_device_buffer_longer_than_its_texts(lib, merges_path, oracle, n, ends, mode):
+    """The bytes of a device buffer behind the last text belong to no text: not counted, in no chunk, and no part of the last
+    text's last segment.  One text and many, ending inside a tile, at its edge, in the last tile and not at all."""
+    import torch
+
+    chunk = 1000
+    rng = np.random.default_rng(n)
+    ends = np.asarray(ends) if isinstance(ends, list) else np.cumsum(rng.integers(0, n // ends * 3 // 2, ends))
+    off = np.concatenate([[0], ends]).astype(np.int64)
+    data = lib.TextGen(9).text(n, mix=lib.MIX_STRESS)
+    cuts = np.unique(np.concatenate([[0], off] + [np.arange(s, e, chunk) for s, e in zip(off[:-1], off[1:])])).astype(np.int64)
+    want, woff = oracle.encode_chunks(data, cuts, mode=MODE_SEGMENTED, threads=NCPU) if len(cuts) > 1 else (np.zeros(0, np.int32), np.zeros(1, np.int64))
+    t = make_tok(lib, merges_path, chunk)
+    d_bytes, d_off = torch.from_numpy(data.copy()).cuda(), torch.from_numpy(off).cuda()
+    d_ids = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    d_coff = torch.full((n // chunk + len(off) + 8,), -1, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    n_ids, n_chunks, _ = t.encode_device(d_bytes.data_ptr(), n, d_off.data_ptr(), len(off) - 1, d_ids.data_ptr(), n, d_coff.data_ptr(),
+                                         d_coff.numel(), mode=lib.GTK_MODE_OPT if mode == "opt" else lib.GTK_MODE_BASE)
+    assert (n_ids, n_chunks) == (len(want), len(woff) - 1)
+    check_chunks(d_ids[:n_ids].cpu().numpy(), d_coff[:n_chunks + 1].cpu().numpy(), want, woff, f"{n} bytes")
+
+
 def test_batch_beyond_2_gib_uses_64_bit_offsets(lib, merges_path, oracle):
     """2.25 GiB in one call (byte positions and id offsets beyond 2^31): every chunk must decode to exactly its own
     bytes (token byte lengths summed per chunk), a seeded sample of chunks must equal the oracle, and the
