@@ -503,11 +503,11 @@ void run_tiles(gtk_tokenizer* h, const gtk::EncodeBuffers& b, bool ready, int64_
   const bool stages = ev != nullptr || h->stage_timing;
   if (!ev) ev = h->ev;
   const bool learned = h->reset_learned;
+  if (stages) GTK_CUDA(cudaEventRecord(ev[0], s));
   if (!ready || learned) {
     *launches += gtk::launch_begin_batch(b, h->dtab.long_words, learned ? h->call_tab.long_words : nullptr, s);
   }
   h->reset_learned = false;
-  if (stages) GTK_CUDA(cudaEventRecord(ev[0], s));
   if (!ready) *launches += gtk::launch_scan_texts(b, learned, s) + gtk::launch_tile_info(b, s);
   if (stages) GTK_CUDA(cudaEventRecord(ev[1], s));
   *launches += gtk::launch_merge_opt(b, h->call_tab, h->opt_grid, s);
@@ -1185,6 +1185,7 @@ int encode_host_tiles(gtk_tokenizer* h, const Source& src, const int64_t* text_o
     p.b.counters        = reinterpret_cast<int32_t*>(dp + 16);
     p.b.group_cnt       = p.b.counters + 16;
     p.b.ticket          = p.b.counters;
+    p.b.starts_clock    = true;
     p.b.text_chunk_base = reinterpret_cast<int64_t*>(dp + o_base);
     p.b.tile_info       = reinterpret_cast<gtk::TileInfo*>(dp + o_info);
     const int64_t seq   = ++h->mid_seq;
@@ -1201,7 +1202,7 @@ int encode_host_tiles(gtk_tokenizer* h, const Source& src, const int64_t* text_o
     if (tot[2] != gtk::kStatusOk) return h->fail(GTK_ERR_KERNEL, status_text(int(tot[2])));
     if (tot[0] != C || tot[1] > n_bytes) return h->fail(GTK_ERR_KERNEL, "inconsistent totals");
     h->res_n_ids   = tot[1];
-    h->stage_ms[4] = float(double(tot[4]) * 1e-6);  // by the kernels' own clock
+    if (attempt == 0) h->stage_ms[4] = float(double(tot[4]) * 1e-6);  // by the kernels' own clock
     if (h->res_n_ids <= room) break;
     h->ids_per_byte = std::min(1.0, 1.1 * double(h->res_n_ids) / double(n_bytes));
     room = h->res_n_ids;
@@ -1295,8 +1296,10 @@ int encode_host_pieces(gtk_tokenizer* h, const Source& src, const int64_t* text_
   h->reset_learned   = false;
   if (n_texts > 1) GTK_CUDA(cudaMemcpyAsync(h->d_text_off.p, text_offsets, size_t(n_texts + 1) * 8, cudaMemcpyHostToDevice, s));
   GTK_CUDA(cudaMemsetAsync(tickets, 0, np * 4, s));
+  GTK_CUDA(cudaEventRecord(h->ev[0], s));
   launches += gtk::launch_begin_batch(b, h->dtab.long_words, learned ? h->call_tab.long_words : nullptr, s);
   launches += gtk::launch_scan_texts(b, learned, s) + gtk::launch_tile_info(b, s);
+  GTK_CUDA(cudaEventRecord(h->ev[1], s));
   GTK_CUDA(cudaGetLastError());
 
   Gather gather(h, src);
@@ -1365,6 +1368,7 @@ int encode_host_pieces(gtk_tokenizer* h, const Source& src, const int64_t* text_
   if (end[2] != gtk::kStatusOk) return h->fail(GTK_ERR_KERNEL, status_text(int(end[2])));
   if (end[0] != C) return h->fail(GTK_ERR_KERNEL, "inconsistent totals");
   GTK_CUDA(cudaEventSynchronize(h->piece_ev[4 * np - 1]));
+  GTK_CUDA(cudaEventElapsedTime(&h->stage_ms[0], h->ev[0], h->ev[1]));
   for (size_t i = 0; i < np; ++i) {
     float merge = 0, pack = 0;
     GTK_CUDA(cudaEventElapsedTime(&merge, h->piece_ev[4 * i + 1], h->piece_ev[4 * i + 2]));
@@ -1372,7 +1376,7 @@ int encode_host_pieces(gtk_tokenizer* h, const Source& src, const int64_t* text_
     h->stage_ms[1] += merge;
     h->stage_ms[3] += pack;
   }
-  h->stage_ms[4]      = h->stage_ms[1] + h->stage_ms[3];
+  h->stage_ms[4]      = h->stage_ms[0] + h->stage_ms[1] + h->stage_ms[3];
   h->result_is_packed = true;
   h->ids_apart        = true;
   h->pack_base        = h->h_out.as<uint8_t>();

@@ -81,6 +81,7 @@ struct EncodeBuffers {
   int64_t n_tiles;
   int64_t tile_lo, tile_hi;  // the launch works on these (all, or those of a piece that starts with a group)
   int32_t* ticket;           // tile ticket of the launch (zero at the start)
+  bool starts_clock;         // the tile kernel is the first of the call: it notes the time, otherwise the launch that resets the counters has
   int64_t* piece_ids;        // nullptr, or [0] ids in front of the piece, [1] the same for the next one (pack kernel)
   // merge outputs
   uint16_t* staging;         // [n_bytes] tokens of a unit, compacted at the unit's first byte
@@ -106,7 +107,7 @@ struct EncodeBuffers {
   int32_t* staging32;        // [n_bytes] 32-bit kernel: tokens of a chunk, compacted at the chunk's first byte
   int64_t seg_scratch_tokens;  // tokens per CTA (two arrays of this length per CTA)
   int64_t* scan_block_sums;  // workspace of the multi-block scan
-  int32_t* counters;         // [0] tile ticket of whole batches, [1] status word, [2] chunk ticket, [8] CTAs done, [12..13] time the tile kernel began
+  int32_t* counters;         // [0] tile ticket of whole batches, [1] status word, [2] chunk ticket, [8] CTAs done, [12..13] time the first kernel of the call began
   int64_t* totals;           // device: [0] n_chunks, [1] n_ids
 };
 
@@ -133,7 +134,7 @@ int launch_tile_info(const EncodeBuffers& b, cudaStream_t stream);
 // done it (learned: whether that was given a learned table): returns 0
 int launch_scan_texts(const EncodeBuffers& b, bool learned, cudaStream_t stream);
 // What follows the tile kernel: ids back to back, offsets of chunks and texts, totals[0] and [1].  publish: where the
-// host waits for the call, or nullptr: {n_chunks, n_ids, status, seq, nanoseconds since the tile kernel began}, seq last;
+// host waits for the call, or nullptr: {n_chunks, n_ids, status, seq, nanoseconds since the first kernel of the call began}, seq last;
 // out_ids, chunk_id_off and text_id_off may then be page-locked host memory.  Uses counters[8] (zero at the start).
 int launch_pack_tiles(const EncodeBuffers& b, int sm_count, bool groups_scanned, int64_t* publish, int64_t seq, cudaStream_t stream);
 // {n_chunks, ids up to the end of the piece, status, seq} to `publish` in page-locked host memory, seq last

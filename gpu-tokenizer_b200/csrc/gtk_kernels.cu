@@ -1028,8 +1028,7 @@ __global__ void __launch_bounds__(kOptThreads, GTK_OPT_CTAS) k_merge_opt(EncodeB
     S.n_tiles = int((n + kTile - 1) / kTile);
     S.tail    = int(n - int64_t(S.n_tiles - 1) * kTile);
   }
-  if (b.tile_lo == 0 && blockIdx.x == 0 && threadIdx.x == 0)
-    *reinterpret_cast<unsigned long long*>(b.counters + 12) = global_timer();
+  if (b.starts_clock && blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long*>(b.counters + 12) = global_timer();
   __syncthreads();
   const int lo = int(b.tile_lo);  // tiles are counted in 32 bits: 8 TB of text
   int k        = lo + int(blockIdx.x);  // the first tile of every CTA, the others by ticket
@@ -1210,11 +1209,18 @@ __global__ void __launch_bounds__(kMediumThreads) k_scan_groups(EncodeBuffers b)
   cta_exclusive_scan_medium(CountsI32{b.group_cnt}, b.n_tiles / kTileGroup + 1, b.group_base, scanbuf, &carry_s, stage);
 }
 
+// Counter i of a call is zero at its start, [12..13] the time of the reset, which is the first launch of the call.
+__device__ __forceinline__ void reset_counter(int32_t* counters, int i)
+{
+  if (i == 12) *reinterpret_cast<unsigned long long*>(counters + 12) = global_timer();
+  else if (i != 13) counters[i] = 0;
+}
+
 // chunks per text, scanned (totals[0], text_chunk_base), for the tile kernel; reset: the call's counters and group counts too
 __global__ void __launch_bounds__(kMediumThreads) k_scan_texts_medium(EncodeBuffers b, int reset)
 {
   if (reset) {
-    if (threadIdx.x < 16) b.counters[threadIdx.x] = 0;
+    if (threadIdx.x < 16) reset_counter(b.counters, threadIdx.x);
     for (int64_t i = threadIdx.x; i <= b.n_tiles / kTileGroup; i += kMediumThreads) b.group_cnt[i] = 0;
     if (b.n_texts == 1) return;
   }
@@ -1837,7 +1843,7 @@ __global__ void __launch_bounds__(512) k_begin_batch(int32_t* counters, int32_t*
                                                      const uint4* __restrict__ from, uint4* __restrict__ to, int n_words)
 {
   const int i0 = blockIdx.x * 512 + threadIdx.x, step = gridDim.x * 512;
-  if (i0 < 16) counters[i0] = 0;
+  if (i0 < 16) reset_counter(counters, i0);
   for (int64_t i = i0; i < n_groups; i += step) group_cnt[i] = 0;
   if (to)
     for (int i = i0; i < n_words; i += 4 * step) {

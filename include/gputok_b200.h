@@ -122,9 +122,10 @@ GTK_API int gtk_table_info_get(const gtk_tokenizer* h, gtk_table_info* out);
  * Copies the batch to the device (fastest from pinned memory, see
  * gtk_pinned_alloc), runs chunker -> merge kernel -> output scan/pack, copies
  * ids and offsets back into pinned buffers owned by the handle.
- * *kernel_ms (optional) receives the device time of the kernel pipeline
- * (cudaEvent pair, as :790-805).  Results stay valid until the next call on
- * the handle; read them with gtk_result_sizes/_view/_copy.
+ * *kernel_ms (optional) receives the device time of the kernel pipeline, from
+ * the first kernel of the call to the end of the last (the reference's event
+ * pair, :790-805; see gtk_last_stage_ms).  Results stay valid until the next
+ * call on the handle; read them with gtk_result_sizes/_view/_copy.
  * An empty batch or a batch of empty texts is not an error: 0 ids, 0 chunks.
  * Small batches (up to 8 KiB and 1024 texts, GTK_MODE_OPT) run as one kernel that reads the text from and
  * writes the results to mapped page-locked memory; the call returns when the kernel's completion mark has
@@ -189,7 +190,10 @@ GTK_API void gtk_result_release(gtk_taken* result);
  * [0] chunker, [1] merge kernel, [2] output scans, [3] pack, [4] whole pipeline.
  * Also the number of kernels launched by that call (for launch accounting).
  * [4] is always measured (it is the kernel_ms the encode entry points return, the reference's one event pair,
- * gputok_binding.cu:790-805).  [0]..[3] are measured for batches that the host path cuts into pieces, and for
+ * gputok_binding.cu:790-805): by the kernels' own clock in GTK_MODE_OPT, by an event pair in the other modes, and as the
+ * sum of the stages for batches that the host path cuts into pieces or slices (their gaps are the link's).  Host batches
+ * whose chunk table the host makes itself (GTK_MODE_OPT below 6 MiB) have no chunker; where the last kernel writes the
+ * results to page-locked memory that is part of its time.  [0]..[3] are measured for batches in pieces or slices, and for
  * batches that run in one piece only after gtk_set_stage_timing(h, 1); otherwise they are 0.  The events between
  * the stages cost a call of a few hundred KiB to a few MiB about a tenth of its time, which is why they are off
  * by default. */

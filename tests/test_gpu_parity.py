@@ -775,6 +775,40 @@ def test_device_buffer_longer_than_its_texts(lib, merges_path, oracle, n, ends, 
     check_chunks(d_ids[:n_ids].cpu().numpy(), d_coff[:n_chunks + 1].cpu().numpy(), want, woff, f"{n} bytes")
 
 
+def test_kernel_ms_covers_the_whole_pipeline(lib, merges_path):
+    """kernel_ms counts from the first kernel of the call: reset, scan of the texts and tile records included, on the device
+    path (50 000 short texts: 67 us, of which 31 in front of the tile kernel) and for host batches in pieces.  The events between
+    the stages add to their sum, 85 us in this batch: 0.79 of it with what is in front, 0.43 without.  Medians of nine calls."""
+    import torch
+
+    n_texts, each = 50_000, 24
+    data = lib.TextGen(4).text(n_texts * each)
+    off = np.arange(0, n_texts * each + 1, each, dtype=np.int64)
+    t = make_tok(lib, merges_path, 2048)
+    d_bytes, d_off = torch.from_numpy(data.copy()).cuda(), torch.from_numpy(off).cuda()
+    d_ids = torch.empty(len(data), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+
+    def medians():
+        rows = []
+        for _ in range(9):
+            ms = t.encode_device(d_bytes.data_ptr(), len(data), d_off.data_ptr(), n_texts, d_ids.data_ptr(), len(data))[2]
+            st = t.stage_ms()
+            rows.append((ms, st["chunker"], st["merge"] + st["scan"] + st["pack"]))
+        return np.median(np.array(rows), axis=0)
+
+    whole = medians()[0]
+    t.set_stage_timing(True)
+    _, front, rest = medians()
+    assert 0.6 * (front + rest) < whole < front + rest, (whole, front, rest)
+    t.set_stage_timing(False)
+    blob = lib.TextGen(5).text(7 << 20)
+    cuts = np.arange(0, len(blob) + 1, 128, dtype=np.int64)
+    ms = t.encode(blob, cuts)[3]
+    st = t.stage_ms()
+    assert st["chunker"] > 0 and ms == pytest.approx(st["chunker"] + st["merge"] + st["scan"] + st["pack"])
+
+
 def test_batch_beyond_2_gib_uses_64_bit_offsets(lib, merges_path, oracle):
     """2.25 GiB in one call (byte positions and id offsets beyond 2^31): every chunk must decode to exactly its own
     bytes (token byte lengths summed per chunk), a seeded sample of chunks must equal the oracle, and the
