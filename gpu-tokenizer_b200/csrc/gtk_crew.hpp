@@ -1,6 +1,8 @@
 // gtk_crew.hpp -- a few helper threads for host work that one core is slow at: gathering strings that lie all over
 // the heap (one core copies them at 9 GB/s, the host link carries 55), and decoding.
 #pragma once
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
 #include <condition_variable>
@@ -16,31 +18,41 @@ namespace gtk {
 
 // Belongs to one handle: started at the first large job, joined with the handle.  One job at a time; whoever finds the
 // crew busy (decoding may run on several threads) does the work alone.
+//
+// A forked child has the memory of the helpers but not the threads, and whatever lock was held at the fork stays held: it
+// neither joins nor touches the team that it has inherited (which is never freed there), and starts one of its own for its first job.
 class Crew {
  public:
   static constexpr int kHelpers = 3;
 
   ~Crew()
   {
+    Team* team = team_.load(std::memory_order_acquire);
+    if (!team || team->pid != getpid()) return;
     {
-      std::lock_guard<std::mutex> lock(mu_);
-      stop_ = true;
+      std::lock_guard<std::mutex> lock(team->mu);
+      team->stop = true;
     }
-    wake_.notify_all();
-    for (std::thread& t : threads_) t.join();
+    team->wake.notify_all();
+    for (std::thread& t : team->threads) t.join();
+    delete team;
   }
 
+ private:
+  struct Team;
+
+ public:
   // Blocks 0 .. n-1 of a job, handed out in order to the helpers and to whoever waits for one.
   class Job {
    public:
-    Job(Crew& crew, int64_t n, std::function<void(int64_t)> work) : crew_(crew), n_(n), work_(std::move(work)), done_(new std::atomic<bool>[size_t(n)])
+    Job(Crew& crew, int64_t n, std::function<void(int64_t)> work) : n_(n), work_(std::move(work)), done_(new std::atomic<bool>[size_t(n)])
     {
       for (int64_t i = 0; i < n; ++i) done_[size_t(i)].store(false, std::memory_order_relaxed);
-      helped_ = n > 1 && crew_.begin(this);
+      if (n > 1) team_ = crew.begin(this);
     }
     ~Job()
     {
-      if (helped_) crew_.end();
+      if (team_) end(*team_);
     }
     Job(const Job&) = delete;
     Job& operator=(const Job&) = delete;
@@ -64,65 +76,79 @@ class Crew {
       done_[size_t(i)].store(true, std::memory_order_release);
       return true;
     }
-    Crew& crew_;
     const int64_t n_;
     std::function<void(int64_t)> work_;
     std::unique_ptr<std::atomic<bool>[]> done_;
     std::atomic<int64_t> next_{0};
     int64_t seen_ = 0;
-    bool helped_  = false;
+    Team* team_   = nullptr;  // that helps
   };
 
  private:
-  bool begin(Job* job)
+  struct Team {
+    const pid_t pid = getpid();  // of the process whose threads they are
+    std::mutex turn;             // one job at a time
+    std::mutex mu;
+    std::condition_variable wake, idle;
+    std::vector<std::thread> threads;
+    Job* job        = nullptr;
+    uint64_t number = 0;
+    int active      = 0;
+    bool stop       = false;
+  };
+
+  Team* team()
   {
-    if (!turn_.try_lock()) return false;
-    std::lock_guard<std::mutex> lock(mu_);
+    Team* t = team_.load(std::memory_order_acquire);
+    while (!t || t->pid != getpid()) {
+      std::unique_ptr<Team> fresh(new Team);
+      if (team_.compare_exchange_strong(t, fresh.get(), std::memory_order_acq_rel)) return fresh.release();
+    }
+    return t;
+  }
+  Team* begin(Job* job)  // nullptr: busy
+  {
+    Team* const t = team();
+    if (!t->turn.try_lock()) return nullptr;
+    std::lock_guard<std::mutex> lock(t->mu);
     const int want = std::min<int>(kHelpers, int(std::thread::hardware_concurrency()) - 1);
     try {
-      while (int(threads_.size()) < want) threads_.emplace_back([this] { serve(); });
+      while (int(t->threads.size()) < want) t->threads.emplace_back([t] { serve(*t); });
     } catch (const std::system_error&) {  // fewer helpers, or none
     }
-    job_ = job;
-    ++number_;
-    wake_.notify_all();
-    return true;
+    t->job = job;
+    ++t->number;
+    t->wake.notify_all();
+    return t;
   }
-  void end()  // no helper touches the job behind this
+  static void end(Team& t)  // no helper touches the job behind this
   {
     {
-      std::unique_lock<std::mutex> lock(mu_);
-      job_ = nullptr;
-      idle_.wait(lock, [this] { return active_ == 0; });
+      std::unique_lock<std::mutex> lock(t.mu);
+      t.job = nullptr;
+      t.idle.wait(lock, [&t] { return t.active == 0; });
     }
-    turn_.unlock();
+    t.turn.unlock();
   }
-  void serve()
+  static void serve(Team& t)
   {
     uint64_t seen = 0;
-    std::unique_lock<std::mutex> lock(mu_);
+    std::unique_lock<std::mutex> lock(t.mu);
     for (;;) {
-      wake_.wait(lock, [&] { return stop_ || (job_ != nullptr && number_ != seen); });
-      if (stop_) return;
-      seen     = number_;
-      Job* job = job_;
-      ++active_;
+      t.wake.wait(lock, [&] { return t.stop || (t.job != nullptr && t.number != seen); });
+      if (t.stop) return;
+      seen     = t.number;
+      Job* job = t.job;
+      ++t.active;
       lock.unlock();
       while (job->step()) {
       }
       lock.lock();
-      if (--active_ == 0) idle_.notify_all();
+      if (--t.active == 0) t.idle.notify_all();
     }
   }
 
-  std::mutex turn_;  // one job at a time
-  std::mutex mu_;
-  std::condition_variable wake_, idle_;
-  std::vector<std::thread> threads_;
-  Job* job_        = nullptr;
-  uint64_t number_ = 0;
-  int active_      = 0;
-  bool stop_       = false;
+  std::atomic<Team*> team_{nullptr};
 };
 
 }  // namespace gtk

@@ -311,6 +311,66 @@ def test_two_rank_sharding_over_gloo(native_built, merges_path, oracle, tmp_path
     assert "SHARDS_OK" in outs[0]
 
 
+FORKS = """
+import os, signal, sys, threading
+sys.path.insert(0, {pkg!r})
+import numpy as np
+import gputok_b200, gputok_gpu
+
+ids = np.arange({n}, dtype=np.int32) % 50000
+
+def check(call):
+    pid = os.fork()
+    if pid == 0:
+        signal.alarm(60)
+        os._exit(0 if call() else 1)
+    status = os.waitpid(pid, 0)[1]
+    assert status == 0, f"child ended with status {{status}}"
+
+want = None
+tok = gputok_b200.Tokenizer({merges!r}, 2048, 50, device=-1)
+want = tok.decode(ids)
+check(lambda: (tok.close(), True)[1])                       # dropped without having been used
+check(lambda: (tok.decode(ids) == want, tok.close())[0])    # used, and dropped with helpers of its own
+assert tok.decode(ids) == want
+
+drop_in = gputok_gpu.GpuTokenizer({merges!r}, device=-1)
+assert drop_in.decode(ids.tolist()) == want
+
+def drop():
+    global drop_in
+    del drop_in
+    return True
+check(drop)
+
+stop = False                                                # forked while another thread is in the middle of a job
+def work():
+    while not stop:
+        assert tok.decode(ids) == want
+thread = threading.Thread(target=work)
+thread.start()
+for _ in range(20):
+    check(lambda: (tok.decode(ids) == want, tok.close())[0])
+stop = True
+thread.join()
+assert tok.decode(ids) == want
+tok.close()
+"""
+
+
+def test_forked_children_use_and_drop_a_tokenizer(native_built, merges_path):
+    """The helper threads of a handle do not exist in a forked child, and its locks may have been held when it was forked: the child
+    drops the handle, or decodes with it, all the same.  300 000 ids: several blocks for the helpers."""
+    import subprocess
+    import sys
+
+    from conftest import PKG
+
+    script = FORKS.format(pkg=PKG, merges=merges_path, n=300_000)
+    done = subprocess.run([sys.executable, "-W", "ignore", "-c", script], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
+
+
 def test_host_table_beyond_16_bits(native_built, merges_path, oracle, novel, tmp_path):
     """A merges file with more than 65 534 merges builds (the reference accepts any file); the host tokenizer
     equals the oracle under that table and the new, high ids really occur."""
