@@ -33,6 +33,7 @@ namespace {
 [[noreturn]] void raise_status(int rc, const std::string& msg)
 {
   if (rc == GTK_ERR_INVALID_ARG) throw std::invalid_argument(msg);
+  if (rc == GTK_ERR_MEMORY) throw std::bad_alloc();
   throw std::runtime_error(msg);
 }
 

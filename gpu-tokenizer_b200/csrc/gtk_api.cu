@@ -270,6 +270,15 @@ struct gtk_tokenizer {
 
 namespace {
 
+// What a failing call does last: its copies and kernels may still be reading the caller's text or the handle's buffers.
+void settle(gtk_tokenizer* h)
+{
+  for (cudaStream_t s : {h->in_stream, h->stream, h->pack_stream, h->out_stream})
+    if (s) cudaStreamSynchronize(s);
+}
+
+int out_of_memory(const gtk_tokenizer* h) { return h->fail(GTK_ERR_MEMORY, "out of memory"); }  // short enough to need none
+
 void upload(DevBuf& buf, const void* src, size_t bytes, cudaStream_t s)
 {
   buf.reserve(bytes);
@@ -970,14 +979,15 @@ struct Source {
   void stream_texts(uint8_t* all, int64_t t, int64_t end) const
   {
     constexpr int64_t kLong = 16 << 10;
-    thread_local std::vector<uint8_t> block;
+    uint8_t block[3 * kLong];
     for (int64_t from = text_offsets[t]; t < end;) {
-      block.clear();
-      int64_t n = 0;
-      for (; t < end && block.size() < size_t(2 * kLong) && (n = text_offsets[t + 1] - text_offsets[t]) < kLong; ++t)
-        block.insert(block.end(), parts[t], parts[t] + n);
-      copy_to_staging(all + from, block.data(), block.size());
-      from += int64_t(block.size());
+      int64_t have = 0, n = 0;
+      for (; t < end && have < 2 * kLong && (n = text_offsets[t + 1] - text_offsets[t]) < kLong; ++t) {
+        if (n) std::memcpy(block + have, parts[t], size_t(n));
+        have += n;
+      }
+      copy_to_staging(all + from, block, size_t(have));
+      from += have;
       if (t < end && n >= kLong) {
         copy_to_staging(all + from, parts[t], size_t(n));
         from += n;
@@ -1327,43 +1337,35 @@ int encode_host_pieces(gtk_tokenizer* h, const Source& src, const int64_t* text_
     have = n;
     return true;
   };
-  try {
-    size_t done = 0;  // pieces collected
-    for (size_t i = 0; i < np; ++i) {
-      cudaEvent_t* ev  = &h->piece_ev[4 * i];
-      const int64_t lo = i ? ends[i - 1] : 0;
-      GTK_CUDA(cudaMemcpyAsync(h->d_bytes.as<uint8_t>() + lo, gather.ready(ends[i]) + lo, size_t(ends[i] - lo), cudaMemcpyHostToDevice, h->in_stream));
-      GTK_CUDA(cudaEventRecord(ev[0], h->in_stream));
-      GTK_CUDA(cudaStreamWaitEvent(s, ev[0], 0));
-      // a tile may need the text to the end of its last chunk: such tiles wait for the next piece
-      const bool last   = i + 1 == np;
-      const int64_t own = ends[i] - gtk::kWindow - std::min(chunk, n_bytes);
-      b.tile_hi         = last ? K : std::max(b.tile_lo, own / gtk::kTile / gtk::kTileGroup * gtk::kTileGroup);
-      b.ticket          = tickets + i;
-      b.piece_ids       = h->d_piece_ids.as<int64_t>() + i;
-      GTK_CUDA(cudaEventRecord(ev[1], s));
-      launches += gtk::launch_merge_opt(b, h->call_tab, h->opt_grid, s);
-      GTK_CUDA(cudaEventRecord(ev[2], s));
-      // a piece without a tile hands the count of the pieces in front of it on
-      launches += gtk::launch_pack_tiles(b, h->sm_count, false, nullptr, 0, s);
-      GTK_CUDA(cudaEventRecord(ev[3], s));
-      GTK_CUDA(cudaStreamWaitEvent(h->pack_stream, ev[3], 0));
-      launches += gtk::launch_publish_piece(b, h->h_marks.as<int64_t>() + 8 * i, int64_t(i) + 1, h->pack_stream);  // page-locked: same address on the device
-      GTK_CUDA(cudaGetLastError());
-      b.tile_lo = b.tile_hi;
-      while (done < i && collect(done, false)) ++done;
-    }
-    while (done < np) collect(done++, true);
-    GTK_CUDA(cudaMemcpyAsync(h->h_out.p, b.text_id_off, size_t(n_texts + 1) * 8, cudaMemcpyDeviceToHost, h->out_stream));
-    GTK_CUDA(cudaMemcpyAsync(h->h_out.as<uint8_t>() + text_b, b.chunk_id_off, size_t(C + 1) * 8, cudaMemcpyDeviceToHost, h->out_stream));
-    GTK_CUDA(cudaStreamSynchronize(h->out_stream));
-  } catch (...) {  // nothing of the call may be in flight when it returns
-    cudaStreamSynchronize(h->in_stream);
-    cudaStreamSynchronize(s);
-    cudaStreamSynchronize(h->pack_stream);
-    cudaStreamSynchronize(h->out_stream);
-    throw;
+  size_t done = 0;  // pieces collected
+  for (size_t i = 0; i < np; ++i) {
+    cudaEvent_t* ev  = &h->piece_ev[4 * i];
+    const int64_t lo = i ? ends[i - 1] : 0;
+    GTK_CUDA(cudaMemcpyAsync(h->d_bytes.as<uint8_t>() + lo, gather.ready(ends[i]) + lo, size_t(ends[i] - lo), cudaMemcpyHostToDevice, h->in_stream));
+    GTK_CUDA(cudaEventRecord(ev[0], h->in_stream));
+    GTK_CUDA(cudaStreamWaitEvent(s, ev[0], 0));
+    // a tile may need the text to the end of its last chunk: such tiles wait for the next piece
+    const bool last   = i + 1 == np;
+    const int64_t own = ends[i] - gtk::kWindow - std::min(chunk, n_bytes);
+    b.tile_hi         = last ? K : std::max(b.tile_lo, own / gtk::kTile / gtk::kTileGroup * gtk::kTileGroup);
+    b.ticket          = tickets + i;
+    b.piece_ids       = h->d_piece_ids.as<int64_t>() + i;
+    GTK_CUDA(cudaEventRecord(ev[1], s));
+    launches += gtk::launch_merge_opt(b, h->call_tab, h->opt_grid, s);
+    GTK_CUDA(cudaEventRecord(ev[2], s));
+    // a piece without a tile hands the count of the pieces in front of it on
+    launches += gtk::launch_pack_tiles(b, h->sm_count, false, nullptr, 0, s);
+    GTK_CUDA(cudaEventRecord(ev[3], s));
+    GTK_CUDA(cudaStreamWaitEvent(h->pack_stream, ev[3], 0));
+    launches += gtk::launch_publish_piece(b, h->h_marks.as<int64_t>() + 8 * i, int64_t(i) + 1, h->pack_stream);  // page-locked: same address on the device
+    GTK_CUDA(cudaGetLastError());
+    b.tile_lo = b.tile_hi;
+    while (done < i && collect(done, false)) ++done;
   }
+  while (done < np) collect(done++, true);
+  GTK_CUDA(cudaMemcpyAsync(h->h_out.p, b.text_id_off, size_t(n_texts + 1) * 8, cudaMemcpyDeviceToHost, h->out_stream));
+  GTK_CUDA(cudaMemcpyAsync(h->h_out.as<uint8_t>() + text_b, b.chunk_id_off, size_t(C + 1) * 8, cudaMemcpyDeviceToHost, h->out_stream));
+  GTK_CUDA(cudaStreamSynchronize(h->out_stream));
   const int64_t* end = h->h_marks.as<int64_t>() + 8 * (np - 1);
   if (end[2] != gtk::kStatusOk) return h->fail(GTK_ERR_KERNEL, status_text(int(end[2])));
   if (end[0] != C) return h->fail(GTK_ERR_KERNEL, "inconsistent totals");
@@ -1670,7 +1672,11 @@ GTK_API int gtk_encode_device(gtk_tokenizer* h, int mode, const uint8_t* d_bytes
     if (kernel_ms) *kernel_ms = h->stage_ms[4];
     return GTK_OK;
   } catch (const CudaFail& f) {
+    settle(h);
     return h->fail(GTK_ERR_CUDA, f.what);
+  } catch (const std::bad_alloc&) {
+    settle(h);
+    return out_of_memory(h);
   }
 }
 
@@ -1777,7 +1783,11 @@ static int encode_host(gtk_tokenizer* h, int mode, const uint8_t* bytes, const u
     if (kernel_ms) *kernel_ms = h->stage_ms[4];
     return GTK_OK;
   } catch (const CudaFail& f) {
+    settle(h);
     return h->fail(GTK_ERR_CUDA, f.what);
+  } catch (const std::bad_alloc&) {
+    settle(h);
+    return out_of_memory(h);
   }
 }
 
@@ -1948,7 +1958,7 @@ GTK_API int gtk_decode(const gtk_tokenizer* h, const int32_t* ids, int64_t n_ids
   // (an unknown id, too little room) is left to the one pass that finds out what.
   constexpr int64_t kBlock = 16384;
   int64_t k = -1;
-  if (n_ids >= 4 * kBlock) {
+  if (n_ids >= 4 * kBlock) try {
     const int64_t nb = (n_ids + kBlock - 1) / kBlock;
     std::vector<int64_t> at(size_t(nb) + 1, 0);
     gtk::Crew::Job(h->crew, nb, [&](int64_t i) {
@@ -1965,6 +1975,7 @@ GTK_API int gtk_decode(const gtk_tokenizer* h, const int32_t* ids, int64_t n_ids
         h->table->decode(ids + i * kBlock, std::min(kBlock, n_ids - i * kBlock), out + at[size_t(i)], at[size_t(i) + 1] - at[size_t(i)]);
       }).finish();
     if (plain) k = at[size_t(nb)];
+  } catch (const std::bad_alloc&) {  // the one pass needs no memory
   }
   if (k < 0) k = h->table->decode(ids, n_ids, out, out_capacity);
   if (k == -1 - n_ids) return h->fail(GTK_ERR_CAPACITY, "decode buffer too small");

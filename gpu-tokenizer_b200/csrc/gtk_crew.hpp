@@ -10,7 +10,6 @@
 #include <functional>
 #include <memory>
 #include <mutex>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -42,7 +41,8 @@ class Crew {
   struct Team;
 
  public:
-  // Blocks 0 .. n-1 of a job, handed out in order to the helpers and to whoever waits for one.
+  // Blocks 0 .. n-1 of a job, handed out in order to the helpers and to whoever waits for one.  The work must not throw (it may
+  // run on a helper, where nobody catches): it works in memory that it is given.
   class Job {
    public:
     Job(Crew& crew, int64_t n, std::function<void(int64_t)> work) : n_(n), work_(std::move(work)), done_(new std::atomic<bool>[size_t(n)])
@@ -114,7 +114,7 @@ class Crew {
     const int want = std::min<int>(kHelpers, int(std::thread::hardware_concurrency()) - 1);
     try {
       while (int(t->threads.size()) < want) t->threads.emplace_back([t] { serve(*t); });
-    } catch (const std::system_error&) {  // fewer helpers, or none
+    } catch (...) {  // no thread or no memory for one: fewer helpers, or none
     }
     t->job = job;
     ++t->number;

@@ -49,7 +49,8 @@ enum {
   GTK_ERR_CAPACITY     = 4, /* a caller-provided output buffer is too small */
   GTK_ERR_TABLE        = 5, /* the entry point does not serve this merge table (see gtk_create) */
   GTK_ERR_NO_DEVICE    = 6, /* GPU entry point called on a host-only handle */
-  GTK_ERR_KERNEL       = 7  /* a kernel reported an internal inconsistency through its status word */
+  GTK_ERR_KERNEL       = 7, /* a kernel reported an internal inconsistency through its status word */
+  GTK_ERR_MEMORY       = 8  /* the host has no memory left (std::bad_alloc in the reference) */
 };
 
 /* which merge kernel serves the call */

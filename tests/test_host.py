@@ -371,6 +371,45 @@ def test_forked_children_use_and_drop_a_tokenizer(native_built, merges_path):
     assert done.returncode == 0, done.stderr[-2000:]
 
 
+SHORT_OF_MEMORY = """
+import ctypes, resource, sys
+sys.path.insert(0, {pkg!r})
+import numpy as np
+import gputok_b200
+
+tok = gputok_b200.Tokenizer({merges!r}, 2048, 50, device=-1)
+n = 1 << 30
+ids = np.zeros(n, dtype=np.int32)            # never written: one page of zeros, whatever its size
+count = ctypes.c_int64()
+decode, handle, at = tok._lib.gtk_decode, tok._h, ids.ctypes.data
+args = (handle, at, n, None, 0, ctypes.byref(count))
+malloc = ctypes.CDLL(None).malloc
+malloc.argtypes, malloc.restype = [ctypes.c_size_t], ctypes.c_void_p
+in_use = int(open("/proc/self/statm").read().split()[0]) * resource.getpagesize()
+old = resource.getrlimit(resource.RLIMIT_AS)
+resource.setrlimit(resource.RLIMIT_AS, (in_use + {room}, old[1]))
+while {room} == 0 and malloc(1 << 17):       # what the heap has left
+    pass
+rc = decode(*args)
+resource.setrlimit(resource.RLIMIT_AS, old)
+assert rc == 0 and count.value == n, (rc, count.value)
+"""
+
+
+@pytest.mark.parametrize("room", [0, 4 << 20])
+def test_decode_without_memory_for_the_helpers(native_built, merges_path, room):
+    """No memory for the table of blocks, or none for the helpers' stacks: the call does the work by itself, as it did when it had no
+    helpers, and nothing is thrown out of a C function."""
+    import subprocess
+    import sys
+
+    from conftest import PKG
+
+    script = SHORT_OF_MEMORY.format(pkg=PKG, merges=merges_path, room=room)
+    done = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, (done.returncode, done.stderr[-2000:])
+
+
 def test_host_table_beyond_16_bits(native_built, merges_path, oracle, novel, tmp_path):
     """A merges file with more than 65 534 merges builds (the reference accepts any file); the host tokenizer
     equals the oracle under that table and the new, high ids really occur."""
