@@ -115,6 +115,7 @@ struct ResultPool {
   size_t taken_bytes = 0, spare_bytes = 0;
   bool closed = false;  // the handle is gone
 
+  ResultPool() { spare.reserve(size_t(kMaxSpare)); }  // give_back allocates nothing: it ends gtk_result_release
   ~ResultPool()
   {
     for (PinBuf& b : spare) b.release();
@@ -1756,8 +1757,6 @@ static int encode_host(gtk_tokenizer* h, int mode, const uint8_t* bytes, const u
       if (!wait_for_mark(tot + 3, seq, s, "result kernel"))
         return h->fail(GTK_ERR_KERNEL, "result kernel ended without publishing its results");
       C = tot[0], N = tot[1], status = int(tot[2]);
-      h->pack_base = h->h_mid.as<uint8_t>() + 64;
-      h->result_bufs[0] = &h->h_mid;
     } else {
       GTK_CUDA(cudaStreamSynchronize(s));
       const int64_t* ht = h->h_totals.as<int64_t>();
@@ -1770,10 +1769,11 @@ static int encode_host(gtk_tokenizer* h, int mode, const uint8_t* bytes, const u
       h->pool->reserve(h->h_out_pack, text_b + chunk_b + size_t(N) * 4 + 64);
       GTK_CUDA(cudaMemcpyAsync(h->h_out_pack.p, dp, text_b + chunk_b + size_t(N) * 4, cudaMemcpyDeviceToHost, s));
       GTK_CUDA(cudaStreamSynchronize(s));
-      h->pack_base = h->h_out_pack.as<uint8_t>();
-      h->result_bufs[0] = &h->h_out_pack;
     }
     collect_stage_times(h, true);
+    // only now is there a result that can be looked at and taken over
+    h->pack_base        = by_kernel ? h->h_mid.as<uint8_t>() + 64 : h->h_out_pack.as<uint8_t>();
+    h->result_bufs[0]   = by_kernel ? &h->h_mid : &h->h_out_pack;
     h->result_is_packed = true;
     h->pack_text_bytes  = text_b;
     h->pack_chunk_bytes = chunk_b;
@@ -1907,14 +1907,14 @@ GTK_API gtk_taken* gtk_result_take(gtk_tokenizer* h)
   size_t bytes = 0;
   for (PinBuf* b : h->result_bufs)
     if (b) bytes += b->cap;
+  std::unique_ptr<gtk_taken> t(new (std::nothrow) gtk_taken());  // in front of the count, which a failure would leave raised
+  if (!t) return nullptr;
   {
     std::lock_guard<std::mutex> plock(h->pool->mu);
     if (h->pool->taken >= ResultPool::kMaxTaken || h->pool->taken_bytes + bytes > ResultPool::kMaxTakenBytes) return nullptr;
     ++h->pool->taken;
     h->pool->taken_bytes += bytes;
   }
-  gtk_taken* t = new (std::nothrow) gtk_taken();
-  if (!t) return nullptr;
   t->pool  = h->pool;
   t->bytes = bytes;
   // the pointers of gtk_result_view stay what they are
@@ -1927,7 +1927,7 @@ GTK_API gtk_taken* gtk_result_take(gtk_tokenizer* h)
     h->result_bufs[i] = nullptr;
   }
   h->result_is_taken = true;
-  return t;
+  return t.release();
 }
 
 GTK_API void gtk_result_release(gtk_taken* t)
