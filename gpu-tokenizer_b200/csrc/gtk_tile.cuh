@@ -945,6 +945,7 @@ __device__ __noinline__ void merge_huge_segments(uint16_t* scratch, int64_t scra
     if (tid < 32) mark_alive_range(S, int(s) + 1, int(s) + len, tid);
     __syncthreads();
   }
+  __syncthreads();  // no_space: the whole CTA decides by it what comes next
 }
 
 // ---- the listed misses and the long segments.  Ends with a barrier when there are any. ----

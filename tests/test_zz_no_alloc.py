@@ -113,3 +113,31 @@ def test_no_alloc_entry_point_matches_regular_path(native_built, merges_path, or
         keep = np.ones(n_chunks, bool)
         keep[skipped] = False
         assert np.array_equal(counts[keep], np.diff(o_off)[keep])
+
+
+@pytest.mark.parametrize("chunk", [300, 1500, 4096])
+def test_chunks_left_to_the_second_kernel(native_built, merges_path, oracle, chunk):
+    """Most chunks hold segments of 273 bytes and more that are no runs, which the first kernel has no workspace for: it puts such a
+    chunk off as a whole CTA, whichever thread finds out, and the second kernel takes it.  One chunk size for each number of threads."""
+    import torch
+    from oracle.loader import MODE_SEGMENTED
+
+    import gputok_b200
+
+    rng = np.random.default_rng(chunk)
+    letters = np.frombuffer(b"etaoinshrdlu", np.uint8)
+    words = [bytes(rng.choice(letters, size=int(k))) for k in list(range(260, 300)) + [600, 1200] + [3] * 20]
+    n = 600_000
+    data = np.frombuffer(b" ".join(words[i] for i in rng.integers(0, len(words), n // 100))[:n], np.uint8)
+    off = np.minimum(np.arange(0, n + chunk, chunk), n).astype(np.int64)
+    want, woff = oracle.encode_chunks(data, off, mode=MODE_SEGMENTED, threads=8)
+    tok = gputok_b200.Tokenizer(merges_path, chunk_tokens=chunk, device=0)
+    d_bytes, d_off = torch.from_numpy(data.copy()).cuda(), torch.from_numpy(off).cuda()
+    for _ in range(3):
+        out_ids = torch.full((n,), -1, dtype=torch.int32, device="cuda")
+        out_cnt = torch.full((len(off) - 1,), -1, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        tok.encode_chunks_noalloc(d_bytes.data_ptr(), n, d_off.data_ptr(), len(off) - 1, chunk, out_ids.data_ptr(), out_cnt.data_ptr())
+        counts = out_cnt.cpu().numpy()
+        assert np.array_equal(counts, np.diff(woff))
+        assert np.array_equal(_unpack(out_ids.cpu().numpy(), counts, off), want)
