@@ -738,7 +738,13 @@ __device__ __noinline__ int recall_run(int s, int L, const DeviceTable& T)
   TileSmem<TH>& S = tile_smem<TH>();
   uint32_t k[4];
   LongSlot at;
-  if (!run_key(S, s, L, k) || !find_long(T, k, kRunCode, at)) return -1;
+  if (!run_key(S, s, L, k)) return -1;
+  // the slot may be filled just now: what the first lane has seen holds for the warp
+  const bool found = find_long(T, k, kRunCode, at);
+  if (!__shfl_sync(0xFFFFFFFFu, found, 0)) return -1;
+  at.v.y = __shfl_sync(0xFFFFFFFFu, at.v.y, 0);
+  at.v.z = __shfl_sync(0xFFFFFFFFu, at.v.z, 0);
+  at.v.w = __shfl_sync(0xFFFFFFFFu, at.v.w, 0);
   const int n0 = int(at.v.y >> 16), n1 = n0 + int(at.v.z >> 16), n2 = n1 + int(at.v.w >> 16);
   for (int j = threadIdx.x & 31; j < n2; j += 32)
     if (GTK_IN(j, L, 16)) S.tok[s + j] = uint16_t(((j < n0 ? at.v.y : j < n1 ? at.v.z : at.v.w) & 0xFFFFu) - 1u);
