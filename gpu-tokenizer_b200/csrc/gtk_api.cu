@@ -164,8 +164,7 @@ struct gtk_taken {
 // Buffers of one in-flight slice of a large host batch (kSliceArenas sets rotate).
 constexpr int kSliceArenas = 4;
 struct SliceArena {
-  DevBuf text_chunk_base, chunk_off, unit_first, unit_cnt, chunk_cnt, scan_sums, counters,
-      totals;
+  DevBuf text_chunk_base, chunk_off, chunk_cnt, scan_sums, counters, totals;
   PinBuf h_totals;  // mapped: written by a kernel
   cudaEvent_t ev[6] = {};          // stage timing
   cudaEvent_t ev_in = nullptr;     // slice text is in HBM
@@ -174,8 +173,7 @@ struct SliceArena {
   cudaEvent_t ev_out = nullptr;    // results of the slice are on the host
   void release()
   {
-    for (DevBuf* b : {&text_chunk_base, &chunk_off, &unit_first, &unit_cnt, &chunk_cnt, &scan_sums,
-                       &counters, &totals})
+    for (DevBuf* b : {&text_chunk_base, &chunk_off, &chunk_cnt, &scan_sums, &counters, &totals})
       b->release();
     h_totals.release();
     for (auto& e : ev)
@@ -208,7 +206,6 @@ struct gtk_tokenizer {
   DevBuf d_staging32, d_seg_scratch32;  // 32-bit kernel
   int id_space = GTK_IDS_REFERENCE;
   gtk::DeviceTable dtab{};
-  bool reset_learned = false;
   gtk::DeviceTable call_tab{};  // what the kernels of the present call get: dtab, or with a long table of the call's own
 
   // arenas
@@ -335,13 +332,11 @@ constexpr int64_t kLearnMinBytes = int64_t(12) << 20;
 
 void begin_call(gtk_tokenizer* h, int mode, int64_t n_bytes)
 {
-  h->call_tab     = h->dtab;
-  h->reset_learned = false;
+  h->call_tab = h->dtab;
   if (h->wide || mode != GTK_MODE_OPT || n_bytes < kLearnMinBytes) return;
   h->d_learned_words.reserve(h->table->long_words.size() * sizeof(gtk::LongWord));
   h->call_tab.long_words = h->d_learned_words.as<uint4>();
-  h->call_tab.learn      = 1;
-  h->reset_learned       = true;  // by the first launch of the call (run_front)
+  h->call_tab.learn      = 1;  // begin_tiles sets it up
 }
 
 // Upper bound on the number of chunks without touching the device: every text
@@ -356,8 +351,11 @@ struct Plan {
   int64_t chunk_cap = 0;
 };
 
+// Which kernels a batch is planned for: each has arrays of its own.
+enum class Kernels { tiles, chunks, small };
+
 // Size the arenas for a batch and fill the kernel argument block.
-Plan plan_batch(gtk_tokenizer* h, const uint8_t* d_bytes, int64_t n_bytes, const int64_t* d_text_off,
+Plan plan_batch(gtk_tokenizer* h, Kernels kernels, const uint8_t* d_bytes, int64_t n_bytes, const int64_t* d_text_off,
                 int64_t n_texts, int32_t* d_out_ids, int64_t out_capacity, int64_t* d_chunk_id_off,
                 bool want_text_id_off)
 {
@@ -367,16 +365,19 @@ Plan plan_batch(gtk_tokenizer* h, const uint8_t* d_bytes, int64_t n_bytes, const
   const int64_t n_tiles = (n_bytes + gtk::kTile - 1) / gtk::kTile;
   p.chunk_cap = chunk_cap;
   h->d_text_chunk_base.reserve(size_t(n_texts + 1) * 8);
-  h->d_chunk_off.reserve(size_t(chunk_cap + 1) * 8);
-  h->d_tile_chunk0.reserve(size_t(gtk::kSmallMaxBytes / gtk::kTile + 1) * 4);
-  h->d_tile_info.reserve(size_t(n_tiles + 1) * sizeof(gtk::TileInfo));
-  h->d_chunk_rel.reserve(size_t(chunk_cap + 1) * 4);
-  h->d_text_rel.reserve(size_t(n_texts + 1) * 4);
-  h->d_group_base.reserve(size_t(n_tiles / gtk::kTileGroup + 2) * 8);
-  h->d_staging.reserve(size_t(n_bytes + 16) * 2);
-  h->d_unit_first.reserve(size_t(n_tiles + 1) * 8);
-  h->d_unit_cnt.reserve(size_t(n_tiles + 1) * 4);
-  h->d_chunk_cnt.reserve(size_t(chunk_cap + 1) * 4);
+  if (kernels == Kernels::tiles) {
+    h->d_tile_info.reserve(size_t(n_tiles + 1) * sizeof(gtk::TileInfo));
+    h->d_chunk_rel.reserve(size_t(chunk_cap + 1) * 4);
+    h->d_text_rel.reserve(size_t(n_texts + 1) * 4);
+    h->d_group_base.reserve(size_t(n_tiles / gtk::kTileGroup + 2) * 8);
+    h->d_unit_first.reserve(size_t(n_tiles + 1) * 8);
+    h->d_unit_cnt.reserve(size_t(n_tiles + 1) * 4);
+  } else {
+    h->d_chunk_off.reserve(size_t(chunk_cap + 1) * 8);
+    h->d_chunk_cnt.reserve(size_t(chunk_cap + 1) * 4);
+    h->d_tile_chunk0.reserve(size_t(gtk::kSmallMaxBytes / gtk::kTile + 1) * 4);
+  }
+  if (kernels != Kernels::small) h->d_staging.reserve(size_t(n_bytes + 16) * 2);
   if (!d_chunk_id_off) {
     h->d_chunk_id_off.reserve(size_t(chunk_cap + 1) * 8);
     d_chunk_id_off = h->d_chunk_id_off.as<int64_t>();
@@ -503,22 +504,23 @@ void run_pack(gtk_tokenizer* h, const gtk::EncodeBuffers& b, int* launches, cuda
   if (chained && totals_by_copy) copy_totals(h, b, nullptr, s);
 }
 
-// The tile kernel and what follows it (GTK_MODE_OPT): reset, chunks per text, tile records, tiles, pack.
-// `ready`: counters, group counts, scanned chunk counts and tile records are in place already.  The pack kernel publishes the totals (see
+// What comes in front of the tile kernel: reset, scan of the texts, tile records.
+void begin_tiles(gtk_tokenizer* h, const gtk::EncodeBuffers& b, int* launches)
+{
+  const bool learned = h->call_tab.learn != 0;
+  *launches += gtk::launch_begin_batch(b, h->dtab.long_words, learned ? h->call_tab.long_words : nullptr, h->stream);
+  *launches += gtk::launch_scan_texts(b, learned, h->stream) + gtk::launch_tile_info(b, h->stream);
+}
+
+// All kernels of a batch in GTK_MODE_OPT.  `ready`: counters, group counts, scanned chunk counts and tile records are in place already.  The pack kernel publishes the totals (see
 // launch_pack_tiles).  The events between the stages are recorded when they are asked for.
-void run_tiles(gtk_tokenizer* h, const gtk::EncodeBuffers& b, bool ready, int64_t* publish, int64_t seq, int* launches,
-               cudaEvent_t* ev = nullptr)
+void run_tiles(gtk_tokenizer* h, const gtk::EncodeBuffers& b, bool ready, int64_t* publish, int64_t seq, int* launches)
 {
   cudaStream_t s    = h->stream;
-  const bool stages = ev != nullptr || h->stage_timing;
-  if (!ev) ev = h->ev;
-  const bool learned = h->reset_learned;
+  const bool stages = h->stage_timing;
+  cudaEvent_t* ev   = h->ev;
   if (stages) GTK_CUDA(cudaEventRecord(ev[0], s));
-  if (!ready || learned) {
-    *launches += gtk::launch_begin_batch(b, h->dtab.long_words, learned ? h->call_tab.long_words : nullptr, s);
-  }
-  h->reset_learned = false;
-  if (!ready) *launches += gtk::launch_scan_texts(b, learned, s) + gtk::launch_tile_info(b, s);
+  if (!ready) begin_tiles(h, b, launches);
   if (stages) GTK_CUDA(cudaEventRecord(ev[1], s));
   *launches += gtk::launch_merge_opt(b, h->call_tab, h->opt_grid, s);
   if (stages) GTK_CUDA(cudaEventRecord(ev[2], s));
@@ -661,13 +663,10 @@ std::vector<SlicePlan> plan_slices(const int64_t* text_off, int64_t n_texts, int
 void slice_arena_prepare(gtk_tokenizer* h, SliceArena& a, int64_t max_bytes, int64_t max_pieces)
 {
   const int64_t chunk_cap = chunk_upper_bound(max_bytes, max_pieces, h->chunk_tokens);
-  const int64_t n_tiles   = (max_bytes + gtk::kTile - 1) / gtk::kTile;
   a.text_chunk_base.reserve(size_t(max_pieces + 1) * 8);
   a.chunk_off.reserve(size_t(chunk_cap + 1) * 8);
-  a.unit_first.reserve(size_t(n_tiles + 1) * 8);
-  a.unit_cnt.reserve(size_t(n_tiles + 1) * 4);
   a.chunk_cnt.reserve(size_t(chunk_cap + 1) * 4);
-  a.scan_sums.reserve(size_t(std::max<int64_t>(std::max(chunk_cap, n_tiles), max_pieces) / 4096 + 2) * 8);
+  a.scan_sums.reserve(size_t(std::max(chunk_cap, max_pieces) / 4096 + 2) * 8);
   a.counters.reserve(64);
   a.totals.reserve(64);
   a.h_totals.reserve_mapped(64);
@@ -697,8 +696,6 @@ gtk::EncodeBuffers slice_buffers(gtk_tokenizer* h, SliceArena& a, const SlicePla
   b.chunk_cap = chunk_upper_bound(n_bytes, pieces, h->chunk_tokens);
   b.n_tiles = (n_bytes + gtk::kTile - 1) / gtk::kTile;
   b.staging = h->d_staging.as<uint16_t>() + dev_off;
-  b.unit_first = a.unit_first.as<int64_t>();
-  b.unit_cnt = a.unit_cnt.as<int32_t>();
   b.chunk_cnt = a.chunk_cnt.as<int32_t>();
   b.chunk_id_off = nullptr;
   b.text_id_off = nullptr;
@@ -1069,7 +1066,7 @@ int encode_host_small(gtk_tokenizer* h, const Source& src, const int64_t* text_o
 {
   std::memcpy(h->small_in_h + kSmallInOff, text_offsets, size_t(n_texts + 1) * 8);
   src.copy_all(h->small_in_h + kSmallInBytes);
-  Plan p = plan_batch(h, h->small_in_d + kSmallInBytes, n_bytes,
+  Plan p = plan_batch(h, Kernels::small, h->small_in_d + kSmallInBytes, n_bytes,
                       reinterpret_cast<const int64_t*>(h->small_in_d + kSmallInOff), n_texts,
                       reinterpret_cast<int32_t*>(h->small_out_d + kSmallOutIds), gtk::kSmallMaxBytes,
                       reinterpret_cast<int64_t*>(h->small_out_d + kSmallOutChunk), false);
@@ -1189,7 +1186,7 @@ int encode_host_tiles(gtk_tokenizer* h, const Source& src, const int64_t* text_o
     h->pool->reserve(h->h_out, 64 + text_b + chunk_b + size_t(room) * 4);
     md = h->h_out.as<uint8_t>();  // page-locked memory has the same address on the device
     std::memset(md, 0, 64);
-    p = plan_batch(h, with_text ? dp + o_text : h->d_bytes.as<uint8_t>(), n_bytes, reinterpret_cast<int64_t*>(dp + o_off), n_texts,
+    p = plan_batch(h, Kernels::tiles, with_text ? dp + o_text : h->d_bytes.as<uint8_t>(), n_bytes, reinterpret_cast<int64_t*>(dp + o_off), n_texts,
                    reinterpret_cast<int32_t*>(md + 64 + text_b + chunk_b), room, reinterpret_cast<int64_t*>(md + 64 + text_b), false);
     p.b.text_id_off     = reinterpret_cast<int64_t*>(md + 64);
     p.b.totals          = reinterpret_cast<int64_t*>(dp);
@@ -1297,19 +1294,16 @@ int encode_host_pieces(gtk_tokenizer* h, const Source& src, const int64_t* text_
     GTK_CUDA(cudaEventCreateWithFlags(&e, h->piece_ev.size() % 4 == 0 ? cudaEventDisableTiming : cudaEventDefault));
     h->piece_ev.push_back(e);
   }
-  gtk::EncodeBuffers b = plan_batch(h, h->d_bytes.as<uint8_t>(), n_bytes, h->d_text_off.as<int64_t>(), n_texts,
+  gtk::EncodeBuffers b = plan_batch(h, Kernels::tiles, h->d_bytes.as<uint8_t>(), n_bytes, h->d_text_off.as<int64_t>(), n_texts,
                                     h->d_out_ids.as<int32_t>(), n_bytes, nullptr, true).b;
   int32_t* tickets = b.group_cnt + groups;
   cudaStream_t s   = h->stream;
   int launches     = 0;
   begin_call(h, GTK_MODE_OPT, n_bytes);
-  const bool learned = h->reset_learned;
-  h->reset_learned   = false;
   if (n_texts > 1) GTK_CUDA(cudaMemcpyAsync(h->d_text_off.p, text_offsets, size_t(n_texts + 1) * 8, cudaMemcpyHostToDevice, s));
   GTK_CUDA(cudaMemsetAsync(tickets, 0, np * 4, s));
   GTK_CUDA(cudaEventRecord(h->ev[0], s));
-  launches += gtk::launch_begin_batch(b, h->dtab.long_words, learned ? h->call_tab.long_words : nullptr, s);
-  launches += gtk::launch_scan_texts(b, learned, s) + gtk::launch_tile_info(b, s);
+  begin_tiles(h, b, &launches);
   GTK_CUDA(cudaEventRecord(h->ev[1], s));
   GTK_CUDA(cudaGetLastError());
 
@@ -1605,10 +1599,12 @@ GTK_API int gtk_encode_device(gtk_tokenizer* h, int mode, const uint8_t* d_bytes
     const int64_t need_chunks = chunk_upper_bound(n_bytes, n_texts, h->chunk_tokens);
     int64_t* chunk_dst = d_out_chunk_offsets;
     if (chunk_dst && chunk_capacity < need_chunks + 1) chunk_dst = nullptr;  // scan into the arena, copy what fits
-    Plan p = plan_batch(h, d_bytes, n_bytes, d_text_offsets, n_texts, d_out_ids, out_capacity, chunk_dst, false);
+    const bool by_tiles = mode == GTK_MODE_OPT && !h->wide;
+    Plan p = plan_batch(h, by_tiles ? Kernels::tiles : Kernels::chunks, d_bytes, n_bytes, d_text_offsets, n_texts, d_out_ids,
+                        out_capacity, chunk_dst, false);
     begin_call(h, mode, n_bytes);
     int launches = 0;
-    if (mode == GTK_MODE_OPT && !h->wide) {
+    if (by_tiles) {
       p.b.text_end = d_text_offsets + n_texts;
       volatile int64_t* tot = h->h_totals.as<int64_t>();
       const int64_t seq     = ++h->mid_seq;
@@ -1735,7 +1731,7 @@ static int encode_host(gtk_tokenizer* h, int mode, const uint8_t* bytes, const u
     const size_t chunk_b = ((size_t(chunk_upper_bound(n_bytes, n_texts, h->chunk_tokens)) + 1) * 8 + 63) & ~size_t(63);
     h->d_out_pack.reserve(text_b + chunk_b + size_t(n_bytes) * 4 + 64);
     uint8_t* dp = h->d_out_pack.as<uint8_t>();
-    Plan p = plan_batch(h, h->d_bytes.as<uint8_t>(), n_bytes, h->d_text_off.as<int64_t>(), n_texts,
+    Plan p = plan_batch(h, Kernels::chunks, h->d_bytes.as<uint8_t>(), n_bytes, h->d_text_off.as<int64_t>(), n_texts,
                         reinterpret_cast<int32_t*>(dp + text_b + chunk_b), n_bytes,
                         reinterpret_cast<int64_t*>(dp + text_b), true);
     p.b.text_id_off = reinterpret_cast<int64_t*>(dp);

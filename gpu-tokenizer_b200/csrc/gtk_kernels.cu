@@ -30,9 +30,6 @@
 namespace gtk {
 namespace {
 
-#ifdef GTK_PHASE_TIMING
-__device__ unsigned long long g_phase_cycles[32];
-#endif
 
 // Checked build (-DGTK_CHECKED): every index into shared memory, the lane scratch, the staging buffer and the
 // per-chunk / per-unit arrays that is computed from data is compared with its limit before it is used.  A
@@ -171,16 +168,16 @@ __device__ __forceinline__ uint32_t lanemask_lt()
 }
 
 // ------------------------------------------------------------------------------------------------
-// A group of NW warps (one warp, or the whole CTA) merges one sequence pass by
-// pass.  tok/rk may point to shared memory or to an HBM workspace.
+// The NW warps of a CTA merge one sequence pass by pass.  tok/rk may point to
+// shared memory or to an HBM workspace.
 //
 // Slots: tok[i] is a token id or the DEAD tombstone; for a live slot rk[i] is the
 // cached rank of the pair (tok[i], next live token), NONE when there is none; a
 // dead slot has rk NONE.  Tombstones stay where they are and the slots are
 // compacted only when an eighth of them is dead, so a pass costs two sweeps over
 // the cached ranks plus work proportional to the number of merges:
-//   (1) group-wide minimum of the cached ranks (four ranks per 64-bit load when
-//       VEC, i.e. when rk is 8-byte aligned; warp redux + cross-warp exchange);
+//   (1) minimum of the cached ranks (four ranks per 64-bit load, rk is 8-byte
+//       aligned; warp redux + cross-warp exchange);
 //   (2) selection of the occurrences of that pair;
 //   (3) every selected occurrence writes the merged id and a tombstone and
 //       remembers its slot;
@@ -198,8 +195,8 @@ constexpr int kMergeList = 64;  // merges of one pass that are re-probed from a 
 struct GroupScratch {
   uint32_t red[2][32];
   uint32_t wsum[32];
-  int dead;  // tombstones since the last compaction (CTA-wide groups)
-  int list[kMergeList];  // slots merged in the current pass (CTA-wide groups)
+  int dead;  // tombstones since the last compaction
+  int list[kMergeList];  // slots merged in the current pass
 };
 
 template <int NW>
@@ -237,7 +234,7 @@ __device__ __forceinline__ int prev_live(const uint16_t* tok, int i)
   return p;
 }
 
-// VEC sweeps read the cached ranks four at a time (one 64-bit load) and reduce them with the packed 16-bit
+// Sweeps read the cached ranks four at a time (one 64-bit load) and reduce them with the packed 16-bit
 // three-input minimum; the up to three slots between n and the next multiple of four hold NONE (pad_ranks).
 __device__ __forceinline__ void pad_ranks(uint16_t* rk, int n, int tid)
 {
@@ -245,27 +242,21 @@ __device__ __forceinline__ void pad_ranks(uint16_t* rk, int n, int tid)
 }
 
 // calls f(i) for every slot i < n whose cached rank equals `pick`
-template <int NW, bool VEC, class F>
+template <int NW, class F>
 __device__ __forceinline__ void for_each_rank(const uint16_t* rk, int n, int tid, uint32_t pick, F f)
 {
-  constexpr int G = NW * 32;
-  if (VEC) {
-    const int nw      = (n + 3) >> 2;
-    const uint32_t p2 = pick | (pick << 16);
-    for (int w = tid; w < nw; w += G) {
-      const uint2 x = reinterpret_cast<const uint2*>(rk)[w];
-      // a half-word of z is zero exactly when one of the four ranks equals pick
-      const uint32_t z = __vimin3_u16x2(x.x ^ p2, x.y ^ p2, 0xFFFFFFFFu);
-      if ((z & 0xFFFFu) == 0u || (z >> 16) == 0u) {
-        const uint32_t q[4] = {x.x & 0xFFFFu, x.x >> 16, x.y & 0xFFFFu, x.y >> 16};
+  const int nw      = (n + 3) >> 2;
+  const uint32_t p2 = pick | (pick << 16);
+  for (int w = tid; w < nw; w += NW * 32) {
+    const uint2 x = reinterpret_cast<const uint2*>(rk)[w];
+    // a half-word of z is zero exactly when one of the four ranks equals pick
+    const uint32_t z = __vimin3_u16x2(x.x ^ p2, x.y ^ p2, 0xFFFFFFFFu);
+    if ((z & 0xFFFFu) == 0u || (z >> 16) == 0u) {
+      const uint32_t q[4] = {x.x & 0xFFFFu, x.x >> 16, x.y & 0xFFFFu, x.y >> 16};
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
-          if (q[k] == pick) f(4 * w + k);
-      }
+      for (int k = 0; k < 4; ++k)
+        if (q[k] == pick) f(4 * w + k);
     }
-  } else {
-    for (int i = tid; i < n; i += G)
-      if (rk[i] == pick) f(i);
   }
 }
 
@@ -290,18 +281,13 @@ __device__ __forceinline__ int group_compact(uint16_t* tok, uint16_t* rk, int n,
       bal[k] = __ballot_sync(0xFFFFFFFFu, t[k] != DEAD);
       wt += __popc(bal[k]);
     }
-    int pre = 0, tot = wt;
-    if (NW > 1) {
-      if (lane == 0) gs->wsum[warp] = uint32_t(wt);
-      __syncthreads();  // all loads of the batch are done, warp totals visible
-      tot = 0;
-      for (int w = 0; w < NW; ++w) {
-        const int x = int(gs->wsum[w]);
-        if (w < warp) pre += x;
-        tot += x;
-      }
-    } else {
-      __syncwarp();
+    if (lane == 0) gs->wsum[warp] = uint32_t(wt);
+    __syncthreads();  // all loads of the batch are done, warp totals visible
+    int pre = 0, tot = 0;
+    for (int w = 0; w < NW; ++w) {
+      const int x = int(gs->wsum[w]);
+      if (w < warp) pre += x;
+      tot += x;
     }
     int o = out + pre;
 #pragma unroll
@@ -314,63 +300,48 @@ __device__ __forceinline__ int group_compact(uint16_t* tok, uint16_t* rk, int n,
       o += __popc(bal[k]);
     }
     out += tot;
-    gsync<NW>();
+    __syncthreads();
   }
   return out;
 }
 
-template <int NW, bool VEC>
+template <int NW>
 __device__ int group_merge(uint16_t* tok, uint16_t* rk, int L, const DeviceTable& T, GroupScratch* gs,
                            int* status)
 {
-  constexpr int G    = NW * 32;
-  constexpr int kMem = 4;  // merged slots a thread remembers per pass; more fall back to a sweep
-  const int lane  = threadIdx.x & 31;
-  const int warp  = (NW == 1) ? 0 : (threadIdx.x >> 5);
-  const int tid   = (NW == 1) ? lane : int(threadIdx.x);
+  constexpr int G = NW * 32;
+  const int tid = int(threadIdx.x), lane = tid & 31, warp = tid >> 5;
   const uint32_t lt = lanemask_lt();
   const bool batch  = T.monotone != 0;
   int parity = 0;
   int n      = L;  // slots in use
   int dead   = 0;  // tombstones among them
-  if (VEC) pad_ranks(rk, n, tid);
-  if (NW > 1) {
-    if (tid == 0) gs->dead = 0;
-    __syncthreads();
-  } else {
-    __syncwarp();
-  }
+  pad_ranks(rk, n, tid);
+  if (tid == 0) gs->dead = 0;
+  __syncthreads();
   for (int pass = 0; pass < L && n - dead >= 2; ++pass) {
     // (1) lowest cached rank
-    uint32_t m = NONE;
-    if (VEC) {
-      const int nw = (n + 3) >> 2;
-      uint32_t m2  = 0xFFFFFFFFu;
-      for (int w = tid; w < nw; w += G) {
-        const uint2 x = reinterpret_cast<const uint2*>(rk)[w];
-        m2 = __vimin3_u16x2(m2, x.x, x.y);
-      }
-      m = min(m2 & 0xFFFFu, m2 >> 16);
-    } else {
-      for (int i = tid; i < n; i += G) m = min(m, uint32_t(rk[i]));
+    uint32_t m2 = 0xFFFFFFFFu;
+    for (int w = tid; w < (n + 3) >> 2; w += G) {
+      const uint2 x = reinterpret_cast<const uint2*>(rk)[w];
+      m2 = __vimin3_u16x2(m2, x.x, x.y);
     }
-    m = group_min<NW>(m, gs, parity, lane, warp);
-    if (m >= SEL) break;
-    const uint32_t r = m;
+    const uint32_t r = group_min<NW>(min(m2 & 0xFFFFu, m2 >> 16), gs, parity, lane, warp);
+    if (r >= SEL) break;
     const uint32_t c = merged_id(T, r);
     const bool same  = batch && (__ldg(T.same_of_rank + r) != 0);
     // (2) selection
     if (!batch) {
       uint32_t p = 0xFFFFFFFFu;
-      for_each_rank<NW, VEC>(rk, n, tid, r, [&](int i) { p = min(p, uint32_t(i)); });
+      for_each_rank<NW>(rk, n, tid, r, [&](int i) { p = min(p, uint32_t(i)); });
       p = group_min<NW>(p, gs, parity, lane, warp);
-      gsync<NW>();
+      __syncthreads();
       if (tid == 0) rk[p] = uint16_t(SEL);
-      gsync<NW>();
+      __syncthreads();
     } else if (same) {
       // occurrences of (a,a) overlap inside a run a a a ...; left to right
       // selection keeps the even offsets of every maximal run of matches
-      for_each_rank<NW, VEC>(rk, n, tid, r, [&](int i) {
+      for_each_rank<NW>(rk, n, tid, r, [&](int i) {
         const int pl = prev_live(tok, i);
         if (pl >= 0) {
           const uint32_t pv = rk[pl];
@@ -386,15 +357,12 @@ __device__ int group_merge(uint16_t* tok, uint16_t* rk, int L, const DeviceTable
           j = j2;
         }
       });
-      gsync<NW>();
+      __syncthreads();
     }
     const uint32_t pick = (!batch || same) ? SEL : r;
-    // (3) apply: the selected occurrences never share a slot, so the writes are disjoint.  A CTA-wide group
-    // collects the merged slots in a shared list (the tombstone counter hands out the places), a single warp
-    // keeps them in registers
-    int mine = 0;
-    int at[kMem];
-    for_each_rank<NW, VEC>(rk, n, tid, pick, [&](int i) {
+    // (3) apply: the selected occurrences never share a slot, so the writes are disjoint.  The merged slots are
+    // collected in a list; the tombstone counter hands out the places
+    for_each_rank<NW>(rk, n, tid, pick, [&](int i) {
       const int j = next_live(tok, i, n);  // exists: the pair has a cached rank
       if (!GTK_IN(i, n, 30)) return;
       tok[i] = uint16_t(c);
@@ -403,15 +371,8 @@ __device__ int group_merge(uint16_t* tok, uint16_t* rk, int L, const DeviceTable
         tok[j] = uint16_t(DEAD);
         rk[j]  = uint16_t(NONE);
       }
-      if (NW > 1) {
-        const int place = atomicAdd(&gs->dead, 1) - dead;
-        if (place < kMergeList) gs->list[place] = i;
-      } else {
-#pragma unroll
-        for (int k = 0; k < kMem; ++k)
-          if (mine == k) at[k] = i;
-        ++mine;
-      }
+      const int place = atomicAdd(&gs->dead, 1) - dead;
+      if (place < kMergeList) gs->list[place] = i;
     });
     // (4) ranks of the two pairs next to every new token
     auto refresh = [&](int i) {
@@ -420,50 +381,28 @@ __device__ int group_merge(uint16_t* tok, uint16_t* rk, int L, const DeviceTable
       const int pl = prev_live(tok, i);
       if (pl >= 0) rk[pl] = uint16_t(probe_rank(T, tok[pl], c));
     };
-    if (NW > 1) {
-      __syncthreads();
-      const int now = gs->dead;
-      if (now == dead) {  // a pass must remove at least one token
-        if (tid == 0 && status) atomicMax(status, int(kStatusBadSegment));
-        break;
-      }
-      const int merged = now - dead;
-      dead = now;
-      if (merged <= kMergeList) {  // the first threads take one merged slot each: one or two warps do the probes
-        if (tid < merged) refresh(gs->list[tid]);
-      } else {
-        for (int i = tid; i < n; i += G)
-          if (tok[i] == c) refresh(i);
-      }
-    } else {
-      const int wsum   = __reduce_add_sync(0xFFFFFFFFu, mine);
-      const bool sweep = __any_sync(0xFFFFFFFFu, mine > kMem) != 0;
-      if (wsum == 0) {
-        if (tid == 0 && status) atomicMax(status, int(kStatusBadSegment));
-        break;
-      }
-      dead += wsum;
-      if (!sweep) {
-#pragma unroll
-        for (int k = 0; k < kMem; ++k)
-          if (k < mine) refresh(at[k]);
-      } else {
-        for (int i = tid; i < n; i += G)
-          if (tok[i] == c) refresh(i);
-      }
+    __syncthreads();
+    const int now = gs->dead;
+    if (now == dead) {  // a pass must remove at least one token
+      if (tid == 0 && status) atomicMax(status, int(kStatusBadSegment));
+      break;
     }
-    gsync<NW>();
+    const int merged = now - dead;
+    dead = now;
+    if (merged <= kMergeList) {  // the first threads take one merged slot each: one or two warps do the probes
+      if (tid < merged) refresh(gs->list[tid]);
+    } else {
+      for (int i = tid; i < n; i += G)
+        if (tok[i] == c) refresh(i);
+    }
+    __syncthreads();
     // (5) compaction when an eighth of the slots is dead
     if (dead * 8 >= n) {
       n    = group_compact<NW>(tok, rk, n, gs, lane, warp, lt);
       dead = 0;
-      if (VEC) pad_ranks(rk, n, tid);
-      if (NW > 1) {
-        if (tid == 0) gs->dead = 0;
-        __syncthreads();
-      } else {
-        __syncwarp();
-      }
+      pad_ranks(rk, n, tid);
+      if (tid == 0) gs->dead = 0;
+      __syncthreads();
     }
   }
   if (dead) n = group_compact<NW>(tok, rk, n, gs, lane, warp, lt);
@@ -817,21 +756,6 @@ __global__ void k_chunk_fill(const int64_t* __restrict__ text_off, const int64_t
 // merge kernel, segment-parallel ("opt")
 // ------------------------------------------------------------------------------------------------
 
-// Optional per-phase cycle accounting of k_merge_opt (build with -DGTK_PHASE_TIMING): thread 0 of
-// every CTA accumulates clock64() deltas between phase boundaries; read with gtk_debug_phase_cycles.
-#ifdef GTK_PHASE_TIMING
-#define GTK_PHASE(k)                                              \
-  do {                                                            \
-    if (threadIdx.x == 0) {                                       \
-      const long long now__ = clock64();                          \
-      atomicAdd(&g_phase_cycles[k], (unsigned long long)(now__ - phase_t0)); \
-      phase_t0 = now__;                                           \
-    }                                                             \
-  } while (0)
-#else
-#define GTK_PHASE(k) do { } while (0)
-#endif
-
 #include "gtk_tile.cuh"
 
 // Window k of a batch walked in tiles of kTile bytes: n_tiles that hold text, `tail` bytes of it in the last of them.
@@ -962,19 +886,13 @@ __device__ __forceinline__ void opt_tile(TileSmem<kOptThreads>& S, const EncodeB
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int* status   = b.counters + 1;
   const Span sp = batch_span(b, k, S.n_tiles, S.tail);
-#ifdef GTK_PHASE_TIMING
-  long long phase_t0 = clock64();
-#endif
   const TileInfo ti = b.tile_info[k];
   tile_cut(S, sp, T, [&](auto mark) { for_each_start(b, ti, sp.lo, sp.wlen, 0, 1, [&](int p, int64_t, int64_t) { mark(p); }); });
-  GTK_PHASE(0);
   tile_lookup(S, sp, T, status);
-  GTK_PHASE(1);
   const int first = S.first;
   const int end   = (S.over_start >= 0) ? S.over_start : S.end;
   uint16_t* ws    = b.seg_scratch ? b.seg_scratch + int64_t(blockIdx.x) * 2 * b.seg_scratch_tokens : nullptr;
   tile_merge(S, T, ws, b.seg_scratch_tokens, status);
-  GTK_PHASE(2);
   const int64_t region_start = sp.lo + min(first, sp.wlen);
   tile_emit<kOptThreads, true>(S, first, end, woff, [&](int off, const uint16_t* ids, int n) {
     uint16_t* dst = b.staging + region_start + off;
@@ -982,7 +900,6 @@ __device__ __forceinline__ void opt_tile(TileSmem<kOptThreads>& S, const EncodeB
       if (GTK_IN(region_start + off + j, b.n_bytes, 22)) dst[j] = ids[j];
   });
   __syncthreads();
-  GTK_PHASE(3);
   const int total = S.total;
   if (S.no_space && tid == 0) atomicMax(status, int(kStatusScratchTooSmall));
   // ids of the tile in front of every chunk and text that starts in it (a chunk start is a segment start, so it lies inside
@@ -992,7 +909,6 @@ __device__ __forceinline__ void opt_tile(TileSmem<kOptThreads>& S, const EncodeB
     if (c >= 0 && GTK_IN(c, b.chunk_cap, 24)) b.chunk_rel[c] = rel;
     if (t >= 0 && GTK_IN(t, b.n_texts, 25)) b.text_rel[t] = rel;
   });
-  GTK_PHASE(4);
   int over = 0;
   if (S.over_start >= 0) {  // CTA-uniform, rare
     const int64_t start = sp.lo + S.over_start;
@@ -1008,7 +924,6 @@ __device__ __forceinline__ void opt_tile(TileSmem<kOptThreads>& S, const EncodeB
     b.unit_cnt[k]   = total + over;
     atomicAdd(b.group_cnt + k / kTileGroup, total + over);
   }
-  GTK_PHASE(5);
 }
 
 // Bound by latency and issue together (see gtk_tile.cuh): about 60 % of the issue slots, DRAM 3 %.  This kernel alone, 128 MiB
@@ -1121,17 +1036,11 @@ __global__ void __launch_bounds__(kMediumThreads) k_chunker_medium(EncodeBuffers
   __shared__ int64_t carry_s;
   __shared__ __align__(16) int stage[4 * kMediumThreads];
   const int tid = threadIdx.x;
-#ifdef GTK_PHASE_TIMING
-  const long long m_t0 = clock64();
-#endif
   // this launch also resets the call's counters and per-chunk counts (two memsets less on the host)
   if (tid < 16) b.counters[tid] = 0;
   for (int64_t c = tid; c <= b.chunk_cap; c += kMediumThreads) b.chunk_cnt[c] = 0;
   const int64_t C = cta_exclusive_scan_medium(ChunksPerText{b.text_off, b.chunk_bytes}, b.n_texts, b.text_chunk_base,
                                               scanbuf, &carry_s, stage);
-#ifdef GTK_PHASE_TIMING
-  if (tid == 0) g_phase_cycles[24] = (unsigned long long)(clock64() - m_t0);
-#endif
   if (tid == 0) b.totals[0] = C;
   if (per_text) {
     // many short texts: every text writes the offsets of its own chunks (no search); a thread takes the texts of up to
@@ -1159,9 +1068,6 @@ __global__ void __launch_bounds__(kMediumThreads) k_chunker_medium(EncodeBuffers
       }
     }
     __syncthreads();
-#ifdef GTK_PHASE_TIMING
-    if (tid == 0) g_phase_cycles[25] = (unsigned long long)(clock64() - m_t0);
-#endif
     const int lane = tid & 31, warp = tid >> 5;
     if (n_long <= kLongTexts) {  // the usual case: the few long texts come from the list
       for (int q = warp; q < n_long; q += kMediumThreads / 32) {
@@ -2084,17 +1990,6 @@ extern "C" __attribute__((visibility("default"))) int gtk_debug_check_words(int 
 }
 #endif
 
-#ifdef GTK_PHASE_TIMING
-extern "C" __attribute__((visibility("default"))) void gtk_debug_phase_cycles(unsigned long long out[32], int reset)
-{
-  cudaDeviceSynchronize();
-  cudaMemcpyFromSymbol(out, g_phase_cycles, sizeof(unsigned long long) * 32);
-  if (reset) {
-    unsigned long long z[32] = {};
-    cudaMemcpyToSymbol(g_phase_cycles, z, sizeof(z));
-  }
-}
-#endif
 
 __global__ void k_publish_totals(const int64_t* totals, const int32_t* counters, int64_t* mapped)
 {
@@ -2282,7 +2177,7 @@ k_merge_chunks_noalloc(const uint8_t* __restrict__ bytes, const int64_t* __restr
       rk[i]  = (i + 1 < L) ? __ldg(T.byte_pair_rank + ((cur << 8) | bytes[cs + i + 1])) : uint16_t(NONE);
     }
     __syncthreads();
-    const int len = group_merge<kBaseThreads / 32, true>(tok, rk, L, T, &gs, header + 1);
+    const int len = group_merge<kBaseThreads / 32>(tok, rk, L, T, &gs, header + 1);
     for (int j = tid; j < len; j += kBaseThreads) {
       const uint32_t t = tok[j];
       out_ids[cs + j]  = int32_t((low_id_map && t < 256u) ? uint32_t(__ldg(low_id_map + t)) : t);

@@ -392,9 +392,6 @@ __device__ __noinline__ void merge_batch(uint32_t ent, int slots, int scratch_wo
                                          uint4* learned)
 {
   TileSmem<TH>& S = tile_smem<TH>();
-#ifdef GTK_PHASE_TIMING
-  const long long batch_t0 = clock64();
-#endif
   const int L = int(ent & 15u) + 1;
   int s       = int(ent >> 4);
   if (!GTK_IN(s + L, S.kWin + 1, 15)) s = 0, ent = 0;
@@ -438,15 +435,7 @@ __device__ __noinline__ void merge_batch(uint32_t ent, int slots, int scratch_wo
   };
   auto set_rank = [&](int i, uint32_t v) { reinterpret_cast<uint16_t*>(scr + (i >> 1) * 32)[i & 1] = uint16_t(v); };
   uint32_t best = lowest();
-#ifdef GTK_PHASE_TIMING
-  const long long loop_t0 = clock64();
-  int trips = 0;
-  if (threadIdx.x == 0) atomicAdd(&g_phase_cycles[13], (unsigned long long)(loop_t0 - batch_t0));
-#endif
   while (__any_sync(0xFFFFFFFFu, best < (SEL << 16))) {
-#ifdef GTK_PHASE_TIMING
-    ++trips;
-#endif
     if (best < (SEL << 16)) {
       const int j = int(best & 0xFFFFu);
       uint32_t t  = alive & (0xFFFFFFFEu << j);
@@ -491,12 +480,6 @@ __device__ __noinline__ void merge_batch(uint32_t ent, int slots, int scratch_wo
       }
     }
   }
-#ifdef GTK_PHASE_TIMING
-  if (threadIdx.x == 0) {
-    atomicAdd(&g_phase_cycles[14], (unsigned long long)(clock64() - loop_t0));
-    atomicAdd(&g_phase_cycles[15], (unsigned long long)trips);
-  }
-#endif
   if (ent) {
     mark_alive(S, s, alive);
     if (learned) learn_segment(S, learned, s, uint32_t(L), alive);
@@ -945,7 +928,7 @@ __device__ __noinline__ void merge_huge_segments(uint16_t* scratch, int64_t scra
       scratch[scratch_tokens + i] = (i + 1 < L) ? __ldg(T.byte_pair_rank + ((u << 8) | S.bytes[17 + s + i])) : uint16_t(NONE);
     }
     __syncthreads();
-    const int len = group_merge<TH / 32, true>(scratch, scratch + scratch_tokens, L, T, S.gs(), status);
+    const int len = group_merge<TH / 32>(scratch, scratch + scratch_tokens, L, T, S.gs(), status);
     __syncthreads();
     for (int i = tid; i < len; i += TH) S.tok[s + i] = scratch[i];
     if (tid < 32) mark_alive_range(S, int(s) + 1, int(s) + len, tid);
@@ -1116,7 +1099,7 @@ __device__ __noinline__ int merge_oversize(const uint8_t* bytes, int64_t start, 
       wrk[i] = (i + 1 < L) ? __ldg(T.byte_pair_rank + ((cur << 8) | bytes[start + i + 1])) : uint16_t(NONE);
     }
     __syncthreads();
-    len = group_merge<TH / 32, true>(wt, wrk, L, T, S.gs(), status);
+    len = group_merge<TH / 32>(wt, wrk, L, T, S.gs(), status);
   }
   __syncthreads();
   return len;
