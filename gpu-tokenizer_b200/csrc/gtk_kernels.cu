@@ -938,16 +938,19 @@ __global__ void __launch_bounds__(kOptThreads, GTK_OPT_CTAS) k_merge_opt(EncodeB
 {
   TileSmem<kOptThreads>& S = tile_smem<kOptThreads>();
   tile_setup(S);
-  if (threadIdx.x == 0) {
-    const int64_t n = text_end(b);
-    S.n_tiles = int((n + kTile - 1) / kTile);
-    S.tail    = int(n - int64_t(S.n_tiles - 1) * kTile);
-  }
-  if (b.starts_clock && blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long*>(b.counters + 12) = global_timer();
-  __syncthreads();
   const int lo = int(b.tile_lo);  // tiles are counted in 32 bits: 8 TB of text
   int k        = lo + int(blockIdx.x);  // the first tile of every CTA, the others by ticket
-  while (k < min(int(b.tile_hi), S.n_tiles)) {
+  {
+    const int64_t n   = text_end(b);
+    const int n_tiles = int((n + kTile - 1) / kTile);
+    if (threadIdx.x == 0) {
+      S.n_tiles = n_tiles;
+      S.tail    = int(n - int64_t(n_tiles - 1) * kTile);
+    }
+    if (k >= min(int(b.tile_hi), n_tiles)) return;
+  }
+  if (b.starts_clock && blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<unsigned long long*>(b.counters + 12) = global_timer();
+  do {
     int next = 0;
     if (threadIdx.x == 0) next = atomicAdd(b.ticket, 1);  // on its way while the tile is worked on
     tile_reset(S);
@@ -956,7 +959,7 @@ __global__ void __launch_bounds__(kOptThreads, GTK_OPT_CTAS) k_merge_opt(EncodeB
     if (threadIdx.x == 0) S.ticket = next;
     __syncthreads();
     k = lo + int(gridDim.x) + S.ticket;
-  }
+  } while (k < min(int(b.tile_hi), S.n_tiles));
 }
 
 // ------------------------------------------------------------------------------------------------
