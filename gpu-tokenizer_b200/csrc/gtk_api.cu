@@ -891,8 +891,13 @@ constexpr size_t kSmallOutText   = 64;
 constexpr size_t kSmallOutChunk  = kSmallOutText + (((size_t(gtk::kSmallMaxTexts) + 1) * 8 + 63) & ~size_t(63));
 constexpr size_t kSmallOutIds    = kSmallOutChunk + (((size_t(kSmallChunkCap) + 1) * 8 + 63) & ~size_t(63));
 constexpr size_t kSmallOutSize   = kSmallOutIds + size_t(gtk::kSmallMaxBytes) * 4 + 64;
-constexpr size_t kMappedResultBytes        = size_t(6) << 20;    // mapped result block of the next size class
-constexpr int64_t kResultsByKernelMaxBytes = int64_t(1) << 20;  // batches up to this size use it: 711 KB in GTK_MODE_BASE 140 us, by two copies 162
+// Host batches of the chunk-by-chunk modes up to this size: a kernel writes the results into a mapped block instead of two copies
+// bringing them.  By kernel / by copies, 64 KiB, 256 KiB, 1, 2, 4 MiB of the novel in GTK_MODE_BASE: 111 / 126, 99 / 111, 140 / 153,
+// 198 / 208, 344 / 349 us; GTK_MODE_LOCALMIN 105 / 115, 92 / 108, 147 / 162, 235 / 244, 410 / 414.  The kernel is ahead at every size
+// measured, by 12 % up to 1 MiB and by 1 % at 4 MiB; the block needs five bytes of page-locked memory per byte of text, so
+// it ends where the gain does.
+constexpr int64_t kResultsByKernelMaxBytes = int64_t(1) << 20;
+constexpr size_t kMappedResultBytes        = size_t(6) << 20;
 
 void small_path_init(gtk_tokenizer* h)
 {
@@ -1046,9 +1051,10 @@ class Gather {
 };
 
 // Ordinary memory from this size on is staged by the crew while the first of it is on the link already; the driver does it
-// on one core.  1 / 4 / 16 MiB per call: 133 / 412 / 1218 us by the driver, 114 / 310 / 860 staged, 94 / 258 / 787 from page-locked
-// memory.  (Staged with stores that go through the caches: 123 / 650 / 1156.)  Beyond the upper bound the staging buffer
-// would be the larger cost.
+// on one core.  256 KiB / 1 / 4 / 16 / 64 MiB per call: 102 / 149 / 427 / 1204 / 6740 us by the driver, 94 / 122 / 324 / 879 / 3009 staged;
+// from page-locked memory 94 / 258 / 787 at 1 / 4 / 16 MiB.  (Staged with stores that go through the caches: 123 / 650 / 1156.)  The upper
+// bound limits the page-locked memory that a handle keeps, not the gain: 96 and 160 MiB take 9.9 and 16.7 ms by the driver, 4.1 and
+// 6.5 staged.
 constexpr int64_t kStageMinBytes = int64_t(512) << 10, kStageMaxBytes = int64_t(64) << 20;
 
 bool is_ordinary_memory(const void* p)

@@ -22,7 +22,11 @@ constexpr int kHalo = 256;
 constexpr int kWindow = kTile + kHalo;
 constexpr int kBaseThreads = 512;
 constexpr int kBaseSmemTokens = 8192;  // chunks up to this length stay in shared memory in the local-minimum and allocation-free kernels
-constexpr int kThreadSegMax = 16;      // longest segment a single thread merges on its own
+// Longest segment a single thread merges on its own; longer ones are a warp's.  A list entry has four bits for the length and the
+// merge scratch room for 16 ranks per lane.  Text with many segments of 17..32 bytes (JSON records 3.0 a tile, Python source 0.7, novel
+// 0.05), 256 KiB / 8 / 64 MiB a call: 62 / 138 / 719, 79 / 139 / 472 and 59 / 112 / 322 us; 73 / 159 / 724, 95 / 168 / 700 and 74 / 142 / 589 us with the
+// tiles before, where a thread took up to 32 bytes.
+constexpr int kThreadSegMax = 16;
 
 // Pointers into HBM, passed by value to every kernel.
 struct DeviceTable {

@@ -5,7 +5,7 @@
 // build_vocab_and_merges (gputok_blockbpe.cu:64-236); the data layout is new:
 // an open-addressing table with 16-byte slots for host lookups, and for the
 // kernels a bucketed pair table answered by one 128-bit load, a dense 256x256
-// table for byte pairs, per-rank merged ids, a never-merge bigram bitmap and a
+// table for byte pairs, per-rank merged ids, a never-merge bigram bitmap and two
 // tables of vocabulary strings that are their own tokenisation.
 #pragma once
 #include <cstdint>
@@ -66,7 +66,7 @@ inline uint32_t short_slot(uint32_t k0, uint32_t k1) { return ((k0 * kShortMulA)
 // token starts at byte i; 0 = empty.  Ids are stored plus one, unused places hold 0xFFFF, so none of the last three
 // words of a filled slot is zero.  The vocabulary's own strings (one id) are placed when the table is built: at slot h,
 // or, when that is taken, at h ^ 1 .. h ^ 7, with kLongMore set in the slots that were passed over.  The kernels
-// of a large batch work on a copy and fill empty slots with segments they have merged (see merge_batch).
+// of a large batch work on a copy and fill empty slots with segments they have merged (see learn_segment).
 struct alignas(32) LongWord {
   uint32_t k[4];
   uint32_t meta;

@@ -13,7 +13,7 @@
 // What bounds it: latency and instruction issue together.  A tile is a chain of table loads between barriers, and the
 // chip holds only as many tiles as shared memory and registers allow; HBM traffic is 1.7 bytes per input byte, a
 // thirtieth of what the memory could carry.  So the layout saves shared memory (what is not used is L1 for the tables),
-// barriers (four in the usual tile) and instructions: the boundary test is one load from an 8 KiB bit matrix (a
+// barriers (six in a tile without listed misses and long segments: reset, cut, list, lookup, emit, ticket) and instructions: the boundary test is one load from an 8 KiB bit matrix (a
 // 128-byte line holds the 32 right bytes of a block for 32 left bytes, so a gather over English text touches three or
 // four lines), and ranks are only formed for the segments that no table knows.  Figures: see k_merge_opt.
 

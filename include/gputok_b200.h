@@ -224,8 +224,8 @@ GTK_API int gtk_set_stream(gtk_tokenizer* h, void* cuda_stream);
 
 /* Threads per CTA of the one-CTA-per-chunk kernel (GTK_MODE_BASE).  Replaces the reference's compile-time
  * BLOCK_SIZE (gputok_blockbpe.cu:313-315, swept by profile_blockbpe_block_sizes.sh:9,22-25 over 128..1024):
- * 0 (default) = one warp per KiB of chunk, 64 / 128 / 256 / 512 / 1024 = that many threads whatever the chunk
- * size; anything else is GTK_ERR_INVALID_ARG.  Results never depend on it. */
+ * 0 (default) = 64 threads for chunks up to 1 KiB, 128 up to 2 KiB, 256 beyond; 64 / 128 / 256 / 512 / 1024 = that many whatever
+ * the chunk size; anything else is GTK_ERR_INVALID_ARG.  Results never depend on it. */
 GTK_API int gtk_set_base_block_size(gtk_tokenizer* h, int threads);
 
 /* Id space of the ids returned by the GPU encode entry points (no counterpart in the reference,

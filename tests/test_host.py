@@ -371,6 +371,49 @@ def test_forked_children_use_and_drop_a_tokenizer(native_built, merges_path):
     assert done.returncode == 0, done.stderr[-2000:]
 
 
+def test_decode_from_many_threads_with_errors_among_them(native_built, merges_path):
+    """Decoding of one handle from several threads, of which one at a time gets the helpers: long lists that are fine, one with an unknown
+    id in its last block, one into a buffer that is a byte too small.  The errors are those of the single pass, and nothing is
+    written behind the buffer."""
+    import ctypes
+    import threading
+
+    from gputok_b200 import GtkError, Tokenizer
+
+    t = Tokenizer(merges_path, 2048, 50, device=-1)
+    ids = np.arange(200_000, dtype=np.int32) % 50_000
+    unknown = ids.copy()
+    unknown[-7] = 60_000
+    want = t.decode(ids)
+    small = np.full(len(want) + 64, 0xEE, dtype=np.uint8)
+    n = ctypes.c_int64()
+    failed = []
+
+    def good():
+        for _ in range(10):
+            if t.decode(ids) != want:
+                failed.append("good")
+
+    def bad():
+        for _ in range(10):
+            try:
+                t.decode(unknown)
+                failed.append("unknown id accepted")
+            except GtkError as e:
+                if e.code != 1 or "60000" not in str(e):
+                    failed.append(str(e))
+            if t._lib.gtk_decode(t._h, ids.ctypes.data, len(ids), small.ctypes.data, len(want) - 1, ctypes.byref(n)) != 4:
+                failed.append("too small a buffer accepted")
+
+    threads = [threading.Thread(target=f) for f in (good, good, good, bad)]
+    for x in threads:
+        x.start()
+    for x in threads:
+        x.join()
+    assert not failed, failed[:3]
+    assert (small[len(want) - 1:] == 0xEE).all()
+
+
 SHORT_OF_MEMORY = """
 import ctypes, resource, sys
 sys.path.insert(0, {pkg!r})
